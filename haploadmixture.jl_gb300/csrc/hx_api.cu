@@ -42,6 +42,10 @@ struct hx_ctx {
     double* slots = nullptr;
     double* h_slots = nullptr;   // pinned
     uint8_t* img = nullptr;      // B-operand image of the tensor-core passes
+    // plain method: partial maxima and out-of-range sums of the passes (hx_f64.cuh)
+    unsigned long long* f64_mx = nullptr;
+    F64Rare rare{nullptr, nullptr, nullptr};
+    int S_qf = 1, spc_qf = 1, S_pf = 1, spc_pf = 1;   // chunks, stages per chunk
     int8_t* qp_ws = nullptr;     // P-side QP working sets, warm start of the next solve
     hx_loop_opts lo{0, 0, 0, -1};  // admixture_qn!/init_em! options
     double ll_tmp = NAN;         // d.ll_tmp of the step control
@@ -194,6 +198,12 @@ void plan(hx_ctx* c) {
     ipc = (ipc + PSTAGE_IND - 1) / PSTAGE_IND * PSTAGE_IND;
     c->ipc_p = (int)ipc;
     c->S_p = (int)((c->I + ipc - 1) / ipc);
+    // plain method's passes: one CTA per SM, chunks within the 64-bit sums' range
+    const int64_t nst_p = (c->I + 31) / 32;
+    c->spc_qf = (int)std::min<int64_t>(F64_MAX_STAGES, pick_chunk(tilesQ, c->JW, nsm, 4));
+    c->S_qf = (c->JW + c->spc_qf - 1) / c->spc_qf;
+    c->spc_pf = (int)std::min<int64_t>(F64_MAX_STAGES, pick_chunk(tilesP, nst_p, nsm, 4));
+    c->S_pf = (int)((nst_p + c->spc_pf - 1) / c->spc_pf);
     // tensor-core passes (stages of one word column, Q, or 32 individuals, P)
     // and the FP32 log-likelihood pass: >= 8 waves with a full last wave
     const int64_t wpc = pick_chunk(tilesQ, c->JW, (int64_t)nsm * tc_resident(c->K, false), 8);
@@ -234,7 +244,21 @@ int stage_pf(hx_ctx* c, const double* p, PassArgs& a) {
     return HX_OK;
 }
 
+// The plain method's pass of one side: maxima, stage images, pass, reduction.
+int pass_f64(hx_ctx* c, bool p_side, const double* q, const double* p, bool hess, double* XtX, double* Xtz) {
+    F64Call f{p_side, hess, pass_args(c, q, p), c->f64_mx, c->rare, c->st};
+    f.a.S = p_side ? c->S_pf : c->S_qf;
+    f.a.per_chunk = p_side ? c->spc_pf : c->spc_qf;
+    f.a.part = p_side ? c->part_p : c->part_q;
+    f.a.XtX = XtX;
+    f.a.Xtz = Xtz;
+    HX_LAUNCH(p_side ? (hess ? HX_KIND_ACCUM_P : HX_KIND_EM_P) : (hess ? HX_KIND_ACCUM_Q : HX_KIND_EM_Q), 4,
+              launch_f64_pass(c->K, f));
+    return HX_OK;
+}
+
 int pass_q(hx_ctx* c, const double* q, const double* p, bool hess, double* XtX, double* Xtz) {
+    if (c->prec == HX_PREC_FP64) return pass_f64(c, false, q, p, hess, XtX, Xtz);
     PassArgs a = pass_args(c, q, p);
     // the gradient-only (EM) Q pass is as fast on the CUDA cores (measured
     // again after the pipeline changes: 6.91 vs 6.90 s of Q passes per C3 fit)
@@ -245,15 +269,14 @@ int pass_q(hx_ctx* c, const double* q, const double* p, bool hess, double* XtX, 
         return HX_OK;
     }
     a.S = c->S_q; a.per_chunk = c->wpc_q; a.part = c->part_q;
-    if (c->prec != HX_PREC_FP64) HX_ST(stage_pf(c, p, a));
-    HX_LAUNCH(hess ? HX_KIND_ACCUM_Q : HX_KIND_EM_Q, 1,
-              c->prec == HX_PREC_FP64 ? launch_accum_q_f64(c->K, hess, a, c->st)
-                                      : launch_accum_q_f32(c->K, hess, a, c->st));
+    HX_ST(stage_pf(c, p, a));
+    HX_LAUNCH(hess ? HX_KIND_ACCUM_Q : HX_KIND_EM_Q, 1, launch_accum_q_f32(c->K, hess, a, c->st));
     HX_LAUNCH(HX_KIND_OTHER, 1, launch_reduce_sym(c->part_q, c->S_q, c->K, hess, c->I, c->Ipad, XtX, Xtz, c->st));
     return HX_OK;
 }
 
 int pass_p(hx_ctx* c, const double* q, const double* p, bool hess, double* XtX, double* Xtz) {
+    if (c->prec == HX_PREC_FP64) return pass_f64(c, true, q, p, hess, XtX, Xtz);
     PassArgs a = pass_args(c, q, p);
     if (c->tc) {
         a.S = c->S_pt; a.per_chunk = c->ipc_pt; a.part = c->part_p; a.XtX = XtX; a.Xtz = Xtz;
@@ -264,9 +287,7 @@ int pass_p(hx_ctx* c, const double* q, const double* p, bool hess, double* XtX, 
         return HX_OK;
     }
     a.S = c->S_p; a.per_chunk = c->ipc_p; a.part = c->part_p; a.XtX = XtX; a.Xtz = Xtz;
-    HX_LAUNCH(hess ? HX_KIND_ACCUM_P : HX_KIND_EM_P, 1,
-              c->prec == HX_PREC_FP64 ? launch_accum_p_f64(c->K, hess, a, c->st)
-                                      : launch_accum_p_f32(c->K, hess, a, c->st));
+    HX_LAUNCH(hess ? HX_KIND_ACCUM_P : HX_KIND_EM_P, 1, launch_accum_p_f32(c->K, hess, a, c->st));
     if (c->S_p > 1)
         HX_LAUNCH(HX_KIND_OTHER, 1,
                   launch_reduce_sym(c->part_p, c->S_p, c->K, hess, 4 * c->J, 4 * c->J, XtX, Xtz, c->st));
@@ -467,6 +488,7 @@ int create_common(const uint8_t* bed, bool bed_on_device, int64_t bps, int64_t n
     HX_CK(cudaEventCreate(&c->ev1));
     HX_CK(init_kernel_attrs());
     HX_CK(init_tc_attrs());
+    if (c->prec == HX_PREC_FP64) HX_CK(f64_attrs(K));
     plan(c);
     if (c->verbose)
         fprintf(stderr,
@@ -490,9 +512,22 @@ int create_common(const uint8_t* bed, bool bed_on_device, int64_t bps, int64_t n
     HX_ST(dalloc(c, &c->Xtzq, (size_t)K * I));
     HX_ST(dalloc(c, &c->XtXp, (size_t)K * K * 4 * J));
     HX_ST(dalloc(c, &c->Xtzp, (size_t)K * 4 * J));
-    HX_ST(dalloc(c, &c->part_q, (size_t)std::max(c->S_q, c->tc ? c->Sq_cap : 1) * NVmax * c->Ipad));
-    const int Sp_max = std::max(c->S_p, c->tc ? c->Sp_cap : 1);
-    if (Sp_max > 1) HX_ST(dalloc(c, &c->part_p, (size_t)Sp_max * NVmax * 4 * J));
+    if (c->prec == HX_PREC_FP64) {
+        const size_t NH = (size_t)K * (K + 1) / 2, rows = (size_t)std::max<int64_t>(I, 4 * J);
+        HX_ST(dalloc(c, &c->part_q, (size_t)c->S_qf * NH * c->Ipad));
+        HX_ST(dalloc(c, &c->part_p, (size_t)c->S_pf * NH * 4 * J));
+        HX_ST(dalloc(c, &c->img, f64_image_bytes(K, I, J)));
+        HX_ST(dalloc(c, &c->f64_mx, (size_t)F_MAXB * F_MXS));
+        HX_ST(dalloc(c, &c->rare.i, 2 * rows * NH));
+        HX_ST(dalloc(c, &c->rare.d, rows * NH));
+        HX_ST(dalloc(c, &c->rare.flag, 1));
+        HX_CK(cudaMemsetAsync(c->rare.i, 0, 2 * rows * NH * sizeof(long long), c->st));
+        HX_CK(cudaMemsetAsync(c->rare.d, 0, rows * NH * sizeof(double), c->st));
+    } else {
+        HX_ST(dalloc(c, &c->part_q, (size_t)std::max(c->S_q, c->tc ? c->Sq_cap : 1) * NVmax * c->Ipad));
+        const int Sp_max = std::max(c->S_p, c->tc ? c->Sp_cap : 1);
+        if (Sp_max > 1) HX_ST(dalloc(c, &c->part_p, (size_t)Sp_max * NVmax * 4 * J));
+    }
     HX_ST(dalloc(c, &c->part_ll, (size_t)std::max<int64_t>((c->Ipad / ACC_THREADS) * c->S_q,
                                                             (int64_t)loglik_f32x2_blocks(c->Ipad, K) *
                                                                 std::max(c->S_ll, c->Sll_cap))));
@@ -629,7 +664,7 @@ int hx_destroy(hx_ctx* c) {
     if (c->st) cudaStreamSynchronize(c->st);
     void* bufs[] = {c->shared_geno ? nullptr : (void*)c->G, c->shared_geno ? nullptr : (void*)c->dm, c->x, c->xn, c->xn2, c->xt, c->xio, c->U, c->V, c->XtXq, c->Xtzq, c->XtXp,
                     c->Xtzp, c->part_q, c->part_p, c->part_ll, c->part_qn, c->coef, c->slots, c->img, c->qp_ws,
-                    c->pf};
+                    c->pf, c->f64_mx, c->rare.i, c->rare.d, c->rare.flag};
     for (void* b : bufs) if (b) cudaFree(b);
     prof_resolve(c);
     for (cudaEvent_t e : c->pool) cudaEventDestroy(e);

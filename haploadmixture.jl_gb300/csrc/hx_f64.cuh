@@ -1,0 +1,697 @@
+// hx_f64.cuh -- the plain (FP64) method's gradient and Hessian passes.
+//
+// GB300's FP64 unit issues 2 operations per clock and SM, 1/64 of the FP32
+// rate, so a pass that does its K(K+1)/2 accumulations per haplotype there
+// costs 90 to 160 clocks per (individual, block) pair (K = 5 .. 8).  These
+// passes keep on the FP64 unit only what has to be there, and only for the
+// haplotypes that a pair's genotypes allow (1.8 of 4 on average):
+//   qp_h = sum_k q[k,i] p[k,4j+h], r_h = 1 / qp_h, and the pair's weights
+//   W_h = c_h r_h^2 (Hessian) or U_h = c_h r_h (gradient only),
+// and form the sums H = sum W v v' (v = p on the Q side, q on the P side;
+// src/loops.jl:328-403) exactly on the tensor cores: the error-free splitting
+// of Ozaki, Ogita, Oishi and Rump (2012).  The vectors are scaled by powers of
+// two, per k and then per reduction index, so that the largest entry is just
+// below 1 in both; W takes the inverse of the index's, which leaves
+// W' = c_h (s / qp_h)^2, s the index's scale: of the order of 1 even for rare
+// haplotypes.  W' is rounded to a multiple of 2^-56 and written as ND_A = 10
+// signed base-256 digits, the scaled products v_k v_k2 to a multiple of 2^-62
+// as ND_B = 8 digits.  Digits are integers in [-128, 127], exact in FP16; a
+// digit product is at most 2^14, and an FP32 accumulator column takes ND_B digit
+// pairs x 128 reduction indices x 2^14 = 2^24 before it is read out, so every
+// accumulation is exact.  Digit pairs (a, b) of equal order a + b share a
+// column; orders 0 .. 9 are kept (an order-10 pair weighs 2^-56 at most, with
+// either sign).  The columns are read out to 64-bit integers, so a chunk's sum
+// does not depend on any order; only the chunk sums and the last digits' cut
+// are rounded, and the error against exact sums is below that of FP64
+// accumulation, whose every add rounds the running total.
+//
+// The gradient needs no sums of its own beside the Hessian: sum_k2 H[k,k2] x_k2
+// = sum W v_k qp = sum U v_k = g_k (x = the row's own vector, qp = v . x), all
+// terms of one sign, formed by the reduction of the chunks.
+//
+// A scaled weight of 2^22 or more (an observed haplotype 2,000 times rarer in
+// the individual's mixture than in one of the ancestries), a negative or a
+// non-finite one does not fit the digits: its products are added in fixed point
+// to 64-bit integers in global memory (order-independent, as every integer
+// sum), and from 2^42 on, or when not finite, to FP64 words there.
+#pragma once
+#include "hx_ops.cuh"
+#include "hx_tc.cuh"
+
+namespace hx {
+namespace {
+using namespace tc;
+
+constexpr int F_GEN_WARPS = 16;                       // generator warps
+constexpr int F_THREADS = 32 * (F_GEN_WARPS + 1);     // + one warp that loads and issues
+constexpr int F_KD = 32;                              // reduction indices per stage
+constexpr int F_RING = 3;
+constexpr int F_WIN = 4;                              // stages per read-out (128 reduction indices)
+constexpr int F_NDA = 10, F_NDB = 8, F_NORD = 10;
+constexpr int F_SA = 56, F_SB = 62;                   // units 2^-SA of W', 2^-SB of the products
+constexpr long long F_BUDGET = 4000000000LL;          // bound of any pipeline wait (clock64 cycles)
+constexpr int F_TOP = 22;                             // W' < 2^TOP: TOP + SA + 1 bits fit ND_A signed bytes
+
+template <int K, bool HESS> struct FDim {
+    static constexpr int NV = HESS ? K * (K + 1) / 2 : K;    // sums per row
+    static constexpr int NG = NV > 48 ? 2 : 1;               // column groups (grid.z): NORD x 48 TMEM columns fit
+    static constexpr int PER = (NV + NG - 1) / NG;           // sums per group
+    static constexpr int NHP = (PER + 15) / 16 * 16;
+    static constexpr int NPC = NHP / 4;                      // columns per order read out by one thread
+    static constexpr int TCOLS = F_NORD * NHP <= 256 ? 256 : 512;
+    static constexpr int KS = (K + 1) | 1;                   // row stride (doubles): odd, so rows differ in banks;
+                                                             // entry K of a stage's row: the index's exponent
+    static constexpr int B_TILE = F_NDB * NHP * F_KD * 2;
+    static constexpr int ROWS = F_KD * KS * 8;
+    static constexpr int IMG = NG * B_TILE + ROWS;           // image bytes per stage
+    static constexpr int SLOT = B_TILE + ROWS + 512;         // + 128 class words
+};
+constexpr int F_LBO_B = 128, F_SBO_B = 512;
+template <bool PS> constexpr int f_lbo() { return PS ? 144 : 128; }   // P side: padded, so that a warp's
+template <bool PS> constexpr int f_sbo() { return 4 * f_lbo<PS>(); }  // 32-bit stores hit distinct banks
+template <bool PS> constexpr int f_atile() { return 16 * f_sbo<PS>(); }
+
+struct FSync {
+    uint64_t full[F_RING];
+    uint64_t gen;        // the generator warps have written a stage's digits (one arrival per warp)
+    uint64_t mma;        // a stage's MMAs are done
+    uint32_t tslot;
+    int bad, issued, loaded;
+};
+
+template <int K, bool HESS, bool PS> constexpr size_t f_smem() {
+    using D = FDim<K, HESS>;
+    return 128 + (size_t)F_NDA * f_atile<PS>() + (size_t)F_RING * D::SLOT + 128 * D::KS * 8 +
+           F_GEN_WARPS * 256 * (8 + 2) + sizeof(FSync);
+}
+
+// Needed haplotypes of a class (all four for the double heterozygote, none for
+// double missing).
+__host__ __device__ constexpr unsigned class_need(unsigned nib) {
+    return nib == NIB_HH ? 0xFu : (class_m1(nib) | class_m2(nib));
+}
+__host__ __device__ constexpr uint64_t make_need() {
+    uint64_t t = 0;
+    for (unsigned n = 0; n < 16; ++n) t |= (uint64_t)class_need(n) << (4 * n);
+    return t;
+}
+constexpr uint64_t TAB_NEED = make_need();
+// Classes whose counts depend on qp: the double heterozygote and one SNP missing.
+__host__ __device__ constexpr unsigned make_cplx() {
+    unsigned t = 0;
+    for (unsigned n = 0; n < 16; ++n)
+        if (n == NIB_HH || ((((n & 3u) == 1u) != ((n >> 2) == 1u)))) t |= 1u << n;
+    return t;
+}
+constexpr unsigned TAB_CPLX = make_cplx();
+
+// 1/x by one step of the cubically convergent form of Newton's iteration
+// (Householder): r (1 + e + e^2), e = 1 - x r, from the hardware's 20-bit
+// reciprocal: e^3 < 2^-56.  Three FP64 operations instead of the eight or more
+// of a division.  Outside 2^-1000 .. 2^1000 (zeros, NaN, infinities) it divides.
+__device__ __forceinline__ double rcp64(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    r = fma(r, fma(e, e, e), r);
+    const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7FFu;
+    if (ex - 23u > 2000u) r = 1.0 / x;
+    return r;
+}
+
+// Largest |v[k]| of each of the K rows of v (K x n), as partial maxima of the
+// bit patterns per block (a NaN's pattern is above infinity's), and beside them
+// whether the block met a zero or a non-finite value; block 0 also clears the
+// flag of out-of-range weights.
+__global__ void __launch_bounds__(256) k_f64_colmax(const double* __restrict__ v, int K, int64_t n,
+                                                    unsigned long long* __restrict__ mx, int* __restrict__ flag) {
+    __shared__ unsigned long long s[HX_KMAX + 1];
+    if (threadIdx.x <= HX_KMAX) s[threadIdx.x] = 0ull;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *flag = 0;
+    __syncthreads();
+    // a stride that is a multiple of K keeps each thread on one k
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x / K * K;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < stride) {
+        unsigned long long m = 0ull;
+        bool odd = false;
+        for (int64_t a = t; a < n * K; a += stride) {
+            const unsigned long long b = (unsigned long long)__double_as_longlong(v[a]) & 0x7FFFFFFFFFFFFFFFull;
+            m = max(m, b);
+            odd |= b == 0ull || b >= 0x7FF0000000000000ull;
+        }
+        atomicMax(&s[t % K], m);
+        if (odd) atomicMax(&s[HX_KMAX], 1ull);
+    }
+    __syncthreads();
+    if (threadIdx.x <= HX_KMAX) mx[(int64_t)blockIdx.x * F_MXS + threadIdx.x] = s[threadIdx.x];
+}
+
+// Exponents e_k with max |v_k| < 2^e_k, from the partial maxima; returns via
+// shared memory of HX_KMAX ints (INT_MAX where a value is not finite).
+__device__ __forceinline__ void f64_exponents(const unsigned long long* __restrict__ mx, int nb, int K, int* se) {
+    if (threadIdx.x < (unsigned)K) {
+        unsigned long long m = 0ull;
+        for (int b = 0; b < nb; ++b) m = max(m, mx[(int64_t)b * F_MXS + threadIdx.x]);
+        const int f = (int)(m >> 52);
+        se[threadIdx.x] = f == 0x7FF ? 0x7FFFFFFF : (f == 0 ? 0 : f - 1022);
+    }
+    __syncthreads();
+}
+
+// Stage images: the digits of the products v_k v_k2 (or of v_k) of 32 reduction
+// indices, in the shared-memory layout of the MMA's B operand, and the FP64
+// vectors.  One warp per stage, lane = reduction index.  Indices past n get
+// zeros (their class nibbles are padding).
+template <int K, bool HESS>
+__global__ void __launch_bounds__(128) k_f64_img(const double* __restrict__ v, int64_t n, int64_t stages,
+                                                 const unsigned long long* __restrict__ mx, int nb,
+                                                 uint8_t* __restrict__ img) {
+    using D = FDim<K, HESS>;
+    __shared__ int se[HX_KMAX];
+    f64_exponents(mx, nb, K, se);
+    const int lane = threadIdx.x & 31;
+    const int64_t st = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (st >= stages) return;
+    const int64_t a = st * F_KD + lane;
+    uint8_t* base = img + st * D::IMG;
+    double x[K], w[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        x[k] = a < n ? v[(int64_t)K * a + k] : 0.0;
+        const int e = se[k];
+        w[k] = e == 0x7FFFFFFF ? 0.0 : scalbn(x[k], -e);
+    }
+    double* rows = reinterpret_cast<double*>(base + D::NG * D::B_TILE) + lane * D::KS;
+#pragma unroll
+    for (int k = 0; k < K; ++k) rows[k] = x[k];
+    // the index's exponent f: max |w| < 2^f
+    double mw = 0.0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) mw = fmax(mw, fabs(w[k]));
+    const int fe = (int)((unsigned long long)__double_as_longlong(mw) >> 52);
+    const int f = fe == 0 || fe == 0x7FF ? 0 : fe - 1022;
+    rows[K] = __longlong_as_double((long long)f);
+#pragma unroll
+    for (int k = 0; k < K; ++k) w[k] = scalbn(w[k], -f);
+    auto put = [&](int c, double y) {   // sum c, value y in (-1, 1)
+        const int g = c / D::PER, col = c - g * D::PER;
+        const unsigned long long u = (unsigned long long)__double2ll_rn(scalbn(y, F_SB)) + 0x8080808080808080ull;
+        uint8_t* tile = base + g * D::B_TILE;
+#pragma unroll
+        for (int b = 0; b < F_NDB; ++b) {
+            const int row = b * D::NHP + col;
+            const int d = (int)((u >> (8 * (F_NDB - 1 - b))) & 0xFF) - 128;
+            uint16_t h;
+            asm("cvt.rn.f16.s32 %0, %1;" : "=h"(h) : "r"(d));
+            *reinterpret_cast<uint16_t*>(tile + (row >> 3) * F_SBO_B + (lane >> 3) * F_LBO_B + (row & 7) * 16 +
+                                         (lane & 7) * 2) = h;
+        }
+    };
+    if (HESS) {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+#pragma unroll
+            for (int k2 = k; k2 < K; ++k2) put(tri_idx<K>(k, k2), w[k] * w[k2]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < K; ++k) put(k, w[k]);
+    }
+    // padding columns are zero
+    for (int g = 0; g < D::NG; ++g)
+        for (int col = min(D::PER, D::NV - g * D::PER); col < D::NHP; ++col)
+            for (int b = 0; b < F_NDB; ++b) {
+                const int row = b * D::NHP + col;
+                *reinterpret_cast<uint16_t*>(base + g * D::B_TILE + (row >> 3) * F_SBO_B + (lane >> 3) * F_LBO_B +
+                                             (row & 7) * 16 + (lane & 7) * 2) = 0;
+            }
+}
+
+// 80-bit fixed point of w 2^sh (0 <= w 2^sh < 2^TOP) in units of 2^-SA, plus 128
+// in every byte: byte d minus 128 is then the signed digit of weight 256^d.
+__device__ __forceinline__ void f64_fix(double w, int sh, uint32_t (&x)[3]) {
+    const uint32_t hi = (uint32_t)__double2hiint(w), lo = (uint32_t)__double2loint(w);
+    const int e = (int)(hi >> 20) - 1023 + (F_SA - 52) + sh;   // of the 53-bit integer m
+    uint64_t m = ((uint64_t)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo;
+    if (hi < 0x100000u) m = 0;                             // zero (subnormals vanish at 2^-SA)
+    const int n = min(63, -e);
+    const uint64_t l = e >= 0 ? m << (e & 63) : (m + (1ull << (n - 1))) >> n;   // rounded to a multiple of 2^-SA
+    const uint32_t h = e > 0 ? (uint32_t)(m >> (64 - e)) : 0u;
+    asm("add.cc.u32 %0, %3, %6;\n\t addc.cc.u32 %1, %4, %6;\n\t addc.u32 %2, %5, %7;"
+        : "=&r"(x[0]), "=&r"(x[1]), "=&r"(x[2])
+        : "r"((uint32_t)l), "r"((uint32_t)(l >> 32)), "r"(h), "r"(0x80808080u), "r"(0x8080u));
+}
+
+__device__ __forceinline__ uint32_t f64_h2(uint32_t pair_bytes, uint32_t sel) {
+    // two digit bytes -> packed FP16 integers: (1024 + byte) - 1152
+    uint32_t h, d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(h) : "r"(pair_bytes), "r"(0x64646464u), "r"(sel));
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(h), "r"(0xE480E480u));
+    return d;
+}
+// The four digits of word w of two elements: digit 4w + t in out[t].
+__device__ __forceinline__ void f64_digits4(uint32_t x0, uint32_t x1, uint32_t (&out)[4]) {
+    const uint32_t p01 = __byte_perm(x0, x1, 0x5140), p23 = __byte_perm(x0, x1, 0x7362);
+    out[0] = f64_h2(p01, 0x4140);
+    out[1] = f64_h2(p01, 0x4342);
+    out[2] = f64_h2(p23, 0x4140);
+    out[3] = f64_h2(p23, 0x4342);
+}
+
+__device__ __forceinline__ bool is_bad_f(const FSync* sy) { return *(volatile const int*)&sy->bad != 0; }
+__device__ __forceinline__ bool f_wait(FSync* sy, uint64_t* bar, int phase, double* slots) {
+    if (mbar_wait(bar, (uint32_t)(phase & 1), F_BUDGET)) return true;
+    *(volatile int*)&sy->bad = 1;
+    slots[S_TC_TIMEOUT] = 1.0;
+    return false;
+}
+
+// Weights of a warp's 2 x 32 pairs: lane = individual, blocks bb = 0, 1 of
+// class nib[bb].  qrow: the 32 individuals' vectors; prow: the 8 columns'
+// vectors (c = 4 bb + h).  The needed (pair, haplotype) items are listed by
+// ballot and spread evenly over the lanes (4 rounds of 32 for 64 pairs instead
+// of 8); then the pairs whose counts depend on qp, again listed, are finished
+// from their reciprocals.  Results in rb[c][lane] (needed items only).
+// A frequency qp_h = 0 makes the Hessian NaN even where the genotypes do not
+// allow h (0 / 0), which the caller reports: with allh (P holds zeros or
+// non-finite values, the only way to such a qp) every haplotype is listed.
+template <int K, bool HESS>
+__device__ __forceinline__ void f64_weights(const unsigned (&nib)[2], const double* qrow, const double* prow,
+                                            double* rb, uint16_t* list, bool allh) {
+    constexpr int KS = FDim<K, HESS>::KS;
+    const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+    int n = 0;
+    unsigned need[2], cpl[2];
+#pragma unroll
+    for (int bb = 0; bb < 2; ++bb) {
+        need[bb] = (unsigned)(TAB_NEED >> (4 * nib[bb])) & 0xFu;
+        cpl[bb] = (TAB_CPLX >> nib[bb]) & 1u;
+        const unsigned tag = lane | (__popc(need[bb]) == 1 ? 256u : 0u) | (cpl[bb] ? 512u : 0u);
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const bool own = (need[bb] >> h) & 1u;
+            const bool has = own || (allh && nib[bb] != NIB_MM);
+            const unsigned bal = __ballot_sync(0xffffffffu, has);
+            if (has)
+                list[n + __popc(bal & lt)] = (uint16_t)((own ? tag : lane | 1024u) | ((4 * bb + h) << 5));
+            n += __popc(bal);
+        }
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int base = 0; base < n; base += 32) {
+        const bool on = base + (int)lane < n;
+        const unsigned it = on ? list[base + lane] : list[n - 1];
+        const double* q = qrow + (it & 31u) * KS;
+        const double* p = prow + ((it >> 5) & 7u) * KS;
+        double s = q[0] * p[0];
+#pragma unroll
+        for (int k = 1; k < K; ++k) s = fma(q[k], p[k], s);
+        const double r = rcp64(s);
+        double w = r;                                   // left for the second part
+        if (!(it & 512u)) {
+            if (HESS) w = r * r;
+            if (it & 256u) {                            // both copies: times 2, by the exponent where that is in range
+                const unsigned ex = ((unsigned)__double2hiint(w) >> 20) & 0x7FFu;
+                w = ex - 1u < 2045u ? __hiloint2double(__double2hiint(w) + 0x00100000, __double2loint(w)) : w + w;
+            }
+            // listed for its zero frequency only (see allh)
+            if (HESS && (it & 1024u)) w = r * 0.0;
+        }
+        if (on) rb[(it & 255u)] = w;                    // it & 255 = 32 c + lane
+    }
+    __syncwarp();
+    // pairs with qp-dependent counts: a <-> b, c <-> d share a factor, with
+    // x = r_a r_b, y = r_c r_d:
+    //   het/het        (0,3,1,2): c_0 = c_3 = y/(x+y), c_1 = c_2 = x/(x+y)
+    //   SNP 1 missing  (0,2,1,3), SNP 2 missing (0,1,2,3):
+    //                  u = f r_a r_b / (r_a + r_b) = f / (qp_a + qp_b), f = copies in that set
+    int nc = 0;
+#pragma unroll
+    for (int bb = 0; bb < 2; ++bb) {
+        const unsigned bal = __ballot_sync(0xffffffffu, cpl[bb] != 0u);
+        if (cpl[bb]) list[nc + __popc(bal & lt)] = (uint16_t)(lane | (nib[bb] << 6) | (bb << 5));
+        nc += __popc(bal);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int base = 0; base < nc; base += 32) {
+        if (base + (int)lane < nc) {
+            const unsigned it = list[base + lane];
+            const unsigned nb = it >> 6, nd = (unsigned)(TAB_NEED >> (4 * nb)) & 0xFu;
+            double* rp = rb + ((it >> 5) & 1u) * 128 + (it & 31u);
+            const bool hh = nb == NIB_HH, m1 = (nb & 3u) == 1u;
+            const int ib = hh ? 3 : (m1 ? 2 : 1), ic = hh || m1 ? 1 : 2, id = hh ? 2 : 3;
+            const bool ab = nd & 1u, cd = (nd >> ic) & 1u;       // a set is needed as a whole
+            const double ra = ab ? rp[0] : 1.0, rbb = ab ? rp[32 * ib] : 1.0;
+            const double rc = cd ? rp[32 * ic] : 1.0, rd = cd ? rp[32 * id] : 1.0;
+            const double x = ra * rbb, y = rc * rd;
+            const double d1 = hh ? x + y : ra + rbb, d2 = hh ? 1.0 : rc + rd;
+            const double t = rcp64(d1 * d2);
+            const double t1 = t * d2, t2 = t * d1;
+            const double e1 = (hh ? y : x) * t1, e2 = (hh ? x : y) * (hh ? t1 : t2);
+            const double f = ab && cd ? 1.0 : 2.0;
+            if (ab) {
+                const double ma = hh ? ra : f, mb = hh ? rbb : f;
+                rp[0] = HESS ? (e1 * ra) * ma : e1 * ma;
+                rp[32 * ib] = HESS ? (e1 * rbb) * mb : e1 * mb;
+            }
+            if (cd) {
+                const double mc = hh ? rc : f, md = hh ? rd : f;
+                rp[32 * ic] = HESS ? (e2 * rc) * mc : e2 * mc;
+                rp[32 * id] = HESS ? (e2 * rd) * md : e2 * md;
+            }
+        }
+    }
+    __syncwarp();
+}
+
+// Whether w 2^sh is outside the digits' range: too large, negative, not finite.
+__device__ __forceinline__ bool f64_out_of_range(double w, int sh) {
+    const int e = (int)((uint32_t)__double2hiint(w) >> 20);
+    return e >= 0x7FF || e + sh >= 1023 + F_TOP;
+}
+
+// A weight outside that range (see the top of the file): its products with the
+// group's vectors, in units of 2^-8 and 2^-56, to the row's integers.
+template <int K, bool HESS>
+__device__ __noinline__ void f64_rare(double w, const double* vrow, const unsigned long long* mx, int nb, int c0,
+                                      int c1, F64Rare ra, int64_t row) {
+    atomicOr(ra.flag, 1);
+    double v[K];
+    for (int k = 0; k < K; ++k) {
+        unsigned long long m = 0ull;
+        for (int b = 0; b < nb; ++b) m = max(m, mx[(int64_t)b * F_MXS + k]);
+        const int f = (int)(m >> 52);
+        v[k] = scalbn(vrow[k], f == 0 || f == 0x7FF ? 0 : 1022 - f);
+    }
+    for (int k = 0; k < K; ++k)
+        for (int k2 = k; k2 < (HESS ? K : k + 1); ++k2) {
+            const int c = HESS ? tri_idx<K>(k, k2) : k;
+            if (c < c0 || c >= c1) continue;
+            const double y = HESS ? w * (v[k] * v[k2]) : w * v[k];
+            const int64_t at = row * FDim<K, HESS>::NV + c;
+            if (fabs(y) < 4398046511104.0) {           // 2^42
+                const long long A = __double2ll_rd(scalbn(y, 8));
+                const long long B = __double2ll_rn(scalbn(y - scalbn((double)A, -8), 56));
+                atomicAdd((unsigned long long*)ra.i + 2 * at, (unsigned long long)A);
+                atomicAdd((unsigned long long*)ra.i + 2 * at + 1, (unsigned long long)B);
+            } else {
+                atomicOr(ra.flag, 2);
+                atomicAdd(ra.d + at, y);
+            }
+        }
+}
+
+// ------------------------------------------------------------------ the pass
+// PS = false (Q side): CTA rows = 128 individuals, stage = one word column (8
+// blocks = 32 columns m); warp w: individuals 32 (w & 3) .. +31, blocks
+// 2 (w >> 2), +1.  PS = true (P side): CTA rows = the 128 columns m of 32
+// blocks, stage = 32 individuals; warp w: blocks 2w, 2w+1.  Chunks of the
+// reduction along grid.y, column groups along grid.z.
+// Bound by the FP64 unit: about (K + 5) operations per needed haplotype.  One
+// CTA per SM (480 of 512 TMEM columns at K = 8); the digit tiles need one
+// buffer only, because a stage's FP64 work (registers and warp-private shared
+// memory) runs while the MMAs of the stage before read it.
+template <int K, bool HESS, bool PS>
+__global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args fa) {
+    using D = FDim<K, HESS>;
+    constexpr int LBO = f_lbo<PS>(), SBO = f_sbo<PS>(), AT = f_atile<PS>();
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+    uint8_t* ring = smem + F_NDA * AT;
+    double* fix = reinterpret_cast<double*>(ring + F_RING * D::SLOT);      // [128][KS]
+    double* rbuf = fix + 128 * D::KS;                                      // [GEN_WARPS][8][32]
+    uint16_t* lists = reinterpret_cast<uint16_t*>(rbuf + F_GEN_WARPS * 256);
+    FSync* sy = reinterpret_cast<FSync*>(lists + F_GEN_WARPS * 256);
+    const uint32_t sA = smem_u32(smem), sR = smem_u32(ring);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int grp = blockIdx.z;
+    const int64_t row0 = (int64_t)blockIdx.x * 128;
+    // stages of this CTA
+    const int64_t s0 = (int64_t)blockIdx.y * a.per_chunk;
+    const int ns = (int)(min(fa.stages, s0 + a.per_chunk) - s0);
+    const int nwc = PS ? (int)min((int64_t)4, (int64_t)a.JW - (int64_t)blockIdx.x * 4) : 1;
+
+    if (warp == F_GEN_WARPS) tmem_alloc<D::TCOLS>(&sy->tslot);
+    if (tid == 0) {
+        for (int r = 0; r < F_RING; ++r) mbar_init(&sy->full[r], 1);
+        mbar_init(&sy->gen, F_GEN_WARPS);
+        mbar_init(&sy->mma, 1);
+        sy->bad = 0;
+        sy->issued = 0;
+        sy->loaded = 0;
+        mbar_fence_init();
+    }
+    // the rows' own vectors
+    const double* own = PS ? a.p : a.q;
+    const int64_t nown = PS ? 4 * a.J : a.I;
+    bool odd_p = false;          // P side: zero or non-finite frequencies among the CTA's own columns
+    for (int t = tid; t < 128 * K; t += F_THREADS) {
+        const int r = t / K, k = t - r * K;
+        const double x = row0 + r < nown ? own[(row0 + r) * K + k] : 0.25;
+        fix[r * D::KS + k] = x;
+        odd_p |= PS && (x == 0.0 || !isfinite(x));
+    }
+    if (!PS)                     // Q side: among all of P
+        for (int b = tid; b < fa.nmx; b += F_THREADS) odd_p |= fa.mx[(int64_t)b * F_MXS + HX_KMAX] != 0ull;
+    fence_before();
+    const bool allh = __syncthreads_or(odd_p) && HESS;
+    fence_after();
+    const uint32_t tmem = sy->tslot;
+
+    if (warp == F_GEN_WARPS) {
+        if (lane == 0) {
+            auto load = [&](int s) {
+                const int slot = s % F_RING;
+                const uint8_t* src = a.img + (s0 + s) * D::IMG;
+                const uint32_t dst = sR + slot * D::SLOT;
+                uint64_t* bar = &sy->full[slot];
+                const uint32_t wb = PS ? 128u * nwc : 512u;
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                             :: "r"(smem_u32(bar)), "r"((uint32_t)(D::B_TILE + D::ROWS) + wb) : "memory");
+                auto copy = [&](uint32_t d, const void* g, uint32_t bytes) {
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                 :: "r"(d), "l"(g), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+                };
+                copy(dst, src + grp * D::B_TILE, D::B_TILE);
+                copy(dst + D::B_TILE, src + D::NG * D::B_TILE, D::ROWS);
+                if (PS) {
+                    for (int w = 0; w < nwc; ++w)
+                        copy(dst + D::B_TILE + D::ROWS + 128 * w,
+                             a.G + ((int64_t)blockIdx.x * 4 + w) * a.Ipad + (s0 + s) * F_KD, 128);
+                } else {
+                    copy(dst + D::B_TILE + D::ROWS, a.G + (s0 + s) * a.Ipad + row0, 512);
+                }
+                *(volatile int*)&sy->loaded = s + 1;
+            };
+            for (int s = 0; s < F_RING && s < ns; ++s) load(s);
+            for (int s = 0; s < ns; ++s) {
+                // all digits of the stage written, and every warp past stage s-1
+                if (!f_wait(sy, &sy->gen, s, a.slots)) break;
+                fence_after();
+                const uint64_t dA = sdesc(sA, LBO, SBO), dB = sdesc(sR + (s % F_RING) * D::SLOT, F_LBO_B, F_SBO_B);
+                // one MMA per digit pair: all of one shape, so that those of one
+                // order (one accumulator) execute in issue order
+#pragma unroll 1
+                for (int d = 0; d < F_NDA; ++d)
+#pragma unroll
+                    for (int b = 0; b < F_NDB; ++b) {
+                        if (d + b >= F_NORD) break;
+#pragma unroll
+                        for (int ks = 0; ks < F_KD / 16; ++ks)
+                            mma_bf16(tmem + (d + b) * D::NHP, dA + (uint64_t)((d * AT + ks * 2 * LBO) >> 4),
+                                     dB + (uint64_t)((b * (D::NHP / 8) * F_SBO_B + ks * 2 * F_LBO_B) >> 4),
+                                     idesc_f16(D::NHP), 1u);
+                    }
+                commit(&sy->mma);
+                *(volatile int*)&sy->issued = s + 1;
+                // the slot of stage s-1: its MMAs are done (every warp waited for
+                // them before it arrived for stage s) and its vectors are read
+                if (s >= 1 && s + 2 < ns) load(s + 2);
+            }
+        }
+        __syncwarp();
+    } else {
+        constexpr int NPC = D::NPC;
+        const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((warp >> 2) * NPC);
+        long long accA[NPC], accB[NPC];
+#pragma unroll
+        for (int c = 0; c < NPC; ++c) { accA[c] = 0; accB[c] = 0; }
+        // the window's columns go to the integer sums (orders 0-4 in units of
+        // 2^-22, orders 5-9 in units of 2^-62) and are cleared
+        auto zero_cols = [&]() {
+#pragma unroll
+            for (int o = 0; o < F_NORD; ++o)
+#pragma unroll
+                for (int c = 0; c < NPC; c += 4)
+                    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %1, %1, %1};"
+                                 :: "r"(tl + (uint32_t)(o * D::NHP + c)), "r"(0u) : "memory");
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            fence_before();
+        };
+        auto read_out = [&]() {
+            fence_after();
+#pragma unroll
+            for (int o = 0; o < F_NORD; ++o) {
+                uint32_t v[NPC];
+#pragma unroll
+                for (int c = 0; c < NPC; c += 4)
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(v[c]), "=r"(v[c + 1]), "=r"(v[c + 2]), "=r"(v[c + 3])
+                                 : "r"(tl + (uint32_t)(o * D::NHP + c)));
+                tmem_wait_ld();
+#pragma unroll
+                for (int c = 0; c < NPC; ++c) {
+                    const int x = __float2int_rz(__uint_as_float(v[c]));
+                    if (o < 5) accA[c] += (long long)x * (1ll << (8 * (4 - o)));
+                    else accB[c] += (long long)x * (1ll << (8 * (9 - o)));
+                }
+            }
+        };
+        zero_cols();
+        const int lr = 32 * (warp & 3) + lane;                          // TMEM lane (row) of this thread
+        double* rb = rbuf + warp * 256;
+        uint16_t* list = lists + warp * 256;
+        int s = 0;
+        for (; s < ns; ++s) {
+            const uint8_t* slot = ring + (s % F_RING) * D::SLOT;
+            if (is_bad_f(sy) || !__all_sync(0xffffffffu, f_wait(sy, &sy->full[s % F_RING], s / F_RING, a.slots))) break;
+            const double* srow = reinterpret_cast<const double*>(slot + D::B_TILE);
+            const uint32_t* words = reinterpret_cast<const uint32_t*>(slot + D::B_TILE + D::ROWS);
+            unsigned nib[2];
+            const double *qrow, *prow;
+            if (PS) {
+                const int64_t j = (int64_t)blockIdx.x * 32 + 2 * warp;
+                const uint32_t word = (warp >> 2) < nwc ? words[32 * (warp >> 2) + lane] : HX_PAD_WORD;
+                const int bit = 8 * (warp & 3);
+                nib[0] = j < a.J ? (word >> bit) & 0xFu : HX_PAD_NIBBLE;
+                nib[1] = j + 1 < a.J ? (word >> (bit + 4)) & 0xFu : HX_PAD_NIBBLE;
+                qrow = srow;
+                prow = fix + 8 * warp * D::KS;
+            } else {
+                const uint32_t word = words[lr];
+                const int bit = 8 * (warp >> 2);
+                nib[0] = (word >> bit) & 0xFu;
+                nib[1] = (word >> (bit + 4)) & 0xFu;
+                qrow = fix + 32 * (warp & 3) * D::KS;
+                prow = srow + 8 * (warp >> 2) * D::KS;
+            }
+            f64_weights<K, HESS>(nib, qrow, prow, rb, list, allh);
+            double W[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const unsigned nd = allh && nib[c >> 2] != NIB_MM ? 0xFu : (unsigned)(TAB_NEED >> (4 * nib[c >> 2])) & 0xFu;
+                W[c] = (nd >> (c & 3)) & 1u ? rb[32 * c + lane] : 0.0;
+            }
+            // powers of two to scale by: the exponents of the reduction indices
+            auto sh = [&](int c) {
+                const double* row = PS ? qrow + lane * D::KS : prow + c * D::KS;
+                return (HESS ? 2 : 1) * (int)__double2loint(row[K]);
+            };
+            bool big = false;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) big |= f64_out_of_range(W[c], sh(c));
+            if (big) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    if (f64_out_of_range(W[c], sh(c))) {
+                        const int c0 = grp * D::PER, c1 = min(D::NV, c0 + D::PER);
+                        if (PS)
+                            f64_rare<K, HESS>(W[c], qrow + lane * D::KS, fa.mx, fa.nmx, c0, c1, fa.rare,
+                                              row0 + 8 * warp + c);
+                        else
+                            f64_rare<K, HESS>(W[c], prow + c * D::KS, fa.mx, fa.nmx, c0, c1, fa.rare, row0 + lr);
+                        W[c] = 0.0;
+                    }
+            }
+            __syncwarp();
+            // the digit tiles and the accumulators are free once stage s-1's MMAs are done
+            if (s > 0) {
+                if (is_bad_f(sy) || !__all_sync(0xffffffffu, f_wait(sy, &sy->mma, s - 1, a.slots))) break;
+                if (s % F_WIN == 0) {
+                    read_out();
+                    zero_cols();
+                }
+            }
+            if (PS) {
+                // lane pairs (2t, 2t+1) share 32-bit words of two reduction
+                // indices: the even lane stores block 0's rows, the odd one block 1's
+                const bool odd = lane & 1;
+                const int shm = sh(0), sho = __shfl_xor_sync(0xffffffffu, shm, 1);
+                uint32_t x0[4][3], x1[4][3];
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const double mine = odd ? W[4 + h] : W[h];
+                    const double other = __shfl_xor_sync(0xffffffffu, odd ? W[h] : W[4 + h], 1);
+                    f64_fix(odd ? other : mine, odd ? sho : shm, x0[h]);
+                    f64_fix(odd ? mine : other, odd ? shm : sho, x1[h]);
+                }
+                const uint32_t at = sA + warp * SBO + (lane >> 3) * LBO + (odd ? 64 : 0) + (lane & 6) * 2;
+#pragma unroll
+                for (int w = 0; w < 3; ++w)
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) {
+                        uint32_t dg[4];
+                        f64_digits4(x0[h][w], x1[h][w], dg);
+#pragma unroll
+                        for (int t = 0; t < (w < 2 ? 4 : 2); ++t)
+                            asm volatile("st.shared.b32 [%0], %1;"
+                                         :: "r"(at + (uint32_t)((F_NDA - 1 - (4 * w + t)) * AT + 16 * h)), "r"(dg[t])
+                                         : "memory");
+                    }
+            } else {
+                uint32_t x[8][3];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) f64_fix(W[c], sh(c), x[c]);
+                const uint32_t at = sA + (lr >> 3) * SBO + (warp >> 2) * LBO + (lr & 7) * 16;
+#pragma unroll
+                for (int w = 0; w < 3; ++w) {
+                    uint32_t dg[4][4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) f64_digits4(x[2 * e][w], x[2 * e + 1][w], dg[e]);
+#pragma unroll
+                    for (int t = 0; t < (w < 2 ? 4 : 2); ++t)
+                        sts128(at + (uint32_t)((F_NDA - 1 - (4 * w + t)) * AT), dg[0][t], dg[1][t], dg[2][t], dg[3][t]);
+                }
+            }
+            fence_async_smem();
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sy->gen);
+        }
+        if (s == ns && ns > 0 && __all_sync(0xffffffffu, f_wait(sy, &sy->mma, ns - 1, a.slots))) read_out();
+        const int64_t rows = PS ? 4 * a.J : a.Ipad;
+        const int64_t row = row0 + lr;
+        if (row < rows) {
+            double* out = a.part + (int64_t)blockIdx.y * D::NV * rows;
+#pragma unroll
+            for (int c = 0; c < NPC; ++c) {
+                const int col = (warp >> 2) * NPC + c;
+                const int v = grp * D::PER + col;
+                if (col < D::PER && v < D::NV)
+                    out[(int64_t)v * rows + row] = scalbn((double)accA[c], -22) + scalbn((double)accB[c], -62);
+            }
+        }
+    }
+    __syncthreads();
+    if (is_bad_f(sy)) {
+        // a wait ran out: let the MMAs and copies that were issued end before
+        // tensor and shared memory are released
+        const int n = sy->issued, l = sy->loaded;
+        if (n > 0) mbar_wait(&sy->mma, (uint32_t)((n - 1) & 1), F_BUDGET);
+        for (int t = (l >= F_RING ? l - F_RING : 0); t < l; ++t)
+            mbar_wait(&sy->full[t % F_RING], (uint32_t)((t / F_RING) & 1), F_BUDGET);
+        __syncthreads();
+    }
+    fence_before();
+    __syncthreads();
+    if (warp == F_GEN_WARPS) {
+        fence_after();
+        tmem_dealloc<D::TCOLS>(tmem);
+    }
+}
+
+}  // namespace
+}  // namespace hx

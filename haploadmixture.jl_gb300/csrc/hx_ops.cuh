@@ -12,8 +12,8 @@ enum Slot {
 };
 
 // pass launchers: precision-specific translation units
-cudaError_t launch_accum_q_f64(int K, bool hess, const PassArgs& a, cudaStream_t st);
-cudaError_t launch_accum_p_f64(int K, bool hess, const PassArgs& a, cudaStream_t st);
+
+
 cudaError_t launch_loglik_f64(int K, const PassArgs& a, cudaStream_t st);
 cudaError_t launch_accum_q_f32(int K, bool hess, const PassArgs& a, cudaStream_t st);
 cudaError_t launch_accum_p_f32(int K, bool hess, const PassArgs& a, cudaStream_t st);
@@ -52,6 +52,39 @@ cudaError_t init_tc_attrs();
 // CTAs of the Hessian tensor-core pass resident on one SM (registers, shared
 // memory and TMEM columns), after init_tc_attrs
 int tc_resident(int K, bool p_side);
+
+// plain (FP64) method's gradient/Hessian passes (hx_f64.cuh): out-of-range
+// weights, kept zero between passes, and what the pass kernel takes beside
+// PassArgs (per_chunk counts stages there).
+struct F64Rare {
+    long long* i;          // [rows][NV][2] fixed-point sums
+    double* d;             // [rows][NV]
+    int* flag;             // bit 0: i was added to, bit 1: d was
+};
+constexpr int F_MXS = 16;  // partial maxima of one block: HX_KMAX values, then a flag
+constexpr int F_MAXB = 64; // blocks of partial maxima
+struct F64Args {
+    int64_t stages;                   // of 32 reduction indices
+    const unsigned long long* mx;     // [nmx][F_MXS]
+    int nmx;
+    F64Rare rare;
+};
+// One pass: partial maxima of v, stage images, the pass (partial sums in
+// a.part, [S][NV][rows]) and their reduction to XtX and Xtz (a.XtX, a.Xtz).
+struct F64Call {
+    bool p_side, hess;
+    PassArgs a;
+    unsigned long long* mx;           // F_MAXB * F_MXS words
+    F64Rare rare;
+    cudaStream_t st;
+};
+cudaError_t launch_f64_pass(int K, const F64Call& c);
+cudaError_t f64_attrs(int K);         // once per device before the first pass
+size_t f64_image_bytes(int K, int64_t I, int64_t J);
+cudaError_t launch_f64_reduce(const double* part, int S, int K, bool hess, int64_t rows, int64_t ld, const double* x,
+                              const unsigned long long* mx, int nmx, const F64Rare& rare, double* XtX, double* Xtz,
+                              cudaStream_t st);
+constexpr int F64_MAX_STAGES = 2048;  // stages per chunk: bounds the 64-bit sums
 
 cudaError_t launch_f2d(const float* a, int64_t n, double* out, cudaStream_t st);
 cudaError_t launch_d2f(const double* a, int64_t n, float* out, cudaStream_t st);

@@ -10,6 +10,7 @@
 
 namespace hx {
 
+#ifdef HX_ACCUM
 cudaError_t HX_CAT(launch_accum_q, HX_SUF)(int K, bool hess, const PassArgs& a, cudaStream_t st) {
     dim3 grid((unsigned)(a.Ipad / ACC_THREADS), (unsigned)a.S);
 #define HX_CASE(KK) \
@@ -29,6 +30,8 @@ cudaError_t HX_CAT(launch_accum_p, HX_SUF)(int K, bool hess, const PassArgs& a, 
 #undef HX_CASE
     return cudaGetLastError();
 }
+
+#endif
 
 cudaError_t HX_CAT(launch_loglik, HX_SUF)(int K, const PassArgs& a, cudaStream_t st) {
     dim3 grid((unsigned)(a.Ipad / ACC_THREADS), (unsigned)a.S);
