@@ -155,6 +155,21 @@ int64_t pick_chunk(int64_t tiles, int64_t units, int64_t slots, int64_t waves) {
     return best;
 }
 
+// Chunk length of the plain method's passes (one CTA per SM): the split with
+// the least time for its last wave, each CTA costing its stages plus about one
+// stage for its start and end.
+int64_t pick_chunk_f64(int64_t tiles, int64_t units, int64_t slots) {
+    int64_t best = std::min<int64_t>(units, F64_MAX_STAGES), bcost = INT64_MAX;
+    for (int64_t s = 1; s <= std::min(units, 16 * slots / tiles + 16); ++s) {
+        const int64_t per = (units + s - 1) / s;
+        if (per > F64_MAX_STAGES) continue;
+        const int64_t sa = (units + per - 1) / per;
+        const int64_t cost = (tiles * sa + slots - 1) / slots * (per + 1);
+        if (cost < bcost) { bcost = cost; best = per; }
+    }
+    return best;
+}
+
 // Chunk lengths (grid.y splits) of the mixed method's three pass kernels that
 // hx_autotune measured fastest, per device, K, I and J, for the whole process.
 struct TuneVal { int wpc_qt, spc_pt, wpc_ll; };
@@ -200,9 +215,9 @@ void plan(hx_ctx* c) {
     c->S_p = (int)((c->I + ipc - 1) / ipc);
     // plain method's passes: one CTA per SM, chunks within the 64-bit sums' range
     const int64_t nst_p = (c->I + 31) / 32;
-    c->spc_qf = (int)std::min<int64_t>(F64_MAX_STAGES, pick_chunk(tilesQ, c->JW, nsm, 4));
+    c->spc_qf = (int)pick_chunk_f64(tilesQ, c->JW, nsm);
     c->S_qf = (c->JW + c->spc_qf - 1) / c->spc_qf;
-    c->spc_pf = (int)std::min<int64_t>(F64_MAX_STAGES, pick_chunk(tilesP, nst_p, nsm, 4));
+    c->spc_pf = (int)pick_chunk_f64(tilesP, nst_p, nsm);
     c->S_pf = (int)((nst_p + c->spc_pf - 1) / c->spc_pf);
     // tensor-core passes (stages of one word column, Q, or 32 individuals, P)
     // and the FP32 log-likelihood pass: >= 8 waves with a full last wave

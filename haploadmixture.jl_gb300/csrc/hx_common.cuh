@@ -187,33 +187,6 @@ __device__ __forceinline__ float pair_lik_tab(unsigned nib, const float qp[4], c
     return F1 * F2;
 }
 
-// Type-generic entry: FP32 uses the indicator table, FP64 the exact select form.
-__device__ __forceinline__ void pair_eval_t(unsigned nib, const float qp[4], float& L, float u[4], const float4* tab) {
-    pair_eval_tab(nib, qp, L, u, tab);
-}
-__device__ __forceinline__ void pair_eval_t(unsigned nib, const double qp[4], double& L, double u[4], const float4*) {
-    pair_eval<double>(nib, qp, L, u);
-}
-
-__device__ __forceinline__ float pair_lik_t(unsigned nib, const float qp[4], const float4* tab) {
-    return pair_lik_tab(nib, qp, tab);
-}
-__device__ __forceinline__ double pair_lik_t(unsigned nib, const double qp[4], const float4*) {
-    const unsigned m1 = (unsigned)(TAB_M1 >> (4 * nib)) & 0xFu;
-    const unsigned m2 = (unsigned)(TAB_M2 >> (4 * nib)) & 0xFu;
-    double F1 = ((((m1 & 1u) ? qp[0] : 0.0) + ((m1 & 2u) ? qp[1] : 0.0)) + ((m1 & 4u) ? qp[2] : 0.0)) +
-                ((m1 & 8u) ? qp[3] : 0.0);
-    double F2 = ((((m2 & 1u) ? qp[0] : 0.0) + ((m2 & 2u) ? qp[1] : 0.0)) + ((m2 & 4u) ? qp[2] : 0.0)) +
-                ((m2 & 8u) ? qp[3] : 0.0);
-    const bool hh = nib == NIB_HH;
-    const bool mm = nib == NIB_MM;
-    const double den = qp[0] * qp[3] + qp[1] * qp[2];
-    F1 = hh ? den : F1;
-    F1 = mm ? 1.0 : F1;
-    F2 = (hh || mm) ? 1.0 : F2;
-    return F1 * F2;
-}
-
 // Packed FP32x2 arithmetic (sm_100+): fma.rn.f32x2 performs two IEEE FMAs,
 // lane by lane, with the results of two fmaf calls.
 __device__ __forceinline__ uint64_t f2_dup(float x) {

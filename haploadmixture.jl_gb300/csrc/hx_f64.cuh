@@ -37,6 +37,7 @@
 #pragma once
 #include "hx_ops.cuh"
 #include "hx_tc.cuh"
+#include "hx_items.cuh"
 
 namespace hx {
 namespace {
@@ -85,37 +86,20 @@ template <int K, bool HESS, bool PS> constexpr size_t f_smem() {
            F_GEN_WARPS * 256 * (8 + 2) + sizeof(FSync);
 }
 
-// Needed haplotypes of a class (all four for the double heterozygote, none for
-// double missing).
-__host__ __device__ constexpr unsigned class_need(unsigned nib) {
-    return nib == NIB_HH ? 0xFu : (class_m1(nib) | class_m2(nib));
-}
-__host__ __device__ constexpr uint64_t make_need() {
-    uint64_t t = 0;
-    for (unsigned n = 0; n < 16; ++n) t |= (uint64_t)class_need(n) << (4 * n);
-    return t;
-}
-constexpr uint64_t TAB_NEED = make_need();
-// Classes whose counts depend on qp: the double heterozygote and one SNP missing.
-__host__ __device__ constexpr unsigned make_cplx() {
-    unsigned t = 0;
-    for (unsigned n = 0; n < 16; ++n)
-        if (n == NIB_HH || ((((n & 3u) == 1u) != ((n >> 2) == 1u)))) t |= 1u << n;
-    return t;
-}
-constexpr unsigned TAB_CPLX = make_cplx();
-
 // 1/x by one step of the cubically convergent form of Newton's iteration
 // (Householder): r (1 + e + e^2), e = 1 - x r, from the hardware's 20-bit
 // reciprocal: e^3 < 2^-56.  Three FP64 operations instead of the eight or more
-// of a division.  Outside 2^-1000 .. 2^1000 (zeros, NaN, infinities) it divides.
+// of a division.  Outside 2^-1000 .. 2^1000 (zeros, NaN, infinities) it divides,
+// out of line: inlined, the division's predicated-off operations still took
+// their issue slots (104 instead of 74 FP64 instructions per 64 pairs at K = 5).
+__device__ __noinline__ double rcp64_edge(double x) { return 1.0 / x; }
 __device__ __forceinline__ double rcp64(double x) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
     const double e = fma(-x, r, 1.0);
     r = fma(r, fma(e, e, e), r);
     const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7FFu;
-    if (ex - 23u > 2000u) r = 1.0 / x;
+    if (ex - 23u > 2000u) r = rcp64_edge(x);
     return r;
 }
 
@@ -313,10 +297,10 @@ __device__ __forceinline__ void f64_weights(const unsigned (&nib)[2], const doub
             if (HESS) w = r * r;
             if (it & 256u) {                            // both copies: times 2, by the exponent where that is in range
                 const unsigned ex = ((unsigned)__double2hiint(w) >> 20) & 0x7FFu;
-                w = ex - 1u < 2045u ? __hiloint2double(__double2hiint(w) + 0x00100000, __double2loint(w)) : w + w;
+                if (ex - 1u < 2045u) w = __hiloint2double(__double2hiint(w) + 0x00100000, __double2loint(w));
             }
-            // listed for its zero frequency only (see allh)
-            if (HESS && (it & 1024u)) w = r * 0.0;
+            // listed for a frequency of zero only (see allh)
+            if (HESS && (it & 1024u)) w = (__double2hiint(r) & 0x7FF00000) == 0x7FF00000 ? NAN : 0.0;
         }
         if (on) rb[(it & 255u)] = w;                    // it & 255 = 32 c + lane
     }

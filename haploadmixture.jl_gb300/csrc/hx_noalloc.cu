@@ -22,11 +22,12 @@ constexpr int NA_THREADS = 128;
 // Scratch of the no-allocation entry point: one FP64 partial per CTA.
 __device__ __align__(256) double g_noalloc_scratch[HX_NOALLOC_SCRATCH];
 
-// One individual per thread over a chunk of blocks, decoding the two SNP codes
+// Mixed method (the plain FP64 one is k_loglik64 in hx_pass_f64.cu): one
+// individual per thread over a chunk of blocks, decoding the two SNP codes
 // of each block straight from the BED bytes (src/loops.jl:55-71); pair
 // likelihoods multiply into an exponent-renormalised product (one log per
 // thread).  Writes one partial per CTA into scratch[blockIdx.y * gridDim.x + blockIdx.x].
-template <int K, typename T>
+template <int K>
 __global__ void __launch_bounds__(NA_THREADS)
 k_loglik_bed(const uint8_t* __restrict__ bed, int64_t bps, int64_t I, int64_t J, const double* __restrict__ q,
              const double* __restrict__ p, int64_t per_chunk, double* __restrict__ scratch) {
@@ -36,10 +37,10 @@ k_loglik_bed(const uint8_t* __restrict__ bed, int64_t bps, int64_t I, int64_t J,
     const bool active = i < I;
     const int64_t j0 = (int64_t)blockIdx.y * per_chunk;
     const int64_t j1 = min(J, j0 + per_chunk);
-    T qi[K];
+    float qi[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) qi[k] = active ? (T)q[(int64_t)K * i + k] : T(1) / T(K);
-    T mant = T(1);
+    for (int k = 0; k < K; ++k) qi[k] = active ? (float)q[(int64_t)K * i + k] : 1.f / K;
+    float mant = 1.f;
     int ex = 0;
     bool zero = false, bad = false;
     if (active) {
@@ -51,17 +52,17 @@ k_loglik_bed(const uint8_t* __restrict__ bed, int64_t bps, int64_t I, int64_t J,
             const unsigned nib = c1 | (c2 << 2);
             if (nib == NIB_MM) continue;
             const double* pj = p + (int64_t)K * 4 * j;
-            T qp[4];
+            float qp[4];
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
-                T s = T(0);
+                float s = 0.f;
 #pragma unroll
-                for (int k = 0; k < K; ++k) s = fma(qi[k], (T)pj[h * K + k], s);
+                for (int k = 0; k < K; ++k) s = fma(qi[k], (float)pj[h * K + k], s);
                 qp[h] = s;
             }
-            T L, u[4];
-            pair_eval<T>(nib, qp, L, u);
-            if (sizeof(T) == 4 && L < T(1.17549435e-38f) && L == L) {
+            float L, u[4];
+            pair_eval<float>(nib, qp, L, u);
+            if (L < 1.17549435e-38f && L == L) {
                 // FP32 pair likelihood below the smallest normal float (caller
                 // Q/P entries far below the fit's 1e-5 floor): the renormaliser
                 // reads the exponent field, so redo this pair in FP64 and fold
@@ -79,12 +80,12 @@ k_loglik_bed(const uint8_t* __restrict__ bed, int64_t bps, int64_t I, int64_t J,
                     if (Ld == 0.0) zero = true; else bad = true;
                     continue;
                 }
-                mant = renorm(mant * (T)renorm(Ld, ex), ex);
+                mant = renorm(mant * (float)renorm(Ld, ex), ex);
                 continue;
             }
-            if (!(L > T(0))) {
-                if (L == T(0)) zero = true; else bad = true;
-                L = T(1);
+            if (!(L > 0.f)) {
+                if (L == 0.f) zero = true; else bad = true;
+                L = 1.f;
             }
             mant = renorm(mant * L, ex);
         }
@@ -120,11 +121,10 @@ __global__ void k_sum_partials(const double* __restrict__ scratch, int64_t n, do
 
 #define HX_NA_FOR_K(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12)
 
-template <typename T>
 cudaError_t launch_bed(int K, dim3 grid, cudaStream_t st, const uint8_t* bed, int64_t bps, int64_t I, int64_t J,
                        const double* q, const double* p, int64_t per_chunk, double* scratch) {
 #define HX_CASE(KK) \
-    case KK: k_loglik_bed<KK, T><<<grid, NA_THREADS, 0, st>>>(bed, bps, I, J, q, p, per_chunk, scratch); break;
+    case KK: k_loglik_bed<KK><<<grid, NA_THREADS, 0, st>>>(bed, bps, I, J, q, p, per_chunk, scratch); break;
     switch (K) { HX_NA_FOR_K(HX_CASE) default: return cudaErrorInvalidValue; }
 #undef HX_CASE
     return cudaGetLastError();
@@ -152,17 +152,29 @@ extern "C" int hx_loglikelihood_noalloc(const uint8_t* d_bed, int64_t bytes_per_
     void* ptr = nullptr;
     if (cudaGetSymbolAddress(&ptr, g_noalloc_scratch) != cudaSuccess || !ptr) return HX_ECUDA;
     double* scratch = (double*)ptr;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (precision == HX_PREC_FP64) {
+        // chunks of whole word columns (8 blocks), as many CTAs as run at once
+        const int64_t JW = (J + 7) / 8;
+        int64_t S = std::max<int64_t>(1, std::min<int64_t>(JW, (1216 + tiles - 1) / tiles));
+        S = std::min<int64_t>(S, HX_NOALLOC_SCRATCH / tiles);
+        const int64_t per = (JW + S - 1) / S;
+        S = (JW + per - 1) / per;
+        PassArgs a{};
+        a.I = I; a.J = J; a.JW = (int)JW;
+        a.q = d_q; a.p = d_p; a.S = (int)S; a.per_chunk = (int)per; a.part = scratch;
+        if (launch_loglik_f64_bed(K, a, d_bed, bytes_per_snp, st) != cudaSuccess) return HX_ECUDA;
+        k_sum_partials<<<1, 256, 0, st>>>(scratch, tiles * S, d_ll);
+        return cudaGetLastError() == cudaSuccess ? HX_OK : HX_ECUDA;
+    }
     const int64_t target = 2048;
     int64_t S = std::max<int64_t>(1, std::min<int64_t>(J, (target + tiles - 1) / tiles));
     S = std::min<int64_t>(S, HX_NOALLOC_SCRATCH / tiles);
     const int64_t per_chunk = (J + S - 1) / S;
     S = (J + per_chunk - 1) / per_chunk;
     dim3 grid((unsigned)tiles, (unsigned)S);
-    cudaStream_t st = (cudaStream_t)stream;
-    cudaError_t e = precision == HX_PREC_FP64
-                        ? launch_bed<double>(K, grid, st, d_bed, bytes_per_snp, I, J, d_q, d_p, per_chunk, scratch)
-                        : launch_bed<float>(K, grid, st, d_bed, bytes_per_snp, I, J, d_q, d_p, per_chunk, scratch);
-    if (e != cudaSuccess) return HX_ECUDA;
+    if (launch_bed(K, grid, st, d_bed, bytes_per_snp, I, J, d_q, d_p, per_chunk, scratch) != cudaSuccess)
+        return HX_ECUDA;
     k_sum_partials<<<1, 256, 0, st>>>(scratch, tiles * S, d_ll);
     if (cudaGetLastError() != cudaSuccess) return HX_ECUDA;
     return HX_OK;

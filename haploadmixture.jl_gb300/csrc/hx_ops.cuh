@@ -1,5 +1,5 @@
 // hx_ops.cuh -- declarations of the non-pass kernels and launchers (hx_ops.cu)
-// and of the pass launchers (hx_pass_f64.cu / hx_pass_f32.cu).
+// and of the pass launchers.
 #pragma once
 #include "hx_pass.cuh"
 
@@ -11,13 +11,12 @@ enum Slot {
     S_ITER = 6, S_TMP = 7, S_QP_FAIL = 8, S_NAN = 9, S_TC_TIMEOUT = 10, HX_NSLOT = 16
 };
 
-// pass launchers: precision-specific translation units
-
-
+// pass launchers
 cudaError_t launch_loglik_f64(int K, const PassArgs& a, cudaStream_t st);
+// the same from BED bytes (first I individuals, 2J SNPs); a.G and a.Ipad unused
+cudaError_t launch_loglik_f64_bed(int K, const PassArgs& a, const uint8_t* bed, int64_t bps, cudaStream_t st);
 cudaError_t launch_accum_q_f32(int K, bool hess, const PassArgs& a, cudaStream_t st);
 cudaError_t launch_accum_p_f32(int K, bool hess, const PassArgs& a, cudaStream_t st);
-cudaError_t launch_loglik_f32(int K, const PassArgs& a, cudaStream_t st);
 cudaError_t launch_loglik_f32x2(int K, const PassArgs& a, cudaStream_t st);   // several individuals per thread
 int loglik_f32x2_blocks(int64_t Ipad, int K);
 int loglik_f32x2_resident(int K);   // CTAs of launch_loglik_f32x2 resident on one SM

@@ -1,10 +1,9 @@
 // hx_pass.cuh -- the streaming passes over the genotype classes (CUDA cores).
 //
-// Three kernels, templated on the number of ancestries K (register-resident
-// accumulators) and on the arithmetic type T:
-//   T = double : the plain FP64 method (the reference's arithmetic class),
-//   T = float  : the mixed method (FP32 products, FP64 cross-chunk totals and
-//                FP64 stage-level promotion of the gradient).
+// Kernels of the mixed method, templated on the number of ancestries K
+// (register-resident accumulators): FP32 products, FP64 cross-chunk totals and
+// FP64 stage-level promotion of the gradient.  (The plain FP64 method's are in
+// hx_f64.cuh and hx_pass_f64.cu.)
 //
 //   k_accum_q  : per individual i over a chunk of blocks (src/loops.jl:328-365,
 //                src/cuda/kernels.jl:104-138):
@@ -14,7 +13,7 @@
 //                (src/loops.jl:367-403, src/cuda/kernels.jl:140-175):
 //                Xtz_p[k,m]    = sum_i c_h q[k,i] / qp_h
 //                XtX_p[k2,k,m] = sum_i c_h q[k,i] q[k2,i] / qp_h^2
-//   k_loglik   : sum over pairs of log L (src/loops.jl:236-258,
+//   k_loglik2  : sum over pairs of log L (src/loops.jl:236-258,
 //                src/cuda/kernels.jl:16-40), as the log of an exponent-
 //                renormalised running product (one log per thread).
 //
@@ -57,12 +56,12 @@ template <int K> __device__ __forceinline__ constexpr int tri(int k, int k2) {
 }
 
 // ------------------------------------------------------------------ Q side
-template <int K, typename T, bool HESS>
+template <int K, bool HESS>
 __global__ void __launch_bounds__(ACC_THREADS)
 k_accum_q(PassArgs a) {
     constexpr int NH = K * (K + 1) / 2;
     constexpr int NV = K + (HESS ? NH : 0);
-    __shared__ T sp[QSTAGE_WORDS * 8 * 4 * K];
+    __shared__ float sp[QSTAGE_WORDS * 8 * 4 * K];
     __shared__ float4 s_snp[4];
     const int tid = threadIdx.x;
     snp_table_init(s_snp, tid);
@@ -70,16 +69,16 @@ k_accum_q(PassArgs a) {
     const int w0 = blockIdx.y * a.per_chunk;
     const int w1 = min(a.JW, w0 + a.per_chunk);
     const bool active = i < a.I;
-    T qi[K];
+    float qi[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) qi[k] = active ? (T)a.q[(int64_t)K * i + k] : T(1) / T(K);
-    T gin[K];
+    for (int k = 0; k < K; ++k) qi[k] = active ? (float)a.q[(int64_t)K * i + k] : 1.f / K;
+    float gin[K];
     double gout[K];
-    T H[HESS ? NH : 1];
+    float H[HESS ? NH : 1];
 #pragma unroll
-    for (int k = 0; k < K; ++k) { gin[k] = T(0); gout[k] = 0.0; }
+    for (int k = 0; k < K; ++k) { gin[k] = 0.f; gout[k] = 0.0; }
 #pragma unroll
-    for (int v = 0; v < (HESS ? NH : 1); ++v) H[v] = T(0);
+    for (int v = 0; v < (HESS ? NH : 1); ++v) H[v] = 0.f;
 
     for (int ws = w0; ws < w1; ws += QSTAGE_WORDS) {
         const int nw = min(QSTAGE_WORDS, w1 - ws);
@@ -92,7 +91,7 @@ k_accum_q(PassArgs a) {
         const int64_t base = (int64_t)ws * 8 * 4 * K;
         const int64_t limit = a.J * 4 * K;
         for (int t = tid; t < nval; t += ACC_THREADS)
-            sp[t] = (base + t < limit) ? ((sizeof(T) == 4 && a.pf) ? (T)a.pf[base + t] : (T)a.p[base + t]) : T(0.25);
+            sp[t] = (base + t < limit) ? (a.pf ? a.pf[base + t] : (float)a.p[base + t]) : 0.25f;
         __syncthreads();
         if (active) {
             for (int w = 0; w < nw; ++w) {
@@ -101,20 +100,20 @@ k_accum_q(PassArgs a) {
                 for (int b = 0; b < 8; ++b) {
                     const unsigned nib = (word >> (4 * b)) & 0xFu;
                     if (nib == NIB_MM) continue;
-                    const T* pb = sp + (w * 8 + b) * 4 * K;
-                    T qp[4];
+                    const float* pb = sp + (w * 8 + b) * 4 * K;
+                    float qp[4];
 #pragma unroll
                     for (int h = 0; h < 4; ++h) {
-                        T s = T(0);
+                        float s = 0.f;
 #pragma unroll
                         for (int k = 0; k < K; ++k) s = fma(qi[k], pb[h * K + k], s);
                         qp[h] = s;
                     }
-                    T L, u[4];
-                    pair_eval_t(nib, qp, L, u, s_snp);
+                    float L, u[4];
+                    pair_eval_tab(nib, qp, L, u, s_snp);
 #pragma unroll
                     for (int k = 0; k < K; ++k) {
-                        T g = gin[k];
+                        float g = gin[k];
                         g = fma(u[0], pb[k], g);
                         g = fma(u[1], pb[K + k], g);
                         g = fma(u[2], pb[2 * K + k], g);
@@ -124,8 +123,8 @@ k_accum_q(PassArgs a) {
                     if (HESS) {
 #pragma unroll
                         for (int h = 0; h < 4; ++h) {
-                            const T wh = u[h] * rcp<T>(qp[h]);
-                            T t[K];
+                            const float wh = u[h] * __frcp_rn(qp[h]);
+                            float t[K];
 #pragma unroll
                             for (int k = 0; k < K; ++k) t[k] = wh * pb[h * K + k];
 #pragma unroll
@@ -138,9 +137,9 @@ k_accum_q(PassArgs a) {
                 }
             }
         }
-        // promote the stage's gradient partial to FP64 (exact for T = double)
+        // promote the stage's gradient partial to FP64
 #pragma unroll
-        for (int k = 0; k < K; ++k) { gout[k] += (double)gin[k]; gin[k] = T(0); }
+        for (int k = 0; k < K; ++k) { gout[k] += (double)gin[k]; gin[k] = 0.f; }
     }
     if (i < a.Ipad) {
         double* out = a.part + (int64_t)blockIdx.y * NV * a.Ipad;
@@ -156,12 +155,12 @@ k_accum_q(PassArgs a) {
 // ------------------------------------------------------------------ P side
 // Thread (b, h) of a CTA owns haplotype column m = 4*(32*blockIdx.x + b) + h;
 // the 4 threads of a block exchange their qp_h by warp shuffles.
-template <int K, typename T, bool HESS>
+template <int K, bool HESS>
 __global__ void __launch_bounds__(ACC_THREADS)
 k_accum_p(PassArgs a) {
     constexpr int NH = K * (K + 1) / 2;
     constexpr int NV = K + (HESS ? NH : 0);
-    __shared__ T sq[PSTAGE_IND * K];
+    __shared__ float sq[PSTAGE_IND * K];
     __shared__ uint32_t sg[4 * PSTAGE_IND];
     __shared__ float4 s_snp[4];
     const int tid = threadIdx.x;
@@ -171,24 +170,24 @@ k_accum_p(PassArgs a) {
     const int64_t j = (int64_t)blockIdx.x * 32 + b;
     const bool valid = j < a.J;
     const int64_t m = 4 * j + h;
-    T pr[K];
+    float pr[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) pr[k] = valid ? (T)a.p[(int64_t)K * m + k] : T(0.25);
+    for (int k = 0; k < K; ++k) pr[k] = valid ? (float)a.p[(int64_t)K * m + k] : 0.25f;
     const int64_t i0 = (int64_t)blockIdx.y * a.per_chunk;
     const int64_t i1 = min(a.I, i0 + (int64_t)a.per_chunk);
     const int bsh = 4 * (b & 7);
-    T gin[K];
+    float gin[K];
     double gout[K];
-    T H[HESS ? NH : 1];
+    float H[HESS ? NH : 1];
 #pragma unroll
-    for (int k = 0; k < K; ++k) { gin[k] = T(0); gout[k] = 0.0; }
+    for (int k = 0; k < K; ++k) { gin[k] = 0.f; gout[k] = 0.0; }
 #pragma unroll
-    for (int v = 0; v < (HESS ? NH : 1); ++v) H[v] = T(0);
+    for (int v = 0; v < (HESS ? NH : 1); ++v) H[v] = 0.f;
 
     for (int64_t is = i0; is < i1; is += PSTAGE_IND) {
         const int n = (int)min((int64_t)PSTAGE_IND, i1 - is);
         __syncthreads();
-        for (int t = tid; t < n * K; t += ACC_THREADS) sq[t] = (T)a.q[(int64_t)K * is + t];
+        for (int t = tid; t < n * K; t += ACC_THREADS) sq[t] = (float)a.q[(int64_t)K * is + t];
         for (int t = tid; t < 4 * PSTAGE_IND; t += ACC_THREADS) {
             const int w = t / PSTAGE_IND, r = t % PSTAGE_IND;
             const int64_t jw = (int64_t)blockIdx.x * 4 + w;
@@ -198,21 +197,21 @@ k_accum_p(PassArgs a) {
 #pragma unroll 1
         for (int r = 0; r < n; ++r) {
             const unsigned nib = (sg[warp * PSTAGE_IND + r] >> bsh) & 0xFu;
-            const T* qr = sq + r * K;
-            T own = T(0);
+            const float* qr = sq + r * K;
+            float own = 0.f;
 #pragma unroll
             for (int k = 0; k < K; ++k) own = fma(qr[k], pr[k], own);
-            T qp[4];
+            float qp[4];
 #pragma unroll
             for (int t = 0; t < 4; ++t) qp[t] = __shfl_sync(0xffffffffu, own, (lane & ~3) | t);
-            T L, u[4];
-            pair_eval_t(nib, qp, L, u, s_snp);
-            const T uh = h == 0 ? u[0] : (h == 1 ? u[1] : (h == 2 ? u[2] : u[3]));
+            float L, u[4];
+            pair_eval_tab(nib, qp, L, u, s_snp);
+            const float uh = h == 0 ? u[0] : (h == 1 ? u[1] : (h == 2 ? u[2] : u[3]));
 #pragma unroll
             for (int k = 0; k < K; ++k) gin[k] = fma(uh, qr[k], gin[k]);
             if (HESS) {
-                const T wh = uh * rcp<T>(own);
-                T t[K];
+                const float wh = uh * __frcp_rn(own);
+                float t[K];
 #pragma unroll
                 for (int k = 0; k < K; ++k) t[k] = wh * qr[k];
 #pragma unroll
@@ -222,7 +221,7 @@ k_accum_p(PassArgs a) {
             }
         }
 #pragma unroll
-        for (int k = 0; k < K; ++k) { gout[k] += (double)gin[k]; gin[k] = T(0); }
+        for (int k = 0; k < K; ++k) { gout[k] += (double)gin[k]; gin[k] = 0.f; }
     }
     if (!valid) return;
     if (a.S == 1) {
@@ -248,82 +247,8 @@ k_accum_p(PassArgs a) {
     }
 }
 
-// ------------------------------------------------------------------ loglik
-template <int K, typename T>
-__global__ void __launch_bounds__(ACC_THREADS)
-k_loglik(PassArgs a) {
-    __shared__ T sp[QSTAGE_WORDS * 8 * 4 * K];
-    __shared__ double red[ACC_THREADS];
-    __shared__ float4 s_snp[4];
-    const int tid = threadIdx.x;
-    snp_table_init(s_snp, tid);
-    const int64_t i = (int64_t)blockIdx.x * ACC_THREADS + tid;
-    const int w0 = blockIdx.y * a.per_chunk;
-    const int w1 = min(a.JW, w0 + a.per_chunk);
-    const bool active = i < a.I;
-    T qi[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) qi[k] = active ? (T)a.q[(int64_t)K * i + k] : T(1) / T(K);
-    T mant = T(1);
-    int ex = 0;
-    bool zero = false, bad = false;
-    for (int ws = w0; ws < w1; ws += QSTAGE_WORDS) {
-        const int nw = min(QSTAGE_WORDS, w1 - ws);
-        uint32_t words[QSTAGE_WORDS];
-#pragma unroll
-        for (int w = 0; w < QSTAGE_WORDS; ++w)
-            words[w] = (w < nw) ? a.G[(int64_t)(ws + w) * a.Ipad + i] : HX_PAD_WORD;
-        __syncthreads();
-        const int nval = nw * 8 * 4 * K;
-        const int64_t base = (int64_t)ws * 8 * 4 * K;
-        const int64_t limit = a.J * 4 * K;
-        for (int t = tid; t < nval; t += ACC_THREADS)
-            sp[t] = (base + t < limit) ? ((sizeof(T) == 4 && a.pf) ? (T)a.pf[base + t] : (T)a.p[base + t]) : T(0.25);
-        __syncthreads();
-        if (active) {
-            for (int w = 0; w < nw; ++w) {
-                const uint32_t word = words[w];
-#pragma unroll 2
-                for (int b = 0; b < 8; ++b) {
-                    const unsigned nib = (word >> (4 * b)) & 0xFu;
-                    if (nib == NIB_MM) continue;
-                    const T* pb = sp + (w * 8 + b) * 4 * K;
-                    T qp[4];
-#pragma unroll
-                    for (int hh = 0; hh < 4; ++hh) {
-                        T s = T(0);
-#pragma unroll
-                        for (int k = 0; k < K; ++k) s = fma(qi[k], pb[hh * K + k], s);
-                        qp[hh] = s;
-                    }
-                    T L = pair_lik_t(nib, qp, s_snp);
-                    if (!(L > T(0))) {
-                        if (L == T(0)) zero = true; else bad = true;
-                        L = T(1);
-                    }
-                    mant = renorm(mant * L, ex);
-                }
-            }
-        }
-    }
-    double v = 0.0;
-    if (active) {
-        v = log((double)mant) + (double)ex * 0.69314718055994530942;
-        if (zero) v = -INFINITY;
-        if (bad) v = NAN;
-    }
-    red[tid] = v;
-    __syncthreads();
-    for (int s = ACC_THREADS / 2; s > 0; s >>= 1) {
-        if (tid < s) red[tid] += red[tid + s];
-        __syncthreads();
-    }
-    if (tid == 0) a.part[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = red[0];
-}
-
 // ------------------------------------------------------------------ loglik, FP32
-// The mixed method's log-likelihood pass (same sums as k_loglik<K, float>):
-// each thread carries NU individuals (i + u ACC_THREADS) that share every
+// The mixed method's log-likelihood pass: each thread carries NU individuals (i + u ACC_THREADS) that share every
 // staged p row, and forms qp for haplotype pairs (h, h+1) with packed FP32x2
 // FMAs (fma.rn.f32x2: two IEEE FMAs per instruction, the same results and
 // order as fmaf).  Stage rows are transposed to [block][k][h] so that one

@@ -84,3 +84,40 @@ def test_non_finite_and_zero_frequencies_reach_the_hessian(hx, O):
     b = O.Bed(c["bed"], I, J)
     assert entry_err(ok[0], O.accum_q(b, K, q, p)[0]) < 1e-13
     d.close()
+
+
+@pytest.mark.parametrize("I,J,K", [(1, 1, 1), (33, 9, 2), (128, 8, 4), (129, 127, 7), (500, 65, 12)])
+def test_loglik_items_and_chunks(hx, O, I, J, K):
+    """Log-likelihood from class words and from BED bytes; a zero frequency of
+    an observed haplotype gives -inf, a NaN one NaN."""
+    import torch
+    c = small_cohort(I, J, K, seed=3 * I + J, miss=0.1)
+    b = O.Bed(c["bed"], I, J)
+    rng = np.random.default_rng(J)
+    q = np.asfortranarray(rng.dirichlet(np.ones(K), size=I).T)
+    p = np.asfortranarray(rng.dirichlet(np.ones(4), size=(K, J)).reshape(K, 4 * J))
+    d = hx.GB300Admix(c["bed"], I, J, K, bytes_per_snp=c["bed"].shape[1], n_snp=c["bed"].shape[0])
+    bed = torch.from_numpy(c["bed"]).cuda()
+    ll = torch.empty((), dtype=torch.float64, device="cuda")
+
+    def noalloc(p):
+        dq, dp = torch.from_numpy(q.T.copy()).cuda(), torch.from_numpy(p.T.copy()).cuda()
+        st = hx.load().hx_loglikelihood_noalloc(bed.data_ptr(), c["bed"].shape[1], I, J, K, dq.data_ptr(),
+                                                dp.data_ptr(), 0, ll.data_ptr(), None)
+        assert st == 0
+        torch.cuda.synchronize()
+        return float(ll)
+
+    want = O.loglik(b, K, q, p)
+    assert d.loglikelihood(q, p) == pytest.approx(want, rel=1e-13)
+    assert noalloc(p) == pytest.approx(want, rel=1e-13)
+    z = p.copy(order="F")
+    z[:, :4] = 0.0
+    want = O.loglik(b, K, q, z)
+    for got in (d.loglikelihood(q, z), noalloc(z)):
+        assert got == want or got == pytest.approx(want, rel=1e-13)
+    z[:, :4] = np.nan
+    want = O.loglik(b, K, q, z)
+    for got in (d.loglikelihood(q, z), noalloc(z)):
+        assert np.isnan(got) == np.isnan(want)
+    d.close()
