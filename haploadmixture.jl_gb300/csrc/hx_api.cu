@@ -501,7 +501,7 @@ int create_common(const uint8_t* bed, bool bed_on_device, int64_t bps, int64_t n
     HX_CK(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking));
     HX_CK(cudaEventCreate(&c->ev0));
     HX_CK(cudaEventCreate(&c->ev1));
-    HX_CK(init_kernel_attrs());
+    HX_CK(init_kernel_attrs(K));
     HX_CK(init_tc_attrs());
     if (c->prec == HX_PREC_FP64) HX_CK(f64_attrs(K));
     plan(c);

@@ -128,8 +128,11 @@ cudaError_t launch_step_q(const double* q, const double* d, int K, int64_t ncol,
                           cudaStream_t st, double factor = 1.0);
 cudaError_t launch_step_p(const double* p, const double* d, int K, int64_t J, double eps, double* out,
                           cudaStream_t st, double factor = 1.0);
-// batched QP (init_kernel_attrs: once per device, before the first launch)
-cudaError_t init_kernel_attrs();
+// batched QP (init_kernel_attrs: before the first launch for this K on a device)
+cudaError_t init_kernel_attrs(int K);
+cudaError_t init_qp_attrs(int K);
+cudaError_t launch_qp_p_pen(int K, int64_t n, const double* XtX, const double* Xtz, const double* p, double rho,
+                            double* pdiff, double* slots, int8_t* ws, cudaStream_t st);
 cudaError_t launch_qp_q(int K, int64_t n, const double* XtX, const double* Xtz, const double* q, double* qdiff,
                         double* slots, cudaStream_t st, double pen_rho = -1.0);
 // eq: the equality form (K equalities per block, rho and ws unused)

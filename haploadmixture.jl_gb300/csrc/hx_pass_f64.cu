@@ -37,6 +37,8 @@ k_loglik64(PassArgs a, const uint8_t* __restrict__ bed, int64_t bps) {
     double* qpb = sp + 32 * KS;               // [WARPS][16][32] qp of the pairs to finish
     uint16_t* lists = reinterpret_cast<uint16_t*>(qpb + L_WARPS * 512);
     __shared__ double red[L_WARPS];
+    __shared__ long long rex[L_WARPS];
+    __shared__ int rfl[L_WARPS];
     const int tid = threadIdx.x, warp = tid >> 5;
     const unsigned lane = tid & 31, lt = (1u << lane) - 1u;
     const int64_t i0 = (int64_t)blockIdx.x * 128, i = i0 + 32 * warp + lane;
@@ -161,16 +163,41 @@ k_loglik64(PassArgs a, const uint8_t* __restrict__ bed, int64_t bps) {
             __syncwarp();
         }
     }
-    double v = log(m1) + (double)e1 * 0.69314718055994530942 + 2.0 * (log(m2) + (double)e2 * 0.69314718055994530942);
-    if (zero) v = -INFINITY;
-    if (bad) v = NAN;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[warp] = v;
+    // the CTA's product, exponents apart, and one log (a log is some 40 FP64
+    // operations, more than a short chunk's own work when every lane takes two)
+    long long ex = (long long)e1 + 2ll * e2;
+    double m = m2;
+    auto mul = [&](double y) {
+        int e = 0;
+        m = renorm(m * y, e);
+        ex += e;
+    };
+    mul(m2);
+    mul(m1);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double y = __shfl_xor_sync(0xffffffffu, m, o);
+        ex += __shfl_xor_sync(0xffffffffu, ex, o);
+        mul(y);
+    }
+    const bool any_zero = __any_sync(0xffffffffu, zero), any_bad = __any_sync(0xffffffffu, bad);
+    if (lane == 0) {
+        red[warp] = m;
+        rex[warp] = ex;
+        rfl[warp] = (any_zero ? 1 : 0) | (any_bad ? 2 : 0);
+    }
     __syncthreads();
     if (tid == 0) {
-        double s = 0.0;
-        for (int x = 0; x < L_WARPS; ++x) s += red[x];
-        a.part[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = s;
+        int fl = rfl[0];
+        for (int x = 1; x < L_WARPS; ++x) {
+            mul(red[x]);
+            ex += rex[x];
+            fl |= rfl[x];
+        }
+        double v = log(m) + (double)ex * 0.69314718055994530942;
+        if (fl & 1) v = -INFINITY;
+        if (fl & 2) v = NAN;
+        a.part[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = v;
     }
 }
 

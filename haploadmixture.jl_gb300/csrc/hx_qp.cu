@@ -1,0 +1,503 @@
+// hx_qp.cu -- batched simplex-constrained QPs of the Q step and of the P step's
+// penalty form (src/algorithms_inner.jl:134-168, 264-305).
+//
+// Exact minimiser of 0.5 d'Hd - z'd, lo <= d <= hi (and sum d = 0 on the Q
+// side), by the primal active-set method of the oracle: solve on the free
+// variables (Cholesky factor of the free block), step to the first bound met
+// (lowest index on ties), and when no bound is met release the bound with the
+// largest multiplier.  GB300's FP64 unit takes 16 clocks of an SM for any warp
+// instruction, however few of its lanes work, so both kernels keep the lanes
+// full: the Q side solves one problem per lane, the P side one per group of 8
+// lanes (16 from K = 9 on).  Both perform, element by element, the operations of
+// the dense factorisation and sweeps of the free block in index order, and leave
+// out only those whose operands are exact zeros, so the results do not depend
+// on this arrangement (the mixed method rounds them to FP32 afterwards, which
+// would turn a last-bit difference into one of 6e-8).
+#include "hx_ops.cuh"
+#include "hx_tc.cuh"
+#include <climits>
+
+namespace hx {
+namespace {
+using tc::tri_idx;
+constexpr unsigned FULL = 0xffffffffu;
+
+// 1 / sqrt(s) as the factorisation uses it: the reciprocal of the rounded root
+__device__ __forceinline__ double inv_root(double s) { return 1.0 / sqrt(s); }
+
+// ------------------------------------------------------------------ Q side
+// One problem per thread, its K x K triangle in shared memory (entry e of
+// thread t at e * QQ_LD + t), factor and vectors in registers.  Rows and
+// columns of fixed variables are zero in the factor, so the code has no
+// data-dependent indices.
+constexpr int QQ_THREADS = 64, QQ_LD = QQ_THREADS + 1;
+
+// Sum of the elements of x (K <= 12) in the order of a butterfly over 16 lanes.
+template <int K> __device__ __forceinline__ double tree_sum(const double (&x)[K]) {
+    double t8[8], t4[4];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) t8[a] = (a < K ? x[a < K ? a : 0] : 0.0) + (a + 8 < K ? x[a + 8 < K ? a + 8 : 0] : 0.0);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) t4[a] = t8[a] + t8[a + 4];
+    return (t4[0] + t4[2]) + (t4[1] + t4[3]);
+}
+
+template <int K>
+__global__ void __launch_bounds__(QQ_THREADS)
+k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz, const double* __restrict__ q,
+       double* __restrict__ qdiff, double* slots, double pen_rho) {
+    constexpr int NT = K * (K + 1) / 2;
+    __shared__ double sH[NT * QQ_LD];
+    __shared__ double sX[K * QQ_THREADS];
+    const int tid = threadIdx.x;
+    const int64_t p0 = (int64_t)blockIdx.x * QQ_THREADS, pr = p0 + tid;
+    const int np = (int)min((int64_t)QQ_THREADS, n - p0);
+    const bool eq = pen_rho < 0.0;               // equality form, else rho on every entry
+    for (int t = tid; t < np * K * K; t += QQ_THREADS) {
+        const int x = t / (K * K), e = t - x * K * K, c = e / K, r = e - c * K;
+        if (r >= c) sH[tri_idx<K>(c, r) * QQ_LD + x] = XtX[p0 * K * K + t] + (eq ? 0.0 : pen_rho);
+    }
+    __syncthreads();
+    if (tid >= np) return;
+    const double* H = sH + tid;
+    double* xs = sX + tid;
+    auto h = [&](int a, int b) { return H[(a <= b ? tri_idx<K>(a, b) : tri_idx<K>(b, a)) * QQ_LD]; };
+    // Sum over the free variables as the list of them is summed: element of rank
+    // r in place r of the butterfly.
+    auto free_sum = [&](const double (&x)[K], unsigned fr) {
+        double y[K];
+        if (fr == (1u << K) - 1u) return tree_sum<K>(x);
+#pragma unroll
+        for (int a = 0; a < K; ++a) xs[a * QQ_THREADS] = 0.0;
+#pragma unroll
+        for (int a = 0; a < K; ++a)
+            if ((fr >> a) & 1u) xs[__popc(fr & ((1u << a) - 1u)) * QQ_THREADS] = x[a];
+#pragma unroll
+        for (int a = 0; a < K; ++a) y[a] = xs[a * QQ_THREADS];
+        return tree_sum<K>(y);
+    };
+    double z[K], d[K], qa[K];
+    unsigned fr = 0u, up = 0u, no = 0u;          // free; at the upper bound; both bounds at 0
+    double tol = 1.0;
+#pragma unroll
+    for (int a = 0; a < K; ++a) {
+        qa[a] = q[pr * K + a];
+        z[a] = Xtz[pr * K + a];
+        tol = fmax(tol, fabs(z[a]));
+        d[a] = 0.0;
+        if (0.0 - qa[a] >= 0.0 && 1.0 - qa[a] <= 0.0) no |= 1u << a;
+        else fr |= 1u << a;
+    }
+    tol *= 1e-12;
+    const int max_iter = 4 * K + 20;
+    bool done = false;
+#pragma unroll 1
+    for (int it = 0; it < max_iter; ++it) {
+        double A[NT], y[K], o[K];
+        double md = 0.0;
+#pragma unroll
+        for (int a = 0; a < K; ++a) {
+            const bool fa = (fr >> a) & 1u;
+            double s = z[a];
+            if (fr != (1u << K) - 1u) {
+#pragma unroll
+                for (int b = 0; b < K; ++b)
+                    if (!((fr >> b) & 1u)) s = fma(-h(a, b), d[b], s);
+            }
+            y[a] = fa ? s : 0.0;
+            o[a] = fa ? 1.0 : 0.0;
+#pragma unroll
+            for (int b = a; b < K; ++b) A[tri_idx<K>(a, b)] = fa && ((fr >> b) & 1u) ? h(a, b) : 0.0;
+            md = fmax(md, fabs(A[tri_idx<K>(a, a)]));
+        }
+        const double fl = 1e-300 + 1e-14 * md;
+        // A = L L': entry (a, b), b > a, ends as L[b, a]; y and o follow through
+        // the forward sweep
+        double iv[K];
+#pragma unroll
+        for (int a = 0; a < K; ++a) {
+            double pv = A[tri_idx<K>(a, a)];
+            if (!(pv > fl)) pv = fl;
+            iv[a] = (fr >> a) & 1u ? inv_root(pv) : 0.0;
+            y[a] *= iv[a];
+            o[a] *= iv[a];
+#pragma unroll
+            for (int b = a + 1; b < K; ++b) A[tri_idx<K>(a, b)] *= iv[a];
+#pragma unroll
+            for (int b = a + 1; b < K; ++b) {
+                const double l = A[tri_idx<K>(a, b)];
+#pragma unroll
+                for (int c = b; c < K; ++c)
+                    A[tri_idx<K>(b, c)] = fma(-l, A[tri_idx<K>(a, c)], A[tri_idx<K>(b, c)]);
+                y[b] = fma(-l, y[a], y[b]);
+                o[b] = fma(-l, o[a], o[b]);
+            }
+        }
+#pragma unroll
+        for (int a = K - 1; a >= 0; --a) {
+            y[a] *= iv[a];
+            o[a] *= iv[a];
+#pragma unroll
+            for (int b = 0; b < a; ++b) {
+                y[b] = fma(-A[tri_idx<K>(b, a)], y[a], y[b]);
+                o[b] = fma(-A[tri_idx<K>(b, a)], o[a], o[b]);
+            }
+        }
+        double nu = 0.0;
+        if (eq && fr) {
+            double f[K];
+#pragma unroll
+            for (int a = 0; a < K; ++a) f[a] = (fr >> a) & 1u ? 0.0 : -d[a];
+            nu = (free_sum(y, fr) - tree_sum<K>(f)) / free_sum(o, fr);
+        }
+        // y becomes the target of the free variables
+        double best = 1.0;
+        int bi = -1;
+        bool bup = false;
+#pragma unroll
+        for (int a = 0; a < K; ++a) {
+            if (!((fr >> a) & 1u)) { y[a] = d[a]; continue; }
+            if (eq) y[a] = fma(-nu, o[a], y[a]);
+            const double s = y[a] - d[a];
+            const bool u = s > 0.0;
+            const double num = u ? (1.0 - qa[a]) - d[a] : (0.0 - qa[a]) - d[a];    // to the bound ahead
+            // a ratio below 1 (or a bound passed by rounding), before dividing
+            if (s != 0.0 && (fabs(num) < fabs(s) || (u ? num < 0.0 : num > 0.0))) {
+                const double ra = num / s;
+                if (ra < best) { best = ra; bi = a; bup = u; }
+            }
+        }
+        if (bi < 0) {
+#pragma unroll
+            for (int a = 0; a < K; ++a) d[a] = y[a];
+            double wv = tol;
+            int rel = -1;
+            if ((fr | no) != (1u << K) - 1u) {
+#pragma unroll
+                for (int a = 0; a < K; ++a) {
+                    if (((fr | no) >> a) & 1u) continue;
+                    double g = -z[a];
+#pragma unroll
+                    for (int b = 0; b < K; ++b) g = fma(h(a, b), d[b], g);
+                    g += nu;
+                    const double v = (up >> a) & 1u ? g : -g;
+                    if (v > wv) { wv = v; rel = a; }
+                }
+            }
+            if (rel < 0) { done = true; break; }
+            fr |= 1u << rel;
+        } else {
+            const double al = best < 0.0 ? 0.0 : best;
+#pragma unroll
+            for (int a = 0; a < K; ++a) {
+                if ((fr >> a) & 1u) d[a] = fma(al, y[a] - d[a], d[a]);
+                if (a == bi) d[a] = bup ? 1.0 - qa[a] : 0.0 - qa[a];
+            }
+            fr &= ~(1u << bi);
+            up = bup ? up | (1u << bi) : up & ~(1u << bi);
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < K; ++a) qdiff[pr * K + a] = d[a];
+    if (!done) atomicAdd(slots + S_QP_FAIL, 1.0);
+}
+
+// ------------------------------------------------------------------ P side
+// Variables (h, k), H = blockdiag(D_0 .. D_3) + rho on equal k.  In the dense
+// factorisation of the free block (order h, then k), the rows of all later
+// haplotypes are alike left of them: before column (h, .) every block
+// (h', h''), h'' >= h, h' > h'', is one and the same K x K matrix T (rho I at
+// first), and so are the rows V of L that haplotype h's columns leave in it.  So
+// the factor takes, per haplotype, its own K x K block, V once, and the update
+// by V V' of T and of the later diagonal blocks: about K^3 x 5 operations
+// instead of 11 K^3.
+// One problem per group of GL lanes; lane k holds row k of each block and the
+// four variables (h, k).
+template <int K> struct PDim {
+    static constexpr int GL = K <= 8 ? 8 : 16;
+    static constexpr int PW = 32 / GL;                      // problems per warp
+    static constexpr int WARPS = 2;
+    // per problem (doubles): D [4][K][K], L [4][K][K], V [3][K][K], iv [4][K], vec [4][K]
+    static constexpr int RAW = 11 * K * K + 8 * K;
+    static constexpr int LD = (RAW + 15) / 16 * 16 + 4;     // problems of a warp start 32 bytes apart modulo 128
+    static constexpr size_t SMEM = (size_t)WARPS * PW * LD * sizeof(double);
+};
+
+template <int K>
+__global__ void __launch_bounds__(32 * PDim<K>::WARPS)
+k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz, const double* __restrict__ p,
+        double rho, double* __restrict__ pdiff, double* slots, int8_t* __restrict__ ws) {
+    using P = PDim<K>;
+    constexpr int GL = P::GL, KK = K * K;
+    extern __shared__ double smem_p[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int k = lane % GL, g = lane / GL;
+    const int64_t j = ((int64_t)blockIdx.x * P::WARPS + warp) * P::PW + g;
+    const bool valid = j < n;
+    const bool row = k < K;
+    const int kc = row ? k : K - 1;                 // index for loads of idle lanes
+    double* D = smem_p + (warp * P::PW + g) * P::LD;   // H(k, b) of block h at h KK + b K + k
+    double* L = D + 4 * KK;                         // L[s, c] of block h at h KK + c K + s
+    double* V = L + 4 * KK;                         // V[k, c] of block h at h KK + c K + k
+    double* iv = V + 3 * KK;                        // reciprocal roots of the pivots (0: fixed)
+    double* vec = iv + 4 * K;
+    for (int t = k; t < 4 * KK; t += GL) D[t] = valid ? XtX[j * 4 * KK + t] : (t % KK / K == t % K ? 1.0 : 0.0);
+    double z[4], d[4], pa[4];
+    unsigned fr = 0u, up = 0u, no = 0u;             // bits h: free; at the upper bound; both bounds at 0
+    double zs = 1.0;
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const int64_t at = (j * 4 + h) * K + kc;
+        pa[h] = valid ? p[at] : 0.25;
+        z[h] = valid ? Xtz[at] : 0.0;
+        d[h] = 0.0;
+        if (row) {
+            zs = fmax(zs, fabs(z[h]));
+            // warm start from the previous solve's working set (bounds only: feasible)
+            int s0 = ws && valid ? (int)ws[at] : 0;
+            if (0.0 - pa[h] >= 0.0 && 1.0 - pa[h] <= 0.0) { no |= 1u << h; s0 = 1; }
+            if (s0 == 0) fr |= 1u << h;
+            if (s0 == 2) up |= 1u << h;
+            d[h] = s0 == 1 ? 0.0 - pa[h] : (s0 == 2 ? 1.0 - pa[h] : 0.0);
+        }
+    }
+#pragma unroll
+    for (int o = GL / 2; o > 0; o >>= 1) zs = fmax(zs, __shfl_xor_sync(FULL, zs, o));
+    const double tol = 1e-12 * zs;
+    const int max_iter = 16 * K + 20;
+    bool done = !valid;
+#pragma unroll 1
+    for (int it = 0; it < max_iter; ++it) {
+        if (__all_sync(FULL, done)) break;
+        __syncwarp();
+        // fixed variables to vec (free ones 0), largest free diagonal
+        double md = 0.0;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const bool f = (fr >> h) & 1u;
+            if (row) vec[h * K + k] = f ? 0.0 : d[h];
+            if (row && f) md = fmax(md, fabs(D[h * KK + kc * K + kc] + rho));
+        }
+#pragma unroll
+        for (int o = GL / 2; o > 0; o >>= 1) md = fmax(md, __shfl_xor_sync(FULL, md, o));
+        const double fl = 1e-300 + 1e-14 * md;
+        __syncwarp();
+        // right-hand sides z - H d over the fixed variables, in index order
+        double x[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            double s = z[h];
+            if (!__all_sync(FULL, !row || done || fr == 0xFu)) {
+#pragma unroll
+                for (int l = 0; l < 4; ++l) {
+                    if (l != h) {
+                        s = fma(-rho, (fr >> l) & 1u ? 0.0 : d[l], s);
+                    } else {
+#pragma unroll
+                        for (int b = 0; b < K; ++b) s = fma(-D[h * KK + b * K + kc], vec[h * K + b], s);
+                    }
+                }
+            }
+            x[h] = row && ((fr >> h) & 1u) ? s : 0.0;
+        }
+        // factorisation, forward sweep alongside
+        double T[K], G[3][K];                        // row k of T and of the diagonal blocks 1 .. 3
+#pragma unroll
+        for (int a = 0; a < K; ++a) {
+            T[a] = a == k ? rho : 0.0;
+#pragma unroll
+            for (int h = 1; h < 4; ++h)
+                G[h - 1][a] = D[h * KK + (a <= kc ? a * K + kc : kc * K + a)] + (a == k ? rho : 0.0);
+        }
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const bool f = row && ((fr >> h) & 1u);
+            const unsigned fm = __ballot_sync(FULL, f) >> (g * GL);      // free indices of this problem's h
+            double M[K], W[K];
+#pragma unroll
+            for (int a = 0; a < K; ++a) {
+                const double m = h == 0 ? D[a <= kc ? a * K + kc : kc * K + a] + (a == k ? rho : 0.0) : G[h > 0 ? h - 1 : 0][a];
+                M[a] = f && ((fm >> a) & 1u) ? m : 0.0;
+                W[a] = T[a];
+            }
+#pragma unroll
+            for (int c = 0; c < K; ++c) {
+                double pv = __shfl_sync(FULL, M[c], c, GL);
+                if (!(pv > fl)) pv = fl;
+                const double ivc = (fm >> c) & 1u ? inv_root(pv) : 0.0;
+                const double l = k > c ? M[c] * ivc : 0.0;
+                if (row) L[h * KK + c * K + k] = l;
+                if (k == c) iv[h * K + c] = ivc;
+                const double xa = __shfl_sync(FULL, x[h], c, GL) * ivc;
+                x[h] = k == c ? xa : fma(-l, xa, x[h]);
+                W[c] *= ivc;                          // V[k, c]
+                if (h < 3) {
+#pragma unroll
+                    for (int b = h + 1; b < 4; ++b) x[b] = fma(-W[c], xa, x[b]);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int s = c + 1; s < K; ++s) {
+                    const double ls = L[h * KK + c * K + s];
+                    M[s] = fma(-l, ls, M[s]);
+                    if (h < 3) W[s] = fma(-W[c], ls, W[s]);
+                }
+            }
+            if (h < 3) {
+                if (row) {
+#pragma unroll
+                    for (int c = 0; c < K; ++c) V[h * KK + c * K + k] = W[c];
+                }
+                __syncwarp();
+#pragma unroll
+                for (int c = 0; c < K; ++c) {
+#pragma unroll
+                    for (int a = 0; a < K; ++a) {
+                        const double va = V[h * KK + c * K + a];
+                        if (h < 2) T[a] = fma(-W[c], va, T[a]);
+#pragma unroll
+                        for (int b = h + 1; b < 4; ++b) G[b - 1][a] = fma(-W[c], va, G[b - 1][a]);
+                    }
+                }
+                // rows of fixed variables get sums too; the masks leave them unused
+#pragma unroll
+                for (int b = h + 1; b < 4; ++b)
+                    if (!((fr >> b) & 1u)) x[b] = 0.0;
+            }
+        }
+        // backward sweep
+#pragma unroll
+        for (int h = 3; h >= 0; --h)
+#pragma unroll
+            for (int c = K - 1; c >= 0; --c) {
+                const double xa = __shfl_sync(FULL, x[h], c, GL) * iv[h * K + c];
+                x[h] = k == c ? xa : (k < c ? fma(-L[h * KK + kc * K + c], xa, x[h]) : x[h]);
+#pragma unroll
+                for (int b = 0; b < h; ++b) x[b] = fma(-V[b * KK + kc * K + c], xa, x[b]);
+            }
+        // targets; ratio test: smallest step ratio < 1, lowest variable index (h, k) on ties
+        double best = 1.0;
+        int bidx = INT_MAX;
+        bool bup = false;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            if (!(row && ((fr >> h) & 1u))) { x[h] = d[h]; continue; }
+            const double s = x[h] - d[h];
+            const bool upw = s > 0.0;
+            const double num = upw ? (1.0 - pa[h]) - d[h] : (0.0 - pa[h]) - d[h];
+            if (s != 0.0 && (fabs(num) < fabs(s) || (upw ? num < 0.0 : num > 0.0))) {
+                const double ra = num / s;
+                if (ra < best) { best = ra; bidx = h * K + k; bup = upw; }
+            }
+        }
+        int bto = bup ? 1 : 0;
+#pragma unroll
+        for (int o = GL / 2; o > 0; o >>= 1) {
+            const double ob = __shfl_xor_sync(FULL, best, o);
+            const int oi = __shfl_xor_sync(FULL, bidx, o), ot = __shfl_xor_sync(FULL, bto, o);
+            if (ob < best || (ob == best && oi < bidx)) { best = ob; bidx = oi; bto = ot; }
+        }
+        const bool blocked = bidx != INT_MAX;
+        if (!done && blocked) {
+            const double al = best < 0.0 ? 0.0 : best;
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                if ((fr >> h) & 1u) d[h] = fma(al, x[h] - d[h], d[h]);
+                if (row && bidx == h * K + k) {
+                    d[h] = bto ? 1.0 - pa[h] : 0.0 - pa[h];
+                    fr &= ~(1u << h);
+                    up = bto ? up | (1u << h) : up & ~(1u << h);
+                }
+            }
+        }
+        // no bound met: take the point, release the largest multiplier
+        if (!done && !blocked) {
+#pragma unroll
+            for (int h = 0; h < 4; ++h) d[h] = x[h];
+        }
+        if (__all_sync(FULL, done || blocked)) continue;
+        __syncwarp();
+        if (row) {
+#pragma unroll
+            for (int h = 0; h < 4; ++h) vec[h * K + k] = d[h];
+        }
+        __syncwarp();
+        double wv = tol;
+        int rel = INT_MAX;
+        if (row && !done && !blocked) {
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                if (((fr | no) >> h) & 1u) continue;
+                double gr = -z[h];
+#pragma unroll
+                for (int l = 0; l < 4; ++l) {
+                    if (l != h) {
+                        gr = fma(rho, d[l], gr);
+                    } else {
+#pragma unroll
+                        for (int b = 0; b < K; ++b)
+                            gr = fma(D[h * KK + b * K + kc] + (b == k ? rho : 0.0), vec[h * K + b], gr);
+                    }
+                }
+                const double v = (up >> h) & 1u ? gr : -gr;
+                if (v > wv) { wv = v; rel = h * K + k; }
+            }
+        }
+#pragma unroll
+        for (int o = GL / 2; o > 0; o >>= 1) {
+            const double ov = __shfl_xor_sync(FULL, wv, o);
+            const int oi = __shfl_xor_sync(FULL, rel, o);
+            if (ov > wv || (ov == wv && oi < rel)) { wv = ov; rel = oi; }
+        }
+        if (!done && !blocked) {
+            if (rel == INT_MAX) done = true;
+            else if (rel % K == k && row) fr |= 1u << (rel / K);
+        }
+    }
+    if (!valid) return;
+    if (row) {
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const int64_t at = (j * 4 + h) * K + k;
+            pdiff[at] = d[h];
+            if (ws) ws[at] = (fr >> h) & 1u ? 0 : ((up >> h) & 1u ? 2 : 1);
+        }
+    }
+    if (!done && k == 0) atomicAdd(slots + S_QP_FAIL, 1.0);
+}
+
+#define HX_FOR_K(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12)
+}  // namespace
+
+cudaError_t launch_qp_q(int K, int64_t n, const double* XtX, const double* Xtz, const double* q, double* qdiff,
+                        double* slots, cudaStream_t st, double pen_rho) {
+    const unsigned g = (unsigned)((n + QQ_THREADS - 1) / QQ_THREADS);
+#define HX_CASE(KK) case KK: k_qp_q<KK><<<g, QQ_THREADS, 0, st>>>(n, XtX, Xtz, q, qdiff, slots, pen_rho); break;
+    switch (K) { HX_FOR_K(HX_CASE) default: return cudaErrorInvalidValue; }
+#undef HX_CASE
+    return cudaGetLastError();
+}
+
+cudaError_t init_qp_attrs(int K) {
+#define HX_CASE(KK)                                                                                     \
+    case KK:                                                                                            \
+        return cudaFuncSetAttribute(k_qp_p4<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PDim<KK>::SMEM);
+    switch (K) { HX_FOR_K(HX_CASE) default: return cudaErrorInvalidValue; }
+#undef HX_CASE
+}
+
+cudaError_t launch_qp_p_pen(int K, int64_t n, const double* XtX, const double* Xtz, const double* p, double rho,
+                            double* pdiff, double* slots, int8_t* ws, cudaStream_t st) {
+#define HX_CASE(KK)                                                                                              \
+    case KK: {                                                                                                   \
+        constexpr int per = PDim<KK>::WARPS * PDim<KK>::PW;                                                      \
+        k_qp_p4<KK><<<(unsigned)((n + per - 1) / per), 32 * PDim<KK>::WARPS, PDim<KK>::SMEM, st>>>(              \
+            n, XtX, Xtz, p, rho, pdiff, slots, ws);                                                              \
+        break;                                                                                                   \
+    }
+    switch (K) { HX_FOR_K(HX_CASE) default: return cudaErrorInvalidValue; }
+#undef HX_CASE
+    return cudaGetLastError();
+}
+
+}  // namespace hx
