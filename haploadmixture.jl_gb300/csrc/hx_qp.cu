@@ -12,8 +12,13 @@
 // the dense factorisation and sweeps of the free block in index order, and leave
 // out only those whose operands are exact zeros, so the results do not depend
 // on this arrangement (the mixed method rounds them to FP32 afterwards, which
-// would turn a last-bit difference into one of 6e-8).
+// would turn a last-bit difference into one of 6e-8).  A free block that is not
+// positive definite to rounding (a mixed-precision Hessian whose entries span
+// more than its 16 bits) has a pivot at its floor, and what follows grows without
+// bound: such a problem is handed to the dense solver, where it is solved from
+// the start.
 #include "hx_ops.cuh"
+#include "hx_qp_dense.cuh"
 #include "hx_tc.cuh"
 #include <climits>
 
@@ -32,6 +37,30 @@ __device__ __forceinline__ double inv_root(double s) { return 1.0 / sqrt(s); }
 // data-dependent indices.
 constexpr int QQ_THREADS = 64, QQ_LD = QQ_THREADS + 1;
 
+// One problem on the dense solver, by a whole warp; base: K^2 + 11 K doubles of
+// shared memory.
+__device__ __noinline__ void qp_q_dense(int K, int64_t pr, const double* XtX, const double* Xtz, const double* q,
+                                        double* qdiff, double* slots, double pen_rho, double* base) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    QPWork w = carve(base, K);
+    for (int a = lane; a < K; a += 32) {
+        const double qa = q[(int64_t)K * pr + a];
+        w.d[a] = 0.0;
+        w.z[a] = Xtz[(int64_t)K * pr + a];
+        w.lo[a] = 0.0 - qa;
+        w.hi[a] = 1.0 - qa;
+        w.st[a] = (w.lo[a] >= 0.0 && w.hi[a] <= 0.0) ? QL : QF;
+    }
+    __syncwarp();
+    HQ H{XtX + (int64_t)K * K * pr, K, pen_rho >= 0.0 ? pen_rho : 0.0};
+    const int it = warp_qp<false>(K, pen_rho < 0.0 ? 1 : 0, H, w);
+    __syncwarp();
+    for (int a = lane; a < K; a += 32) qdiff[(int64_t)K * pr + a] = w.d[a];
+    if (it < 0 && lane == 0) atomicAdd(slots + S_QP_FAIL, 1.0);
+    __syncwarp();
+}
+
 // Sum of the elements of x (K <= 12) in the order of a butterfly over 16 lanes.
 template <int K> __device__ __forceinline__ double tree_sum(const double (&x)[K]) {
     double t8[8], t4[4];
@@ -48,7 +77,7 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
        double* __restrict__ qdiff, double* slots, double pen_rho) {
     constexpr int NT = K * (K + 1) / 2;
     __shared__ double sH[NT * QQ_LD];
-    __shared__ double sX[K * QQ_THREADS];
+    __shared__ double sX[K * QQ_THREADS];        // per warp: ranks, then the dense solver's work
     const int tid = threadIdx.x;
     const int64_t p0 = (int64_t)blockIdx.x * QQ_THREADS, pr = p0 + tid;
     const int np = (int)min((int64_t)QQ_THREADS, n - p0);
@@ -58,9 +87,9 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
         if (r >= c) sH[tri_idx<K>(c, r) * QQ_LD + x] = XtX[p0 * K * K + t] + (eq ? 0.0 : pen_rho);
     }
     __syncthreads();
-    if (tid >= np) return;
-    const double* H = sH + tid;
-    double* xs = sX + tid;
+    const bool mine = tid < np;
+    const double* H = sH + (mine ? tid : 0);
+    double* xs = sX + (tid >> 5) * 32 * K + (tid & 31);
     auto h = [&](int a, int b) { return H[(a <= b ? tri_idx<K>(a, b) : tri_idx<K>(b, a)) * QQ_LD]; };
     // Sum over the free variables as the list of them is summed: element of rank
     // r in place r of the butterfly.
@@ -68,12 +97,12 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
         double y[K];
         if (fr == (1u << K) - 1u) return tree_sum<K>(x);
 #pragma unroll
-        for (int a = 0; a < K; ++a) xs[a * QQ_THREADS] = 0.0;
+        for (int a = 0; a < K; ++a) xs[a * 32] = 0.0;
 #pragma unroll
         for (int a = 0; a < K; ++a)
-            if ((fr >> a) & 1u) xs[__popc(fr & ((1u << a) - 1u)) * QQ_THREADS] = x[a];
+            if ((fr >> a) & 1u) xs[__popc(fr & ((1u << a) - 1u)) * 32] = x[a];
 #pragma unroll
-        for (int a = 0; a < K; ++a) y[a] = xs[a * QQ_THREADS];
+        for (int a = 0; a < K; ++a) y[a] = xs[a * 32];
         return tree_sum<K>(y);
     };
     double z[K], d[K], qa[K];
@@ -81,8 +110,8 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
     double tol = 1.0;
 #pragma unroll
     for (int a = 0; a < K; ++a) {
-        qa[a] = q[pr * K + a];
-        z[a] = Xtz[pr * K + a];
+        qa[a] = mine ? q[pr * K + a] : 0.0;
+        z[a] = mine ? Xtz[pr * K + a] : 0.0;
         tol = fmax(tol, fabs(z[a]));
         d[a] = 0.0;
         if (0.0 - qa[a] >= 0.0 && 1.0 - qa[a] <= 0.0) no |= 1u << a;
@@ -90,9 +119,9 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
     }
     tol *= 1e-12;
     const int max_iter = 4 * K + 20;
-    bool done = false;
+    bool done = !mine, floored = false;
 #pragma unroll 1
-    for (int it = 0; it < max_iter; ++it) {
+    for (int it = 0; it < max_iter && !done; ++it) {
         double A[NT], y[K], o[K];
         double md = 0.0;
 #pragma unroll
@@ -116,9 +145,10 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
         double iv[K];
 #pragma unroll
         for (int a = 0; a < K; ++a) {
-            double pv = A[tri_idx<K>(a, a)];
-            if (!(pv > fl)) pv = fl;
-            iv[a] = (fr >> a) & 1u ? inv_root(pv) : 0.0;
+            const double pv = A[tri_idx<K>(a, a)];
+            const bool fa = (fr >> a) & 1u;
+            if (fa && !(pv > fl)) floored = true;
+            iv[a] = fa ? inv_root(pv) : 0.0;
             y[a] *= iv[a];
             o[a] *= iv[a];
 #pragma unroll
@@ -143,6 +173,7 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
                 o[b] = fma(-A[tri_idx<K>(b, a)], o[a], o[b]);
             }
         }
+        if (floored) break;
         double nu = 0.0;
         if (eq && fr) {
             double f[K];
@@ -197,9 +228,17 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
             up = bup ? up | (1u << bi) : up & ~(1u << bi);
         }
     }
+    if (mine && !floored) {
 #pragma unroll
-    for (int a = 0; a < K; ++a) qdiff[pr * K + a] = d[a];
-    if (!done) atomicAdd(slots + S_QP_FAIL, 1.0);
+        for (int a = 0; a < K; ++a) qdiff[pr * K + a] = d[a];
+        if (!done) atomicAdd(slots + S_QP_FAIL, 1.0);
+    }
+    unsigned left = __ballot_sync(FULL, floored);
+    while (left) {
+        const int b = __ffs(left) - 1;
+        left &= left - 1;
+        qp_q_dense(K, pr - (tid & 31) + b, XtX, Xtz, q, qdiff, slots, pen_rho, sX + (tid >> 5) * 32 * K);
+    }
 }
 
 // ------------------------------------------------------------------ P side
@@ -222,6 +261,35 @@ template <int K> struct PDim {
     static constexpr int LD = (RAW + 15) / 16 * 16 + 4;     // problems of a warp start 32 bytes apart modulo 128
     static constexpr size_t SMEM = (size_t)WARPS * PW * LD * sizeof(double);
 };
+
+// One block on the dense solver, by a whole warp; base: 16 K^2 + 44 K doubles.
+__device__ __noinline__ void qp_p_dense(int K, int64_t j, const double* XtX, const double* Xtz, const double* p,
+                                        double rho, double* pdiff, double* slots, int8_t* ws, double* base) {
+    const int lane = threadIdx.x & 31, nv = 4 * K;
+    __syncwarp();
+    QPWork w = carve(base, nv);
+    for (int a = lane; a < nv; a += 32) {
+        const double pa = p[(int64_t)nv * j + a];
+        w.d[a] = 0.0;
+        w.z[a] = Xtz[(int64_t)nv * j + a];
+        w.lo[a] = 0.0 - pa;
+        w.hi[a] = 1.0 - pa;
+        int s0 = ws ? (int)ws[(int64_t)nv * j + a] : QF;
+        if (w.lo[a] >= 0.0 && w.hi[a] <= 0.0) s0 = QL;
+        w.st[a] = s0;
+        w.d[a] = s0 == QL ? w.lo[a] : (s0 == QH ? w.hi[a] : 0.0);
+    }
+    __syncwarp();
+    HP H{XtX + (int64_t)K * K * 4 * j, K, rho};
+    const int it = warp_qp<false>(nv, 0, H, w);
+    __syncwarp();
+    for (int a = lane; a < nv; a += 32) {
+        pdiff[(int64_t)nv * j + a] = w.d[a];
+        if (ws) ws[(int64_t)nv * j + a] = (int8_t)w.st[a];
+    }
+    if (it < 0 && lane == 0) atomicAdd(slots + S_QP_FAIL, 1.0);
+    __syncwarp();
+}
 
 template <int K>
 __global__ void __launch_bounds__(32 * PDim<K>::WARPS)
@@ -265,7 +333,7 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
     for (int o = GL / 2; o > 0; o >>= 1) zs = fmax(zs, __shfl_xor_sync(FULL, zs, o));
     const double tol = 1e-12 * zs;
     const int max_iter = 16 * K + 20;
-    bool done = !valid;
+    bool done = !valid, floored = false;            // floored: left to the dense solver
 #pragma unroll 1
     for (int it = 0; it < max_iter; ++it) {
         if (__all_sync(FULL, done)) break;
@@ -322,8 +390,8 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
             }
 #pragma unroll
             for (int c = 0; c < K; ++c) {
-                double pv = __shfl_sync(FULL, M[c], c, GL);
-                if (!(pv > fl)) pv = fl;
+                const double pv = __shfl_sync(FULL, M[c], c, GL);
+                if (((fm >> c) & 1u) && !done && !(pv > fl)) floored = true;
                 const double ivc = (fm >> c) & 1u ? inv_root(pv) : 0.0;
                 const double l = k > c ? M[c] * ivc : 0.0;
                 if (row) L[h * KK + c * K + k] = l;
@@ -365,6 +433,7 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
                     if (!((fr >> b) & 1u)) x[b] = 0.0;
             }
         }
+        done |= floored;
         // backward sweep
 #pragma unroll
         for (int h = 3; h >= 0; --h)
@@ -454,8 +523,7 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
             else if (rel % K == k && row) fr |= 1u << (rel / K);
         }
     }
-    if (!valid) return;
-    if (row) {
+    if (valid && row && !floored) {
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
             const int64_t at = (j * 4 + h) * K + k;
@@ -463,7 +531,13 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
             if (ws) ws[at] = (fr >> h) & 1u ? 0 : ((up >> h) & 1u ? 2 : 1);
         }
     }
-    if (!done && k == 0) atomicAdd(slots + S_QP_FAIL, 1.0);
+    if (valid && !done && k == 0) atomicAdd(slots + S_QP_FAIL, 1.0);
+    unsigned left = __ballot_sync(FULL, floored && k == 0);
+    while (left) {
+        const int b = __ffs(left) - 1;
+        left &= left - 1;
+        qp_p_dense(K, __shfl_sync(FULL, j, b), XtX, Xtz, p, rho, pdiff, slots, ws, smem_p + warp * P::PW * P::LD);
+    }
 }
 
 #define HX_FOR_K(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12)
