@@ -156,38 +156,6 @@ __device__ __forceinline__ void pair_eval_tab(unsigned nib, const float qp[4], f
     u[3] = fmaf(hr, qp[0], fmaf(x11, tb.y, x21 * tb.w));
 }
 
-// scale * u of pair_eval_tab (scale a power of two, e.g. 1/4), without the
-// likelihood: the scale is folded into the two reciprocals, and since every
-// later operation is a product or a sum of scaled terms the result has the
-// same bits as u * scale, two multiplications cheaper than scaling u.
-__device__ __forceinline__ void pair_u_tab(unsigned nib, const float qp[4], float u[4], const float4* tab,
-                                           float scale) {
-    const float4 ta = tab[nib & 3u], tb = tab[(nib >> 2) & 3u];
-    const float v10 = fmaf(tb.y, qp[1], tb.x * qp[0]), v11 = fmaf(tb.y, qp[3], tb.x * qp[2]);
-    const float v20 = fmaf(tb.w, qp[1], tb.z * qp[0]), v21 = fmaf(tb.w, qp[3], tb.z * qp[2]);
-    float F1 = fmaf(ta.y, v11, ta.x * v10);
-    float F2 = fmaf(ta.w, v21, ta.z * v20);
-    const bool hh = nib == NIB_HH;
-    const bool mm = nib == NIB_MM;
-    const float den = fmaf(qp[1], qp[2], qp[0] * qp[3]);
-    F1 = hh ? den : F1;
-    F1 = mm ? 1.f : F1;
-    F2 = (hh || mm) ? 1.f : F2;
-    float r1, r2;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(F1));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r2) : "f"(F2));
-    r1 *= scale;
-    r2 *= scale;
-    const float hr = hh ? r1 : 0.f;
-    r1 = (hh || mm) ? 0.f : r1;
-    r2 = (hh || mm) ? 0.f : r2;
-    const float x10 = ta.x * r1, x11 = ta.y * r1, x20 = ta.z * r2, x21 = ta.w * r2;
-    u[0] = fmaf(hr, qp[3], fmaf(x10, tb.x, x20 * tb.z));
-    u[1] = fmaf(hr, qp[2], fmaf(x10, tb.y, x20 * tb.w));
-    u[2] = fmaf(hr, qp[1], fmaf(x11, tb.x, x21 * tb.z));
-    u[3] = fmaf(hr, qp[0], fmaf(x11, tb.y, x21 * tb.w));
-}
-
 // Likelihood only (log-likelihood passes).
 __device__ __forceinline__ float pair_lik_tab(unsigned nib, const float qp[4], const float4* tab) {
     const float4 ta = tab[nib & 3u], tb = tab[(nib >> 2) & 3u];
@@ -221,8 +189,66 @@ __device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t f2_sub(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 __device__ __forceinline__ void f2_split(uint64_t v, float& lo, float& hi) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
+// Class rows: for each class the 0/1 membership of the four haplotypes in the
+// first copy's set (class_m1) and, CLS_COPY2 bytes on, in the second copy's
+// (class_m2), as FP32.  A kernel keeps them in shared memory (cls_table_init by
+// its first 128 threads, then a barrier) and addresses a row by 16 * class.
+constexpr int CLS_COPY2 = 256;
+__device__ __forceinline__ void cls_table_init(float* tab, int tid) {
+    if (tid < 128) {
+        const unsigned nib = (tid & 63) >> 2;
+        const unsigned m = (unsigned)((tid < 64 ? TAB_M1 : TAB_M2) >> (4 * nib)) & 0xFu;
+        tab[tid] = (m >> (tid & 3)) & 1u ? 1.f : 0.f;
+    }
+}
+
+// scale * u (scale a power of two) of the class at byte offset off = 16 * class,
+// from packed (qp0, qp1), (qp2, qp3), in packed FP32x2 arithmetic: the same
+// results as pair_eval_tab's u * scale, bit for bit (a copy's set has at most
+// two members, so each factor rounds once in either order of the sum; scaling
+// by a power of two is exact).  The double heterozygote takes its operands
+// (qp3, qp2, qp1, qp0) / den through the first copy's row.
+__device__ __forceinline__ void pair_u_cls(unsigned off, uint64_t z01, uint64_t z23, uint64_t& u01, uint64_t& u23,
+                                           const float* tab, float scale) {
+    const char* row = reinterpret_cast<const char*>(tab) + off;
+    const ulonglong2 c1 = *reinterpret_cast<const ulonglong2*>(row);
+    const ulonglong2 c2 = *reinterpret_cast<const ulonglong2*>(row + CLS_COPY2);
+    float q0, q1, q2, q3, a, b;
+    f2_split(z01, q0, q1);
+    f2_split(z23, q2, q3);
+    f2_split(f2_fma(c1.y, z23, f2_mul(c1.x, z01)), a, b);
+    float F1 = a + b;
+    f2_split(f2_fma(c2.y, z23, f2_mul(c2.x, z01)), a, b);
+    float F2 = a + b;
+    const bool hh = off == 16u * NIB_HH, mm = off == 16u * NIB_MM;
+    const float den = fmaf(q1, q2, q0 * q3);
+    F1 = hh ? den : F1;
+    F1 = mm ? 1.f : F1;
+    F2 = hh || mm ? 1.f : F2;
+    float r1, r2;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(F1));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r2) : "f"(F2));
+    const uint64_t r1d = f2_dup(r1 * scale), r2d = f2_dup(r2 * scale);
+    float x0, x1, x2, x3;
+    f2_split(c1.x, x0, x1);
+    f2_split(c1.y, x2, x3);
+    const uint64_t s01 = f2_pack(hh ? q3 : x0, hh ? q2 : x1), s23 = f2_pack(hh ? q1 : x2, hh ? q0 : x3);
+    u01 = f2_fma(s01, r1d, f2_mul(c2.x, r2d));
+    u23 = f2_fma(s23, r1d, f2_mul(c2.y, r2d));
 }
 
 // Exact exponent/mantissa split used to accumulate products of likelihoods

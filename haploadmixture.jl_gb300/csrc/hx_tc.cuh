@@ -9,6 +9,7 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+#include "hx_common.cuh"
 
 namespace hx {
 namespace tc {
@@ -139,6 +140,26 @@ __device__ __forceinline__ void split2_f16(float x0, float x1, uint32_t& hi2, ui
     asm("{ .reg .b16 a, b; mov.b32 {a, b}, %2; cvt.f32.f16 %0, a; cvt.f32.f16 %1, b; }"
         : "=f"(h0), "=f"(h1) : "r"(hi2));
     asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(lo2) : "f"(x1 - h1), "f"(x0 - h0));
+}
+
+// The two splits of a packed pair.
+__device__ __forceinline__ void split2(uint64_t x, uint32_t& hi2, uint32_t& lo2) {
+    float x0, x1;
+    f2_split(x, x0, x1);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi2) : "f"(x1), "f"(x0));
+    float d0, d1;
+    f2_split(f2_sub(x, f2_pack(__uint_as_float(hi2 << 16), __uint_as_float(hi2 & 0xFFFF0000u))), d0, d1);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo2) : "f"(d1), "f"(d0));
+}
+__device__ __forceinline__ void split2_f16(uint64_t x, uint32_t& hi2, uint32_t& lo2) {
+    float x0, x1, h0, h1;
+    f2_split(x, x0, x1);
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(hi2) : "f"(x1), "f"(x0));
+    asm("{ .reg .b16 a, b; mov.b32 {a, b}, %2; cvt.f32.f16 %0, a; cvt.f32.f16 %1, b; }"
+        : "=f"(h0), "=f"(h1) : "r"(hi2));
+    float d0, d1;
+    f2_split(f2_sub(x, f2_pack(h0, h1)), d0, d1);
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(lo2) : "f"(d1), "f"(d0));
 }
 
 __device__ __forceinline__ void sts128(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {

@@ -576,13 +576,19 @@ __device__ __forceinline__ void final_fold(Sync* sy, double* slots, long long bu
 // CTA's q tile by the stage's p tile into a double-buffered 32-column TMEM
 // tile, issued two stages ahead; each thread reads its row's 16 values.
 
-// One pair from its qp: U and W, both times U_SCALE.
+// One pair from its packed qp (byte offset off = 16 * class): U and W as packed
+// pairs of haplotypes, both times U_SCALE.
 template <bool HESS>
-__device__ __forceinline__ void gen_pair_qp(unsigned nib, const float* qp, float* U4, float* W4, const float4* tab) {
-    pair_u_tab(nib, qp, U4, tab, U_SCALE);          // U * U_SCALE
-#pragma unroll
-    for (int h = 0; h < 4; ++h)
-        if (HESS) W4[h] = U4[h] * rcp_approx(qp[h]);   // W * U_SCALE
+__device__ __forceinline__ void gen_pair_qp(unsigned off, uint64_t z01, uint64_t z23, uint64_t* U, uint64_t* W,
+                                            const float* tab) {
+    pair_u_cls(off, z01, z23, U[0], U[1], tab, U_SCALE);
+    if (HESS) {
+        float q0, q1, q2, q3;
+        f2_split(z01, q0, q1);
+        f2_split(z23, q2, q3);
+        W[0] = f2_mul(U[0], f2_pack(rcp_approx(q0), rcp_approx(q1)));
+        W[1] = f2_mul(U[1], f2_pack(rcp_approx(q2), rcp_approx(q3)));
+    }
 }
 
 template <int K, bool HESS>
@@ -600,7 +606,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pass
     const uint32_t sRq = sR + RING * GBM;                            // ring [QRING][GBQ]
     uint32_t* SW = (uint32_t*)(smem + (sRq - sA) + QRING * GBQ);     // [RING][128]
     Sync* sy = (Sync*)(SW + RING * 128);
-    __shared__ float4 s_snp[4];
+    __shared__ __align__(16) float s_cls[128];
     const long long budget = a.budget;
 
     const int tid = threadIdx.x, warp = tid >> 5;
@@ -610,7 +616,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pass
     const int w0 = blockIdx.y * a.per_chunk;
     const int ns = min(a.JW, w0 + a.per_chunk) - w0;     // one word per stage
     const int64_t i0 = (int64_t)blockIdx.x * 128;
-    snp_table_init(s_snp, tid);
+    cls_table_init(s_cls, tid);
 
     // stage t's inputs: the word column's B tile and the CTA's 128 class words;
     // separately, 4 stages ahead, the tf32 p tile of its qp MMA
@@ -711,7 +717,9 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pass
             uint32_t raw[16];
             tmem_ld8_async(taddr_lane + (uint32_t)(2 * D::WQ + b * 32 + hf * 16), raw);
             tmem_ld8_async(taddr_lane + (uint32_t)(2 * D::WQ + b * 32 + hf * 16 + 8), raw + 8);
+            // the half's four classes from bit 4 on: class bb times 16 is (word >> 4 bb) & 0xF0
             word = SW[slot * 128 + r];
+            word = __funnelshift_r(word, word, (16 * hf + 28) & 31);
             tmem_wait_ld();
 #pragma unroll
             for (int t = 0; t < 16; ++t) qpv[t] = __uint_as_float(raw[t]);
@@ -719,18 +727,19 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pass
         const uint32_t aB = sA + b * 4 * A_TILE_STD;
 #pragma unroll
         for (int t2 = 0; t2 < 2; ++t2) {
-            float W[8], U[8];
+            uint64_t W[4], U[4];                              // haplotype pairs
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int bb = 2 * t2 + e;                    // block within this thread's half
-                gen_pair_qp<HESS>((word >> (4 * (hf * 4 + bb))) & 0xFu, qpv + 4 * bb, U + 4 * e, W + 4 * e, s_snp);
+                gen_pair_qp<HESS>((word >> (4 * bb)) & 0xF0u, f2_pack(qpv[4 * bb], qpv[4 * bb + 1]),
+                                  f2_pack(qpv[4 * bb + 2], qpv[4 * bb + 3]), U + 2 * e, W + 2 * e, s_cls);
             }
             const uint32_t off = (r >> 3) * SBO_STD + (hf * 2 + t2) * LBO_STD + (r & 7) * 16;
             uint32_t wh[4], wl[4], uh[4], ul[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                if (HESS) split2(W[2 * e], W[2 * e + 1], wh[e], wl[e]);
-                split2_f16(U[2 * e], U[2 * e + 1], uh[e], ul[e]);
+                if (HESS) split2(W[e], wh[e], wl[e]);
+                split2_f16(U[e], uh[e], ul[e]);
             }
             if (HESS) {
                 sts128(aB + off, wh[0], wh[1], wh[2], wh[3]);
@@ -798,21 +807,22 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pass
 // pr2[2k+1] = (p[k,4j+2], p[k,4j+3]): the packed FMAs form qp_h for h pairs
 // in the order of the fmaf chain sum_k q_k p[k,m].
 template <int K, bool HESS>
-__device__ __forceinline__ void gen_pair(unsigned nib, const uint64_t* qd, const uint64_t* pr2, float* U4, float* W4,
-                                         const float4* tab) {
+__device__ __forceinline__ void gen_pair(unsigned off, const uint64_t* qd, const uint64_t* pr2, float* U4, float* W4,
+                                         const float* tab) {
     uint64_t z01 = 0ull, z23 = 0ull;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         z01 = f2_fma(qd[k], pr2[2 * k], z01);
         z23 = f2_fma(qd[k], pr2[2 * k + 1], z23);
     }
-    float qp[4];
-    f2_split(z01, qp[0], qp[1]);
-    f2_split(z23, qp[2], qp[3]);
-    pair_u_tab(nib, qp, U4, tab, U_SCALE);          // U * U_SCALE
-#pragma unroll
-    for (int h = 0; h < 4; ++h)
-        if (HESS) W4[h] = U4[h] * rcp_approx(qp[h]);   // W * U_SCALE
+    uint64_t U[2], W[2];
+    gen_pair_qp<HESS>(off, z01, z23, U, W, tab);
+    f2_split(U[0], U4[0], U4[1]);
+    f2_split(U[1], U4[2], U4[3]);
+    if (HESS) {
+        f2_split(W[0], W4[0], W4[1]);
+        f2_split(W[1], W4[2], W4[3]);
+    }
 }
 
 template <int K, bool HESS>
@@ -829,7 +839,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pass
     const uint32_t sR = sA + 2 * 4 * A_TILE_PAD;                     // ring [RING][GB]
     uint32_t* SW = (uint32_t*)(smem + (sR - sA) + RING * GB);        // [RING][4][KD]
     Sync* sy = (Sync*)(SW + RING * 4 * KD);
-    __shared__ float4 s_snp[4];
+    __shared__ __align__(16) float s_cls[128];
     const long long budget = a.budget;
 
     const int tid = threadIdx.x, warp = tid >> 5;
@@ -843,7 +853,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pass
     const int64_t g0 = i0 / KD;
     const int64_t jw0 = (int64_t)blockIdx.x * 4;
     const int nwc = (int)min((int64_t)4, (int64_t)a.JW - jw0);     // word columns inside the matrix
-    snp_table_init(s_snp, tid);
+    cls_table_init(s_cls, tid);
 
     // stage t's inputs: the 32 individuals' image and their class words of the
     // CTA's word columns (columns past JW are never read: their blocks are
@@ -887,7 +897,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pass
     for (int c = 0; c < D::HALF; ++c) acc[c] = 0.f;
 #pragma unroll
     for (int c = 0; c < D::NG; ++c) comp[c] = 0.f;
-    const int bsh = 4 * (jl & 7);
+    const int bsh = (4 * (jl & 7) + 28) & 31;     // rotates the block's class to bits 4 .. 7
 
     for (int s = 0; s < ns; ++s) {
         const int b = s & 1, slot = s % RING;
@@ -904,7 +914,8 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pass
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int ii = ig * 4 + e;
-            const unsigned nib = valid ? (Ws[ii] >> bsh) & 0xFu : HX_PAD_NIBBLE;
+            // 16 * class
+            const unsigned off = valid ? __funnelshift_r(Ws[ii], Ws[ii], bsh) & 0xF0u : 16u * HX_PAD_NIBBLE;
             uint64_t qd[(K + 1) / 2 * 2];
             const ulonglong2* q2 = reinterpret_cast<const ulonglong2*>(Qs + qrow_slot(ii) * QSTR);
 #pragma unroll
@@ -914,7 +925,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pass
                 qd[2 * c + 1] = x.y;
             }
             float u4[4], w4[4];
-            gen_pair<K, HESS>(nib, qd, pr2, u4, w4, s_snp);
+            gen_pair<K, HESS>(off, qd, pr2, u4, w4, s_cls);
 #pragma unroll
             for (int h = 0; h < 4; ++h) { U[h][e] = u4[h]; if (HESS) W[h][e] = w4[h]; }
         }
