@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
     FSync* sy = reinterpret_cast<FSync*>(lists + F_GEN_WARPS * 256);
     const uint32_t sA = smem_u32(smem), sR = smem_u32(ring);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int grp = blockIdx.z;
     const int64_t row0 = (int64_t)blockIdx.x * 128;
     // stages of this CTA
@@ -426,58 +426,58 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
     fence_before();
     const bool allh = __syncthreads_or(odd_p) && HESS;
     fence_after();
-    const uint32_t tmem = sy->tslot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, sy->tslot, 0);
 
     if (warp == F_GEN_WARPS) {
-        if (lane == 0) {
-            auto load = [&](int s) {
-                const int slot = s % F_RING;
-                const uint8_t* src = a.img + (s0 + s) * D::IMG;
-                const uint32_t dst = sR + slot * D::SLOT;
-                uint64_t* bar = &sy->full[slot];
-                const uint32_t wb = PS ? 128u * nwc : 512u;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                             :: "r"(smem_u32(bar)), "r"((uint32_t)(D::B_TILE + D::ROWS) + wb) : "memory");
-                auto copy = [&](uint32_t d, const void* g, uint32_t bytes) {
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                                 :: "r"(d), "l"(g), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-                };
-                copy(dst, src + grp * D::B_TILE, D::B_TILE);
-                copy(dst + D::B_TILE, src + D::NG * D::B_TILE, D::ROWS);
-                if (PS) {
-                    for (int w = 0; w < nwc; ++w)
-                        copy(dst + D::B_TILE + D::ROWS + 128 * w,
-                             a.G + ((int64_t)blockIdx.x * 4 + w) * a.Ipad + (s0 + s) * F_KD, 128);
-                } else {
-                    copy(dst + D::B_TILE + D::ROWS, a.G + (s0 + s) * a.Ipad + row0, 512);
-                }
-                *(volatile int*)&sy->loaded = s + 1;
+        const uint32_t el = elect_lane();
+        auto load = [&](int s) {
+            const int slot = s % F_RING;
+            const uint8_t* src = a.img + (s0 + s) * D::IMG;
+            const uint32_t dst = sR + slot * D::SLOT;
+            uint64_t* bar = &sy->full[slot];
+            const uint32_t wb = PS ? 128u * nwc : 512u;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                         :: "r"(smem_u32(bar)), "r"((uint32_t)(D::B_TILE + D::ROWS) + wb) : "memory");
+            auto copy = [&](uint32_t d, const void* g, uint32_t bytes) {
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                             :: "r"(d), "l"(g), "r"(bytes), "r"(smem_u32(bar)) : "memory");
             };
-            for (int s = 0; s < F_RING && s < ns; ++s) load(s);
-            for (int s = 0; s < ns; ++s) {
-                // all digits of the stage written, and every warp past stage s-1
-                if (!f_wait(sy, &sy->gen, s, a.slots)) break;
-                fence_after();
-                const uint64_t dA = sdesc(sA, LBO, SBO), dB = sdesc(sR + (s % F_RING) * D::SLOT, F_LBO_B, F_SBO_B);
-                // one MMA per digit pair: all of one shape, so that those of one
-                // order (one accumulator) execute in issue order
-#pragma unroll 1
-                for (int d = 0; d < F_NDA; ++d)
-#pragma unroll
-                    for (int b = 0; b < F_NDB; ++b) {
-                        if (d + b >= F_NORD) break;
-#pragma unroll
-                        for (int ks = 0; ks < F_KD / 16; ++ks)
-                            mma_bf16(tmem + (d + b) * D::NHP, dA + (uint64_t)((d * AT + ks * 2 * LBO) >> 4),
-                                     dB + (uint64_t)((b * (D::NHP / 8) * F_SBO_B + ks * 2 * F_LBO_B) >> 4),
-                                     idesc_f16(D::NHP), 1u);
-                    }
-                commit(&sy->mma);
-                *(volatile int*)&sy->issued = s + 1;
-                // the slot of stage s-1: its MMAs are done (every warp waited for
-                // them before it arrived for stage s) and its vectors are read
-                if (s >= 1 && s + 2 < ns) load(s + 2);
+            copy(dst, src + grp * D::B_TILE, D::B_TILE);
+            copy(dst + D::B_TILE, src + D::NG * D::B_TILE, D::ROWS);
+            if (PS) {
+                for (int w = 0; w < nwc; ++w)
+                    copy(dst + D::B_TILE + D::ROWS + 128 * w,
+                         a.G + ((int64_t)blockIdx.x * 4 + w) * a.Ipad + (s0 + s) * F_KD, 128);
+            } else {
+                copy(dst + D::B_TILE + D::ROWS, a.G + (s0 + s) * a.Ipad + row0, 512);
             }
+            *(volatile int*)&sy->loaded = s + 1;
+        };
+        if (el)
+            for (int s = 0; s < F_RING && s < ns; ++s) load(s);
+        for (int s = 0; s < ns; ++s) {
+            // all digits of the stage written, and every warp past stage s-1
+            if (!__all_sync(0xffffffffu, f_wait(sy, &sy->gen, s, a.slots))) break;
+            fence_after();
+            const uint64_t dA = sdesc(sA, LBO, SBO), dB = sdesc(sR + (s % F_RING) * D::SLOT, F_LBO_B, F_SBO_B);
+            // one MMA per digit pair: all of one shape, so that those of one
+            // order (one accumulator) execute in issue order
+#pragma unroll 1
+            for (int d = 0; d < F_NDA; ++d)
+#pragma unroll
+                for (int b = 0; b < F_NDB; ++b) {
+                    if (d + b >= F_NORD) break;
+#pragma unroll
+                    for (int ks = 0; ks < F_KD / 16; ++ks)
+                        mma_bf16(tmem + (d + b) * D::NHP, dA + (uint64_t)((d * AT + ks * 2 * LBO) >> 4),
+                                 dB + (uint64_t)((b * (D::NHP / 8) * F_SBO_B + ks * 2 * F_LBO_B) >> 4),
+                                 idesc_f16(D::NHP), 1u, el);
+                }
+            commit(&sy->mma, el);
+            if (el) *(volatile int*)&sy->issued = s + 1;
+            // the slot of stage s-1: its MMAs are done (every warp waited for
+            // them before it arrived for stage s) and its vectors are read
+            if (el && s >= 1 && s + 2 < ns) load(s + 2);
         }
         __syncwarp();
     } else {

@@ -36,10 +36,21 @@ __host__ __device__ constexpr uint32_t idesc_f16(int N) {
 __host__ __device__ constexpr uint32_t idesc_tf32(int N) {
     return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(N >> 3) << 17) | ((128u >> 4) << 24);
 }
-__device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-    asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p; }"
-                 :: "r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(acc));
+// The MMAs and their commits are issued by one elected lane of a warp that runs
+// the issuing code as a whole: in convergent code the descriptors stay in
+// uniform registers.  Under a branch on one lane each operand was moved there
+// instruction by instruction, about 90 clocks per MMA.
+// 1 in the elected lane, 0 in the others.
+__device__ __forceinline__ uint32_t elect_lane() {
+    uint32_t e;
+    asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(e));
+    return e;
+}
+__device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc,
+                                         uint32_t el) {
+    asm volatile("{ .reg .pred p, q; setp.ne.b32 p, %4, 0; setp.ne.b32 q, %5, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p; }"
+                 :: "r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(el));
 }
 // FP32 rounded to TF32 precision (10 stored mantissa bits, ties away from
 // zero), so that the tensor core reads it exactly.
@@ -47,14 +58,16 @@ __device__ __forceinline__ float tf32_round(float x) {
     return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
 }
 
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-    asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }"
-                 :: "r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(acc));
+__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc,
+                                         uint32_t el) {
+    asm volatile("{ .reg .pred p, q; setp.ne.b32 p, %4, 0; setp.ne.b32 q, %5, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }"
+                 :: "r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(el));
 }
-__device__ __forceinline__ void commit(uint64_t* mbar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                 :: "r"(smem_u32(mbar)) : "memory");
+__device__ __forceinline__ void commit(uint64_t* mbar, uint32_t el) {
+    asm volatile("{ .reg .pred q; setp.ne.b32 q, %1, 0;\n\t"
+                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0]; }"
+                 :: "r"(smem_u32(mbar)), "r"(el) : "memory");
 }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }

@@ -138,8 +138,8 @@ __device__ __forceinline__ bool is_bad(const Sync* sy) { return *(volatile const
 
 // Arrival on the stage buffer, one atomic per warp: after __syncwarp (which
 // orders the warp's tile stores, each already fenced to the async proxy), lane
-// 0 adds to the buffer's counter; the lane 0 of the last of the TC_THREADS/32
-// warps of this use of the buffer returns true (the counter only grows, so no
+// 0 adds to the buffer's counter; all lanes of the last of the TC_THREADS/32
+// warps of this use of the buffer return true (the counter only grows, so no
 // reset races with the next use).  Release/acquire ordering of the atomic makes
 // every warp's stores visible to the MMAs that the last arriver issues.
 __device__ __forceinline__ bool arrive_last(uint32_t* ctr) {
@@ -150,7 +150,7 @@ __device__ __forceinline__ bool arrive_last(uint32_t* ctr) {
         asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(old) : "r"(smem_u32(ctr)) : "memory");
         last = (old % (TC_THREADS / 32)) == TC_THREADS / 32 - 1;
     }
-    return last;
+    return __any_sync(0xffffffffu, last);
 }
 
 // True in lane 0 of the first warp of the CTA to reach this point of a stage
@@ -277,7 +277,7 @@ __device__ __forceinline__ void compensate(float* acc, const float* comp) {
 // (bit-reproducible).
 template <int K, int HG>
 __device__ __forceinline__ void issue_stage_group(uint32_t tmem, int dcol, uint32_t aBase, int aStride, int aLBO,
-                                                  int aSBO, uint32_t bBase, bool first) {
+                                                  int aSBO, uint32_t bBase, bool first, uint32_t el) {
     using D = TcDims<K>;
     constexpr uint32_t idH = idesc_bf16(D::NHP);
     constexpr uint32_t idG = idesc_f16(D::NG);
@@ -292,13 +292,13 @@ __device__ __forceinline__ void issue_stage_group(uint32_t tmem, int dcol, uint3
         const uint32_t acc0 = (first && ks == 0) ? 0u : 1u;
         const uint64_t aWh = dA + ao, aWl = aWh + oS, aUh = aWh + 2 * oS, aUl = aWh + 3 * oS;
         if (HG == 0) {
-            mma_bf16(dH, aWh, dB + bo, idH, acc0);
-            mma_bf16(dH, aWh, dB + oBl + bo, idH, 1u);
-            mma_bf16(dH, aWl, dB + bo, idH, 1u);
+            mma_bf16(dH, aWh, dB + bo, idH, acc0, el);
+            mma_bf16(dH, aWh, dB + oBl + bo, idH, 1u, el);
+            mma_bf16(dH, aWl, dB + bo, idH, 1u, el);
         } else {
-            mma_bf16(dG, aUh, dB + oPh + bo, idG, acc0);
-            mma_bf16(dG + D::NG, aUh, dB + oPh + oBl + bo, idG, acc0);   // lo products: own columns
-            mma_bf16(dG + D::NG, aUl, dB + oPh + bo, idG, 1u);
+            mma_bf16(dG, aUh, dB + oPh + bo, idG, acc0, el);
+            mma_bf16(dG + D::NG, aUh, dB + oPh + oBl + bo, idG, acc0, el);   // lo products: own columns
+            mma_bf16(dG + D::NG, aUl, dB + oPh + bo, idG, 1u, el);
         }
     }
 }
@@ -309,7 +309,7 @@ __device__ __forceinline__ void issue_stage_group(uint32_t tmem, int dcol, uint3
 // the hi.hi columns.  Eight MMAs per 32-deep stage instead of twelve.
 template <int K, bool HESS>
 __device__ __forceinline__ void issue_stage_stacked(uint32_t tmem, int dcol, uint32_t aBase, int aStride, int aLBO,
-                                                    int aSBO, uint32_t bBase, bool first) {
+                                                    int aSBO, uint32_t bBase, bool first, uint32_t el) {
     using D = TcDims<K>;
     constexpr uint32_t idH2 = idesc_bf16(2 * D::NHP), idH = idesc_bf16(D::NHP);
     constexpr uint32_t idG2 = idesc_f16(2 * D::NG), idG = idesc_f16(D::NG);
@@ -327,16 +327,16 @@ __device__ __forceinline__ void issue_stage_stacked(uint32_t tmem, int dcol, uin
         // written once per k-step (every MMA write rounds its accumulator,
         // not to nearest)
         if (HESS) {
-            mma_bf16(dH, aWh, dB + bo, idH2, acc0);
-            mma_bf16(dH + D::NHP, aWl, dB + bo, idH, 1u);
+            mma_bf16(dH, aWh, dB + bo, idH2, acc0, el);
+            mma_bf16(dH + D::NHP, aWl, dB + bo, idH, 1u, el);
         }
-        mma_bf16(dG, aUh, dB + oG + bo, idG2, acc0);
-        mma_bf16(dG + D::NG, aUl, dB + oG + bo, idG, 1u);
+        mma_bf16(dG, aUh, dB + oG + bo, idG2, acc0, el);
+        mma_bf16(dG + D::NG, aUl, dB + oG + bo, idG, 1u, el);
     }
 }
 
 template <int K>
-__device__ __forceinline__ void issue_qp(uint32_t tmem_col, uint32_t sAq, uint32_t sBq_buf) {
+__device__ __forceinline__ void issue_qp(uint32_t tmem_col, uint32_t sAq, uint32_t sBq_buf, uint32_t el) {
     using QD = QpDims<K>;
     constexpr uint32_t id = idesc_tf32(32);
 #pragma unroll
@@ -344,9 +344,9 @@ __device__ __forceinline__ void issue_qp(uint32_t tmem_col, uint32_t sAq, uint32
         const uint32_t o = ks * 256;
         const uint64_t ah = sdesc(sAq + o, 128, QD::SBO), al = sdesc(sAq + QD::A_T + o, 128, QD::SBO);
         const uint64_t bh = sdesc(sBq_buf + o, 128, QD::SBO), bl = sdesc(sBq_buf + QD::B_T + o, 128, QD::SBO);
-        mma_tf32(tmem_col, ah, bh, id, ks > 0 ? 1u : 0u);
-        mma_tf32(tmem_col, ah, bl, id, 1u);
-        mma_tf32(tmem_col, al, bh, id, 1u);
+        mma_tf32(tmem_col, ah, bh, id, ks > 0 ? 1u : 0u, el);
+        mma_tf32(tmem_col, ah, bl, id, 1u, el);
+        mma_tf32(tmem_col, al, bh, id, 1u, el);
     }
 }
 
@@ -499,12 +499,12 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_
                  :: "r"(dst), "l"(src), "r"(bytes), "r"(smem_u32(mbar)) : "memory");
 }
 
-// Window bookkeeping after a stage's MMAs were issued by this thread.
-__device__ __forceinline__ void commit_stage(Sync* sy, int s, int ns, int b, bool window = true) {
+// Window bookkeeping after a stage's MMAs were issued by this warp's elected lane.
+__device__ __forceinline__ void commit_stage(Sync* sy, int s, int ns, int b, uint32_t el, bool window = true) {
     const int d = (s / TC_FLUSH) & 1;
-    commit(&sy->mma_done[b]);
-    if (window && ((s % TC_FLUSH) == TC_FLUSH - 1 || s == ns - 1)) commit(&sy->flush_done[d]);
-    atomicMax(&sy->issued, s + 1);
+    commit(&sy->mma_done[b], el);
+    if (window && ((s % TC_FLUSH) == TC_FLUSH - 1 || s == ns - 1)) commit(&sy->flush_done[d], el);
+    if (el) atomicMax(&sy->issued, s + 1);
 }
 
 // Every generator warp has written its part of stage s's A tiles (buffer b):
@@ -515,9 +515,9 @@ __device__ __forceinline__ void arrive_generated(Sync* sy, int b) {
     __syncwarp();
     if ((threadIdx.x & 31) == 0) mbar_arrive(&sy->gen_full[b]);
 }
-// An issuer (lane 0 of a fixed warp) waits until the whole stage is generated.
+// An issuing warp waits until the whole stage is generated.
 __device__ __forceinline__ bool wait_generated(Sync* sy, int s, int b, double* slots, long long budget) {
-    if (!mbar_wait(&sy->gen_full[b], (s >> 1) & 1, budget)) { set_bad(sy, slots); return false; }
+    if (!__all_sync(0xffffffffu, mbar_wait(&sy->gen_full[b], (s >> 1) & 1, budget))) { set_bad(sy, slots); return false; }
     fence_after();
     return true;
 }
@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pass
     __shared__ __align__(16) float s_cls[128];
     const long long budget = a.budget;
 
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // uniform
     const int r = tid & 127, hf = tid >> 7;
     const int64_t i = (int64_t)blockIdx.x * 128 + r;
     const bool active = i < a.I;
@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pass
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tmem = sy->tslot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, sy->tslot, 0);
     const uint32_t tq = tmem + 2 * D::WQ;                 // qp tiles: columns [2WQ, 2WQ + 64)
     const uint32_t taddr_lane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
     if (tid == 0) {
@@ -680,8 +680,8 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pass
         for (int t = 0; t < 2 && t < ns; ++t) {
             if (!mbar_wait(&sy->fullq[t], 0, budget)) { set_bad(sy, a.slots); break; }
             fence_after();
-            issue_qp<K>(tq + t * 32, sAq, sRq + t * GBQ);
-            commit(&sy->qp_done[t]);
+            issue_qp<K>(tq + t * 32, sAq, sRq + t * GBQ, 1u);
+            commit(&sy->qp_done[t], 1u);
         }
     }
 
@@ -749,33 +749,36 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pass
             sts128(aB + 3 * A_TILE_STD + off, ul[0], ul[1], ul[2], ul[3]);
         }
         arrive_generated(sy, b);
-        // Three issuers, lane 0 of warps 0, 2 and 4, each with its own TMEM
-        // columns: the Hessian MMAs, the gradient MMAs, and the qp MMA of stage
+        // Three issuers, warps 0, 2 and 4 (one elected lane each), each with its own
+        // TMEM columns: the Hessian MMAs, the gradient MMAs, and the qp MMA of stage
         // s+2 into this stage's qp columns (every thread has read them).  Each
         // commits to mma_done, which therefore also covers the qp MMA.
-        if ((tid & 31) == 0 && (warp == 2 || warp == 4 || (HESS && warp == 0))) {
+        if (warp == 2 || warp == 4 || (HESS && warp == 0)) {
             if (wait_generated(sy, s, b, a.slots, budget)) {
+                const uint32_t el = elect_lane();
                 const int d = (s / TC_FLUSH) & 1;
                 if (warp == 4) {
                     if (s + 2 < ns) {
                         const int qs = (s + 2) % QRING;
-                        if (!mbar_wait(&sy->fullq[qs], ((s + 2) / QRING) & 1, budget)) set_bad(sy, a.slots);
-                        else issue_qp<K>(tq + b * 32, sAq, sRq + qs * GBQ);
+                        if (!__all_sync(0xffffffffu, mbar_wait(&sy->fullq[qs], ((s + 2) / QRING) & 1, budget)))
+                            set_bad(sy, a.slots);
+                        else issue_qp<K>(tq + b * 32, sAq, sRq + qs * GBQ, el);
                     }
-                    commit_stage(sy, s, ns, b, false);
+                    commit_stage(sy, s, ns, b, el, false);
                     // the qp tile slots of stages 0 and 1 (their MMAs came from the
                     // prologue, every thread waited for them); later ones are
                     // refilled by the first warp of the stage
-                    if (s < 2 && s + QRING < ns) load_qtile(s + QRING);
+                    if (el && s < 2 && s + QRING < ns) load_qtile(s + QRING);
                 } else {
                     const bool first = (s % TC_FLUSH) == 0;
                     if (warp == 0)
-                        issue_stage_group<K, 0>(tmem, d * D::WQ, aB, A_TILE_STD, LBO_STD, SBO_STD, sR + slot * GBM, first);
+                        issue_stage_group<K, 0>(tmem, d * D::WQ, aB, A_TILE_STD, LBO_STD, SBO_STD, sR + slot * GBM, first, el);
                     else
-                        issue_stage_group<K, 1>(tmem, d * D::WQ, aB, A_TILE_STD, LBO_STD, SBO_STD, sR + slot * GBM, first);
-                    commit_stage(sy, s, ns, b);
+                        issue_stage_group<K, 1>(tmem, d * D::WQ, aB, A_TILE_STD, LBO_STD, SBO_STD, sR + slot * GBM, first, el);
+                    commit_stage(sy, s, ns, b, el);
                 }
             }
+            __syncwarp();
         }
         maybe_fold<K, false>(sy, a.slots, budget, hf, s, taddr_lane, acc, comp);
     }
@@ -842,7 +845,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pass
     __shared__ __align__(16) float s_cls[128];
     const long long budget = a.budget;
 
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // uniform
     const int jl = tid >> 3, ig = tid & 7;
     const int hf = tid >> 7;
     const int64_t j = (int64_t)blockIdx.x * 32 + jl;
@@ -880,7 +883,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pass
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tmem = sy->tslot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, sy->tslot, 0);
     const uint32_t taddr_lane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
     if (tid == 0)
         for (int t = 0; t < RING && t < ns; ++t) load_stage(t);
@@ -955,9 +958,10 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pass
         if (arrive_last(&sy->arrived[b])) {
             fence_after();
             const int d = (s / TC_FLUSH) & 1;
+            const uint32_t el = elect_lane();
             issue_stage_stacked<K, HESS>(tmem, d * D::WS, aB, A_TILE_PAD, LBO_PAD, SBO_PAD, sR + slot * GB,
-                                         (s % TC_FLUSH) == 0);
-            commit_stage(sy, s, ns, b);
+                                         (s % TC_FLUSH) == 0, el);
+            commit_stage(sy, s, ns, b, el);
         }
         maybe_fold<K, true>(sy, a.slots, budget, hf, s, taddr_lane, acc, comp);
     }
