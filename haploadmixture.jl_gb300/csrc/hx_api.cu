@@ -32,6 +32,7 @@ struct hx_ctx {
     int64_t nx = 0;        // K * (I + 4J)
     cudaStream_t st = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    uint8_t* arena = nullptr;    // all device buffers of this context
     uint32_t* G = nullptr;
     unsigned long long* dm = nullptr;
     double *x = nullptr, *xn = nullptr, *xn2 = nullptr, *xt = nullptr, *xio = nullptr;
@@ -41,6 +42,7 @@ struct hx_ctx {
     float* pf = nullptr;                     // mixed: FP32 copy of the pass's p (K x 4J)
     double* slots = nullptr;
     double* h_slots = nullptr;   // pinned
+    int pin_slot = -1;           // its place in the process's pinned page, or -1
     uint8_t* img = nullptr;      // B-operand image of the tensor-core passes
     // plain method: partial maxima and out-of-range sums of the passes (hx_f64.cuh)
     unsigned long long* f64_mx = nullptr;
@@ -49,7 +51,6 @@ struct hx_ctx {
     int8_t* qp_ws = nullptr;     // P-side QP working sets, warm start of the next solve
     hx_loop_opts lo{0, 0, 0, -1};  // admixture_qn!/init_em! options
     double ll_tmp = NAN;         // d.ll_tmp of the step control
-    bool shared_geno = false;    // G and dm belong to the parent context (hx_create_shared)
     int S_q = 1, wpc_q = 1, S_p = 1, ipc_p = 1;
     int S_ll = 1, wpc_ll = 1;                // FP32 log-likelihood pass
     bool tc = false;                         // Hessian passes on the tensor cores
@@ -132,6 +133,48 @@ void prof_resolve(hx_ctx* c) {
         HX_CK(expr);             \
         prof_end(c, kind, n);    \
     } while (0)
+
+// Pinned host memory of a context's scalar block.  Allocating and releasing it
+// costs 270 us, most of the time of opening a small cohort, so the process
+// keeps one page with room for PIN_SLOTS contexts; slots go back when their
+// context is destroyed, and further contexts allocate their own.  The page is
+// looked up before a slot is handed out: a device reset in between frees it.
+constexpr int PIN_SLOTS = 32;
+std::mutex g_pin_mu;
+double* g_pin = nullptr;
+uint32_t g_pin_used = 0;
+
+cudaError_t pin_get(hx_ctx* c) {
+    std::lock_guard<std::mutex> g(g_pin_mu);
+    if (g_pin && g_pin_used == 0) {
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, g_pin) != cudaSuccess || at.type != cudaMemoryTypeHost) {
+            cudaGetLastError();
+            g_pin = nullptr;
+        }
+    }
+    if (!g_pin) {
+        const cudaError_t e = cudaHostAlloc((void**)&g_pin, PIN_SLOTS * HX_NSLOT * sizeof(double), cudaHostAllocPortable);
+        if (e != cudaSuccess) { g_pin = nullptr; return e; }
+        g_pin_used = 0;
+    }
+    for (int s = 0; s < PIN_SLOTS; ++s)
+        if (!((g_pin_used >> s) & 1u)) {
+            g_pin_used |= 1u << s;
+            c->pin_slot = s;
+            c->h_slots = g_pin + s * HX_NSLOT;
+            return cudaSuccess;
+        }
+    return cudaMallocHost((void**)&c->h_slots, HX_NSLOT * sizeof(double));
+}
+void pin_put(hx_ctx* c) {
+    if (c->pin_slot < 0) {
+        if (c->h_slots) cudaFreeHost(c->h_slots);
+        return;
+    }
+    std::lock_guard<std::mutex> g(g_pin_mu);
+    g_pin_used &= ~(1u << c->pin_slot);
+}
 
 inline double* qof(double* x) { return x; }
 inline double* pof(hx_ctx* c, double* x) { return x + (int64_t)c->K * c->I; }
@@ -467,10 +510,22 @@ int check_qp(hx_ctx* c) {
     return HX_OK;
 }
 
+// The context's device memory is one allocation: need() notes a buffer and its
+// size, alloc_all() allocates and places them (256-byte boundaries).  An
+// allocation and its release cost some 20 us each, and a context has up to 30
+// buffers.
+struct Request { void** p; size_t bytes; };
 template <class T>
-int dalloc(hx_ctx* c, T** p, size_t n) {
-    cudaError_t e = cudaMalloc((void**)p, std::max<size_t>(n, 1) * sizeof(T));
+void need(std::vector<Request>& rq, T** p, size_t n) {
+    rq.push_back({(void**)p, (std::max<size_t>(n, 1) * sizeof(T) + 255) / 256 * 256});
+}
+int alloc_all(hx_ctx* c, const std::vector<Request>& rq) {
+    size_t total = 0;
+    for (const Request& r : rq) total += r.bytes;
+    cudaError_t e = cudaMalloc((void**)&c->arena, total);
     if (e != cudaSuccess) return cuda_fail(c, "cudaMalloc", e);
+    uint8_t* at = c->arena;
+    for (const Request& r : rq) { *r.p = at; at += r.bytes; }
     return HX_OK;
 }
 
@@ -502,7 +557,7 @@ int create_common(const uint8_t* bed, bool bed_on_device, int64_t bps, int64_t n
     HX_CK(cudaEventCreate(&c->ev0));
     HX_CK(cudaEventCreate(&c->ev1));
     HX_CK(init_kernel_attrs(K));
-    HX_CK(init_tc_attrs());
+    if (c->tc) HX_CK(init_tc_attrs(K));
     if (c->prec == HX_PREC_FP64) HX_CK(f64_attrs(K));
     plan(c);
     if (c->verbose)
@@ -512,71 +567,80 @@ int create_common(const uint8_t* bed, bool bed_on_device, int64_t bps, int64_t n
                 c->S_q, c->S_p, c->S_qt, c->S_pt, c->S_ll, tc_resident(K, false), tc_resident(K, true),
                 loglik_f32x2_resident(K));
     const int NVmax = K + K * (K + 1) / 2;
+    std::vector<Request> rq;
     if (parent) {
         c->G = parent->G;
         c->dm = parent->dm;
-        c->shared_geno = true;
     } else {
-        HX_ST(dalloc(c, &c->G, (size_t)c->JW * c->Ipad));
-        HX_ST(dalloc(c, &c->dm, (size_t)I));
+        need(rq, &c->G, (size_t)c->JW * c->Ipad);
+        need(rq, &c->dm, (size_t)I);
     }
-    for (double** b : {&c->x, &c->xn, &c->xn2, &c->xt, &c->xio}) HX_ST(dalloc(c, b, (size_t)c->nx));
-    HX_ST(dalloc(c, &c->U, (size_t)c->nx * c->Qs));
-    HX_ST(dalloc(c, &c->V, (size_t)c->nx * c->Qs));
-    HX_ST(dalloc(c, &c->XtXq, (size_t)K * K * I));
-    HX_ST(dalloc(c, &c->Xtzq, (size_t)K * I));
-    HX_ST(dalloc(c, &c->XtXp, (size_t)K * K * 4 * J));
-    HX_ST(dalloc(c, &c->Xtzp, (size_t)K * 4 * J));
+    for (double** b : {&c->x, &c->xn, &c->xn2, &c->xt, &c->xio}) need(rq, b, (size_t)c->nx);
+    // secants; the BED matrix passes through here on its way in, in slices
+    const size_t nuv = (size_t)c->nx * c->Qs;
+    size_t stage = 0;
+    if (!parent && !bed_on_device)
+        stage = std::max<size_t>((size_t)16 * bps, std::min<size_t>((size_t)bps * nsnp, (size_t)32 << 20));
+    need(rq, &c->U, std::max(2 * nuv, (stage + 7) / 8));
+    stage = std::max(stage, 2 * nuv * sizeof(double));
+    need(rq, &c->XtXq, (size_t)K * K * I);
+    need(rq, &c->Xtzq, (size_t)K * I);
+    need(rq, &c->XtXp, (size_t)K * K * 4 * J);
+    need(rq, &c->Xtzp, (size_t)K * 4 * J);
+    const size_t NH = (size_t)K * (K + 1) / 2, rows = (size_t)std::max<int64_t>(I, 4 * J);
     if (c->prec == HX_PREC_FP64) {
-        const size_t NH = (size_t)K * (K + 1) / 2, rows = (size_t)std::max<int64_t>(I, 4 * J);
-        HX_ST(dalloc(c, &c->part_q, (size_t)c->S_qf * NH * c->Ipad));
-        HX_ST(dalloc(c, &c->part_p, (size_t)c->S_pf * NH * 4 * J));
-        HX_ST(dalloc(c, &c->img, f64_image_bytes(K, I, J)));
-        HX_ST(dalloc(c, &c->f64_mx, (size_t)F_MAXB * F_MXS));
-        HX_ST(dalloc(c, &c->rare.i, 2 * rows * NH));
-        HX_ST(dalloc(c, &c->rare.d, rows * NH));
-        HX_ST(dalloc(c, &c->rare.flag, 1));
+        need(rq, &c->part_q, (size_t)c->S_qf * NH * c->Ipad);
+        need(rq, &c->part_p, (size_t)c->S_pf * NH * 4 * J);
+        need(rq, &c->img, f64_image_bytes(K, I, J));
+        need(rq, &c->f64_mx, (size_t)F_MAXB * F_MXS);
+        need(rq, &c->rare.i, 2 * rows * NH);
+        need(rq, &c->rare.d, rows * NH);
+        need(rq, &c->rare.flag, 1);
+    } else {
+        need(rq, &c->part_q, (size_t)std::max(c->S_q, c->tc ? c->Sq_cap : 1) * NVmax * c->Ipad);
+        const int Sp_max = std::max(c->S_p, c->tc ? c->Sp_cap : 1);
+        if (Sp_max > 1) need(rq, &c->part_p, (size_t)Sp_max * NVmax * 4 * J);
+        if (c->tc) need(rq, &c->img, tc_image_bytes(K, I, J));
+        need(rq, &c->pf, (size_t)K * 4 * J);
+    }
+    need(rq, &c->part_ll, (size_t)std::max<int64_t>((c->Ipad / ACC_THREADS) * c->S_q,
+                                                    (int64_t)loglik_f32x2_blocks(c->Ipad, K) *
+                                                        std::max(c->S_ll, c->Sll_cap)));
+    need(rq, &c->part_qn, (size_t)qn_dots_blocks(c->nx) * (2 * HX_QMAX * HX_QMAX + HX_QMAX));
+    need(rq, &c->coef, HX_QMAX);
+    need(rq, &c->slots, HX_NSLOT);
+    need(rq, &c->qp_ws, (size_t)4 * K * J);
+    HX_ST(alloc_all(c, rq));
+    c->V = c->U + nuv;
+    if (c->prec == HX_PREC_FP64) {
         HX_CK(cudaMemsetAsync(c->rare.i, 0, 2 * rows * NH * sizeof(long long), c->st));
         HX_CK(cudaMemsetAsync(c->rare.d, 0, rows * NH * sizeof(double), c->st));
-    } else {
-        HX_ST(dalloc(c, &c->part_q, (size_t)std::max(c->S_q, c->tc ? c->Sq_cap : 1) * NVmax * c->Ipad));
-        const int Sp_max = std::max(c->S_p, c->tc ? c->Sp_cap : 1);
-        if (Sp_max > 1) HX_ST(dalloc(c, &c->part_p, (size_t)Sp_max * NVmax * 4 * J));
     }
-    HX_ST(dalloc(c, &c->part_ll, (size_t)std::max<int64_t>((c->Ipad / ACC_THREADS) * c->S_q,
-                                                            (int64_t)loglik_f32x2_blocks(c->Ipad, K) *
-                                                                std::max(c->S_ll, c->Sll_cap))));
-    HX_ST(dalloc(c, &c->part_qn, (size_t)qn_dots_blocks(c->nx) * (2 * HX_QMAX * HX_QMAX + HX_QMAX)));
-    HX_ST(dalloc(c, &c->coef, HX_QMAX));
-    HX_ST(dalloc(c, &c->slots, HX_NSLOT));
-    if (c->tc) HX_ST(dalloc(c, &c->img, tc_image_bytes(K, I, J)));
-    if (c->prec != HX_PREC_FP64) HX_ST(dalloc(c, &c->pf, (size_t)K * 4 * J));
-    HX_ST(dalloc(c, &c->qp_ws, (size_t)4 * K * J));
     HX_CK(cudaMemsetAsync(c->qp_ws, 0, (size_t)4 * K * J, c->st));
-    HX_CK(cudaMallocHost((void**)&c->h_slots, HX_NSLOT * sizeof(double)));
-    HX_CK(cudaMemsetAsync(c->U, 0, (size_t)c->nx * c->Qs * sizeof(double), c->st));
-    HX_CK(cudaMemsetAsync(c->V, 0, (size_t)c->nx * c->Qs * sizeof(double), c->st));
+    HX_CK(pin_get(c));
     for (int s = 0; s < HX_NSLOT; ++s) c->h_slots[s] = 0.0;
     c->h_slots[S_LL_NEW] = NAN;
     HX_CK(cudaMemcpyAsync(c->slots, c->h_slots, HX_NSLOT * sizeof(double), cudaMemcpyHostToDevice, c->st));
-    if (parent) {
-        HX_CK(cudaStreamSynchronize(c->st));
-        return HX_OK;
+    if (!parent) {
+        // the BED matrix (first 2J SNPs used by the fit; all n_snp SNPs for the
+        // double-missing count, as count_double_missing! reads the whole file)
+        HX_CK(cudaMemsetAsync(c->dm, 0, (size_t)I * sizeof(unsigned long long), c->st));
+        const int64_t Jf = nsnp / 2, cols = (Jf + 7) / 8;
+        if (bed_on_device) {
+            HX_CK(launch_pack(bed, bps, bps * nsnp, I, J, Jf, c->Ipad, c->JW, 0, cols, c->G, c->dm, c->st));
+        } else {
+            // whole word columns (16 SNPs) at a time through the secants' memory
+            uint8_t* buf = (uint8_t*)c->U;
+            const int64_t step = std::max<int64_t>(1, (int64_t)(stage / (16 * (size_t)bps)));
+            for (int64_t w = 0; w < cols; w += step) {
+                const int64_t n = std::min(step, cols - w), s0 = 16 * w, s1 = std::min(nsnp, s0 + 16 * n);
+                HX_CK(cudaMemcpyAsync(buf, bed + s0 * bps, (size_t)(s1 - s0) * bps, cudaMemcpyHostToDevice, c->st));
+                HX_CK(launch_pack(buf, bps, bps * (s1 - s0), I, J, Jf, c->Ipad, c->JW, w, n, c->G, c->dm, c->st));
+            }
+        }
     }
-    HX_CK(cudaMemsetAsync(c->dm, 0, (size_t)I * sizeof(unsigned long long), c->st));
-    // stage the BED matrix (first 2J SNPs used by the fit; all n_snp SNPs for
-    // the double-missing count, as count_double_missing! reads the whole file)
-    const uint8_t* dbed = bed;
-    uint8_t* tmp = nullptr;
-    if (!bed_on_device) {
-        HX_ST(dalloc(c, &tmp, (size_t)bps * nsnp));
-        HX_CK(cudaMemcpyAsync(tmp, bed, (size_t)bps * nsnp, cudaMemcpyHostToDevice, c->st));
-        dbed = tmp;
-    }
-    HX_CK(launch_pack(dbed, bps, I, J, c->Ipad, c->JW, c->G, c->st));
-    HX_CK(launch_double_missing(dbed, bps, I, nsnp, c->dm, c->st));
+    HX_CK(cudaMemsetAsync(c->U, 0, 2 * nuv * sizeof(double), c->st));
     HX_CK(cudaStreamSynchronize(c->st));
-    if (tmp) HX_CK(cudaFree(tmp));
     return HX_OK;
 }
 
@@ -677,13 +741,10 @@ int hx_create_device(const uint8_t* d_bed, int64_t bps, int64_t nsnp, int64_t I,
 int hx_destroy(hx_ctx* c) {
     if (!c) return HX_OK;
     if (c->st) cudaStreamSynchronize(c->st);
-    void* bufs[] = {c->shared_geno ? nullptr : (void*)c->G, c->shared_geno ? nullptr : (void*)c->dm, c->x, c->xn, c->xn2, c->xt, c->xio, c->U, c->V, c->XtXq, c->Xtzq, c->XtXp,
-                    c->Xtzp, c->part_q, c->part_p, c->part_ll, c->part_qn, c->coef, c->slots, c->img, c->qp_ws,
-                    c->pf, c->f64_mx, c->rare.i, c->rare.d, c->rare.flag};
-    for (void* b : bufs) if (b) cudaFree(b);
+    if (c->arena) cudaFree(c->arena);
     prof_resolve(c);
     for (cudaEvent_t e : c->pool) cudaEventDestroy(e);
-    if (c->h_slots) cudaFreeHost(c->h_slots);
+    pin_put(c);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->st) cudaStreamDestroy(c->st);
@@ -739,14 +800,12 @@ int hx_get_ll(hx_ctx* c, double* ll) {
 
 int hx_census(hx_ctx* c, uint64_t counts[16]) {
     if (!c || !counts) return HX_EINVAL;
-    int st = HX_OK;
-    Tmp t;
-    unsigned long long* d = t.get<unsigned long long>(c, 16, &st);
-    if (!d) return st;
+    unsigned long long* d = (unsigned long long*)c->part_ll;   // scratch of the log-likelihood (256 bytes at least)
     HX_CK(cudaMemsetAsync(d, 0, 16 * sizeof(unsigned long long), c->st));
-    HX_CK(launch_census(c->G, c->Ipad, c->I, c->J, c->JW, d, c->st));
+    HX_CK(launch_census(c->G, c->Ipad, c->JW, d, c->st));
     HX_CK(cudaMemcpyAsync(counts, d, 16 * sizeof(uint64_t), cudaMemcpyDeviceToHost, c->st));
     HX_CK(cudaStreamSynchronize(c->st));
+    counts[15] -= (uint64_t)(c->Ipad * c->JW * 8 - c->I * c->J);   // padding counts as double missing
     return HX_OK;
 }
 

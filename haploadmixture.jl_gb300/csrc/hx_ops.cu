@@ -3,6 +3,7 @@
 // arithmetic is floating point).
 #include "hx_ops.cuh"
 #include "hx_qp_dense.cuh"
+#include <algorithm>
 #include <climits>
 
 namespace hx {
@@ -11,66 +12,150 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 
 // ------------------------------------------------------------------ decode
-// One thread per (word column jw, BED byte column c): reads the 16 SNP rows of
-// the word column at byte c (4 individuals) and writes 4 class words.
-__global__ void k_pack(const uint8_t* __restrict__ bed, int64_t bps, int64_t I, int64_t J, int64_t Ipad,
-                       uint32_t* __restrict__ G) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t jw = blockIdx.y;
-    if (c >= Ipad / 4) return;
-    uint32_t w[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-    for (int t = 0; t < 16; ++t) {
-        const int64_t s = 16 * jw + t;
-        const int64_t j = s >> 1;
-        const uint8_t byte = (j < J && c < bps) ? bed[s * bps + c] : (uint8_t)0x55;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            uint32_t code = (byte >> (2 * r)) & 3u;
-            if (4 * c + r >= I) code = 1u;
-            w[r] |= code << (4 * (t >> 1) + 2 * (t & 1));
-        }
-    }
-    uint4 v = make_uint4(w[0], w[1], w[2], w[3]);
-    *reinterpret_cast<uint4*>(G + jw * Ipad + 4 * c) = v;
+// Four bytes (16 individuals) of a SNP row from byte address a on; bytes at or
+// past end read as 0.
+__device__ __noinline__ uint32_t load_codes(const uint8_t* a, const uint8_t* end) {
+    uint32_t v = 0u;
+    for (int b = 0; b < 4; ++b)
+        if (a + b < end) v |= (uint32_t)a[b] << (8 * b);
+    return v;
 }
 
-__global__ void k_census(const uint32_t* __restrict__ G, int64_t Ipad, int64_t I, int64_t J,
-                         unsigned long long* __restrict__ counts) {
+// One round of a 16 x 16 transpose of 2-bit elements: exchanges the blocks off the
+// diagonal of each 2H x 2H block (m: the columns of its first half).
+template <int H>
+__device__ __forceinline__ void swap_round(uint32_t (&x)[16], uint32_t m) {
+#pragma unroll
+    for (int t = 0; t < 16; ++t)
+        if (!(t & H)) {
+            const uint32_t a = x[t], b = x[t + H < 16 ? t + H : t];
+            x[t] = (a & m) | ((b & m) << (2 * H));
+            x[t + H < 16 ? t + H : t] = ((a >> (2 * H)) & m) | (b & ~m);
+        }
+}
+
+// Decodes word columns jw0 .. jw0+ncol-1 (the 16 SNP rows of word column jw0 + w
+// start at bed + 16 w bps) into class words, and counts the blocks whose two SNPs
+// are both missing (src/utils.jl:1-18: over all Jf blocks of the file, beyond
+// the J that the fit uses).  Thread: 16 individuals x `per` word columns; the 16
+// rows' words are transposed as a 16 x 16 matrix of 2-bit codes in registers (four
+// rounds of swaps), so the matrix is read once, in words, and each row of 16
+// class words is written whole.  Memory-bound.
+__global__ void __launch_bounds__(128)
+k_pack(const uint8_t* __restrict__ bed, int64_t bps, const uint8_t* end, int64_t I, int64_t J, int64_t Jf, int64_t Ipad,
+       int JW, int64_t jw0, int64_t ncol, int per, uint32_t* __restrict__ G, unsigned long long* __restrict__ dm) {
+    __shared__ uint4 swap[128 * 4];
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t i0 = 16 * c;              // individuals past Ipad (the last warps) are neither read nor written
+    const int nv = (int)min((int64_t)16, max((int64_t)0, I - i0));        // individuals here
+    const bool aligned = ((reinterpret_cast<uintptr_t>(bed) | (uintptr_t)bps) & 3u) == 0;
+    const uint32_t vmask = nv == 16 ? 0xFFFFFFFFu : (1u << (2 * nv)) - 1u;
+    unsigned cnt[16];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) cnt[r] = 0u;
+    const int64_t w1 = min(ncol, ((int64_t)blockIdx.y + 1) * per);
+    for (int64_t w = (int64_t)blockIdx.y * per; w < w1; ++w) {
+        const int64_t jw = jw0 + w;
+        // codes of the 16 rows; rows past the file read as homozygous, individuals
+        // past I as missing.  Away from the buffer's end the loads need no checks
+        // of their own, so they are all in flight together.
+        uint32_t x[16];
+        const uint8_t* row = bed + 16 * w * bps + 4 * c;
+        if (nv > 0 && 16 * jw + 15 < 2 * Jf && row + 15 * bps + 8 <= end) {
+            if (aligned) {
+#pragma unroll
+                for (int t = 0; t < 16; ++t) x[t] = *reinterpret_cast<const uint32_t*>(row + t * bps);
+            } else {
+                uint32_t y[16];
+#pragma unroll
+                for (int t = 0; t < 16; ++t) {
+                    const uint32_t* p = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(row + t * bps) & ~(uintptr_t)3);
+                    x[t] = p[0];
+                    y[t] = p[1];
+                }
+#pragma unroll
+                for (int t = 0; t < 16; ++t)
+                    x[t] = __funnelshift_r(x[t], y[t], 8 * (unsigned)(reinterpret_cast<uintptr_t>(row + t * bps) & 3u));
+            }
+        } else {
+#pragma unroll
+            for (int t = 0; t < 16; ++t)
+                x[t] = nv > 0 && 16 * jw + t < 2 * Jf ? load_codes(row + t * bps, end) : 0u;
+        }
+#pragma unroll
+        for (int t = 0; t < 16; ++t) x[t] = (x[t] & vmask) | (0x55555555u & ~vmask);
+        swap_round<8>(x, 0x0000FFFFu);
+        swap_round<4>(x, 0x00FF00FFu);
+        swap_round<2>(x, 0x0F0F0F0Fu);
+        swap_round<1>(x, 0x33333333u);
+        // x[r]: individual i0 + r, nibble b the class of block 8 jw + b
+        const int nb = (int)min((int64_t)8, max((int64_t)0, J - 8 * jw));   // blocks of the fit in this column
+        const uint32_t keep = nb == 8 ? 0xFFFFFFFFu : (1u << (4 * nb)) - 1u;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+            const uint32_t d = x[r] ^ HX_PAD_WORD, e = d | (d >> 1);
+            cnt[r] += 8 - __popc((e | (e >> 2)) & 0x11111111u);
+            x[r] = (x[r] & keep) | (HX_PAD_WORD & ~keep);
+        }
+        if (jw < JW) {
+            // through shared memory, so that a warp's stores cover whole lines
+            uint4* buf = swap + (threadIdx.x & ~31u) * 4;
+            const int lane = threadIdx.x & 31;
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                buf[4 * lane + (r ^ ((lane >> 1) & 3))] = make_uint4(x[4 * r], x[4 * r + 1], x[4 * r + 2], x[4 * r + 3]);
+            __syncwarp();
+            uint4* out = reinterpret_cast<uint4*>(G + jw * Ipad + 16 * (c - lane));
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int u = 32 * r + lane;
+                if (16 * (c - lane) + 4 * u < Ipad) out[u] = buf[(u & ~3) + ((u & 3) ^ ((u >> 3) & 3))];
+            }
+            __syncwarp();
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 16; ++r)
+        if (r < nv && cnt[r]) atomicAdd(dm + i0 + r, (unsigned long long)cnt[r]);
+}
+
+// Counts of the 16 classes over n4 x 4 class words, padding included (the caller
+// subtracts it).  Four words at a time: each code's positions of the two SNPs as
+// bits, the words' bits side by side in one mask, one population count per class.
+__global__ void __launch_bounds__(256) k_census(const uint4* __restrict__ G, int64_t n4,
+                                                unsigned long long* __restrict__ counts) {
     __shared__ unsigned hist[16];
     if (threadIdx.x < 16) hist[threadIdx.x] = 0u;
     __syncthreads();
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t jw = blockIdx.y;
-    if (i < I) {
-        const uint32_t word = G[jw * Ipad + i];
-        for (int b = 0; b < 8; ++b) {
-            if (8 * jw + b >= J) break;
-            const unsigned nib = (word >> (4 * b)) & 0xFu;
-            const int g1 = code_g(nib & 3), g2 = code_g(nib >> 2);
-            atomicAdd(&hist[g1 * 4 + g2], 1u);
-        }
+    unsigned n[16];
+#pragma unroll
+    for (int a = 0; a < 16; ++a) n[a] = 0u;
+    for (int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x; t < n4; t += (int64_t)gridDim.x * 256) {
+        const uint4 v = G[t];
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        // bit planes of the nibbles: word q's bit plane p at bits 4 b + q
+        uint32_t p[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const uint32_t x = w[q] & (0x11111111u << b);
+                p[b] |= q >= b ? x << (q - b) : x >> (b - q);
+            }
+        const uint32_t s1[4] = {~p[0] & ~p[1], p[0] & ~p[1], ~p[0] & p[1], p[0] & p[1]};
+        const uint32_t s2[4] = {~p[2] & ~p[3], p[2] & ~p[3], ~p[2] & p[3], p[2] & p[3]};
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) n[code_g(a) * 4 + code_g(b)] += __popc(s1[a] & s2[b]);
+    }
+#pragma unroll
+    for (int a = 0; a < 16; ++a) {
+        const unsigned s = __reduce_add_sync(FULL, n[a]);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&hist[a], s);
     }
     __syncthreads();
     if (threadIdx.x < 16 && hist[threadIdx.x]) atomicAdd(counts + threadIdx.x, (unsigned long long)hist[threadIdx.x]);
-}
-
-// src/utils.jl:1-18: per individual, blocks (over the whole SNP range) whose
-// two SNPs are both missing.  Thread per (byte column, chunk of blocks).
-__global__ void k_double_missing(const uint8_t* __restrict__ bed, int64_t bps, int64_t I, int64_t Jf, int64_t chunk,
-                                 unsigned long long* __restrict__ dm) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= bps) return;
-    const int64_t j0 = (int64_t)blockIdx.y * chunk, j1 = min(Jf, j0 + chunk);
-    unsigned cnt[4] = {0u, 0u, 0u, 0u};
-    for (int64_t j = j0; j < j1; ++j) {
-        const uint8_t b1 = bed[(2 * j) * bps + c], b2 = bed[(2 * j + 1) * bps + c];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) cnt[r] += (((b1 >> (2 * r)) & 3) == 1 && ((b2 >> (2 * r)) & 3) == 1) ? 1u : 0u;
-    }
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-        if (4 * c + r < I && cnt[r]) atomicAdd(dm + 4 * c + r, (unsigned long long)cnt[r]);
 }
 
 // ------------------------------------------------------------------ synthetic
@@ -431,25 +516,21 @@ inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 }  // namespace
 
 // ================================================================== launchers
-cudaError_t launch_pack(const uint8_t* bed, int64_t bps, int64_t I, int64_t J, int64_t Ipad, int JW, uint32_t* G,
+cudaError_t launch_pack(const uint8_t* bed, int64_t bps, int64_t nbytes, int64_t I, int64_t J, int64_t Jf,
+                        int64_t Ipad, int JW, int64_t jw0, int64_t ncol, uint32_t* G, unsigned long long* dm,
                         cudaStream_t st) {
-    dim3 grid(nblk(Ipad / 4, 256), JW);
-    k_pack<<<grid, 256, 0, st>>>(bed, bps, I, J, Ipad, G);
+    if (ncol <= 0) return cudaSuccess;
+    // word columns per thread: enough CTAs to fill the chip, few additions to dm
+    const unsigned gx = nblk(Ipad / 16, 128);
+    const int64_t per = std::max<int64_t>(1, std::min<int64_t>(64, ncol * gx / 2432));
+    dim3 grid(gx, nblk(ncol, (int)per));
+    k_pack<<<grid, 128, 0, st>>>(bed, bps, bed + nbytes, I, J, Jf, Ipad, JW, jw0, ncol, (int)per, G, dm);
     return cudaGetLastError();
 }
-cudaError_t launch_census(const uint32_t* G, int64_t Ipad, int64_t I, int64_t J, int JW, unsigned long long* counts,
-                          cudaStream_t st) {
-    dim3 grid(nblk(I, 256), JW);
-    k_census<<<grid, 256, 0, st>>>(G, Ipad, I, J, counts);
-    return cudaGetLastError();
-}
-cudaError_t launch_double_missing(const uint8_t* bed, int64_t bps, int64_t I, int64_t nsnp, unsigned long long* dm,
-                                  cudaStream_t st) {
-    const int64_t Jf = nsnp / 2;
-    if (Jf == 0) return cudaSuccess;
-    const int64_t chunk = 512;
-    dim3 grid(nblk(bps, 256), (unsigned)((Jf + chunk - 1) / chunk));
-    k_double_missing<<<grid, 256, 0, st>>>(bed, bps, I, Jf, chunk, dm);
+cudaError_t launch_census(const uint32_t* G, int64_t Ipad, int JW, unsigned long long* counts, cudaStream_t st) {
+    const int64_t n4 = Ipad / 4 * JW;
+    k_census<<<(unsigned)std::min<int64_t>((n4 + 255) / 256, 1216), 256, 0, st>>>(reinterpret_cast<const uint4*>(G), n4,
+                                                                              counts);
     return cudaGetLastError();
 }
 cudaError_t launch_synth(uint64_t seed, int64_t I, int64_t J, int K, const uint64_t* thrQ, const uint64_t* thrP,

@@ -47,7 +47,7 @@ cudaError_t tc_run_g2(TcCall& c);   // K = 8, 9
 cudaError_t tc_run_g3(TcCall& c);   // K = 10
 cudaError_t tc_run_g4(TcCall& c);   // K = 11
 cudaError_t tc_run_g5(TcCall& c);   // K = 12
-cudaError_t init_tc_attrs();
+cudaError_t init_tc_attrs(int K);
 // CTAs of the Hessian tensor-core pass resident on one SM (registers, shared
 // memory and TMEM columns), after init_tc_attrs
 int tc_resident(int K, bool p_side);
@@ -104,12 +104,14 @@ cudaError_t launch_accum_p_tc(int K, bool hess, const PassArgs& a, cudaStream_t 
 size_t tc_image_bytes(int K, int64_t I, int64_t J);
 
 // decode / checks / synthetic data
-cudaError_t launch_pack(const uint8_t* bed, int64_t bps, int64_t I, int64_t J, int64_t Ipad, int JW, uint32_t* G,
+// word columns jw0 .. jw0+ncol-1, whose SNP rows start at bed (nbytes readable
+// bytes); dm (zero at the start) takes the double-missing counts over all Jf
+// blocks of the file
+cudaError_t launch_pack(const uint8_t* bed, int64_t bps, int64_t nbytes, int64_t I, int64_t J, int64_t Jf,
+                        int64_t Ipad, int JW, int64_t jw0, int64_t ncol, uint32_t* G, unsigned long long* dm,
                         cudaStream_t st);
-cudaError_t launch_census(const uint32_t* G, int64_t Ipad, int64_t I, int64_t J, int JW,
-                          unsigned long long* counts, cudaStream_t st);
-cudaError_t launch_double_missing(const uint8_t* bed, int64_t bps, int64_t I, int64_t nsnp,
-                                  unsigned long long* dm, cudaStream_t st);
+// counts over all class words, padding included
+cudaError_t launch_census(const uint32_t* G, int64_t Ipad, int JW, unsigned long long* counts, cudaStream_t st);
 cudaError_t launch_synth(uint64_t seed, int64_t I, int64_t J, int K, const uint64_t* thrQ, const uint64_t* thrP,
                          double miss, uint8_t* bed, cudaStream_t st);
 

@@ -15,13 +15,9 @@ cudaError_t tc_run_any(TcCall& c) {
 }
 }  // namespace
 
-cudaError_t init_tc_attrs() {
-    for (int K = 1; K <= 12; ++K) {
-        TcCall c{TC_ATTRS, K, true, nullptr, nullptr, 0, 0, 0};
-        const cudaError_t e = tc_run_any(c);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+cudaError_t init_tc_attrs(int K) {
+    TcCall c{TC_ATTRS, K, true, nullptr, nullptr, 0, 0, 0};
+    return tc_run_any(c);
 }
 
 int tc_resident(int K, bool p_side) {
