@@ -208,24 +208,37 @@ __global__ void k_synth(uint64_t seed, int64_t I, int64_t J, int K, const uint64
 }
 
 // ------------------------------------------------------------------ reductions
-__global__ void k_reduce_sym(const double* __restrict__ part, int S, int K, int NV, int64_t rows, int64_t ld,
-                             double* __restrict__ XtX, double* __restrict__ Xtz) {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    for (int k = 0; k < K; ++k) {
+// Chunk sums [S][NV][ld] (values 0 .. K-1 the gradient, then the Hessian's upper
+// triangle) added in chunk order -> Xtz and both triangles of XtX.  Block: 32
+// rows; a warp sums one value of 32 consecutive rows (coalesced), and the
+// results leave through shared memory, so that the K x K blocks are written in
+// order too (each thread walking all values of its own row took 83 us for 5,000
+// rows of 20 values and 61 chunks: 20 blocks of uncoalesced stores).
+constexpr int RS_ROWS = 32;
+__global__ void __launch_bounds__(256) k_reduce_sym(const double* __restrict__ part, int S, int K, int NV, int64_t rows,
+                                                    int64_t ld, double* __restrict__ XtX, double* __restrict__ Xtz) {
+    extern __shared__ double tile[];   // [NV][RS_ROWS + 1]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int64_t r0 = (int64_t)blockIdx.x * RS_ROWS, r = r0 + lane;
+    for (int v = warp; v < NV; v += 8) {
         double s = 0.0;
-        for (int c = 0; c < S; ++c) s += part[((int64_t)c * NV + k) * ld + r];
-        Xtz[(int64_t)K * r + k] = s;
-    }
-    if (NV == K) return;
-    int v = K;
-    for (int k = 0; k < K; ++k)
-        for (int k2 = k; k2 < K; ++k2, ++v) {
-            double s = 0.0;
-            for (int c = 0; c < S; ++c) s += part[((int64_t)c * NV + v) * ld + r];
-            XtX[(int64_t)K * K * r + k2 + K * k] = s;
-            XtX[(int64_t)K * K * r + k + K * k2] = s;
+        if (r < rows) {
+            const double* src = part + (int64_t)v * ld + r;
+#pragma unroll 8
+            for (int c = 0; c < S; ++c) s += src[(int64_t)c * NV * ld];
         }
+        tile[v * (RS_ROWS + 1) + lane] = s;
+    }
+    __syncthreads();
+    const int nr = (int)min((int64_t)RS_ROWS, rows - r0);
+    for (int t = tid; t < nr * K; t += 256) Xtz[r0 * K + t] = tile[(t % K) * (RS_ROWS + 1) + t / K];
+    if (NV == K) return;
+    const int KK = K * K;
+    for (int t = tid; t < nr * KK; t += 256) {
+        const int row = t / KK, e = t - row * KK, a = e / K, b = e - a * K;
+        const int lo = min(a, b), hi = max(a, b);
+        XtX[r0 * KK + t] = tile[(K + lo * K - lo * (lo - 1) / 2 + hi - lo) * (RS_ROWS + 1) + row];
+    }
 }
 
 __global__ void k_reduce_sum(const double* __restrict__ part, int64_t n, double* __restrict__ out) {
@@ -545,7 +558,8 @@ cudaError_t launch_synth(uint64_t seed, int64_t I, int64_t J, int K, const uint6
 cudaError_t launch_reduce_sym(const double* part, int S, int K, bool hess, int64_t rows, int64_t ld, double* XtX,
                               double* Xtz, cudaStream_t st) {
     const int NV = K + (hess ? K * (K + 1) / 2 : 0);
-    k_reduce_sym<<<nblk(rows, 256), 256, 0, st>>>(part, S, K, NV, rows, ld, XtX, Xtz);
+    const size_t smem = (size_t)NV * (RS_ROWS + 1) * sizeof(double);   // <= 23.8 KB (K = 12)
+    k_reduce_sym<<<nblk(rows, RS_ROWS), 256, smem, st>>>(part, S, K, NV, rows, ld, XtX, Xtz);
     return cudaGetLastError();
 }
 cudaError_t launch_reduce_sum(const double* part, int64_t n, double* out, cudaStream_t st) {
