@@ -213,6 +213,19 @@ int64_t pick_chunk_f64(int64_t tiles, int64_t units, int64_t slots) {
     return best;
 }
 
+// Chunk length (word columns) of the FP32 log-likelihood: the split with the
+// least time for its last wave of CTAs, where a CTA costs its columns plus about
+// 4 for its start (q, the first p rows) and its end (the product's log).
+int64_t pick_chunk_ll(int64_t tiles, int64_t units, int64_t slots) {
+    int64_t best = units, bcost = INT64_MAX;
+    for (int64_t s = 1; s <= std::min(units, 32 * slots / tiles + 32); ++s) {
+        const int64_t per = (units + s - 1) / s, sa = (units + per - 1) / per;
+        const int64_t cost = (tiles * sa + slots - 1) / slots * (per + 4);
+        if (cost < bcost) { bcost = cost; best = per; }
+    }
+    return best;
+}
+
 // Chunk lengths (grid.y splits) of the mixed method's three pass kernels that
 // hx_autotune measured fastest, per device, K, I and J, for the whole process.
 struct TuneVal { int wpc_qt, spc_pt, wpc_ll; };
@@ -272,7 +285,7 @@ void plan(hx_ctx* c) {
     c->ipc_pt = (int)(spc * 32);
     c->S_pt = (int)((nst + spc - 1) / spc);
     const int64_t tilesL = loglik_f32x2_blocks(c->Ipad, c->K);
-    c->wpc_ll = (int)pick_chunk(tilesL, c->JW, (int64_t)nsm * loglik_f32x2_resident(c->K), 8);
+    c->wpc_ll = (int)pick_chunk_ll(tilesL, c->JW, (int64_t)nsm * loglik_f32x2_resident(c->K));
     c->S_ll = (c->JW + c->wpc_ll - 1) / c->wpc_ll;
     c->Sq_cap = std::min(c->JW, 2 * c->S_qt);
     c->Sp_cap = (int)std::min<int64_t>(nst, 2 * (int64_t)c->S_pt);

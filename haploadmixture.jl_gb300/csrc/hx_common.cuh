@@ -156,7 +156,7 @@ __device__ __forceinline__ void pair_eval_tab(unsigned nib, const float qp[4], f
     u[3] = fmaf(hr, qp[0], fmaf(x11, tb.y, x21 * tb.w));
 }
 
-// Likelihood only (log-likelihood passes).
+// Likelihood only.
 __device__ __forceinline__ float pair_lik_tab(unsigned nib, const float qp[4], const float4* tab) {
     const float4 ta = tab[nib & 3u], tb = tab[(nib >> 2) & 3u];
     const float v10 = fmaf(tb.y, qp[1], tb.x * qp[0]), v11 = fmaf(tb.y, qp[3], tb.x * qp[2]);
@@ -203,38 +203,56 @@ __device__ __forceinline__ void f2_split(uint64_t v, float& lo, float& hi) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
 
-// Class rows: for each class the 0/1 membership of the four haplotypes in the
-// first copy's set (class_m1) and, CLS_COPY2 bytes on, in the second copy's
-// (class_m2), as FP32.  A kernel keeps them in shared memory (cls_table_init by
-// its first 128 threads, then a barrier) and addresses a row by 16 * class.
-constexpr int CLS_COPY2 = 256;
-__device__ __forceinline__ void cls_table_init(float* tab, int tid) {
-    if (tid < 128) {
-        const unsigned nib = (tid & 63) >> 2;
-        const unsigned m = (unsigned)((tid < 64 ? TAB_M1 : TAB_M2) >> (4 * nib)) & 0xFu;
-        tab[tid] = (m >> (tid & 3)) & 1u ? 1.f : 0.f;
+// Class rows: for each class the membership of the four haplotypes in the first
+// copy's set (class_m1, bytes 0-3) and in the second copy's (class_m2, bytes
+// 4-7), 0x40 or 0: the byte as the top byte of a float is 2.0f or 0.0f.  Sixteen
+// rows of 8 bytes fill the 32 banks once, so a warp's lookups never conflict and
+// take two wavefronts (FP32 rows of 16 bytes took about eleven, and shared-memory
+// wavefronts were what bound the P pass and the log-likelihood: 80% of the
+// clocks).  Kept in shared memory (cls_table_init by the first 32 threads, then a
+// barrier); a row is addressed by 8 * class.
+__device__ __forceinline__ void cls_table_init(uint32_t* tab, int tid) {
+    if (tid < 32) {
+        const unsigned nib = tid >> 1;
+        const unsigned m = (unsigned)((tid & 1 ? TAB_M2 : TAB_M1) >> (4 * nib)) & 0xFu;
+        tab[tid] = (m & 1u ? 0x40u : 0u) | (m & 2u ? 0x4000u : 0u) | (m & 4u ? 0x400000u : 0u) | (m & 8u ? 0x40000000u : 0u);
     }
 }
+struct ClsRow { uint64_t a01, a23, b01, b23; };   // 2.0f or 0.0f: first copy's set, second copy's
+__device__ __forceinline__ ClsRow cls_row(const uint32_t* tab, unsigned off) {
+    const uint2 r = *reinterpret_cast<const uint2*>(reinterpret_cast<const char*>(tab) + off);
+    auto f = [](uint32_t x, unsigned sel) { return __uint_as_float(__byte_perm(x, 0u, sel)); };
+    ClsRow c;
+    c.a01 = f2_pack(f(r.x, 0x0444), f(r.x, 0x1444));
+    c.a23 = f2_pack(f(r.x, 0x2444), f(r.x, 0x3444));
+    c.b01 = f2_pack(f(r.y, 0x0444), f(r.y, 0x1444));
+    c.b23 = f2_pack(f(r.y, 0x2444), f(r.y, 0x3444));
+    return c;
+}
+// Twice the two copies' factors F1, F2 (0 for the double heterozygote and double
+// missing).
+__device__ __forceinline__ void cls_factors(const ClsRow& c, uint64_t z01, uint64_t z23, float& F1, float& F2) {
+    float a, b;
+    f2_split(f2_fma(c.a23, z23, f2_mul(c.a01, z01)), a, b);
+    F1 = a + b;
+    f2_split(f2_fma(c.b23, z23, f2_mul(c.b01, z01)), a, b);
+    F2 = a + b;
+}
 
-// scale * u (scale a power of two) of the class at byte offset off = 16 * class,
+// scale * u (scale a power of two) of the class at byte offset off = 8 * class,
 // from packed (qp0, qp1), (qp2, qp3), in packed FP32x2 arithmetic: the same
 // results as pair_eval_tab's u * scale, bit for bit (a copy's set has at most
-// two members, so each factor rounds once in either order of the sum; scaling
-// by a power of two is exact).  The double heterozygote takes its operands
-// (qp3, qp2, qp1, qp0) / den through the first copy's row.
+// two members, so each factor rounds once in either order of the sum; the
+// powers of two are exact: 2 / (2 F)).  The double heterozygote takes its operands
+// (qp3, qp2, qp1, qp0) / den in the place of the first copy's row.
 __device__ __forceinline__ void pair_u_cls(unsigned off, uint64_t z01, uint64_t z23, uint64_t& u01, uint64_t& u23,
-                                           const float* tab, float scale) {
-    const char* row = reinterpret_cast<const char*>(tab) + off;
-    const ulonglong2 c1 = *reinterpret_cast<const ulonglong2*>(row);
-    const ulonglong2 c2 = *reinterpret_cast<const ulonglong2*>(row + CLS_COPY2);
-    float q0, q1, q2, q3, a, b;
+                                           const uint32_t* tab, float scale) {
+    const ClsRow c = cls_row(tab, off);
+    float q0, q1, q2, q3, F1, F2;
     f2_split(z01, q0, q1);
     f2_split(z23, q2, q3);
-    f2_split(f2_fma(c1.y, z23, f2_mul(c1.x, z01)), a, b);
-    float F1 = a + b;
-    f2_split(f2_fma(c2.y, z23, f2_mul(c2.x, z01)), a, b);
-    float F2 = a + b;
-    const bool hh = off == 16u * NIB_HH, mm = off == 16u * NIB_MM;
+    cls_factors(c, z01, z23, F1, F2);
+    const bool hh = off == 8u * NIB_HH, mm = off == 8u * NIB_MM;
     const float den = fmaf(q1, q2, q0 * q3);
     F1 = hh ? den : F1;
     F1 = mm ? 1.f : F1;
@@ -244,11 +262,11 @@ __device__ __forceinline__ void pair_u_cls(unsigned off, uint64_t z01, uint64_t 
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r2) : "f"(F2));
     const uint64_t r1d = f2_dup(r1 * scale), r2d = f2_dup(r2 * scale);
     float x0, x1, x2, x3;
-    f2_split(c1.x, x0, x1);
-    f2_split(c1.y, x2, x3);
+    f2_split(c.a01, x0, x1);
+    f2_split(c.a23, x2, x3);
     const uint64_t s01 = f2_pack(hh ? q3 : x0, hh ? q2 : x1), s23 = f2_pack(hh ? q1 : x2, hh ? q0 : x3);
-    u01 = f2_fma(s01, r1d, f2_mul(c2.x, r2d));
-    u23 = f2_fma(s23, r1d, f2_mul(c2.y, r2d));
+    u01 = f2_fma(s01, r1d, f2_mul(c.b01, r2d));
+    u23 = f2_fma(s23, r1d, f2_mul(c.b23, r2d));
 }
 
 // Exact exponent/mantissa split used to accumulate products of likelihoods

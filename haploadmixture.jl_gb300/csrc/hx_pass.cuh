@@ -258,7 +258,8 @@ template <int K, int NU>
 __global__ void __launch_bounds__(ACC_THREADS)
 k_loglik2(PassArgs a) {
     __shared__ __align__(16) float spt[QSTAGE_WORDS * 8 * 4 * K];
-    __shared__ double red[ACC_THREADS];
+    __shared__ double red[ACC_THREADS / 32];
+    __shared__ long long rex[ACC_THREADS / 32];
     __shared__ float4 s_snp[4];
     const int tid = threadIdx.x;
     snp_table_init(s_snp, tid);
@@ -327,23 +328,46 @@ k_loglik2(PassArgs a) {
             }
         }
     }
-    double v = 0.0;
+    // the CTA's product, exponents apart, and one log (two FP64 logs per thread
+    // took 20% of the narrow FP64 unit at short chunks); padding individuals
+    // hold likelihoods of 1
+    double m = 1.0;
+    long long e = 0;
+    bool zero = false, bad = false;
 #pragma unroll
     for (int u = 0; u < NU; ++u) {
-        if (ii[u] < a.I) {
-            double x = log((double)mant[u]) + (double)ex[u] * 0.69314718055994530942;
-            if (lmin[u] == 0.f) x = -INFINITY;
-            if (lmin[u] < 0.f || chk[u] != chk[u]) x = NAN;
-            v += x;
+        m *= (double)mant[u];
+        e += ex[u];
+        zero |= lmin[u] == 0.f;
+        bad |= lmin[u] < 0.f || chk[u] != chk[u];
+    }
+    auto mul = [&](double y) {
+        int x = 0;
+        m = renorm(m * y, x);
+        e += x;
+    };
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double y = __shfl_xor_sync(0xffffffffu, m, o);
+        e += __shfl_xor_sync(0xffffffffu, e, o);
+        mul(y);
+    }
+    if ((tid & 31) == 0) {
+        red[tid >> 5] = m;
+        rex[tid >> 5] = e;
+    }
+    const bool any_zero = __syncthreads_or(zero), any_bad = __syncthreads_or(bad);
+    if (tid == 0) {
+#pragma unroll
+        for (int x = 1; x < ACC_THREADS / 32; ++x) {
+            mul(red[x]);
+            e += rex[x];
         }
+        double v = log(m) + (double)e * 0.69314718055994530942;
+        if (any_zero) v = -INFINITY;
+        if (any_bad) v = NAN;
+        a.part[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = v;
     }
-    red[tid] = v;
-    __syncthreads();
-    for (int s = ACC_THREADS / 2; s > 0; s >>= 1) {
-        if (tid < s) red[tid] += red[tid + s];
-        __syncthreads();
-    }
-    if (tid == 0) a.part[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = red[0];
 }
 
 }  // namespace hx

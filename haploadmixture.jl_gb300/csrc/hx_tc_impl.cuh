@@ -576,11 +576,11 @@ __device__ __forceinline__ void final_fold(Sync* sy, double* slots, long long bu
 // CTA's q tile by the stage's p tile into a double-buffered 32-column TMEM
 // tile, issued two stages ahead; each thread reads its row's 16 values.
 
-// One pair from its packed qp (byte offset off = 16 * class): U and W as packed
+// One pair from its packed qp (byte offset off = 8 * class): U and W as packed
 // pairs of haplotypes, both times U_SCALE.
 template <bool HESS>
 __device__ __forceinline__ void gen_pair_qp(unsigned off, uint64_t z01, uint64_t z23, uint64_t* U, uint64_t* W,
-                                            const float* tab) {
+                                            const uint32_t* tab) {
     pair_u_cls(off, z01, z23, U[0], U[1], tab, U_SCALE);
     if (HESS) {
         float q0, q1, q2, q3;
@@ -606,7 +606,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pass
     const uint32_t sRq = sR + RING * GBM;                            // ring [QRING][GBQ]
     uint32_t* SW = (uint32_t*)(smem + (sRq - sA) + QRING * GBQ);     // [RING][128]
     Sync* sy = (Sync*)(SW + RING * 128);
-    __shared__ __align__(16) float s_cls[128];
+    __shared__ __align__(128) uint32_t s_cls[32];
     const long long budget = a.budget;
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // uniform
@@ -717,9 +717,9 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pass
             uint32_t raw[16];
             tmem_ld8_async(taddr_lane + (uint32_t)(2 * D::WQ + b * 32 + hf * 16), raw);
             tmem_ld8_async(taddr_lane + (uint32_t)(2 * D::WQ + b * 32 + hf * 16 + 8), raw + 8);
-            // the half's four classes from bit 4 on: class bb times 16 is (word >> 4 bb) & 0xF0
+            // the half's four classes from bit 3 on: class bb times 8 is (word >> 4 bb) & 0x78
             word = SW[slot * 128 + r];
-            word = __funnelshift_r(word, word, (16 * hf + 28) & 31);
+            word = __funnelshift_r(word, word, (16 * hf + 29) & 31);
             tmem_wait_ld();
 #pragma unroll
             for (int t = 0; t < 16; ++t) qpv[t] = __uint_as_float(raw[t]);
@@ -731,7 +731,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pass
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int bb = 2 * t2 + e;                    // block within this thread's half
-                gen_pair_qp<HESS>((word >> (4 * bb)) & 0xF0u, f2_pack(qpv[4 * bb], qpv[4 * bb + 1]),
+                gen_pair_qp<HESS>((word >> (4 * bb)) & 0x78u, f2_pack(qpv[4 * bb], qpv[4 * bb + 1]),
                                   f2_pack(qpv[4 * bb + 2], qpv[4 * bb + 3]), U + 2 * e, W + 2 * e, s_cls);
             }
             const uint32_t off = (r >> 3) * SBO_STD + (hf * 2 + t2) * LBO_STD + (r & 7) * 16;
@@ -811,7 +811,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pass
 // in the order of the fmaf chain sum_k q_k p[k,m].
 template <int K, bool HESS>
 __device__ __forceinline__ void gen_pair(unsigned off, const uint64_t* qd, const uint64_t* pr2, float* U4, float* W4,
-                                         const float* tab) {
+                                         const uint32_t* tab) {
     uint64_t z01 = 0ull, z23 = 0ull;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
@@ -842,7 +842,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pass
     const uint32_t sR = sA + 2 * 4 * A_TILE_PAD;                     // ring [RING][GB]
     uint32_t* SW = (uint32_t*)(smem + (sR - sA) + RING * GB);        // [RING][4][KD]
     Sync* sy = (Sync*)(SW + RING * 4 * KD);
-    __shared__ __align__(16) float s_cls[128];
+    __shared__ __align__(128) uint32_t s_cls[32];
     const long long budget = a.budget;
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // uniform
@@ -900,7 +900,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pass
     for (int c = 0; c < D::HALF; ++c) acc[c] = 0.f;
 #pragma unroll
     for (int c = 0; c < D::NG; ++c) comp[c] = 0.f;
-    const int bsh = (4 * (jl & 7) + 28) & 31;     // rotates the block's class to bits 4 .. 7
+    const int bsh = (4 * (jl & 7) + 29) & 31;     // rotates the block's class to bits 3 .. 6
 
     for (int s = 0; s < ns; ++s) {
         const int b = s & 1, slot = s % RING;
@@ -917,8 +917,8 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pass
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int ii = ig * 4 + e;
-            // 16 * class
-            const unsigned off = valid ? __funnelshift_r(Ws[ii], Ws[ii], bsh) & 0xF0u : 16u * HX_PAD_NIBBLE;
+            // 8 * class
+            const unsigned off = valid ? __funnelshift_r(Ws[ii], Ws[ii], bsh) & 0x78u : 8u * HX_PAD_NIBBLE;
             uint64_t qd[(K + 1) / 2 * 2];
             const ulonglong2* q2 = reinterpret_cast<const ulonglong2*>(Qs + qrow_slot(ii) * QSTR);
 #pragma unroll
