@@ -47,7 +47,9 @@ namespace hx {
 namespace {
 using namespace tc;
 
-constexpr int TC_THREADS = 256;
+constexpr int TC_THREADS = 256;             // generating threads
+constexpr int TC_WARPS = TC_THREADS / 32;
+constexpr int TCQ_THREADS = TC_THREADS + 32;   // Q side: and a warp that copies and issues
 constexpr int TC_FLUSH = 8;                // stages per TMEM window (256 reduction indices)
 constexpr long long TC_BUDGET = 4000000000LL;
 constexpr int RING = 3;                    // stage-input ring depth
@@ -88,6 +90,7 @@ template <int K> struct TcDims {
     static constexpr int TCOLS_S = (2 * WS <= 32) ? 32 : (2 * WS <= 64) ? 64 : (2 * WS <= 128) ? 128 : (2 * WS <= 256) ? 256 : 512;
     // CTAs per SM: 2 while the generators fit in 128 registers, else 1
     static constexpr int MINB = K <= 8 ? 2 : 1;
+    static constexpr int MINB_Q = MINB;             // 96 registers at K <= 8, the limit of two CTAs of nine warps
 };
 
 // qp of the Q side from the tensor core (kind::tf32), see k_accum_q_tc.
@@ -132,6 +135,19 @@ struct Sync {
     int64_t gstride;       // words between word columns (Ipad)
     int nwc;               // word columns (P side)
     uint32_t tx;           // bytes per stage
+};
+
+// Q side
+struct SyncQ {
+    uint64_t full[RING];     // B tile landed
+    uint64_t fullq[QRING];   // p tile of the qp MMA landed
+    uint64_t fullw[QRING];   // class words landed
+    uint64_t go[2];          // stage may be generated: words here; qp and the MMAs of stage s-2 done
+    uint64_t gen[2];         // the generating warps have written stage buffer b (one arrival per warp)
+    uint64_t flush_done[2];  // an accumulator window is complete
+    uint64_t end;            // everything issued is done
+    uint32_t tslot;
+    int bad;
 };
 
 __device__ __forceinline__ bool is_bad(const Sync* sy) { return *(volatile const int*)&sy->bad != 0; }
@@ -591,8 +607,8 @@ __device__ __forceinline__ void gen_pair_qp(unsigned off, uint64_t z01, uint64_t
     }
 }
 
-template <int K, bool HESS>
-__global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_q_tc(PassArgs a) {
+template <int K>
+__global__ void __launch_bounds__(TCQ_THREADS, TcDims<K>::MINB_Q) k_accum_q_tc(PassArgs a) {
     using D = TcDims<K>;
     using QD = QpDims<K>;
     constexpr int GB = qimg_bytes<K>();
@@ -604,198 +620,211 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pass
     const uint32_t sAq = sA + 2 * 4 * A_TILE_STD;                    // [2 hi/lo][A_T]
     const uint32_t sR = sAq + 2 * QD::A_T;                           // ring [RING][GBM]
     const uint32_t sRq = sR + RING * GBM;                            // ring [QRING][GBQ]
-    uint32_t* SW = (uint32_t*)(smem + (sRq - sA) + QRING * GBQ);     // [RING][128]
-    Sync* sy = (Sync*)(SW + RING * 128);
+    uint32_t* SW = (uint32_t*)(smem + (sRq - sA) + QRING * GBQ);     // [QRING][128]
+    SyncQ* sy = (SyncQ*)(SW + QRING * 128);
     __shared__ __align__(128) uint32_t s_cls[32];
     const long long budget = a.budget;
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // uniform
     const int r = tid & 127, hf = tid >> 7;
     const int64_t i = (int64_t)blockIdx.x * 128 + r;
-    const bool active = i < a.I;
     const int w0 = blockIdx.y * a.per_chunk;
     const int ns = min(a.JW, w0 + a.per_chunk) - w0;     // one word per stage
     const int64_t i0 = (int64_t)blockIdx.x * 128;
     cls_table_init(s_cls, tid);
 
-    // stage t's inputs: the word column's B tile and the CTA's 128 class words;
-    // separately, 4 stages ahead, the tf32 p tile of its qp MMA
-    auto load_stage = [&](int t) {
-        const int slot = t % RING;
-        expect_tx(&sy->full[slot], (uint32_t)(GBM + 512));
-        bulk_copy(sR + slot * GBM, sy->img0 + (int64_t)t * GB, GBM, &sy->full[slot]);
-        bulk_copy(smem_u32(SW + slot * 128), sy->g0 + (int64_t)t * sy->gstride, 512, &sy->full[slot]);
-        atomicMax(&sy->loaded, t + 1);   // refills come from different warps
-    };
-    auto load_qtile = [&](int t) {
-        const int slot = t % QRING;
-        expect_tx(&sy->fullq[slot], (uint32_t)GBQ);
-        bulk_copy(sRq + slot * GBQ, sy->img0 + (int64_t)t * GB + GBM, GBQ, &sy->fullq[slot]);
-        atomicMax(&sy->loadedq, t + 1);
-    };
-
-    if (warp == 0) tmem_alloc<QD::TCOLS>(&sy->tslot);
-    init_sync(sy, tid, HESS ? 3 : 2, HESS ? 2 : 1);   // issuers: Hessian, gradient, qp
+    if (warp == TC_WARPS) tmem_alloc<QD::TCOLS>(&sy->tslot);
     if (tid == 0) {
-        sy->img0 = a.img + (int64_t)w0 * GB;
-        sy->g0 = a.G + (int64_t)w0 * a.Ipad + i0;
-        sy->gstride = a.Ipad;
+        for (int t = 0; t < RING; ++t) mbar_init(&sy->full[t], 1);
+        for (int t = 0; t < QRING; ++t) { mbar_init(&sy->fullq[t], 1); mbar_init(&sy->fullw[t], 1); }
+        for (int t = 0; t < 2; ++t) {
+            mbar_init(&sy->go[t], 2);
+            mbar_init(&sy->gen[t], TC_WARPS);
+            mbar_init(&sy->flush_done[t], 1);
+        }
+        mbar_init(&sy->end, 1);
+        sy->bad = 0;
+        mbar_fence_init();
     }
-    // zero the q tile (reduction padding k >= K stays zero)
-    for (int t = tid; t < (2 * QD::A_T) / 4; t += TC_THREADS)
-        asm volatile("st.shared.b32 [%0], %1;" :: "r"(sAq + 4 * t), "r"(0u) : "memory");
-    fence_before();
-    __syncthreads();
-    fence_after();
-    const uint32_t tmem = __shfl_sync(0xffffffffu, sy->tslot, 0);
-    const uint32_t tq = tmem + 2 * D::WQ;                 // qp tiles: columns [2WQ, 2WQ + 64)
-    const uint32_t taddr_lane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-    if (tid == 0) {
-        for (int t = 0; t < RING && t < ns; ++t) load_stage(t);
-        for (int t = 0; t < QRING && t < ns; ++t) load_qtile(t);
-    }
-
-    // q tile (tf32 hi/lo), once per CTA
-    if (hf == 0) {
+    // q tile (tf32 hi/lo), once per CTA; the reduction's padding k >= K is zero
+    if (tid < 128) {
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const float x = active ? (float)a.q[(int64_t)K * i + k] : 1.f / K;
+        for (int k = 0; k < QD::KP; ++k) {
+            const float x = k >= K ? 0.f : (i < a.I ? (float)a.q[(int64_t)K * i + k] : 1.f / K);
             const float hi = tf32_round(x), lo = tf32_round(x - hi);
             const uint32_t off = (r >> 3) * QD::SBO + (k >> 2) * 128 + (r & 7) * 16 + (k & 3) * 4;
             asm volatile("st.shared.b32 [%0], %1;" :: "r"(sAq + off), "f"(hi) : "memory");
             asm volatile("st.shared.b32 [%0], %1;" :: "r"(sAq + QD::A_T + off), "f"(lo) : "memory");
         }
     }
-    float acc[D::HALF], comp[D::NG];
-#pragma unroll
-    for (int c = 0; c < D::HALF; ++c) acc[c] = 0.f;
-#pragma unroll
-    for (int c = 0; c < D::NG; ++c) comp[c] = 0.f;
-
     fence_async_smem();
     fence_before();
     __syncthreads();
-    // qp of stages 0 and 1; stage t's qp is then issued at stage t-2
-    if (tid == 0) {
-        for (int t = 0; t < 2 && t < ns; ++t) {
-            if (!mbar_wait(&sy->fullq[t], 0, budget)) { set_bad(sy, a.slots); break; }
-            fence_after();
-            issue_qp<K>(tq + t * 32, sAq, sRq + t * GBQ, 1u);
-            commit(&sy->qp_done[t], 1u);
-        }
-    }
+    fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, sy->tslot, 0);
+    const uint32_t tq = tmem + 2 * D::WQ;                 // qp tiles: columns [2WQ, 2WQ + 64)
 
-    for (int s = 0; s < ns; ++s) {
-        const int b = s & 1, slot = s % RING;
-        if (!mbar_wait(&sy->full[slot], (s / RING) & 1, budget)) set_bad(sy, a.slots);
-        // A buffer b was last read by the MMAs of stage s-2
-        if (s >= 2 && !is_bad(sy))
-            if (!mbar_wait(&sy->mma_done[b], ((s - 2) >> 1) & 1, budget)) set_bad(sy, a.slots);
-        if (is_bad(sy)) break;
-        // ring refill: the slot of stage s-2 is free (its MMAs are done -- just
-        // waited for -- and they were issued after every thread had read it).
-        // The first warp here loads it, which keeps the refill off the last
-        // arriving warp of stage s-1 (the MMA issuer, still issuing).
-        // The qp tile slot of stage s is free too: its MMA (issued with the
-        // MMAs of stage s-2) is done.
-        if (s >= 2 && first_at_stage(&sy->started[b])) {
-            if (s - 2 + RING < ns) load_stage(s - 2 + RING);
-            if (s + QRING < ns) load_qtile(s + QRING);
-        }
-        // this stage's qp: 16 columns of this thread's row.  From stage 2 on it
-        // was issued with the MMAs of stage s-2 and is covered by their
-        // mma_done, just waited for; stages 0 and 1 wait for the prologue's.
-        // Both loads go out before one wait, with the class word read between.
-        float qpv[16];
-        uint32_t word;
-        {
-            if (s < 2) {
-                const bool ok = __all_sync(0xffffffffu, mbar_wait(&sy->qp_done[b], 0, budget));
-                if (!ok) { set_bad(sy, a.slots); break; }
-            }
+    if (warp == TC_WARPS) {
+        // ---- the issuing warp: all copies and MMAs of the CTA.  A generating
+        // warp that issued them was held until the tensor core took them (about
+        // 48 clocks per MMA however small, shared by the SM's two CTAs: 1,200
+        // clocks a stage), and the others waited for it.
+        const uint32_t el = elect_lane();
+        const uint8_t* img = a.img + (int64_t)w0 * GB;
+        const uint32_t* g = a.G + (int64_t)w0 * a.Ipad + i0;
+        auto load_b = [&](int t) {        // stage t's B tile
+            if (!el) return;
+            expect_tx(&sy->full[t % RING], (uint32_t)GBM);
+            bulk_copy(sR + (t % RING) * GBM, img + (int64_t)t * GB, GBM, &sy->full[t % RING]);
+        };
+        auto load_q = [&](int t) {        // the tf32 p tile of its qp MMA
+            if (!el) return;
+            expect_tx(&sy->fullq[t % QRING], (uint32_t)GBQ);
+            bulk_copy(sRq + (t % QRING) * GBQ, img + (int64_t)t * GB + GBM, GBQ, &sy->fullq[t % QRING]);
+        };
+        auto load_w = [&](int t) {        // its class words
+            if (!el) return;
+            expect_tx(&sy->fullw[t % QRING], 512u);
+            bulk_copy(smem_u32(SW + (t % QRING) * 128), g + (int64_t)t * a.Ipad, 512, &sy->fullw[t % QRING]);
+        };
+        auto wait = [&](uint64_t* bar, int phase) {
+            if (__all_sync(0xffffffffu, mbar_wait(bar, (uint32_t)(phase & 1), budget))) return true;
+            if (el) { *(volatile int*)&sy->bad = 1; a.slots[S_TC_TIMEOUT] = 1.0; }
+            return false;
+        };
+        int lb = 0, lq = 0;               // stages loaded: B tiles; p tiles and words
+        for (; lq < QRING && lq < ns; ++lq) { load_q(lq); load_w(lq); }
+        for (; lb < RING && lb < ns; ++lb) load_b(lb);
+        // stage t may start: its words are here, its qp and the MMAs of stage t-2
+        // (its A buffer) are done -- the second arrival comes from their commit
+        auto start = [&](int t) {
+            if (!wait(&sy->fullq[t % QRING], t / QRING)) return false;
             fence_after();
-            uint32_t raw[16];
-            tmem_ld8_async(taddr_lane + (uint32_t)(2 * D::WQ + b * 32 + hf * 16), raw);
-            tmem_ld8_async(taddr_lane + (uint32_t)(2 * D::WQ + b * 32 + hf * 16 + 8), raw + 8);
-            // the half's four classes from bit 3 on: class bb times 8 is (word >> 4 bb) & 0x78
-            word = SW[slot * 128 + r];
-            word = __funnelshift_r(word, word, (16 * hf + 29) & 31);
-            tmem_wait_ld();
-#pragma unroll
-            for (int t = 0; t < 16; ++t) qpv[t] = __uint_as_float(raw[t]);
+            issue_qp<K>(tq + (t & 1) * 32, sAq, sRq + (t % QRING) * GBQ, el);
+            commit(&sy->go[t & 1], el);
+            if (!wait(&sy->fullw[t % QRING], t / QRING)) return false;
+            if (el) mbar_arrive(&sy->go[t & 1]);
+            return true;
+        };
+        bool ok = true;
+        for (int t = 0; t < 2 && t < ns && ok; ++t) ok = start(t);
+        for (int s = 0; s < ns && ok; ++s) {
+            const int b = s & 1, slot = s % RING, d = (s / TC_FLUSH) & 1;
+            // every warp has written its part of stage s's A tiles, read its qp and words
+            ok = wait(&sy->gen[b], s >> 1) && wait(&sy->full[slot], s / RING);
+            if (!ok) break;
+            fence_after();
+            const bool first = (s % TC_FLUSH) == 0;
+            issue_stage_group<K, 0>(tmem, d * D::WQ, sA + b * 4 * A_TILE_STD, A_TILE_STD, LBO_STD, SBO_STD, sR + slot * GBM, first, el);
+            issue_stage_group<K, 1>(tmem, d * D::WQ, sA + b * 4 * A_TILE_STD, A_TILE_STD, LBO_STD, SBO_STD, sR + slot * GBM, first, el);
+            if ((s % TC_FLUSH) == TC_FLUSH - 1 || s == ns - 1) commit(&sy->flush_done[d], el);
+            // the slots of stage s's p tile and words are free, and that of stage
+            // s-2's B tile (every warp passed go for stage s)
+            if (lq < ns) { load_q(lq); load_w(lq); ++lq; }
+            if (s >= 2 && lb < ns) { load_b(lb); ++lb; }
+            if (s + 2 < ns) ok = start(s + 2);
         }
-        const uint32_t aB = sA + b * 4 * A_TILE_STD;
-#pragma unroll
-        for (int t2 = 0; t2 < 2; ++t2) {
-            uint64_t W[4], U[4];                              // haplotype pairs
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int bb = 2 * t2 + e;                    // block within this thread's half
-                gen_pair_qp<HESS>((word >> (4 * bb)) & 0x78u, f2_pack(qpv[4 * bb], qpv[4 * bb + 1]),
-                                  f2_pack(qpv[4 * bb + 2], qpv[4 * bb + 3]), U + 2 * e, W + 2 * e, s_cls);
+        // nothing of this warp's is left in flight when the CTA releases its memory
+        commit(&sy->end, el);
+        mbar_wait(&sy->end, 0u, TC_BUDGET);
+        if (!ok) {
+            for (int t = (lb >= RING ? lb - RING : 0); t < lb; ++t) mbar_wait(&sy->full[t % RING], (t / RING) & 1, TC_BUDGET);
+            for (int t = (lq >= QRING ? lq - QRING : 0); t < lq; ++t) {
+                mbar_wait(&sy->fullq[t % QRING], (t / QRING) & 1, TC_BUDGET);
+                mbar_wait(&sy->fullw[t % QRING], (t / QRING) & 1, TC_BUDGET);
             }
-            const uint32_t off = (r >> 3) * SBO_STD + (hf * 2 + t2) * LBO_STD + (r & 7) * 16;
-            uint32_t wh[4], wl[4], uh[4], ul[4];
+        }
+        __syncwarp();
+    } else {
+        const uint32_t taddr_lane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+        float acc[D::HALF], comp[D::NG];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                if (HESS) split2(W[e], wh[e], wl[e]);
-                split2_f16(U[e], uh[e], ul[e]);
+        for (int c = 0; c < D::HALF; ++c) acc[c] = 0.f;
+#pragma unroll
+        for (int c = 0; c < D::NG; ++c) comp[c] = 0.f;
+        bool ok = true;
+        for (int s = 0; s < ns; ++s) {
+            const int b = s & 1;
+            ok = __all_sync(0xffffffffu, mbar_wait(&sy->go[b], (s >> 1) & 1, budget));
+            if (!ok) break;
+            fence_after();
+            // this stage's qp: 16 columns of this thread's row; both loads go out
+            // before one wait, with the class word read between
+            float qpv[16];
+            uint32_t word;
+            {
+                uint32_t raw[16];
+                tmem_ld8_async(taddr_lane + (uint32_t)(2 * D::WQ + b * 32 + hf * 16), raw);
+                tmem_ld8_async(taddr_lane + (uint32_t)(2 * D::WQ + b * 32 + hf * 16 + 8), raw + 8);
+                // the half's four classes from bit 3 on: class bb times 8 is (word >> 4 bb) & 0x78
+                word = SW[(s % QRING) * 128 + r];
+                word = __funnelshift_r(word, word, (16 * hf + 29) & 31);
+                tmem_wait_ld();
+#pragma unroll
+                for (int t = 0; t < 16; ++t) qpv[t] = __uint_as_float(raw[t]);
             }
-            if (HESS) {
+            const uint32_t aB = sA + b * 4 * A_TILE_STD;
+#pragma unroll
+            for (int t2 = 0; t2 < 2; ++t2) {
+                uint64_t W[4], U[4];                              // haplotype pairs
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int bb = 2 * t2 + e;                    // block within this thread's half
+                    gen_pair_qp<true>((word >> (4 * bb)) & 0x78u, f2_pack(qpv[4 * bb], qpv[4 * bb + 1]),
+                                      f2_pack(qpv[4 * bb + 2], qpv[4 * bb + 3]), U + 2 * e, W + 2 * e, s_cls);
+                }
+                const uint32_t off = (r >> 3) * SBO_STD + (hf * 2 + t2) * LBO_STD + (r & 7) * 16;
+                uint32_t wh[4], wl[4], uh[4], ul[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    split2(W[e], wh[e], wl[e]);
+                    split2_f16(U[e], uh[e], ul[e]);
+                }
                 sts128(aB + off, wh[0], wh[1], wh[2], wh[3]);
                 sts128(aB + A_TILE_STD + off, wl[0], wl[1], wl[2], wl[3]);
+                sts128(aB + 2 * A_TILE_STD + off, uh[0], uh[1], uh[2], uh[3]);
+                sts128(aB + 3 * A_TILE_STD + off, ul[0], ul[1], ul[2], ul[3]);
             }
-            sts128(aB + 2 * A_TILE_STD + off, uh[0], uh[1], uh[2], uh[3]);
-            sts128(aB + 3 * A_TILE_STD + off, ul[0], ul[1], ul[2], ul[3]);
-        }
-        arrive_generated(sy, b);
-        // Three issuers, warps 0, 2 and 4 (one elected lane each), each with its own
-        // TMEM columns: the Hessian MMAs, the gradient MMAs, and the qp MMA of stage
-        // s+2 into this stage's qp columns (every thread has read them).  Each
-        // commits to mma_done, which therefore also covers the qp MMA.
-        if (warp == 2 || warp == 4 || (HESS && warp == 0)) {
-            if (wait_generated(sy, s, b, a.slots, budget)) {
-                const uint32_t el = elect_lane();
-                const int d = (s / TC_FLUSH) & 1;
-                if (warp == 4) {
-                    if (s + 2 < ns) {
-                        const int qs = (s + 2) % QRING;
-                        if (!__all_sync(0xffffffffu, mbar_wait(&sy->fullq[qs], ((s + 2) / QRING) & 1, budget)))
-                            set_bad(sy, a.slots);
-                        else issue_qp<K>(tq + b * 32, sAq, sRq + qs * GBQ, el);
-                    }
-                    commit_stage(sy, s, ns, b, el, false);
-                    // the qp tile slots of stages 0 and 1 (their MMAs came from the
-                    // prologue, every thread waited for them); later ones are
-                    // refilled by the first warp of the stage
-                    if (el && s < 2 && s + QRING < ns) load_qtile(s + QRING);
-                } else {
-                    const bool first = (s % TC_FLUSH) == 0;
-                    if (warp == 0)
-                        issue_stage_group<K, 0>(tmem, d * D::WQ, aB, A_TILE_STD, LBO_STD, SBO_STD, sR + slot * GBM, first, el);
-                    else
-                        issue_stage_group<K, 1>(tmem, d * D::WQ, aB, A_TILE_STD, LBO_STD, SBO_STD, sR + slot * GBM, first, el);
-                    commit_stage(sy, s, ns, b, el);
-                }
-            }
+            fence_async_smem();
+            fence_before();
             __syncwarp();
+            if ((tid & 31) == 0) mbar_arrive(&sy->gen[b]);
+            // window fold, see FOLD_OFF
+            if (s >= TC_FLUSH + FOLD_OFF && (s - FOLD_OFF) % TC_FLUSH == 0) {
+                const int wp = (s - FOLD_OFF) / TC_FLUSH - 1;
+                ok = __all_sync(0xffffffffu, mbar_wait(&sy->flush_done[wp & 1], (wp >> 1) & 1, budget));
+                if (!ok) break;
+                fence_after();
+                fold_half<K, false>(hf, taddr_lane, (wp & 1) * D::WQ, acc, comp);
+                fence_before();
+            }
         }
-        maybe_fold<K, false>(sy, a.slots, budget, hf, s, taddr_lane, acc, comp);
-    }
-    final_fold<K, false>(sy, a.slots, budget, hf, ns, taddr_lane, acc, comp);
-    // write partials: v < K gradient, v = K + tri index Hessian
-    constexpr int NV = K + (HESS ? D::NH : 0);
-    double* out = a.part + (int64_t)blockIdx.y * NV * a.Ipad;
+        if (ok && ns > 0) {
+            // windows not folded in the loop: the last one and possibly the one before
+            const int wl = (ns - 1) / TC_FLUSH;
+            for (int w = ns - 1 >= FOLD_OFF ? (ns - 1 - FOLD_OFF) / TC_FLUSH : 0; w <= wl && ok; ++w) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&sy->flush_done[w & 1], (w >> 1) & 1, budget));
+                if (!ok) break;
+                fence_after();
+                fold_half<K, false>(hf, taddr_lane, (w & 1) * D::WQ, acc, comp);
+            }
+        }
+        if (!ok) { *(volatile int*)&sy->bad = 1; a.slots[S_TC_TIMEOUT] = 1.0; }
+        fence_before();
+        if (hf == 0) compensate<K, 0>(acc, comp);
+        else compensate<K, 1>(acc, comp);
+        // write partials: v < K gradient, v = K + tri index Hessian
+        constexpr int NV = K + D::NH;
+        double* out = a.part + (int64_t)blockIdx.y * NV * a.Ipad;
 #pragma unroll
-    for (int c = 0; c < D::HALF; ++c) {
-        const int col = hf * D::HALF + c;
-        if (col < D::NH) {
-            if (HESS) out[(int64_t)(K + col) * a.Ipad + i] = (double)acc[c];
-        } else if (col >= D::NHP && col < D::NHP + K) {
-            out[(int64_t)(col - D::NHP) * a.Ipad + i] = (double)acc[c] * G_UNSCALE;
+        for (int c = 0; c < D::HALF; ++c) {
+            const int col = hf * D::HALF + c;
+            if (col < D::NH) out[(int64_t)(K + col) * a.Ipad + i] = (double)acc[c];
+            else if (col >= D::NHP && col < D::NHP + K) out[(int64_t)(col - D::NHP) * a.Ipad + i] = (double)acc[c] * G_UNSCALE;
         }
     }
-    if (warp == 0) {
+    __syncthreads();
+    if (warp == TC_WARPS) {
         fence_after();
         tmem_dealloc<QD::TCOLS>(tmem);
     }
@@ -1002,7 +1031,7 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pass
 template <int K> constexpr size_t smem_q() {
     using QD = QpDims<K>;
     return 1024 + 2 * 4 * A_TILE_STD + 2 * QD::A_T + RING * 2 * TcDims<K>::B_TILE + QRING * 2 * QD::B_T +
-           RING * 128 * 4 + sizeof(Sync);
+           QRING * 128 * 4 + sizeof(SyncQ);
 }
 template <int K> constexpr size_t smem_p() {
     return 1024 + 2 * 4 * A_TILE_PAD + RING * pimg_bytes<K>() + RING * 4 * KD * 4 + sizeof(Sync);
@@ -1013,11 +1042,8 @@ template <int K>
 cudaError_t tc_run(TcCall& c) {
     switch (c.op) {
     case TC_ATTRS: {
-        cudaError_t e = cudaFuncSetAttribute(k_accum_q_tc<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(k_accum_q_tc<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem_q<K>());
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_accum_q_tc<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem_q<K>());
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k_accum_p_tc<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem_p<K>());
@@ -1027,7 +1053,7 @@ cudaError_t tc_run(TcCall& c) {
         return e;
     }
     case TC_RESIDENT_Q:
-        c.bytes = (size_t)resident_ctas((const void*)k_accum_q_tc<K, true>, TC_THREADS, smem_q<K>(), QpDims<K>::TCOLS);
+        c.bytes = (size_t)TcDims<K>::MINB_Q;
         return cudaSuccess;
     case TC_RESIDENT_P:
         c.bytes = (size_t)resident_ctas((const void*)k_accum_p_tc<K, true>, TC_THREADS, smem_p<K>(), TcDims<K>::TCOLS_S);
@@ -1042,8 +1068,7 @@ cudaError_t tc_run(TcCall& c) {
         const unsigned gi = (unsigned)(((int64_t)a.JW * 4 + 127) / 128);
         dim3 grid((unsigned)(a.Ipad / 128), (unsigned)a.S);
         k_qimg<K><<<gi, 128, 0, c.st>>>(a.p, a.J, a.JW, a.img);
-        if (c.hess) k_accum_q_tc<K, true><<<grid, TC_THREADS, smem_q<K>(), c.st>>>(a);
-        else k_accum_q_tc<K, false><<<grid, TC_THREADS, smem_q<K>(), c.st>>>(a);
+        k_accum_q_tc<K><<<grid, TCQ_THREADS, smem_q<K>(), c.st>>>(a);
         return cudaGetLastError();
     }
     case TC_P: {
