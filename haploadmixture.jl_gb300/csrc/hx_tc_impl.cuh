@@ -49,11 +49,11 @@ using namespace tc;
 
 constexpr int TC_THREADS = 256;             // generating threads
 constexpr int TC_WARPS = TC_THREADS / 32;
-constexpr int TCQ_THREADS = TC_THREADS + 32;   // Q side: and a warp that copies and issues
+constexpr int TCI_THREADS = TC_THREADS + 32;   // and a warp that copies and issues
 constexpr int TC_FLUSH = 8;                // stages per TMEM window (256 reduction indices)
 constexpr long long TC_BUDGET = 4000000000LL;
 constexpr int RING = 3;                    // stage-input ring depth
-constexpr int QRING = 4;                   // Q side: ring of the qp MMA's p tiles, loaded 4 stages ahead
+constexpr int IRING = 4;                   // ring of what the generators read (words, qp tiles or q rows)
 constexpr int KD = 32;                     // reduction indices per stage
 constexpr int LBO_STD = 128;
 constexpr int SBO_STD = (KD / 8) * LBO_STD;      // 512
@@ -90,7 +90,6 @@ template <int K> struct TcDims {
     static constexpr int TCOLS_S = (2 * WS <= 32) ? 32 : (2 * WS <= 64) ? 64 : (2 * WS <= 128) ? 128 : (2 * WS <= 256) ? 256 : 512;
     // CTAs per SM: 2 while the generators fit in 128 registers, else 1
     static constexpr int MINB = K <= 8 ? 2 : 1;
-    static constexpr int MINB_Q = MINB;             // 96 registers at K <= 8, the limit of two CTAs of nine warps
 };
 
 // qp of the Q side from the tensor core (kind::tf32), see k_accum_q_tc.
@@ -115,34 +114,11 @@ __host__ __device__ constexpr int qrow_slot(int ii) { return 8 * (ii & 3) + (ii 
 template <int K> constexpr int qimg_bytes() { return 2 * TcDims<K>::B_TILE + 2 * QpDims<K>::B_T; }
 template <int K> constexpr int pimg_bytes() { return 2 * TcDims<K>::B_TILE + KD * qstr<K>() * 4; }
 
-struct Sync {
-    uint64_t full[RING];   // stage inputs landed (transaction-count barrier)
-    uint64_t fullq[QRING]; // Q side: p tile of the qp MMA landed
-    uint64_t mma_done[2];
-    uint64_t flush_done[2];
-    uint64_t qp_done[2];
-    uint64_t gen_full[2];  // the 8 generator warps have written stage buffer b (one arrival per warp)
-    uint32_t tslot;
-    int bad;
-    int issued;            // stages whose MMAs have been issued
-    int loaded;            // stages whose input copies have been issued
-    int loadedq;           // Q side: stages whose qp p tile copy has been issued
-    uint32_t arrived[2];   // generator arrivals on stage buffer b (monotonic)
-    uint32_t started[2];   // warps past the waits of a stage, by stage parity (the first one refills)
-    // stage-input sources, read only by the thread that issues a refill
-    const uint8_t* img0;   // image slice of stage 0
-    const uint32_t* g0;    // class words of stage 0
-    int64_t gstride;       // words between word columns (Ipad)
-    int nwc;               // word columns (P side)
-    uint32_t tx;           // bytes per stage
-};
-
-// Q side
-struct SyncQ {
-    uint64_t full[RING];     // B tile landed
-    uint64_t fullq[QRING];   // p tile of the qp MMA landed
-    uint64_t fullw[QRING];   // class words landed
-    uint64_t go[2];          // stage may be generated: words here; qp and the MMAs of stage s-2 done
+struct SyncI {
+    uint64_t full[RING];     // B tile landed (transaction-count barrier)
+    uint64_t fullq[IRING];   // Q side: p tile of the qp MMA landed
+    uint64_t fullw[IRING];   // class words (P side: and q rows) landed
+    uint64_t go[2];          // stage may be generated: its inputs are here, the MMAs of stage s-2 (its A buffer) done
     uint64_t gen[2];         // the generating warps have written stage buffer b (one arrival per warp)
     uint64_t flush_done[2];  // an accumulator window is complete
     uint64_t end;            // everything issued is done
@@ -150,56 +126,24 @@ struct SyncQ {
     int bad;
 };
 
-__device__ __forceinline__ bool is_bad(const Sync* sy) { return *(volatile const int*)&sy->bad != 0; }
-
-// Arrival on the stage buffer, one atomic per warp: after __syncwarp (which
-// orders the warp's tile stores, each already fenced to the async proxy), lane
-// 0 adds to the buffer's counter; all lanes of the last of the TC_THREADS/32
-// warps of this use of the buffer return true (the counter only grows, so no
-// reset races with the next use).  Release/acquire ordering of the atomic makes
-// every warp's stores visible to the MMAs that the last arriver issues.
-__device__ __forceinline__ bool arrive_last(uint32_t* ctr) {
-    __syncwarp();
-    bool last = false;
-    if ((threadIdx.x & 31) == 0) {
-        uint32_t old;
-        asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(old) : "r"(smem_u32(ctr)) : "memory");
-        last = (old % (TC_THREADS / 32)) == TC_THREADS / 32 - 1;
+__device__ __forceinline__ void sync_init(SyncI* sy) {
+    for (int t = 0; t < RING; ++t) mbar_init(&sy->full[t], 1);
+    for (int t = 0; t < IRING; ++t) { mbar_init(&sy->fullq[t], 1); mbar_init(&sy->fullw[t], 1); }
+    for (int t = 0; t < 2; ++t) {
+        mbar_init(&sy->go[t], 2);          // the inputs; the MMAs' commit
+        mbar_init(&sy->gen[t], TC_WARPS);
+        mbar_init(&sy->flush_done[t], 1);
     }
-    return __any_sync(0xffffffffu, last);
+    mbar_init(&sy->end, 1);
+    sy->bad = 0;
+    mbar_fence_init();
 }
-
-// True in lane 0 of the first warp of the CTA to reach this point of a stage
-// (one atomic per warp).  Counted by stage parity like arrive_last: a warp
-// reaches stage s+2 only after every warp has passed this point of stage s.
-__device__ __forceinline__ bool first_at_stage(uint32_t* ctr) {
-    __syncwarp();
-    bool first = false;
-    if ((threadIdx.x & 31) == 0) {
-        uint32_t old;
-        asm volatile("atom.relaxed.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(old) : "r"(smem_u32(ctr)) : "memory");
-        first = (old % (TC_THREADS / 32)) == 0;
-    }
-    return first;
-}
-
-__device__ __forceinline__ void set_bad(Sync* sy, double* slots) {
-    *(volatile int*)&sy->bad = 1;
-    if (slots) slots[S_TC_TIMEOUT] = 1.0;
-}
-
-// After a timeout: wait (bounded) until the MMAs of the last two issued stages
-// and the bulk copies of the last RING loaded stages have completed, so that
-// TMEM and shared memory are not released under them.  Only operations that
-// were issued are waited for, so each wait ends as soon as the hardware does.
-__device__ __forceinline__ void drain(Sync* sy) {
-    __syncthreads();
-    if (!is_bad(sy)) return;
-    const int n = sy->issued, l = sy->loaded, lq = sy->loadedq;
-    for (int s = (n >= 2 ? n - 2 : 0); s < n; ++s) mbar_wait(&sy->mma_done[s & 1], (s >> 1) & 1, TC_BUDGET);
-    for (int s = (l >= RING ? l - RING : 0); s < l; ++s) mbar_wait(&sy->full[s % RING], (s / RING) & 1, TC_BUDGET);
-    for (int s = (lq >= QRING ? lq - QRING : 0); s < lq; ++s)
-        mbar_wait(&sy->fullq[s % QRING], (s / QRING) & 1, TC_BUDGET);
+// A wait of the issuing warp; on timeout it records the fact.
+__device__ __forceinline__ bool wait_or_bad(SyncI* sy, uint64_t* bar, int phase, double* slots, long long budget,
+                                            uint32_t el) {
+    if (__all_sync(0xffffffffu, mbar_wait(bar, (uint32_t)(phase & 1), budget))) return true;
+    if (el) { *(volatile int*)&sy->bad = 1; slots[S_TC_TIMEOUT] = 1.0; }
+    return false;
 }
 
 // TMEM window fold: this thread's lane, columns [HF*HALF, HF*HALF + HALF) of the
@@ -485,28 +429,6 @@ __global__ void __launch_bounds__(128) k_pimg(const double* __restrict__ q, int6
 }
 
 // ------------------------------------------------------------------ shared helpers
-// n_mma: issuers that commit each stage to mma_done; n_flush: those that
-// commit each accumulator window to flush_done
-__device__ __forceinline__ void init_sync(Sync* sy, int tid, int n_mma, int n_flush) {
-    if (tid == 0) {
-        for (int r = 0; r < RING; ++r) mbar_init(&sy->full[r], 1);
-        for (int r = 0; r < QRING; ++r) mbar_init(&sy->fullq[r], 1);
-        sy->loadedq = 0;
-        mbar_init(&sy->mma_done[0], n_mma); mbar_init(&sy->mma_done[1], n_mma);
-        mbar_init(&sy->flush_done[0], n_flush); mbar_init(&sy->flush_done[1], n_flush);
-        mbar_init(&sy->gen_full[0], TC_THREADS / 32); mbar_init(&sy->gen_full[1], TC_THREADS / 32);
-        mbar_init(&sy->qp_done[0], 1); mbar_init(&sy->qp_done[1], 1);
-        sy->bad = 0;
-        sy->issued = 0;
-        sy->loaded = 0;
-        sy->arrived[0] = 0;
-        sy->arrived[1] = 0;
-        sy->started[0] = 0;
-        sy->started[1] = 0;
-        mbar_fence_init();
-    }
-}
-
 __device__ __forceinline__ void expect_tx(uint64_t* mbar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(smem_u32(mbar)), "r"(bytes) : "memory");
 }
@@ -515,27 +437,13 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_
                  :: "r"(dst), "l"(src), "r"(bytes), "r"(smem_u32(mbar)) : "memory");
 }
 
-// Window bookkeeping after a stage's MMAs were issued by this warp's elected lane.
-__device__ __forceinline__ void commit_stage(Sync* sy, int s, int ns, int b, uint32_t el, bool window = true) {
-    const int d = (s / TC_FLUSH) & 1;
-    commit(&sy->mma_done[b], el);
-    if (window && ((s % TC_FLUSH) == TC_FLUSH - 1 || s == ns - 1)) commit(&sy->flush_done[d], el);
-    if (el) atomicMax(&sy->issued, s + 1);
-}
-
-// Every generator warp has written its part of stage s's A tiles (buffer b):
+// Every generator warp has written its part of the stage's A tiles (buffer b):
 // one arrival per warp, after the tiles are made visible to the tensor core.
-__device__ __forceinline__ void arrive_generated(Sync* sy, int b) {
+__device__ __forceinline__ void arrive_generated(SyncI* sy, int b) {
     fence_async_smem();
     fence_before();
     __syncwarp();
-    if ((threadIdx.x & 31) == 0) mbar_arrive(&sy->gen_full[b]);
-}
-// An issuing warp waits until the whole stage is generated.
-__device__ __forceinline__ bool wait_generated(Sync* sy, int s, int b, double* slots, long long budget) {
-    if (!__all_sync(0xffffffffu, mbar_wait(&sy->gen_full[b], (s >> 1) & 1, budget))) { set_bad(sy, slots); return false; }
-    fence_after();
-    return true;
+    if ((threadIdx.x & 31) == 0) mbar_arrive(&sy->gen[b]);
 }
 
 // Fold of TMEM window w at stage (w+1)*TC_FLUSH + FOLD_OFF: half a window
@@ -544,44 +452,31 @@ __device__ __forceinline__ bool wait_generated(Sync* sy, int s, int b, double* s
 // once every thread has arrived there).
 constexpr int FOLD_OFF = TC_FLUSH / 2;
 template <int K, bool STACK>
-__device__ __forceinline__ void maybe_fold(Sync* sy, double* slots, long long budget, int hf, int s, uint32_t taddr_lane, float* acc,
-                                           float* comp) {
+__device__ __forceinline__ bool fold_window(SyncI* sy, long long budget, int hf, int w, uint32_t taddr_lane, float* acc,
+                                            float* comp) {
     using D = TcDims<K>;
     constexpr int WC = STACK ? D::WS : D::WQ;   // TMEM columns per window
-    if (s >= TC_FLUSH + FOLD_OFF && (s - FOLD_OFF) % TC_FLUSH == 0) {
-        const int wp = (s - FOLD_OFF) / TC_FLUSH - 1;
-        const bool ok = __all_sync(0xffffffffu, mbar_wait(&sy->flush_done[wp & 1], (wp >> 1) & 1, budget));
-        if (!ok) set_bad(sy, slots);
-        else {
-            fence_after();
-            fold_half<K, STACK>(hf, taddr_lane, (wp & 1) * WC, acc, comp);
-        }
-        fence_before();
-    }
-}
-
-template <int K, bool STACK>
-__device__ __forceinline__ void final_fold(Sync* sy, double* slots, long long budget, int hf, int ns, uint32_t taddr_lane, float* acc,
-                                           float* comp) {
-    using D = TcDims<K>;
-    constexpr int WC = STACK ? D::WS : D::WQ;
-    __syncthreads();
-    if (ns > 0 && !is_bad(sy)) {
-        // windows not folded in the loop: the last one and possibly the one before
-        const int wl = (ns - 1) / TC_FLUSH;
-        const int nf = ns - 1 >= FOLD_OFF ? (ns - 1 - FOLD_OFF) / TC_FLUSH : 0;
-        for (int w = nf; w <= wl; ++w) {
-            const bool ok = __all_sync(0xffffffffu, mbar_wait(&sy->flush_done[w & 1], (w >> 1) & 1, budget));
-            if (!ok) { set_bad(sy, slots); break; }
-            fence_after();
-            fold_half<K, STACK>(hf, taddr_lane, (w & 1) * WC, acc, comp);
-        }
-    }
-    drain(sy);
+    if (!__all_sync(0xffffffffu, mbar_wait(&sy->flush_done[w & 1], (w >> 1) & 1, budget))) return false;
+    fence_after();
+    fold_half<K, STACK>(hf, taddr_lane, (w & 1) * WC, acc, comp);
     fence_before();
-    __syncthreads();
-    if (hf == 0) compensate<K, 0>(acc, comp);
-    else compensate<K, 1>(acc, comp);
+    return true;
+}
+template <int K, bool STACK>
+__device__ __forceinline__ bool maybe_fold(SyncI* sy, long long budget, int hf, int s, uint32_t taddr_lane, float* acc,
+                                           float* comp) {
+    if (s < TC_FLUSH + FOLD_OFF || (s - FOLD_OFF) % TC_FLUSH != 0) return true;
+    return fold_window<K, STACK>(sy, budget, hf, (s - FOLD_OFF) / TC_FLUSH - 1, taddr_lane, acc, comp);
+}
+// Windows not folded in the loop: the last one and possibly the one before.
+template <int K, bool STACK>
+__device__ __forceinline__ bool final_fold(SyncI* sy, long long budget, int hf, int ns, uint32_t taddr_lane, float* acc,
+                                           float* comp) {
+    bool ok = true;
+    if (ns > 0)
+        for (int w = ns - 1 >= FOLD_OFF ? (ns - 1 - FOLD_OFF) / TC_FLUSH : 0; w <= (ns - 1) / TC_FLUSH && ok; ++w)
+            ok = fold_window<K, STACK>(sy, budget, hf, w, taddr_lane, acc, comp);
+    return ok;
 }
 
 // ------------------------------------------------------------------ Q side
@@ -608,7 +503,7 @@ __device__ __forceinline__ void gen_pair_qp(unsigned off, uint64_t z01, uint64_t
 }
 
 template <int K>
-__global__ void __launch_bounds__(TCQ_THREADS, TcDims<K>::MINB_Q) k_accum_q_tc(PassArgs a) {
+__global__ void __launch_bounds__(TCI_THREADS, TcDims<K>::MINB) k_accum_q_tc(PassArgs a) {
     using D = TcDims<K>;
     using QD = QpDims<K>;
     constexpr int GB = qimg_bytes<K>();
@@ -619,9 +514,9 @@ __global__ void __launch_bounds__(TCQ_THREADS, TcDims<K>::MINB_Q) k_accum_q_tc(P
     constexpr int GBQ = 2 * QD::B_T;                                 // qp ring slot: tf32 p tile
     const uint32_t sAq = sA + 2 * 4 * A_TILE_STD;                    // [2 hi/lo][A_T]
     const uint32_t sR = sAq + 2 * QD::A_T;                           // ring [RING][GBM]
-    const uint32_t sRq = sR + RING * GBM;                            // ring [QRING][GBQ]
-    uint32_t* SW = (uint32_t*)(smem + (sRq - sA) + QRING * GBQ);     // [QRING][128]
-    SyncQ* sy = (SyncQ*)(SW + QRING * 128);
+    const uint32_t sRq = sR + RING * GBM;                            // ring [IRING][GBQ]
+    uint32_t* SW = (uint32_t*)(smem + (sRq - sA) + IRING * GBQ);     // [IRING][128]
+    SyncI* sy = (SyncI*)(SW + IRING * 128);
     __shared__ __align__(128) uint32_t s_cls[32];
     const long long budget = a.budget;
 
@@ -634,18 +529,7 @@ __global__ void __launch_bounds__(TCQ_THREADS, TcDims<K>::MINB_Q) k_accum_q_tc(P
     cls_table_init(s_cls, tid);
 
     if (warp == TC_WARPS) tmem_alloc<QD::TCOLS>(&sy->tslot);
-    if (tid == 0) {
-        for (int t = 0; t < RING; ++t) mbar_init(&sy->full[t], 1);
-        for (int t = 0; t < QRING; ++t) { mbar_init(&sy->fullq[t], 1); mbar_init(&sy->fullw[t], 1); }
-        for (int t = 0; t < 2; ++t) {
-            mbar_init(&sy->go[t], 2);
-            mbar_init(&sy->gen[t], TC_WARPS);
-            mbar_init(&sy->flush_done[t], 1);
-        }
-        mbar_init(&sy->end, 1);
-        sy->bad = 0;
-        mbar_fence_init();
-    }
+    if (tid == 0) sync_init(sy);
     // q tile (tf32 hi/lo), once per CTA; the reduction's padding k >= K is zero
     if (tid < 128) {
 #pragma unroll
@@ -679,30 +563,26 @@ __global__ void __launch_bounds__(TCQ_THREADS, TcDims<K>::MINB_Q) k_accum_q_tc(P
         };
         auto load_q = [&](int t) {        // the tf32 p tile of its qp MMA
             if (!el) return;
-            expect_tx(&sy->fullq[t % QRING], (uint32_t)GBQ);
-            bulk_copy(sRq + (t % QRING) * GBQ, img + (int64_t)t * GB + GBM, GBQ, &sy->fullq[t % QRING]);
+            expect_tx(&sy->fullq[t % IRING], (uint32_t)GBQ);
+            bulk_copy(sRq + (t % IRING) * GBQ, img + (int64_t)t * GB + GBM, GBQ, &sy->fullq[t % IRING]);
         };
         auto load_w = [&](int t) {        // its class words
             if (!el) return;
-            expect_tx(&sy->fullw[t % QRING], 512u);
-            bulk_copy(smem_u32(SW + (t % QRING) * 128), g + (int64_t)t * a.Ipad, 512, &sy->fullw[t % QRING]);
+            expect_tx(&sy->fullw[t % IRING], 512u);
+            bulk_copy(smem_u32(SW + (t % IRING) * 128), g + (int64_t)t * a.Ipad, 512, &sy->fullw[t % IRING]);
         };
-        auto wait = [&](uint64_t* bar, int phase) {
-            if (__all_sync(0xffffffffu, mbar_wait(bar, (uint32_t)(phase & 1), budget))) return true;
-            if (el) { *(volatile int*)&sy->bad = 1; a.slots[S_TC_TIMEOUT] = 1.0; }
-            return false;
-        };
+        auto wait = [&](uint64_t* bar, int phase) { return wait_or_bad(sy, bar, phase, a.slots, budget, el); };
         int lb = 0, lq = 0;               // stages loaded: B tiles; p tiles and words
-        for (; lq < QRING && lq < ns; ++lq) { load_q(lq); load_w(lq); }
+        for (; lq < IRING && lq < ns; ++lq) { load_q(lq); load_w(lq); }
         for (; lb < RING && lb < ns; ++lb) load_b(lb);
         // stage t may start: its words are here, its qp and the MMAs of stage t-2
         // (its A buffer) are done -- the second arrival comes from their commit
         auto start = [&](int t) {
-            if (!wait(&sy->fullq[t % QRING], t / QRING)) return false;
+            if (!wait(&sy->fullq[t % IRING], t / IRING)) return false;
             fence_after();
-            issue_qp<K>(tq + (t & 1) * 32, sAq, sRq + (t % QRING) * GBQ, el);
+            issue_qp<K>(tq + (t & 1) * 32, sAq, sRq + (t % IRING) * GBQ, el);
             commit(&sy->go[t & 1], el);
-            if (!wait(&sy->fullw[t % QRING], t / QRING)) return false;
+            if (!wait(&sy->fullw[t % IRING], t / IRING)) return false;
             if (el) mbar_arrive(&sy->go[t & 1]);
             return true;
         };
@@ -729,9 +609,9 @@ __global__ void __launch_bounds__(TCQ_THREADS, TcDims<K>::MINB_Q) k_accum_q_tc(P
         mbar_wait(&sy->end, 0u, TC_BUDGET);
         if (!ok) {
             for (int t = (lb >= RING ? lb - RING : 0); t < lb; ++t) mbar_wait(&sy->full[t % RING], (t / RING) & 1, TC_BUDGET);
-            for (int t = (lq >= QRING ? lq - QRING : 0); t < lq; ++t) {
-                mbar_wait(&sy->fullq[t % QRING], (t / QRING) & 1, TC_BUDGET);
-                mbar_wait(&sy->fullw[t % QRING], (t / QRING) & 1, TC_BUDGET);
+            for (int t = (lq >= IRING ? lq - IRING : 0); t < lq; ++t) {
+                mbar_wait(&sy->fullq[t % IRING], (t / IRING) & 1, TC_BUDGET);
+                mbar_wait(&sy->fullw[t % IRING], (t / IRING) & 1, TC_BUDGET);
             }
         }
         __syncwarp();
@@ -757,7 +637,7 @@ __global__ void __launch_bounds__(TCQ_THREADS, TcDims<K>::MINB_Q) k_accum_q_tc(P
                 tmem_ld8_async(taddr_lane + (uint32_t)(2 * D::WQ + b * 32 + hf * 16), raw);
                 tmem_ld8_async(taddr_lane + (uint32_t)(2 * D::WQ + b * 32 + hf * 16 + 8), raw + 8);
                 // the half's four classes from bit 3 on: class bb times 8 is (word >> 4 bb) & 0x78
-                word = SW[(s % QRING) * 128 + r];
+                word = SW[(s % IRING) * 128 + r];
                 word = __funnelshift_r(word, word, (16 * hf + 29) & 31);
                 tmem_wait_ld();
 #pragma unroll
@@ -785,30 +665,11 @@ __global__ void __launch_bounds__(TCQ_THREADS, TcDims<K>::MINB_Q) k_accum_q_tc(P
                 sts128(aB + 2 * A_TILE_STD + off, uh[0], uh[1], uh[2], uh[3]);
                 sts128(aB + 3 * A_TILE_STD + off, ul[0], ul[1], ul[2], ul[3]);
             }
-            fence_async_smem();
-            fence_before();
-            __syncwarp();
-            if ((tid & 31) == 0) mbar_arrive(&sy->gen[b]);
-            // window fold, see FOLD_OFF
-            if (s >= TC_FLUSH + FOLD_OFF && (s - FOLD_OFF) % TC_FLUSH == 0) {
-                const int wp = (s - FOLD_OFF) / TC_FLUSH - 1;
-                ok = __all_sync(0xffffffffu, mbar_wait(&sy->flush_done[wp & 1], (wp >> 1) & 1, budget));
-                if (!ok) break;
-                fence_after();
-                fold_half<K, false>(hf, taddr_lane, (wp & 1) * D::WQ, acc, comp);
-                fence_before();
-            }
+            arrive_generated(sy, b);
+            ok = maybe_fold<K, false>(sy, budget, hf, s, taddr_lane, acc, comp);
+            if (!ok) break;
         }
-        if (ok && ns > 0) {
-            // windows not folded in the loop: the last one and possibly the one before
-            const int wl = (ns - 1) / TC_FLUSH;
-            for (int w = ns - 1 >= FOLD_OFF ? (ns - 1 - FOLD_OFF) / TC_FLUSH : 0; w <= wl && ok; ++w) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&sy->flush_done[w & 1], (w >> 1) & 1, budget));
-                if (!ok) break;
-                fence_after();
-                fold_half<K, false>(hf, taddr_lane, (w & 1) * D::WQ, acc, comp);
-            }
-        }
+        if (ok) ok = final_fold<K, false>(sy, budget, hf, ns, taddr_lane, acc, comp);
         if (!ok) { *(volatile int*)&sy->bad = 1; a.slots[S_TC_TIMEOUT] = 1.0; }
         fence_before();
         if (hf == 0) compensate<K, 0>(acc, comp);
@@ -858,171 +719,194 @@ __device__ __forceinline__ void gen_pair(unsigned off, const uint64_t* qd, const
 }
 
 template <int K, bool HESS>
-__global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_p_tc(PassArgs a) {
+__global__ void __launch_bounds__(TCI_THREADS, TcDims<K>::MINB) k_accum_p_tc(PassArgs a) {
     using D = TcDims<K>;
     constexpr int QSTR = qstr<K>();
     constexpr int GB = pimg_bytes<K>();
+    constexpr int GBM = 2 * D::B_TILE;                               // image slice: the B tile, then
+    constexpr int GBR = KD * QSTR * 4;                               // the q rows
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // aligned by an offset from the shared array (no integer round trip), so
     // that the compiler keeps every derived pointer in the shared space:
     // 32-bit shared loads instead of generic ones (fewer registers, no spills)
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const uint32_t sA = smem_u32(smem);                              // [2][4][A_TILE_PAD]
-    const uint32_t sR = sA + 2 * 4 * A_TILE_PAD;                     // ring [RING][GB]
-    uint32_t* SW = (uint32_t*)(smem + (sR - sA) + RING * GB);        // [RING][4][KD]
-    Sync* sy = (Sync*)(SW + RING * 4 * KD);
+    const uint32_t sR = sA + 2 * 4 * A_TILE_PAD;                     // ring [RING][GBM]
+    uint8_t* rows = smem + 2 * 4 * A_TILE_PAD + RING * GBM;          // ring [IRING][GBR]
+    uint32_t* SW = (uint32_t*)(rows + IRING * GBR);                  // ring [IRING][4][KD]
+    SyncI* sy = (SyncI*)(SW + IRING * 4 * KD);
     __shared__ __align__(128) uint32_t s_cls[32];
     const long long budget = a.budget;
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // uniform
-    const int jl = tid >> 3, ig = tid & 7;
-    const int hf = tid >> 7;
-    const int64_t j = (int64_t)blockIdx.x * 32 + jl;
-    const bool valid = j < a.J;
     const int64_t i0 = (int64_t)blockIdx.y * a.per_chunk;
     const int64_t i1 = min(a.I, i0 + (int64_t)a.per_chunk);
     const int ns = (int)((i1 - i0 + KD - 1) / KD);
-    const int64_t g0 = i0 / KD;
-    const int64_t jw0 = (int64_t)blockIdx.x * 4;
-    const int nwc = (int)min((int64_t)4, (int64_t)a.JW - jw0);     // word columns inside the matrix
     cls_table_init(s_cls, tid);
 
-    // stage t's inputs: the 32 individuals' image and their class words of the
-    // CTA's word columns (columns past JW are never read: their blocks are
-    // past J and evaluate as padding)
-    auto load_stage = [&](int t) {
-        const int slot = t % RING;
-        expect_tx(&sy->full[slot], sy->tx);
-        bulk_copy(sR + slot * GB, sy->img0 + (int64_t)t * GB, GB, &sy->full[slot]);
-        for (int w = 0; w < sy->nwc; ++w)
-            bulk_copy(smem_u32(SW + (slot * 4 + w) * KD), sy->g0 + w * sy->gstride + (int64_t)KD * t, 128,
-                      &sy->full[slot]);
-        atomicMax(&sy->loaded, t + 1);   // refills come from different warps
-    };
-
-    if (warp == 0) tmem_alloc<D::TCOLS_S>(&sy->tslot);
-    init_sync(sy, tid, 1, 1);
-    if (tid == 0) {
-        sy->img0 = a.img + g0 * GB;
-        sy->g0 = a.G + jw0 * a.Ipad + i0;
-        sy->gstride = a.Ipad;
-        sy->nwc = nwc;
-        sy->tx = (uint32_t)(GB + 128 * nwc);
-    }
+    if (warp == TC_WARPS) tmem_alloc<D::TCOLS_S>(&sy->tslot);
+    if (tid == 0) sync_init(sy);
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, sy->tslot, 0);
-    const uint32_t taddr_lane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-    if (tid == 0)
-        for (int t = 0; t < RING && t < ns; ++t) load_stage(t);
 
-    uint64_t pr2[2 * K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const double* pj = a.p + (int64_t)K * 4 * j + k;
-        pr2[2 * k] = valid ? f2_pack((float)pj[0], (float)pj[K]) : f2_dup(0.25f);
-        pr2[2 * k + 1] = valid ? f2_pack((float)pj[2 * K], (float)pj[3 * K]) : f2_dup(0.25f);
-    }
-    float acc[D::HALF], comp[D::NG];
-#pragma unroll
-    for (int c = 0; c < D::HALF; ++c) acc[c] = 0.f;
-#pragma unroll
-    for (int c = 0; c < D::NG; ++c) comp[c] = 0.f;
-    const int bsh = (4 * (jl & 7) + 29) & 31;     // rotates the block's class to bits 3 .. 6
-
-    for (int s = 0; s < ns; ++s) {
-        const int b = s & 1, slot = s % RING;
-        if (!mbar_wait(&sy->full[slot], (s / RING) & 1, budget)) set_bad(sy, a.slots);
-        if (s >= 2 && !is_bad(sy))
-            if (!mbar_wait(&sy->mma_done[b], ((s - 2) >> 1) & 1, budget)) set_bad(sy, a.slots);
-        if (is_bad(sy)) break;
-        // ring refill by the first warp here (see the Q side)
-        if (s >= 2 && s - 2 + RING < ns && first_at_stage(&sy->started[b])) load_stage(s - 2 + RING);
-        const float* Qs = reinterpret_cast<const float*>(smem + (sR - sA) + slot * GB + 2 * D::B_TILE);
-        const uint32_t* Ws = SW + slot * 4 * KD + (jl >> 3) * KD;
-        // A = W^T tile: rows m = 4*jl + h, reduction over the stage's individuals
-        float W[4][4], U[4][4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int ii = ig * 4 + e;
-            // 8 * class
-            const unsigned off = valid ? __funnelshift_r(Ws[ii], Ws[ii], bsh) & 0x78u : 8u * HX_PAD_NIBBLE;
-            uint64_t qd[(K + 1) / 2 * 2];
-            const ulonglong2* q2 = reinterpret_cast<const ulonglong2*>(Qs + qrow_slot(ii) * QSTR);
-#pragma unroll
-            for (int c = 0; c < (K + 1) / 2; ++c) {
-                const ulonglong2 x = q2[c];
-                qd[2 * c] = x.x;
-                qd[2 * c + 1] = x.y;
-            }
-            float u4[4], w4[4];
-            gen_pair<K, HESS>(off, qd, pr2, u4, w4, s_cls);
-#pragma unroll
-            for (int h = 0; h < 4; ++h) { U[h][e] = u4[h]; if (HESS) W[h][e] = w4[h]; }
+    if (warp == TC_WARPS) {
+        // ---- the issuing warp, as on the Q side
+        const uint32_t el = elect_lane();
+        const uint8_t* img = a.img + (i0 / KD) * GB;
+        const int64_t jw0 = (int64_t)blockIdx.x * 4;
+        const int nwc = (int)min((int64_t)4, (int64_t)a.JW - jw0);   // word columns inside the matrix; later ones
+                                                                     // are never read (their blocks are past J)
+        const uint32_t* g = a.G + jw0 * a.Ipad + i0;
+        auto load_b = [&](int t) {        // stage t's B tile
+            if (!el) return;
+            expect_tx(&sy->full[t % RING], (uint32_t)GBM);
+            bulk_copy(sR + (t % RING) * GBM, img + (int64_t)t * GB, GBM, &sy->full[t % RING]);
+        };
+        auto load_i = [&](int t) {        // its q rows and class words
+            if (!el) return;
+            const int slot = t % IRING;
+            expect_tx(&sy->fullw[slot], (uint32_t)(GBR + 128 * nwc));
+            bulk_copy(smem_u32(rows + slot * GBR), img + (int64_t)t * GB + GBM, GBR, &sy->fullw[slot]);
+            for (int w = 0; w < nwc; ++w)
+                bulk_copy(smem_u32(SW + (slot * 4 + w) * KD), g + w * a.Ipad + (int64_t)KD * t, 128, &sy->fullw[slot]);
+        };
+        auto wait = [&](uint64_t* bar, int phase) { return wait_or_bad(sy, bar, phase, a.slots, budget, el); };
+        int lb = 0, li = 0;               // stages loaded
+        for (; li < IRING && li < ns; ++li) load_i(li);
+        for (; lb < RING && lb < ns; ++lb) load_b(lb);
+        bool ok = true;
+        for (int t = 0; t < 2 && t < ns && ok; ++t) {
+            if (el) mbar_arrive(&sy->go[t]);      // no MMAs before them
+            ok = wait(&sy->fullw[t], 0);
+            if (ok && el) mbar_arrive(&sy->go[t]);
         }
-        const uint32_t aB = sA + b * 4 * A_TILE_PAD;
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            const int m = 4 * jl + h;
-            const uint32_t off = (m >> 3) * SBO_PAD + (ig >> 1) * LBO_PAD + (m & 7) * 16 + (ig & 1) * 8;
-            uint32_t wh[2], wl[2], uh[2], ul[2];
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                if (HESS) split2(W[h][2 * e], W[h][2 * e + 1], wh[e], wl[e]);
-                split2_f16(U[h][2 * e], U[h][2 * e + 1], uh[e], ul[e]);
-            }
-            if (HESS) {
-                asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(aB + off), "r"(wh[0]), "r"(wh[1]) : "memory");
-                asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(aB + A_TILE_PAD + off), "r"(wl[0]), "r"(wl[1]) : "memory");
-            }
-            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(aB + 2 * A_TILE_PAD + off), "r"(uh[0]), "r"(uh[1]) : "memory");
-            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(aB + 3 * A_TILE_PAD + off), "r"(ul[0]), "r"(ul[1]) : "memory");
-        }
-        // One issuer, the last warp to arrive: on this side two issuers were
-        // measured slower (the SM's MMA issue rate, not one thread, is the
-        // limit, and the fixed issuer warps fall behind on generation)
-        fence_async_smem();
-        fence_before();
-        if (arrive_last(&sy->arrived[b])) {
+        for (int s = 0; s < ns && ok; ++s) {
+            const int b = s & 1, slot = s % RING, d = (s / TC_FLUSH) & 1;
+            ok = wait(&sy->gen[b], s >> 1) && wait(&sy->full[slot], s / RING);
+            if (!ok) break;
             fence_after();
-            const int d = (s / TC_FLUSH) & 1;
-            const uint32_t el = elect_lane();
-            issue_stage_stacked<K, HESS>(tmem, d * D::WS, aB, A_TILE_PAD, LBO_PAD, SBO_PAD, sR + slot * GB,
-                                         (s % TC_FLUSH) == 0, el);
-            commit_stage(sy, s, ns, b, el);
+            issue_stage_stacked<K, HESS>(tmem, d * D::WS, sA + b * 4 * A_TILE_PAD, A_TILE_PAD, LBO_PAD, SBO_PAD,
+                                         sR + slot * GBM, (s % TC_FLUSH) == 0, el);
+            if (s + 2 < ns) commit(&sy->go[b], el);
+            if ((s % TC_FLUSH) == TC_FLUSH - 1 || s == ns - 1) commit(&sy->flush_done[d], el);
+            if (li < ns) { load_i(li); ++li; }
+            if (s >= 2 && lb < ns) { load_b(lb); ++lb; }
+            if (s + 2 < ns) {
+                ok = wait(&sy->fullw[(s + 2) % IRING], (s + 2) / IRING);
+                if (ok && el) mbar_arrive(&sy->go[b]);
+            }
         }
-        maybe_fold<K, true>(sy, a.slots, budget, hf, s, taddr_lane, acc, comp);
-    }
-    final_fold<K, true>(sy, a.slots, budget, hf, ns, taddr_lane, acc, comp);
-    // rows m of this CTA: TMEM lane r
-    const int r = tid & 127;
-    const int64_t m = (int64_t)blockIdx.x * 128 + r;
-    if (m < 4 * a.J) {
-        constexpr int NV = K + (HESS ? D::NH : 0);
-        const int64_t rows = 4 * a.J;
+        commit(&sy->end, el);
+        mbar_wait(&sy->end, 0u, TC_BUDGET);
+        if (!ok) {
+            for (int t = (lb >= RING ? lb - RING : 0); t < lb; ++t) mbar_wait(&sy->full[t % RING], (t / RING) & 1, TC_BUDGET);
+            for (int t = (li >= IRING ? li - IRING : 0); t < li; ++t) mbar_wait(&sy->fullw[t % IRING], (t / IRING) & 1, TC_BUDGET);
+        }
+        __syncwarp();
+    } else {
+        const int jl = tid >> 3, ig = tid & 7, hf = tid >> 7;
+        const int64_t j = (int64_t)blockIdx.x * 32 + jl;
+        const bool valid = j < a.J;
+        const uint32_t taddr_lane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+        uint64_t pr2[2 * K];
 #pragma unroll
-        for (int c = 0; c < D::HALF; ++c) {
-            const int col = hf * D::HALF + c;
-            if (col < D::NH) {
-                if (!HESS) continue;
-                const double val = (double)acc[c];
-                if (a.S == 1) {
-                    int k, k2;
-                    tri_pair<K>(col, k, k2);
-                    a.XtX[(int64_t)K * K * m + k2 + K * k] = val;
-                    a.XtX[(int64_t)K * K * m + k + K * k2] = val;
-                } else {
-                    a.part[((int64_t)blockIdx.y * NV + K + col) * rows + m] = val;
+        for (int k = 0; k < K; ++k) {
+            const double* pj = a.p + (int64_t)K * 4 * j + k;
+            pr2[2 * k] = valid ? f2_pack((float)pj[0], (float)pj[K]) : f2_dup(0.25f);
+            pr2[2 * k + 1] = valid ? f2_pack((float)pj[2 * K], (float)pj[3 * K]) : f2_dup(0.25f);
+        }
+        float acc[D::HALF], comp[D::NG];
+#pragma unroll
+        for (int c = 0; c < D::HALF; ++c) acc[c] = 0.f;
+#pragma unroll
+        for (int c = 0; c < D::NG; ++c) comp[c] = 0.f;
+        const int bsh = (4 * (jl & 7) + 29) & 31;     // rotates the block's class to bits 3 .. 6
+        bool ok = true;
+        for (int s = 0; s < ns; ++s) {
+            const int b = s & 1, slot = s % IRING;
+            ok = __all_sync(0xffffffffu, mbar_wait(&sy->go[b], (s >> 1) & 1, budget));
+            if (!ok) break;
+            const float* Qs = reinterpret_cast<const float*>(rows + slot * GBR);
+            const uint32_t* Ws = SW + slot * 4 * KD + (jl >> 3) * KD;
+            // A = W^T tile: rows m = 4*jl + h, reduction over the stage's individuals
+            float W[4][4], U[4][4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int ii = ig * 4 + e;
+                // 8 * class
+                const unsigned off = valid ? __funnelshift_r(Ws[ii], Ws[ii], bsh) & 0x78u : 8u * HX_PAD_NIBBLE;
+                uint64_t qd[(K + 1) / 2 * 2];
+                const ulonglong2* q2 = reinterpret_cast<const ulonglong2*>(Qs + qrow_slot(ii) * QSTR);
+#pragma unroll
+                for (int c = 0; c < (K + 1) / 2; ++c) {
+                    const ulonglong2 x = q2[c];
+                    qd[2 * c] = x.x;
+                    qd[2 * c + 1] = x.y;
                 }
-            } else if (col >= D::NHP && col < D::NHP + K) {
-                const double val = (double)acc[c] * G_UNSCALE;
-                if (a.S == 1) a.Xtz[(int64_t)K * m + (col - D::NHP)] = val;
-                else a.part[((int64_t)blockIdx.y * NV + (col - D::NHP)) * rows + m] = val;
+                float u4[4], w4[4];
+                gen_pair<K, HESS>(off, qd, pr2, u4, w4, s_cls);
+#pragma unroll
+                for (int h = 0; h < 4; ++h) { U[h][e] = u4[h]; if (HESS) W[h][e] = w4[h]; }
+            }
+            const uint32_t aB = sA + b * 4 * A_TILE_PAD;
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const int m = 4 * jl + h;
+                const uint32_t off = (m >> 3) * SBO_PAD + (ig >> 1) * LBO_PAD + (m & 7) * 16 + (ig & 1) * 8;
+                uint32_t wh[2], wl[2], uh[2], ul[2];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    if (HESS) split2(W[h][2 * e], W[h][2 * e + 1], wh[e], wl[e]);
+                    split2_f16(U[h][2 * e], U[h][2 * e + 1], uh[e], ul[e]);
+                }
+                if (HESS) {
+                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(aB + off), "r"(wh[0]), "r"(wh[1]) : "memory");
+                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(aB + A_TILE_PAD + off), "r"(wl[0]), "r"(wl[1]) : "memory");
+                }
+                asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(aB + 2 * A_TILE_PAD + off), "r"(uh[0]), "r"(uh[1]) : "memory");
+                asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(aB + 3 * A_TILE_PAD + off), "r"(ul[0]), "r"(ul[1]) : "memory");
+            }
+            arrive_generated(sy, b);
+            ok = maybe_fold<K, true>(sy, budget, hf, s, taddr_lane, acc, comp);
+            if (!ok) break;
+        }
+        if (ok) ok = final_fold<K, true>(sy, budget, hf, ns, taddr_lane, acc, comp);
+        if (!ok) { *(volatile int*)&sy->bad = 1; a.slots[S_TC_TIMEOUT] = 1.0; }
+        fence_before();
+        if (hf == 0) compensate<K, 0>(acc, comp);
+        else compensate<K, 1>(acc, comp);
+        // rows m of this CTA: TMEM lane r
+        const int r = tid & 127;
+        const int64_t m = (int64_t)blockIdx.x * 128 + r;
+        if (m < 4 * a.J) {
+            constexpr int NV = K + (HESS ? D::NH : 0);
+            const int64_t nrow = 4 * a.J;
+#pragma unroll
+            for (int c = 0; c < D::HALF; ++c) {
+                const int col = hf * D::HALF + c;
+                if (col < D::NH) {
+                    if (!HESS) continue;
+                    const double val = (double)acc[c];
+                    if (a.S == 1) {
+                        int k, k2;
+                        tri_pair<K>(col, k, k2);
+                        a.XtX[(int64_t)K * K * m + k2 + K * k] = val;
+                        a.XtX[(int64_t)K * K * m + k + K * k2] = val;
+                    } else {
+                        a.part[((int64_t)blockIdx.y * NV + K + col) * nrow + m] = val;
+                    }
+                } else if (col >= D::NHP && col < D::NHP + K) {
+                    const double val = (double)acc[c] * G_UNSCALE;
+                    if (a.S == 1) a.Xtz[(int64_t)K * m + (col - D::NHP)] = val;
+                    else a.part[((int64_t)blockIdx.y * NV + (col - D::NHP)) * nrow + m] = val;
+                }
             }
         }
     }
-    if (warp == 0) {
+    __syncthreads();
+    if (warp == TC_WARPS) {
         fence_after();
         tmem_dealloc<D::TCOLS_S>(tmem);
     }
@@ -1030,11 +914,11 @@ __global__ void __launch_bounds__(TC_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pass
 
 template <int K> constexpr size_t smem_q() {
     using QD = QpDims<K>;
-    return 1024 + 2 * 4 * A_TILE_STD + 2 * QD::A_T + RING * 2 * TcDims<K>::B_TILE + QRING * 2 * QD::B_T +
-           QRING * 128 * 4 + sizeof(SyncQ);
+    return 1024 + 2 * 4 * A_TILE_STD + 2 * QD::A_T + RING * 2 * TcDims<K>::B_TILE + IRING * 2 * QD::B_T +
+           IRING * 128 * 4 + sizeof(SyncI);
 }
 template <int K> constexpr size_t smem_p() {
-    return 1024 + 2 * 4 * A_TILE_PAD + RING * pimg_bytes<K>() + RING * 4 * KD * 4 + sizeof(Sync);
+    return 1024 + 2 * 4 * A_TILE_PAD + RING * 2 * TcDims<K>::B_TILE + IRING * KD * (qstr<K>() + 4) * 4 + sizeof(SyncI);
 }
 
 // One entry for every host-side operation on the K instantiation.
@@ -1053,10 +937,10 @@ cudaError_t tc_run(TcCall& c) {
         return e;
     }
     case TC_RESIDENT_Q:
-        c.bytes = (size_t)TcDims<K>::MINB_Q;
+        c.bytes = (size_t)TcDims<K>::MINB;
         return cudaSuccess;
     case TC_RESIDENT_P:
-        c.bytes = (size_t)resident_ctas((const void*)k_accum_p_tc<K, true>, TC_THREADS, smem_p<K>(), TcDims<K>::TCOLS_S);
+        c.bytes = (size_t)TcDims<K>::MINB;
         return cudaSuccess;
     case TC_IMG_BYTES: {
         const int64_t JW = (c.J + 7) / 8, ng = (c.I + KD - 1) / KD;
@@ -1068,7 +952,7 @@ cudaError_t tc_run(TcCall& c) {
         const unsigned gi = (unsigned)(((int64_t)a.JW * 4 + 127) / 128);
         dim3 grid((unsigned)(a.Ipad / 128), (unsigned)a.S);
         k_qimg<K><<<gi, 128, 0, c.st>>>(a.p, a.J, a.JW, a.img);
-        k_accum_q_tc<K><<<grid, TCQ_THREADS, smem_q<K>(), c.st>>>(a);
+        k_accum_q_tc<K><<<grid, TCI_THREADS, smem_q<K>(), c.st>>>(a);
         return cudaGetLastError();
     }
     case TC_P: {
@@ -1076,8 +960,8 @@ cudaError_t tc_run(TcCall& c) {
         const unsigned gi = (unsigned)((((a.I + KD - 1) / KD) * 4 + 127) / 128);
         dim3 grid((unsigned)((a.J + 31) / 32), (unsigned)a.S);
         k_pimg<K><<<gi, 128, 0, c.st>>>(a.q, a.I, a.img);
-        if (c.hess) k_accum_p_tc<K, true><<<grid, TC_THREADS, smem_p<K>(), c.st>>>(a);
-        else k_accum_p_tc<K, false><<<grid, TC_THREADS, smem_p<K>(), c.st>>>(a);
+        if (c.hess) k_accum_p_tc<K, true><<<grid, TCI_THREADS, smem_p<K>(), c.st>>>(a);
+        else k_accum_p_tc<K, false><<<grid, TCI_THREADS, smem_p<K>(), c.st>>>(a);
         return cudaGetLastError();
     }
     }
