@@ -77,7 +77,6 @@ template <int K> struct TcDims {
     static constexpr int NG = 16;
     static constexpr int NT = NHP + NG;
     static constexpr int TCOLS = (2 * NT <= 32) ? 32 : (2 * NT <= 64) ? 64 : (2 * NT <= 128) ? 128 : 256;
-    static constexpr int HALF = NT / 2;
     // Q side: one TMEM window = [Hessian NHP | gradient hi.hi NG | gradient
     // hi.lo + lo.hi NG].  Every MMA write rounds the accumulator it adds to,
     // not to nearest, so the small lo products get columns of their own:
@@ -146,86 +145,81 @@ __device__ __forceinline__ bool wait_or_bad(SyncI* sy, uint64_t* bar, int phase,
     return false;
 }
 
-// TMEM window fold: this thread's lane, columns [HF*HALF, HF*HALF + HALF) of the
-// accumulator at column base dcol.  Hessian columns add plainly; gradient
-// columns (>= NHP) use Kahan compensation in comp[col - NHP].
+// Columns that the threads of half hf of a CTA keep in registers, in chunks of 8:
+// the ceil(NH / 8) Hessian chunks, then the ceil(K / 8) gradient chunks.  The
+// padding that the MMAs' column counts (multiples of 16) add is not read: at
+// K = 8 a thread holds 24 sums and 8 compensations, not 32 and 16, and the
+// gradient-only form 8 and 8.
+template <int K, bool HESS> struct Kept {
+    using D = TcDims<K>;
+    static constexpr int CH = HESS ? (D::NH + 7) / 8 : 0, CG = (K + 7) / 8;
+    static constexpr int NC = CH + CG, HC = (NC + 1) / 2, N = 8 * HC;
+    // logical column of chunk ci (gradient columns start at NHP)
+    static __host__ __device__ constexpr int col(int ci) { return ci < CH ? 8 * ci : D::NHP + 8 * (ci - CH); }
+};
+
+// TMEM window fold: this thread's lane, its half's columns of the window at
+// column dcol, added to the FP32 registers; gradient columns (>= NHP) use Kahan
+// compensation in comp[col - NHP].
 // With STACK (P side) logical column c sums two physical columns: c and
 // NHP + c for the Hessian, 2NHP + g and 2NHP + NG + g for gradient column g.
-template <int K, int HF, bool STACK>
+// Otherwise (Q side) gradient column g has its lo products in column NT + g.
+template <int K, bool HESS, int HF, bool STACK>
 __device__ __forceinline__ void fold(uint32_t taddr_lane, int dcol, float* acc, float* comp) {
     using D = TcDims<K>;
-    uint32_t raw[D::HALF];
-    if (!STACK) {
+    using C = Kept<K, HESS>;
+    constexpr int CB = HF * C::HC, CE = CB + C::HC < C::NC ? CB + C::HC : C::NC;
+    uint32_t raw[C::N];
 #pragma unroll
-        for (int c = 0; c < D::HALF / 8; ++c)
-            tmem_ld8_async(taddr_lane + (uint32_t)(dcol + HF * D::HALF + 8 * c), raw + 8 * c);
-        tmem_wait_ld();
-        // gradient columns: add their lo-product columns [NT, NT + NG)
+    for (int ci = CB; ci < CE; ++ci) {
+        const int col = C::col(ci), p0 = STACK && ci >= C::CH ? 2 * D::NHP + (col - D::NHP) : col;
+        tmem_ld8_async(taddr_lane + (uint32_t)(dcol + p0), raw + 8 * (ci - CB));
+    }
+    tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < D::HALF / 8; ++c) {
-            const int col = HF * D::HALF + 8 * c;     // chunks never straddle NHP (a multiple of 16)
-            if (col >= D::NHP) {
-                uint32_t r2[8];
-                tmem_ld8_async(taddr_lane + (uint32_t)(dcol + D::NT + (col - D::NHP)), r2);
-                tmem_wait_ld();
-#pragma unroll
-                for (int t = 0; t < 8; ++t)
-                    raw[8 * c + t] = __float_as_uint(__uint_as_float(raw[8 * c + t]) + __uint_as_float(r2[t]));
-            }
-        }
-    } else {
-#pragma unroll
-        for (int c = 0; c < D::HALF / 8; ++c) {
-            const int col = HF * D::HALF + 8 * c;     // chunks never straddle NHP (a multiple of 16)
-            const int p0 = col < D::NHP ? col : 2 * D::NHP + (col - D::NHP);
-            tmem_ld8_async(taddr_lane + (uint32_t)(dcol + p0), raw + 8 * c);
-        }
+    for (int ci = CB; ci < CE; ++ci) {
+        if (!STACK && ci < C::CH) continue;
+        const int col = C::col(ci);
+        const int p1 = !STACK ? D::NT + (col - D::NHP) : ci < C::CH ? D::NHP + col : 2 * D::NHP + D::NG + (col - D::NHP);
+        uint32_t r2[8];
+        tmem_ld8_async(taddr_lane + (uint32_t)(dcol + p1), r2);
         tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < D::HALF / 8; ++c) {
-            const int col = HF * D::HALF + 8 * c;
-            const int p1 = col < D::NHP ? D::NHP + col : 2 * D::NHP + D::NG + (col - D::NHP);
-            uint32_t r2[8];
-            tmem_ld8_async(taddr_lane + (uint32_t)(dcol + p1), r2);
-            tmem_wait_ld();
-#pragma unroll
-            for (int t = 0; t < 8; ++t)
-                raw[8 * c + t] = __float_as_uint(__uint_as_float(raw[8 * c + t]) + __uint_as_float(r2[t]));
-        }
+        for (int t = 0; t < 8; ++t)
+            raw[8 * (ci - CB) + t] = __float_as_uint(__uint_as_float(raw[8 * (ci - CB) + t]) + __uint_as_float(r2[t]));
     }
 #pragma unroll
-    for (int c = 0; c < D::HALF / 8; ++c) {
-        float v[8];
-#pragma unroll
-        for (int t = 0; t < 8; ++t) v[t] = __uint_as_float(raw[8 * c + t]);
+    for (int ci = CB; ci < CE; ++ci) {
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
-            const int col = HF * D::HALF + 8 * c + t;
-            if (col >= D::NHP) {
-                const float y = v[t] - comp[col - D::NHP];
-                const float s = acc[8 * c + t] + y;
-                comp[col - D::NHP] = (s - acc[8 * c + t]) - y;
-                acc[8 * c + t] = s;
+            float& x = acc[8 * (ci - CB) + t];
+            const float v = __uint_as_float(raw[8 * (ci - CB) + t]);
+            if (ci >= C::CH) {
+                float& cc = comp[8 * (ci - C::CH) + t];
+                const float y = v - cc;
+                const float s = x + y;
+                cc = (s - x) - y;
+                x = s;
             } else {
-                acc[8 * c + t] += v[t];
+                x += v;
             }
         }
     }
 }
-template <int K, bool STACK>
+template <int K, bool HESS, bool STACK>
 __device__ __forceinline__ void fold_half(int hf, uint32_t taddr_lane, int dcol, float* acc, float* comp) {
-    if (hf == 0) fold<K, 0, STACK>(taddr_lane, dcol, acc, comp);
-    else fold<K, 1, STACK>(taddr_lane, dcol, acc, comp);
+    if (hf == 0) fold<K, HESS, 0, STACK>(taddr_lane, dcol, acc, comp);
+    else fold<K, HESS, 1, STACK>(taddr_lane, dcol, acc, comp);
 }
 // Applies the Kahan compensation to the gradient columns: acc then holds the sums.
-template <int K, int HF>
+template <int K, bool HESS, int HF>
 __device__ __forceinline__ void compensate(float* acc, const float* comp) {
-    using D = TcDims<K>;
+    using C = Kept<K, HESS>;
 #pragma unroll
-    for (int c = 0; c < D::HALF; ++c) {
-        const int col = HF * D::HALF + c;
-        if (col >= D::NHP) acc[c] -= comp[col - D::NHP];
-    }
+    for (int ci = HF * C::HC; ci < HF * C::HC + C::HC && ci < C::NC; ++ci)
+        if (ci >= C::CH)
+#pragma unroll
+            for (int t = 0; t < 8; ++t) acc[8 * (ci - HF * C::HC) + t] -= comp[8 * (ci - C::CH) + t];
 }
 
 // The 3 split products of one 32-deep stage into D (TMEM cols dcol..):
@@ -451,31 +445,31 @@ __device__ __forceinline__ void arrive_generated(SyncI* sy, int b) {
 // and before window w+2 reuses its columns (issued at stage (w+2)*TC_FLUSH,
 // once every thread has arrived there).
 constexpr int FOLD_OFF = TC_FLUSH / 2;
-template <int K, bool STACK>
+template <int K, bool HESS, bool STACK>
 __device__ __forceinline__ bool fold_window(SyncI* sy, long long budget, int hf, int w, uint32_t taddr_lane, float* acc,
                                             float* comp) {
     using D = TcDims<K>;
     constexpr int WC = STACK ? D::WS : D::WQ;   // TMEM columns per window
     if (!__all_sync(0xffffffffu, mbar_wait(&sy->flush_done[w & 1], (w >> 1) & 1, budget))) return false;
     fence_after();
-    fold_half<K, STACK>(hf, taddr_lane, (w & 1) * WC, acc, comp);
+    fold_half<K, HESS, STACK>(hf, taddr_lane, (w & 1) * WC, acc, comp);
     fence_before();
     return true;
 }
-template <int K, bool STACK>
+template <int K, bool HESS, bool STACK>
 __device__ __forceinline__ bool maybe_fold(SyncI* sy, long long budget, int hf, int s, uint32_t taddr_lane, float* acc,
                                            float* comp) {
     if (s < TC_FLUSH + FOLD_OFF || (s - FOLD_OFF) % TC_FLUSH != 0) return true;
-    return fold_window<K, STACK>(sy, budget, hf, (s - FOLD_OFF) / TC_FLUSH - 1, taddr_lane, acc, comp);
+    return fold_window<K, HESS, STACK>(sy, budget, hf, (s - FOLD_OFF) / TC_FLUSH - 1, taddr_lane, acc, comp);
 }
 // Windows not folded in the loop: the last one and possibly the one before.
-template <int K, bool STACK>
+template <int K, bool HESS, bool STACK>
 __device__ __forceinline__ bool final_fold(SyncI* sy, long long budget, int hf, int ns, uint32_t taddr_lane, float* acc,
                                            float* comp) {
     bool ok = true;
     if (ns > 0)
         for (int w = ns - 1 >= FOLD_OFF ? (ns - 1 - FOLD_OFF) / TC_FLUSH : 0; w <= (ns - 1) / TC_FLUSH && ok; ++w)
-            ok = fold_window<K, STACK>(sy, budget, hf, w, taddr_lane, acc, comp);
+            ok = fold_window<K, HESS, STACK>(sy, budget, hf, w, taddr_lane, acc, comp);
     return ok;
 }
 
@@ -505,6 +499,7 @@ __device__ __forceinline__ void gen_pair_qp(unsigned off, uint64_t z01, uint64_t
 template <int K>
 __global__ void __launch_bounds__(TCI_THREADS, TcDims<K>::MINB) k_accum_q_tc(PassArgs a) {
     using D = TcDims<K>;
+    using C = Kept<K, true>;
     using QD = QpDims<K>;
     constexpr int GB = qimg_bytes<K>();
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -617,11 +612,11 @@ __global__ void __launch_bounds__(TCI_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pas
         __syncwarp();
     } else {
         const uint32_t taddr_lane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-        float acc[D::HALF], comp[D::NG];
+        float acc[C::N], comp[8 * C::CG];
 #pragma unroll
-        for (int c = 0; c < D::HALF; ++c) acc[c] = 0.f;
+        for (int c = 0; c < C::N; ++c) acc[c] = 0.f;
 #pragma unroll
-        for (int c = 0; c < D::NG; ++c) comp[c] = 0.f;
+        for (int c = 0; c < 8 * C::CG; ++c) comp[c] = 0.f;
         bool ok = true;
         for (int s = 0; s < ns; ++s) {
             const int b = s & 1;
@@ -666,20 +661,22 @@ __global__ void __launch_bounds__(TCI_THREADS, TcDims<K>::MINB) k_accum_q_tc(Pas
                 sts128(aB + 3 * A_TILE_STD + off, ul[0], ul[1], ul[2], ul[3]);
             }
             arrive_generated(sy, b);
-            ok = maybe_fold<K, false>(sy, budget, hf, s, taddr_lane, acc, comp);
+            ok = maybe_fold<K, true, false>(sy, budget, hf, s, taddr_lane, acc, comp);
             if (!ok) break;
         }
-        if (ok) ok = final_fold<K, false>(sy, budget, hf, ns, taddr_lane, acc, comp);
+        if (ok) ok = final_fold<K, true, false>(sy, budget, hf, ns, taddr_lane, acc, comp);
         if (!ok) { *(volatile int*)&sy->bad = 1; a.slots[S_TC_TIMEOUT] = 1.0; }
         fence_before();
-        if (hf == 0) compensate<K, 0>(acc, comp);
-        else compensate<K, 1>(acc, comp);
+        if (hf == 0) compensate<K, true, 0>(acc, comp);
+        else compensate<K, true, 1>(acc, comp);
         // write partials: v < K gradient, v = K + tri index Hessian
         constexpr int NV = K + D::NH;
         double* out = a.part + (int64_t)blockIdx.y * NV * a.Ipad;
 #pragma unroll
-        for (int c = 0; c < D::HALF; ++c) {
-            const int col = hf * D::HALF + c;
+        for (int c = 0; c < C::N; ++c) {
+            const int ci = hf * C::HC + c / 8;
+            if (ci >= C::NC) break;
+            const int col = C::col(ci) + c % 8;
             if (col < D::NH) out[(int64_t)(K + col) * a.Ipad + i] = (double)acc[c];
             else if (col >= D::NHP && col < D::NHP + K) out[(int64_t)(col - D::NHP) * a.Ipad + i] = (double)acc[c] * G_UNSCALE;
         }
@@ -721,6 +718,7 @@ __device__ __forceinline__ void gen_pair(unsigned off, const uint64_t* qd, const
 template <int K, bool HESS>
 __global__ void __launch_bounds__(TCI_THREADS, TcDims<K>::MINB) k_accum_p_tc(PassArgs a) {
     using D = TcDims<K>;
+    using C = Kept<K, HESS>;
     constexpr int QSTR = qstr<K>();
     constexpr int GB = pimg_bytes<K>();
     constexpr int GBM = 2 * D::B_TILE;                               // image slice: the B tile, then
@@ -817,11 +815,11 @@ __global__ void __launch_bounds__(TCI_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pas
             pr2[2 * k] = valid ? f2_pack((float)pj[0], (float)pj[K]) : f2_dup(0.25f);
             pr2[2 * k + 1] = valid ? f2_pack((float)pj[2 * K], (float)pj[3 * K]) : f2_dup(0.25f);
         }
-        float acc[D::HALF], comp[D::NG];
+        float acc[C::N], comp[8 * C::CG];
 #pragma unroll
-        for (int c = 0; c < D::HALF; ++c) acc[c] = 0.f;
+        for (int c = 0; c < C::N; ++c) acc[c] = 0.f;
 #pragma unroll
-        for (int c = 0; c < D::NG; ++c) comp[c] = 0.f;
+        for (int c = 0; c < 8 * C::CG; ++c) comp[c] = 0.f;
         const int bsh = (4 * (jl & 7) + 29) & 31;     // rotates the block's class to bits 3 .. 6
         bool ok = true;
         for (int s = 0; s < ns; ++s) {
@@ -869,14 +867,14 @@ __global__ void __launch_bounds__(TCI_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pas
                 asm volatile("st.shared.v2.b32 [%0], {%1, %2};" :: "r"(aB + 3 * A_TILE_PAD + off), "r"(ul[0]), "r"(ul[1]) : "memory");
             }
             arrive_generated(sy, b);
-            ok = maybe_fold<K, true>(sy, budget, hf, s, taddr_lane, acc, comp);
+            ok = maybe_fold<K, HESS, true>(sy, budget, hf, s, taddr_lane, acc, comp);
             if (!ok) break;
         }
-        if (ok) ok = final_fold<K, true>(sy, budget, hf, ns, taddr_lane, acc, comp);
+        if (ok) ok = final_fold<K, HESS, true>(sy, budget, hf, ns, taddr_lane, acc, comp);
         if (!ok) { *(volatile int*)&sy->bad = 1; a.slots[S_TC_TIMEOUT] = 1.0; }
         fence_before();
-        if (hf == 0) compensate<K, 0>(acc, comp);
-        else compensate<K, 1>(acc, comp);
+        if (hf == 0) compensate<K, HESS, 0>(acc, comp);
+        else compensate<K, HESS, 1>(acc, comp);
         // rows m of this CTA: TMEM lane r
         const int r = tid & 127;
         const int64_t m = (int64_t)blockIdx.x * 128 + r;
@@ -884,8 +882,10 @@ __global__ void __launch_bounds__(TCI_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pas
             constexpr int NV = K + (HESS ? D::NH : 0);
             const int64_t nrow = 4 * a.J;
 #pragma unroll
-            for (int c = 0; c < D::HALF; ++c) {
-                const int col = hf * D::HALF + c;
+            for (int c = 0; c < C::N; ++c) {
+                const int ci = hf * C::HC + c / 8;
+            if (ci >= C::NC) break;
+            const int col = C::col(ci) + c % 8;
                 if (col < D::NH) {
                     if (!HESS) continue;
                     const double val = (double)acc[c];
