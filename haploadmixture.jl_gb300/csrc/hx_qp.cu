@@ -5,10 +5,13 @@
 // side), by the primal active-set method of the oracle: solve on the free
 // variables (Cholesky factor of the free block), step to the first bound met
 // (lowest index on ties), and when no bound is met release the bound with the
-// largest multiplier.  GB300's FP64 unit takes 16 clocks of an SM for any warp
-// instruction, however few of its lanes work, so both kernels keep the lanes
-// full: the Q side solves one problem per lane, the P side one per group of 8
-// lanes (16 from K = 9 on).  Both perform, element by element, the operations of
+// largest multiplier.  An FP64 operation of a warp takes 64 clocks of its quarter of
+// an SM, however few of its lanes work and whether or not the next one waits for
+// it, so both kernels keep the lanes full: the Q side solves one problem per lane,
+// the P side one per group of K lanes; and the pivots' roots and all comparisons
+// (FP64 operations too) are done in integers.  P side, 20,000 blocks at K = 10:
+// 2.10 ms with 16 lanes per problem, 1.50 with 10, 1.27 with the integer forms;
+// 4,000 blocks at K = 5: 0.59, 0.45, 0.39.  Both perform, element by element, the operations of
 // the dense factorisation and sweeps of the free block in index order, and leave
 // out only those whose operands are exact zeros, so the results do not depend
 // on this arrangement (the mixed method rounds them to FP32 afterwards, which
@@ -27,8 +30,61 @@ namespace {
 using tc::tri_idx;
 constexpr unsigned FULL = 0xffffffffu;
 
-// 1 / sqrt(s) as the factorisation uses it: the reciprocal of the rounded root
-__device__ __forceinline__ double inv_root(double s) { return 1.0 / sqrt(s); }
+// 1 / sqrt(s) as the factorisation uses it: the reciprocal of the rounded root,
+// both correctly rounded.  In fixed point: with s = m 4^k, 1 <= m < 4, one
+// cubically convergent step y (1 + e/2 + 3 e^2/8), e = 1 - m y^2, from the
+// hardware's FP32 reciprocal root leaves y ~ 1 / sqrt(m) within 2^-53, and
+// G ~ sqrt(m) = m y; the remainders m - G^2 and 1 - G R, exact in the low 64 bits
+// of the products, then tell how far G and R are from the nearest 53-bit numbers
+// (1 and 2 units at most).  Outside 2^-600 .. 2^600 the operators, out of line.
+__device__ __noinline__ double inv_root_edge(double s) { return 1.0 / sqrt(s); }
+__device__ __forceinline__ double inv_root(double s) {
+    typedef unsigned long long u64;
+    typedef long long i64;
+    const int hi = __double2hiint(s);
+    if (((unsigned)hi >> 20) - 423u > 1200u) return inv_root_edge(s);
+    const int ex = (hi >> 20) - 1023, odd = ex & 1, half = (ex - odd) >> 1;
+    const u64 b = ((u64)__double_as_longlong(s) & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+    const u64 m = b << (10 + odd);                                     // m 2^62
+    float y0;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(__uint2float_rn((unsigned)(m >> 32)) * 0x1p-30f));
+    const unsigned Y0 = __float2uint_rz(y0 * 0x1p31f);                 // y 2^31, at most 2^31 (1 + 2^-22)
+    const i64 e = (i64)((1ull << 60) - __umul64hi(m, (u64)Y0 * Y0));   // 2^60, |e| < 2^39
+    const int e1 = (int)(e >> 24);                                     // 2^36
+    const i64 t = (e >> 1) + (((i64)e1 * e1 * 3) >> 15);               // e/2 + 3 e^2/8, 2^60
+    const int t1 = (int)((t + 64) >> 7);                               // 2^53
+    const u64 y = ((u64)Y0 << 31) + (u64)(((i64)Y0 * t1) >> 22);       // 2^62
+    u64 G = (__umul64hi(m, y) + 128) >> 8;                             // sqrt(m) 2^52
+    const i64 r = (i64)((m << 42) - G * G);
+    G = G + (r > (i64)G) - (r <= -(i64)G);
+    u64 R = (y + 256) >> 9;                                            // 2^53 / sqrt(m)
+    const i64 g = (i64)G, q = -2 * (i64)(R * G);                       // 2 (2^105 - R G)
+    R = R + (q > g) + (q > 3 * g) - (q < -g) - (q < -3 * g);
+    return __longlong_as_double((i64)(R + ((u64)(1021 - half) << 52)));
+}
+// x > f for f > 0
+__device__ __forceinline__ bool above(double x, double f) {
+    const long long b = __double_as_longlong(x);
+    return b > __double_as_longlong(f) && b <= 0x7FF0000000000000ll;
+}
+__device__ __forceinline__ long long abs_bits(double x) { return __double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll; }
+constexpr long long INF_BITS = 0x7FF0000000000000ll;
+// The larger of two magnitudes, as bits
+__device__ __forceinline__ long long max_bits(long long a, long long b) { return a > b ? a : b; }
+// x > 0, and x < 0
+__device__ __forceinline__ bool positive(double x) { return __double_as_longlong(x) > 0 && abs_bits(x) <= INF_BITS; }
+__device__ __forceinline__ bool negative(double x) {
+    return __double2hiint(x) < 0 && abs_bits(x) > 0 && abs_bits(x) <= INF_BITS;
+}
+// |a| < |b|
+__device__ __forceinline__ bool smaller(double a, double b) { return abs_bits(a) < abs_bits(b) && abs_bits(b) <= INF_BITS; }
+// Whether the step s from d passes the bound ahead (upper bound 1 - v, lower 0 - v):
+// a ratio num / s below 1, or a bound passed by rounding, before dividing
+__device__ __forceinline__ bool passes(double s, double v, double d, bool& upw, double& num) {
+    upw = positive(s);
+    num = ((upw ? 1.0 : 0.0) - v) - d;
+    return abs_bits(s) != 0 && (smaller(num, s) || (upw ? negative(num) : positive(num)));
+}
 
 // ------------------------------------------------------------------ Q side
 // One problem per thread, its K x K triangle in shared memory (entry e of
@@ -123,7 +179,7 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
 #pragma unroll 1
     for (int it = 0; it < max_iter && !done; ++it) {
         double A[NT], y[K], o[K];
-        double md = 0.0;
+        long long mb = 0;
 #pragma unroll
         for (int a = 0; a < K; ++a) {
             const bool fa = (fr >> a) & 1u;
@@ -137,9 +193,9 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
             o[a] = fa ? 1.0 : 0.0;
 #pragma unroll
             for (int b = a; b < K; ++b) A[tri_idx<K>(a, b)] = fa && ((fr >> b) & 1u) ? h(a, b) : 0.0;
-            md = fmax(md, fabs(A[tri_idx<K>(a, a)]));
+            mb = max_bits(mb, abs_bits(A[tri_idx<K>(a, a)]));
         }
-        const double fl = 1e-300 + 1e-14 * md;
+        const double fl = 1e-300 + 1e-14 * __longlong_as_double(mb);
         // A = L L': entry (a, b), b > a, ends as L[b, a]; y and o follow through
         // the forward sweep
         double iv[K];
@@ -147,7 +203,7 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
         for (int a = 0; a < K; ++a) {
             const double pv = A[tri_idx<K>(a, a)];
             const bool fa = (fr >> a) & 1u;
-            if (fa && !(pv > fl)) floored = true;
+            if (fa && !above(pv, fl)) floored = true;
             iv[a] = fa ? inv_root(pv) : 0.0;
             y[a] *= iv[a];
             o[a] *= iv[a];
@@ -190,10 +246,9 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
             if (!((fr >> a) & 1u)) { y[a] = d[a]; continue; }
             if (eq) y[a] = fma(-nu, o[a], y[a]);
             const double s = y[a] - d[a];
-            const bool u = s > 0.0;
-            const double num = u ? (1.0 - qa[a]) - d[a] : (0.0 - qa[a]) - d[a];    // to the bound ahead
-            // a ratio below 1 (or a bound passed by rounding), before dividing
-            if (s != 0.0 && (fabs(num) < fabs(s) || (u ? num < 0.0 : num > 0.0))) {
+            bool u;
+            double num;
+            if (passes(s, qa[a], d[a], u, num)) {
                 const double ra = num / s;
                 if (ra < best) { best = ra; bi = a; bup = u; }
             }
@@ -212,7 +267,7 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
                     for (int b = 0; b < K; ++b) g = fma(h(a, b), d[b], g);
                     g += nu;
                     const double v = (up >> a) & 1u ? g : -g;
-                    if (v > wv) { wv = v; rel = a; }
+                    if (above(v, wv)) { wv = v; rel = a; }
                 }
             }
             if (rel < 0) { done = true; break; }
@@ -250,15 +305,15 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
 // the factor takes, per haplotype, its own K x K block, V once, and the update
 // by V V' of T and of the later diagonal blocks: about K^3 x 5 operations
 // instead of 11 K^3.
-// One problem per group of GL lanes; lane k holds row k of each block and the
+// One problem per group of K lanes; lane k holds row k of each block and the
 // four variables (h, k).
 template <int K> struct PDim {
-    static constexpr int GL = K <= 8 ? 8 : 16;
-    static constexpr int PW = 32 / GL;                      // problems per warp
+    static constexpr int PW = 32 / K;                       // problems per warp
     static constexpr int WARPS = 2;
     // per problem (doubles): D [4][K][K], L [4][K][K], V [3][K][K], iv [4][K], vec [4][K]
     static constexpr int RAW = 11 * K * K + 8 * K;
-    static constexpr int LD = (RAW + 15) / 16 * 16 + 4;     // problems of a warp start 32 bytes apart modulo 128
+    // problems of a warp start in different banks
+    static constexpr int LD = (RAW + 15) / 16 * 16 + (K % 4 == 0 ? 4 : K);
     static constexpr size_t SMEM = (size_t)WARPS * PW * LD * sizeof(double);
 };
 
@@ -296,10 +351,10 @@ __global__ void __launch_bounds__(32 * PDim<K>::WARPS)
 k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz, const double* __restrict__ p,
         double rho, double* __restrict__ pdiff, double* slots, int8_t* __restrict__ ws) {
     using P = PDim<K>;
-    constexpr int GL = P::GL, KK = K * K;
+    constexpr int KK = K * K;
     extern __shared__ double smem_p[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int k = lane % GL, g = lane / GL;
+    const int g = min(lane / K, P::PW - 1), k = lane - g * K, base = g * K;     // k >= K: idle lane
     const int64_t j = ((int64_t)blockIdx.x * P::WARPS + warp) * P::PW + g;
     const bool valid = j < n;
     const bool row = k < K;
@@ -309,7 +364,9 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
     double* V = L + 4 * KK;                         // V[k, c] of block h at h KK + c K + k
     double* iv = V + 3 * KK;                        // reciprocal roots of the pivots (0: fixed)
     double* vec = iv + 4 * K;
-    for (int t = k; t < 4 * KK; t += GL) D[t] = valid ? XtX[j * 4 * KK + t] : (t % KK / K == t % K ? 1.0 : 0.0);
+    if (row) for (int t = k; t < 4 * KK; t += K) D[t] = valid ? XtX[j * 4 * KK + t] : (t % KK / K == t % K ? 1.0 : 0.0);
+    // lane o places on in the group, round its end: ceil(log2 K) such steps reach every lane
+    auto next = [&](int o) { return base + (row ? k + o - (k + o < K ? 0 : K) : o); };
     double z[4], d[4], pa[4];
     unsigned fr = 0u, up = 0u, no = 0u;             // bits h: free; at the upper bound; both bounds at 0
     double zs = 1.0;
@@ -330,25 +387,29 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
         }
     }
 #pragma unroll
-    for (int o = GL / 2; o > 0; o >>= 1) zs = fmax(zs, __shfl_xor_sync(FULL, zs, o));
+    for (int o = 1; o < K; o *= 2) zs = fmax(zs, __shfl_sync(FULL, zs, next(o)));
     const double tol = 1e-12 * zs;
     const int max_iter = 16 * K + 20;
+    __syncwarp();
+    double dk[4];                                   // diagonal of H
+#pragma unroll
+    for (int h = 0; h < 4; ++h) dk[h] = D[h * KK + kc * K + kc] + rho;
     bool done = !valid, floored = false;            // floored: left to the dense solver
 #pragma unroll 1
     for (int it = 0; it < max_iter; ++it) {
         if (__all_sync(FULL, done)) break;
         __syncwarp();
         // fixed variables to vec (free ones 0), largest free diagonal
-        double md = 0.0;
+        long long mb = 0;
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
             const bool f = (fr >> h) & 1u;
             if (row) vec[h * K + k] = f ? 0.0 : d[h];
-            if (row && f) md = fmax(md, fabs(D[h * KK + kc * K + kc] + rho));
+            if (row && f) mb = max_bits(mb, abs_bits(dk[h]));
         }
 #pragma unroll
-        for (int o = GL / 2; o > 0; o >>= 1) md = fmax(md, __shfl_xor_sync(FULL, md, o));
-        const double fl = 1e-300 + 1e-14 * md;
+        for (int o = 1; o < K; o *= 2) mb = max_bits(mb, __shfl_sync(FULL, mb, next(o)));
+        const double fl = 1e-300 + 1e-14 * __longlong_as_double(mb);
         __syncwarp();
         // right-hand sides z - H d over the fixed variables, in index order
         double x[4];
@@ -368,82 +429,118 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
             }
             x[h] = row && ((fr >> h) & 1u) ? s : 0.0;
         }
-        // factorisation, forward sweep alongside
-        double T[K], G[3][K];                        // row k of T and of the diagonal blocks 1 .. 3
+        // factorisation, forward sweep alongside.  One copy of the code serves the
+        // four haplotypes, with C, the later blocks G and the right-hand sides
+        // moved up by one after each (written out four times, the loop was 210 KB
+        // of code at K = 10, and 6% slower)
+        double T[K], C[K], G[3][K];                  // row k of T, of this and of the later diagonal blocks
 #pragma unroll
         for (int a = 0; a < K; ++a) {
             T[a] = a == k ? rho : 0.0;
+            const int at = a <= kc ? a * K + kc : kc * K + a;
+            C[a] = a == k ? dk[0] : D[at];
 #pragma unroll
-            for (int h = 1; h < 4; ++h)
-                G[h - 1][a] = D[h * KK + (a <= kc ? a * K + kc : kc * K + a)] + (a == k ? rho : 0.0);
+            for (int h = 1; h < 4; ++h) G[h - 1][a] = a == k ? dk[h] : D[h * KK + at];
         }
-#pragma unroll
+        __syncwarp();
+#pragma unroll 1
         for (int h = 0; h < 4; ++h) {
+            double *Lh = L + h * KK, *Vh = V + h * KK;
             const bool f = row && ((fr >> h) & 1u);
-            const unsigned fm = __ballot_sync(FULL, f) >> (g * GL);      // free indices of this problem's h
+            const unsigned fm = __ballot_sync(FULL, f) >> base;          // free indices of this problem's h
             double M[K], W[K];
 #pragma unroll
             for (int a = 0; a < K; ++a) {
-                const double m = h == 0 ? D[a <= kc ? a * K + kc : kc * K + a] + (a == k ? rho : 0.0) : G[h > 0 ? h - 1 : 0][a];
-                M[a] = f && ((fm >> a) & 1u) ? m : 0.0;
+                M[a] = f && ((fm >> a) & 1u) ? C[a] : 0.0;
                 W[a] = T[a];
             }
 #pragma unroll
             for (int c = 0; c < K; ++c) {
-                const double pv = __shfl_sync(FULL, M[c], c, GL);
-                if (((fm >> c) & 1u) && !done && !(pv > fl)) floored = true;
+                const double pv = __shfl_sync(FULL, M[c], base + c);
+                if (((fm >> c) & 1u) && !done && !above(pv, fl)) floored = true;
                 const double ivc = (fm >> c) & 1u ? inv_root(pv) : 0.0;
                 const double l = k > c ? M[c] * ivc : 0.0;
-                if (row) L[h * KK + c * K + k] = l;
+                if (row) Lh[c * K + k] = l;
                 if (k == c) iv[h * K + c] = ivc;
-                const double xa = __shfl_sync(FULL, x[h], c, GL) * ivc;
-                x[h] = k == c ? xa : fma(-l, xa, x[h]);
+                const double xa = __shfl_sync(FULL, x[0], base + c) * ivc;
+                x[0] = k == c ? xa : fma(-l, xa, x[0]);
                 W[c] *= ivc;                          // V[k, c]
-                if (h < 3) {
-#pragma unroll
-                    for (int b = h + 1; b < 4; ++b) x[b] = fma(-W[c], xa, x[b]);
-                }
                 __syncwarp();
 #pragma unroll
                 for (int s = c + 1; s < K; ++s) {
-                    const double ls = L[h * KK + c * K + s];
+                    const double ls = Lh[c * K + s];
                     M[s] = fma(-l, ls, M[s]);
-                    if (h < 3) W[s] = fma(-W[c], ls, W[s]);
+                    W[s] = fma(-W[c], ls, W[s]);
                 }
             }
-            if (h < 3) {
-                if (row) {
+            if (row) vec[h * K + k] = x[0];
+            if (h == 3) break;
+            if (row) {
 #pragma unroll
-                    for (int c = 0; c < K; ++c) V[h * KK + c * K + k] = W[c];
-                }
-                __syncwarp();
+                for (int c = 0; c < K; ++c) Vh[c * K + k] = W[c];
+            }
+            __syncwarp();
+#pragma unroll 1
+            for (int c = 0; c < K; ++c) {
+                const double w = -Vh[c * K + kc], xa = vec[h * K + c];
+                const double* v = Vh + c * K;
+                x[1] = fma(w, xa, x[1]);
 #pragma unroll
-                for (int c = 0; c < K; ++c) {
+                for (int a = 0; a < K; ++a) G[0][a] = fma(w, v[a], G[0][a]);
+                if (h < 2) {
+                    x[2] = fma(w, xa, x[2]);
 #pragma unroll
                     for (int a = 0; a < K; ++a) {
-                        const double va = V[h * KK + c * K + a];
-                        if (h < 2) T[a] = fma(-W[c], va, T[a]);
-#pragma unroll
-                        for (int b = h + 1; b < 4; ++b) G[b - 1][a] = fma(-W[c], va, G[b - 1][a]);
+                        T[a] = fma(w, v[a], T[a]);
+                        G[1][a] = fma(w, v[a], G[1][a]);
                     }
                 }
-                // rows of fixed variables get sums too; the masks leave them unused
+                if (h == 0) {
+                    x[3] = fma(w, xa, x[3]);
 #pragma unroll
-                for (int b = h + 1; b < 4; ++b)
-                    if (!((fr >> b) & 1u)) x[b] = 0.0;
+                    for (int a = 0; a < K; ++a) G[2][a] = fma(w, v[a], G[2][a]);
+                }
             }
+#pragma unroll
+            for (int a = 0; a < K; ++a) {
+                C[a] = G[0][a];
+                G[0][a] = G[1][a];
+                G[1][a] = G[2][a];
+            }
+            // rows of fixed variables get sums too; the masks leave them unused
+            x[0] = (fr >> (h + 1)) & 1u ? x[1] : 0.0;
+            x[1] = (fr >> (h + 2)) & 1u ? x[2] : 0.0;
+            x[2] = (fr >> (h + 3)) & 1u ? x[3] : 0.0;
         }
         done |= floored;
-        // backward sweep
+        __syncwarp();
+        // backward sweep, the same way: x[b] belongs to haplotype h - b
 #pragma unroll
-        for (int h = 3; h >= 0; --h)
+        for (int b = 0; b < 4; ++b) x[b] = vec[(3 - b) * K + kc];
+#pragma unroll 1
+        for (int h = 3; h >= 0; --h) {
+            const double *Lh = L + h * KK, *Vh = V + h * KK;
 #pragma unroll
             for (int c = K - 1; c >= 0; --c) {
-                const double xa = __shfl_sync(FULL, x[h], c, GL) * iv[h * K + c];
-                x[h] = k == c ? xa : (k < c ? fma(-L[h * KK + kc * K + c], xa, x[h]) : x[h]);
-#pragma unroll
-                for (int b = 0; b < h; ++b) x[b] = fma(-V[b * KK + kc * K + c], xa, x[b]);
+                const double xa = __shfl_sync(FULL, x[0], base + c) * iv[h * K + c];
+                x[0] = k == c ? xa : (k < c ? fma(-Lh[kc * K + c], xa, x[0]) : x[0]);
             }
+            __syncwarp();
+            if (row) vec[h * K + k] = x[0];
+            __syncwarp();
+#pragma unroll 1
+            for (int c = K - 1; c >= 0; --c) {
+                const double xa = vec[h * K + c];
+                const double* v = Vh + kc * K + c;
+                if (h > 0) x[1] = fma(-v[-KK], xa, x[1]);
+                if (h > 1) x[2] = fma(-v[-2 * KK], xa, x[2]);
+                if (h > 2) x[3] = fma(-v[-3 * KK], xa, x[3]);
+            }
+#pragma unroll
+            for (int b = 0; b < 3; ++b) x[b] = x[b + 1];
+        }
+#pragma unroll
+        for (int h = 0; h < 4; ++h) x[h] = vec[h * K + kc];
         // targets; ratio test: smallest step ratio < 1, lowest variable index (h, k) on ties
         double best = 1.0;
         int bidx = INT_MAX;
@@ -452,23 +549,25 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
         for (int h = 0; h < 4; ++h) {
             if (!(row && ((fr >> h) & 1u))) { x[h] = d[h]; continue; }
             const double s = x[h] - d[h];
-            const bool upw = s > 0.0;
-            const double num = upw ? (1.0 - pa[h]) - d[h] : (0.0 - pa[h]) - d[h];
-            if (s != 0.0 && (fabs(num) < fabs(s) || (upw ? num < 0.0 : num > 0.0))) {
+            bool upw;
+            double num;
+            if (passes(s, pa[h], d[h], upw, num)) {
                 const double ra = num / s;
                 if (ra < best) { best = ra; bidx = h * K + k; bup = upw; }
             }
         }
+        long long bb = __double_as_longlong(best);       // as an integer in the same order
+        if (bb < 0) bb = abs_bits(best) == 0 ? 0 : bb ^ 0x7FFFFFFFFFFFFFFFll;
         int bto = bup ? 1 : 0;
 #pragma unroll
-        for (int o = GL / 2; o > 0; o >>= 1) {
-            const double ob = __shfl_xor_sync(FULL, best, o);
-            const int oi = __shfl_xor_sync(FULL, bidx, o), ot = __shfl_xor_sync(FULL, bto, o);
-            if (ob < best || (ob == best && oi < bidx)) { best = ob; bidx = oi; bto = ot; }
+        for (int o = 1; o < K; o *= 2) {
+            const long long ob = __shfl_sync(FULL, bb, next(o));
+            const int oi = __shfl_sync(FULL, bidx, next(o)), ot = __shfl_sync(FULL, bto, next(o));
+            if (ob < bb || (ob == bb && oi < bidx)) { bb = ob; bidx = oi; bto = ot; }
         }
         const bool blocked = bidx != INT_MAX;
         if (!done && blocked) {
-            const double al = best < 0.0 ? 0.0 : best;
+            const double al = bb < 0 ? 0.0 : __longlong_as_double(bb);
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
                 if ((fr >> h) & 1u) d[h] = fma(al, x[h] - d[h], d[h]);
@@ -505,18 +604,19 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
                     } else {
 #pragma unroll
                         for (int b = 0; b < K; ++b)
-                            gr = fma(D[h * KK + b * K + kc] + (b == k ? rho : 0.0), vec[h * K + b], gr);
+                            gr = fma(b == k ? dk[h] : D[h * KK + b * K + kc], vec[h * K + b], gr);
                     }
                 }
                 const double v = (up >> h) & 1u ? gr : -gr;
-                if (v > wv) { wv = v; rel = h * K + k; }
+                if (above(v, wv)) { wv = v; rel = h * K + k; }
             }
         }
 #pragma unroll
-        for (int o = GL / 2; o > 0; o >>= 1) {
-            const double ov = __shfl_xor_sync(FULL, wv, o);
-            const int oi = __shfl_xor_sync(FULL, rel, o);
-            if (ov > wv || (ov == wv && oi < rel)) { wv = ov; rel = oi; }
+        for (int o = 1; o < K; o *= 2) {
+            const double ov = __shfl_sync(FULL, wv, next(o));
+            const int oi = __shfl_sync(FULL, rel, next(o));
+            const long long bo = __double_as_longlong(ov), bw = __double_as_longlong(wv);    // tol or above
+            if (bo > bw || (bo == bw && oi < rel)) { wv = ov; rel = oi; }
         }
         if (!done && !blocked) {
             if (rel == INT_MAX) done = true;

@@ -1,5 +1,6 @@
-"""Batched QPs at the edges of their lane layout (8 and 16 lanes per problem,
-64 problems per CTA) and on problems whose bounds bind, against the oracle's
+"""Batched QPs at the edges of their lane layout (K lanes per problem on
+the P side, with idle lanes where K does not divide 32; 64 problems per CTA on
+the Q side) and on problems whose bounds bind, against the oracle's
 solver.  The minimiser is unique, so both find the same point; 1e-9 is the
 bound the QP tests of this suite use for K up to 12."""
 import numpy as np
@@ -21,7 +22,7 @@ def problems(K, n, cols, seed):
     return X, z, rng
 
 
-@pytest.mark.parametrize("K", [1, 2, 7, 8, 9, 12])
+@pytest.mark.parametrize("K", [1, 2, 3, 7, 8, 9, 10, 12])
 @pytest.mark.parametrize("n", [1, 63, 65])
 def test_bounds_bind_and_last_groups(hx, O, K, n):
     c = small_cohort(40, 8, K, seed=K)
