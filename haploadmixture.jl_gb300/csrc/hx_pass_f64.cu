@@ -54,8 +54,10 @@ k_loglik64(PassArgs a, const uint8_t* __restrict__ bed, int64_t bps) {
     int e1 = 0, e2 = 0;
     bool zero = false, bad = false;
     auto times = [&](double v, bool twice) {
-        if (!(v > 0.0)) {
-            if (v == 0.0) zero = true; else bad = true;
+        // v > 0 in integers: a comparison takes an FP64 operation's time
+        const long long vb = __double_as_longlong(v);
+        if ((unsigned long long)(vb - 1) >= 0x7FF0000000000000ull) {
+            if ((vb << 1) == 0) zero = true; else bad = true;
             v = 1.0;
         }
         int e = 0;
