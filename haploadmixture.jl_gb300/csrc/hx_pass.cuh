@@ -19,7 +19,7 @@
 //
 // The EM numerators of em_loop!/em_kernel! (src/loops.jl:260-295,
 // src/cuda/kernels.jl:42-73) are q[k,i] * Xtz_q[k,i] and p[k,m] * Xtz_p[k,m],
-// so EM runs the gradient-only instances of the two accumulation kernels.
+// so EM runs the gradient-only forms of the two (k_grad_q and k_accum_p without HESS).
 //
 // No atomics: each output element has exactly one owner thread per chunk and
 // chunks are combined by a fixed-order FP64 reduction, so every pass is
@@ -56,11 +56,11 @@ template <int K> __device__ __forceinline__ constexpr int tri(int k, int k2) {
 }
 
 // ------------------------------------------------------------------ Q side
-template <int K, bool HESS>
+template <int K>
 __global__ void __launch_bounds__(ACC_THREADS)
 k_accum_q(PassArgs a) {
     constexpr int NH = K * (K + 1) / 2;
-    constexpr int NV = K + (HESS ? NH : 0);
+    constexpr int NV = K + NH;
     __shared__ float sp[QSTAGE_WORDS * 8 * 4 * K];
     __shared__ float4 s_snp[4];
     const int tid = threadIdx.x;
@@ -74,11 +74,11 @@ k_accum_q(PassArgs a) {
     for (int k = 0; k < K; ++k) qi[k] = active ? (float)a.q[(int64_t)K * i + k] : 1.f / K;
     float gin[K];
     double gout[K];
-    float H[HESS ? NH : 1];
+    float H[NH];
 #pragma unroll
     for (int k = 0; k < K; ++k) { gin[k] = 0.f; gout[k] = 0.0; }
 #pragma unroll
-    for (int v = 0; v < (HESS ? NH : 1); ++v) H[v] = 0.f;
+    for (int v = 0; v < NH; ++v) H[v] = 0.f;
 
     for (int ws = w0; ws < w1; ws += QSTAGE_WORDS) {
         const int nw = min(QSTAGE_WORDS, w1 - ws);
@@ -120,19 +120,17 @@ k_accum_q(PassArgs a) {
                         g = fma(u[3], pb[3 * K + k], g);
                         gin[k] = g;
                     }
-                    if (HESS) {
 #pragma unroll
-                        for (int h = 0; h < 4; ++h) {
-                            const float wh = u[h] * __frcp_rn(qp[h]);
-                            float t[K];
+                    for (int h = 0; h < 4; ++h) {
+                        const float wh = u[h] * __frcp_rn(qp[h]);
+                        float t[K];
 #pragma unroll
-                            for (int k = 0; k < K; ++k) t[k] = wh * pb[h * K + k];
+                        for (int k = 0; k < K; ++k) t[k] = wh * pb[h * K + k];
 #pragma unroll
-                            for (int k = 0; k < K; ++k)
+                        for (int k = 0; k < K; ++k)
 #pragma unroll
-                                for (int k2 = k; k2 < K; ++k2)
-                                    H[tri<K>(k, k2)] = fma(t[k], pb[h * K + k2], H[tri<K>(k, k2)]);
-                        }
+                            for (int k2 = k; k2 < K; ++k2)
+                                H[tri<K>(k, k2)] = fma(t[k], pb[h * K + k2], H[tri<K>(k, k2)]);
                     }
                 }
             }
@@ -145,11 +143,100 @@ k_accum_q(PassArgs a) {
         double* out = a.part + (int64_t)blockIdx.y * NV * a.Ipad;
 #pragma unroll
         for (int k = 0; k < K; ++k) out[(int64_t)k * a.Ipad + i] = gout[k];
-        if (HESS) {
 #pragma unroll
-            for (int v = 0; v < (HESS ? NH : 1); ++v) out[(int64_t)(K + v) * a.Ipad + i] = (double)H[v];
-        }
+        for (int v = 0; v < NH; ++v) out[(int64_t)(K + v) * a.Ipad + i] = (double)H[v];
     }
+}
+
+// Gradient only (EM): the same sums in the same order, with k_loglik2's layout of p
+// (one 16-byte load gives p[k, 4j..4j+3], used for qp and for the gradient), class
+// rows in packed FP32x2 arithmetic and the next stage's p and class words loaded
+// while this one is summed.  Bound by issue slots: 2 K packed FMAs, 4 K FMAs and
+// about 35 operations on the class per pair.  Per 1,000 pairs, against k_accum_q's
+// loop without its Hessian: K = 3 3.04 -> 2.27 ns, K = 5 3.71 -> 2.84, K = 8
+// 4.82 -> 3.75, K = 10 5.81 -> 4.44.
+template <int K>
+__global__ void __launch_bounds__(ACC_THREADS)
+k_grad_q(PassArgs a) {
+    __shared__ __align__(16) float spt[QSTAGE_WORDS * 8 * 4 * K];
+    __shared__ __align__(128) uint32_t s_cls[32];
+    const int tid = threadIdx.x;
+    cls_table_init(s_cls, tid);
+    const int64_t i = (int64_t)blockIdx.x * ACC_THREADS + tid;
+    const int w0 = blockIdx.y * a.per_chunk;
+    const int w1 = min(a.JW, w0 + a.per_chunk);
+    uint64_t qd[K];
+    float gin[K];
+    double gout[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        qd[k] = f2_dup(i < a.I ? (float)a.q[(int64_t)K * i + k] : 1.f / K);
+        gout[k] = 0.0;
+    }
+    const int64_t limit = a.J * 4 * K;
+    float nxt[2 * K];
+    auto fetch = [&](int ws) {
+        const int nval = min(QSTAGE_WORDS, w1 - ws) * 8 * 4 * K;
+        const int64_t base = (int64_t)ws * 8 * 4 * K;
+#pragma unroll
+        for (int v = 0; v < 2 * K; ++v) {
+            const int t = v * ACC_THREADS + tid;
+            nxt[v] = t < nval && base + t < limit ? a.pf[base + t] : 0.25f;
+        }
+    };
+    uint32_t nword = HX_PAD_WORD;
+    if (w0 < w1) {
+        fetch(w0);
+        nword = a.G[(int64_t)w0 * a.Ipad + i];
+    }
+    for (int ws = w0; ws < w1; ws += QSTAGE_WORDS) {
+        const int nw = min(QSTAGE_WORDS, w1 - ws);
+        __syncthreads();
+#pragma unroll
+        for (int v = 0; v < 2 * K; ++v) {
+            const int t = v * ACC_THREADS + tid, blk = t / (4 * K), r = t - blk * 4 * K, h = r / K, k = r - h * K;
+            spt[blk * 4 * K + k * 4 + h] = nxt[v];
+        }
+        __syncthreads();
+        if (ws + QSTAGE_WORDS < w1) fetch(ws + QSTAGE_WORDS);
+#pragma unroll
+        for (int k = 0; k < K; ++k) gin[k] = 0.f;
+#pragma unroll 1
+        for (int w = 0; w < nw; ++w) {
+            const uint32_t word = nword;
+            if (ws + w + 1 < w1) nword = a.G[(int64_t)(ws + w + 1) * a.Ipad + i];
+            const ulonglong2* pw = reinterpret_cast<const ulonglong2*>(spt + w * 8 * 4 * K);
+#pragma unroll 2
+            for (int b = 0; b < 8; ++b) {
+                ulonglong2 pk[K];
+                uint64_t z01 = 0ull, z23 = 0ull;
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    pk[k] = pw[b * K + k];
+                    z01 = f2_fma(qd[k], pk[k].x, z01);
+                    z23 = f2_fma(qd[k], pk[k].y, z23);
+                }
+                uint64_t u01, u23;
+                pair_u_cls(((word >> (4 * b)) & 0xFu) << 3, z01, z23, u01, u23, s_cls, 1.f);
+                float u0, u1, u2, u3;
+                f2_split(u01, u0, u1);
+                f2_split(u23, u2, u3);
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    float p0, p1, p2, p3;
+                    f2_split(pk[k].x, p0, p1);
+                    f2_split(pk[k].y, p2, p3);
+                    gin[k] = fmaf(u3, p3, fmaf(u2, p2, fmaf(u1, p1, fmaf(u0, p0, gin[k]))));
+                }
+            }
+        }
+        // promote the stage's gradient partial to FP64
+#pragma unroll
+        for (int k = 0; k < K; ++k) gout[k] += (double)gin[k];
+    }
+    double* out = a.part + (int64_t)blockIdx.y * K * a.Ipad;
+#pragma unroll
+    for (int k = 0; k < K; ++k) out[(int64_t)k * a.Ipad + i] = gout[k];
 }
 
 // ------------------------------------------------------------------ P side
