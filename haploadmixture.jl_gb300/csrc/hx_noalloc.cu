@@ -18,20 +18,46 @@ namespace hx {
 namespace {
 
 constexpr int NA_THREADS = 128;
+constexpr int NA_STAGE = 16;        // blocks whose p a CTA stages at a time
 
 // Scratch of the no-allocation entry point: one FP64 partial per CTA.
 __device__ __align__(256) double g_noalloc_scratch[HX_NOALLOC_SCRATCH];
+
+// One pair again in FP64, its mantissa and exponent folded in separately.
+template <int K>
+__device__ __noinline__ void redo_f64(unsigned nib, const double* qr, const double* pj, float& mant, int& ex, bool& zero,
+                                      bool& bad) {
+    double qd[4], Ld, ud[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < K; ++k) s = fma(qr[k], pj[h * K + k], s);
+        qd[h] = s;
+    }
+    pair_eval<double>(nib, qd, Ld, ud);
+    if (!(Ld > 0.0)) {
+        if (Ld == 0.0) zero = true; else bad = true;
+        return;
+    }
+    mant = renorm(mant * (float)renorm(Ld, ex), ex);
+}
 
 // Mixed method (the plain FP64 one is k_loglik64 in hx_pass_f64.cu): one
 // individual per thread over a chunk of blocks, decoding the two SNP codes
 // of each block straight from the BED bytes (src/loops.jl:55-71); pair
 // likelihoods multiply into an exponent-renormalised product (one log per
-// thread).  Writes one partial per CTA into scratch[blockIdx.y * gridDim.x + blockIdx.x].
+// CTA).  The CTA converts p to FP32 once per stage: a conversion is an FP64
+// operation, 64 clocks of a quarter of an SM for a warp, and with 4 K of them per
+// pair the kernel did little else (20,000 individuals x 10,000 blocks, K = 8:
+// 11.2 -> 0.90 ms).  Writes one partial per CTA into scratch[blockIdx.y * gridDim.x + blockIdx.x].
 template <int K>
 __global__ void __launch_bounds__(NA_THREADS)
 k_loglik_bed(const uint8_t* __restrict__ bed, int64_t bps, int64_t I, int64_t J, const double* __restrict__ q,
              const double* __restrict__ p, int64_t per_chunk, double* __restrict__ scratch) {
-    __shared__ double red[NA_THREADS];
+    __shared__ float sp[NA_STAGE * 4 * K];
+    __shared__ double red[NA_THREADS / 32];
+    __shared__ long long rex[NA_THREADS / 32];
     const int tid = threadIdx.x;
     const int64_t i = (int64_t)blockIdx.x * NA_THREADS + tid;
     const bool active = i < I;
@@ -43,21 +69,33 @@ k_loglik_bed(const uint8_t* __restrict__ bed, int64_t bps, int64_t I, int64_t J,
     float mant = 1.f;
     int ex = 0;
     bool zero = false, bad = false;
-    if (active) {
-        const int64_t byte = i >> 2;
-        const int sh = 2 * (int)(i & 3);
-        for (int64_t j = j0; j < j1; ++j) {
-            const unsigned c1 = (bed[(2 * j) * bps + byte] >> sh) & 3u;
-            const unsigned c2 = (bed[(2 * j + 1) * bps + byte] >> sh) & 3u;
-            const unsigned nib = c1 | (c2 << 2);
+    const int64_t byte = active ? i >> 2 : 0;
+    const int sh = 2 * (int)(i & 3);
+    for (int64_t js = j0; js < j1; js += NA_STAGE) {
+        const int nb = (int)min((int64_t)NA_STAGE, j1 - js);
+        unsigned codes[NA_STAGE];               // both codes of each block of the stage
+#pragma unroll
+        for (int b = 0; b < NA_STAGE; ++b) {
+            codes[b] = NIB_MM;
+            if (active && b < nb) {
+                const uint8_t* r = bed + 2 * (js + b) * bps + byte;
+                codes[b] = ((r[0] >> sh) & 3u) | (((r[bps] >> sh) & 3u) << 2);
+            }
+        }
+        __syncthreads();
+        for (int t = tid; t < nb * 4 * K; t += NA_THREADS) sp[t] = (float)p[(int64_t)K * 4 * js + t];
+        __syncthreads();
+#pragma unroll
+        for (int b = 0; b < NA_STAGE; ++b) {
+            const unsigned nib = codes[b];
             if (nib == NIB_MM) continue;
-            const double* pj = p + (int64_t)K * 4 * j;
+            const float* pj = sp + 4 * K * b;
             float qp[4];
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
                 float s = 0.f;
 #pragma unroll
-                for (int k = 0; k < K; ++k) s = fma(qi[k], (float)pj[h * K + k], s);
+                for (int k = 0; k < K; ++k) s = fma(qi[k], pj[h * K + k], s);
                 qp[h] = s;
             }
             float L, u[4];
@@ -67,20 +105,7 @@ k_loglik_bed(const uint8_t* __restrict__ bed, int64_t bps, int64_t I, int64_t J,
                 // Q/P entries far below the fit's 1e-5 floor): the renormaliser
                 // reads the exponent field, so redo this pair in FP64 and fold
                 // its mantissa and exponent in separately
-                double qd[4], Ld, ud[4];
-#pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    double s = 0.0;
-#pragma unroll
-                    for (int k = 0; k < K; ++k) s = fma((double)q[(int64_t)K * i + k], pj[h * K + k], s);
-                    qd[h] = s;
-                }
-                pair_eval<double>(nib, qd, Ld, ud);
-                if (!(Ld > 0.0)) {
-                    if (Ld == 0.0) zero = true; else bad = true;
-                    continue;
-                }
-                mant = renorm(mant * (float)renorm(Ld, ex), ex);
+                redo_f64<K>(nib, q + (int64_t)K * i, p + (int64_t)K * 4 * (js + b), mant, ex, zero, bad);
                 continue;
             }
             if (!(L > 0.f)) {
@@ -90,19 +115,30 @@ k_loglik_bed(const uint8_t* __restrict__ bed, int64_t bps, int64_t I, int64_t J,
             mant = renorm(mant * L, ex);
         }
     }
-    double v = 0.0;
-    if (active) {
-        v = log((double)mant) + (double)ex * 0.69314718055994530942;
-        if (zero) v = -INFINITY;
-        if (bad) v = NAN;
+    // the CTA's product, exponents apart, and one log
+    double m = mant;
+    long long e = ex;
+    auto mul = [&](double y) {
+        int x = 0;
+        m = renorm(m * y, x);
+        e += x;
+    };
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double y = __shfl_xor_sync(0xffffffffu, m, o);
+        e += __shfl_xor_sync(0xffffffffu, e, o);
+        mul(y);
     }
-    red[tid] = v;
+    const bool any_zero = __syncthreads_or(zero), any_bad = __syncthreads_or(bad);
+    if ((tid & 31) == 0) { red[tid >> 5] = m; rex[tid >> 5] = e; }
     __syncthreads();
-    for (int s = NA_THREADS / 2; s > 0; s >>= 1) {
-        if (tid < s) red[tid] += red[tid + s];
-        __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < NA_THREADS / 32; ++w) { e += rex[w]; mul(red[w]); }
+        double v = log(m) + (double)e * 0.69314718055994530942;
+        if (any_zero) v = -INFINITY;
+        if (any_bad) v = NAN;
+        scratch[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = v;
     }
-    if (tid == 0) scratch[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = red[0];
 }
 
 // Sums the n partials in a fixed order into *out (one CTA).
