@@ -62,21 +62,30 @@ template <typename T> __device__ __forceinline__ T rcp(T x);
 template <> __device__ __forceinline__ float rcp<float>(float x) { return __frcp_rn(x); }
 template <> __device__ __forceinline__ double rcp<double>(double x) { return 1.0 / x; }
 
-// 1/x by one step of the cubically convergent form of Newton's iteration
-// (Householder): r (1 + e + e^2), e = 1 - x r, from the hardware's 20-bit
-// reciprocal: e^3 < 2^-56.  Three FP64 operations instead of the eight or more
-// of a division.  Outside 2^-1000 .. 2^1000 (zeros, NaN, infinities) it divides,
-// out of line: inlined, the division's predicated-off operations still took
-// their issue slots (104 instead of 74 FP64 instructions per 64 pairs at K = 5).
+// 1/x in fixed point, to 0.5001 ulp: from the hardware's FP32 reciprocal y of the
+// significand m cut to 24 bits, one step y (1 + e + e^2), e = 1 - m y < 2^-22 (the
+// cubically convergent form of Newton's iteration; e, from the low 64 bits of the
+// product, is exact), and one rounding.  About 30 integer operations, which find free
+// issue slots where an FP64 operation takes 64 clocks of its quarter of an SM: the
+// same step in FP64 was 3 of the K + 4 operations per item of the plain passes,
+// and those were what bound them.  Outside 2^-1000 .. 2^1000 (zeros, NaN,
+// infinities) and below zero it divides, out of line.
 static __device__ __noinline__ double rcp64_edge(double x) { return 1.0 / x; }
 __device__ __forceinline__ double rcp64(double x) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    const double e = fma(-x, r, 1.0);
-    r = fma(r, fma(e, e, e), r);
-    const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7FFu;
-    if (ex - 23u > 2000u) r = rcp64_edge(x);
-    return r;
+    typedef long long i64;
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), ex = hi >> 20;
+    if (ex - 23u > 2000u) return rcp64_edge(x);
+    float y0;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0)
+        : "f"(__uint_as_float(0x3F800000u | ((hi & 0xFFFFFu) << 3) | (lo >> 29))));
+    const unsigned Y = (__float_as_uint(fminf(y0, 0x1.fffffep-1f)) << 7) ^ 0xC0000000u;    // y 2^31
+    const unsigned long long m = ((unsigned long long)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo;   // 2^52
+    const i64 e = -(i64)(m * Y);                                // 2^83
+    const int e1 = (int)(e >> 37);                              // 2^46
+    const i64 d = e + (((i64)e1 * e1) >> 9);                    // e + e^2, 2^83
+    const i64 c = (i64)(int)(d >> 32) * Y + __umulhi((unsigned)d, Y);    // y d, 2^82
+    const i64 r = (i64)((unsigned long long)Y << 22) + ((c + (1ll << 28)) >> 29);          // 2^53 / m
+    return __longlong_as_double(r + ((i64)(2044u - ex) << 52));
 }
 
 // Per-pair evaluation.  Given the class nibble and the mixed haplotype

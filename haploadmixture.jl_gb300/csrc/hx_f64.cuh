@@ -301,33 +301,25 @@ __device__ __forceinline__ void f64_weights(const unsigned (&nib)[2], const doub
         nc += __popc(bal);
     }
     __syncwarp();
+    // two lanes per pair, one for each set
 #pragma unroll 1
-    for (int base = 0; base < nc; base += 32) {
-        if (base + (int)lane < nc) {
-            const unsigned it = list[base + lane];
-            const unsigned nb = it >> 6, nd = (unsigned)(TAB_NEED >> (4 * nb)) & 0xFu;
-            double* rp = rb + ((it >> 5) & 1u) * 128 + (it & 31u);
-            const bool hh = nb == NIB_HH, m1 = (nb & 3u) == 1u;
-            const int ib = hh ? 3 : (m1 ? 2 : 1), ic = hh || m1 ? 1 : 2, id = hh ? 2 : 3;
-            const bool ab = nd & 1u, cd = (nd >> ic) & 1u;       // a set is needed as a whole
-            const double ra = ab ? rp[0] : 1.0, rbb = ab ? rp[32 * ib] : 1.0;
-            const double rc = cd ? rp[32 * ic] : 1.0, rd = cd ? rp[32 * id] : 1.0;
-            const double x = ra * rbb, y = rc * rd;
-            const double d1 = hh ? x + y : ra + rbb, d2 = hh ? 1.0 : rc + rd;
-            const double t = rcp64(d1 * d2);
-            const double t1 = t * d2, t2 = t * d1;
-            const double e1 = (hh ? y : x) * t1, e2 = (hh ? x : y) * (hh ? t1 : t2);
-            const double f = ab && cd ? 1.0 : 2.0;
-            if (ab) {
-                const double ma = hh ? ra : f, mb = hh ? rbb : f;
-                rp[0] = HESS ? (e1 * ra) * ma : e1 * ma;
-                rp[32 * ib] = HESS ? (e1 * rbb) * mb : e1 * mb;
-            }
-            if (cd) {
-                const double mc = hh ? rc : f, md = hh ? rd : f;
-                rp[32 * ic] = HESS ? (e2 * rc) * mc : e2 * mc;
-                rp[32 * id] = HESS ? (e2 * rd) * md : e2 * md;
-            }
+    for (int base = 0; base < 2 * nc; base += 32) {
+        const int slot = base + (int)lane;
+        const unsigned it = list[min(slot >> 1, nc - 1)], set = lane & 1u;
+        const unsigned nb = it >> 6, nd = (unsigned)(TAB_NEED >> (4 * nb)) & 0xFu;
+        const bool hh = nb == NIB_HH, m1 = (nb & 3u) == 1u;
+        const int ia = set ? (hh || m1 ? 1 : 2) : 0, ib = set ? (hh ? 2 : 3) : (hh ? 3 : (m1 ? 2 : 1));
+        double* rp = rb + ((it >> 5) & 1u) * 128 + (it & 31u);
+        const bool mine = slot < 2 * nc && ((nd >> ia) & 1u);    // a set is needed as a whole
+        const bool both = __shfl_xor_sync(0xffffffffu, mine, 1) && mine;
+        const double ra = mine ? rp[32 * ia] : 1.0, rbb = mine ? rp[32 * ib] : 1.0;
+        const double own = ra * rbb, oth = __shfl_xor_sync(0xffffffffu, own, 1);
+        const double e = (hh ? oth : own) * rcp64((hh ? own : ra) + (hh ? oth : rbb));
+        const double f = both ? 1.0 : 2.0;
+        const double ma = hh ? ra : f, mb = hh ? rbb : f;
+        if (mine) {
+            rp[32 * ia] = HESS ? (e * ra) * ma : e * ma;
+            rp[32 * ib] = HESS ? (e * rbb) * mb : e * mb;
         }
     }
     __syncwarp();
