@@ -1,11 +1,13 @@
 // hx_f64.cuh -- the plain (FP64) method's gradient and Hessian passes.
 //
-// GB300's FP64 unit issues 2 operations per clock and SM, 1/64 of the FP32
-// rate, so a pass that does its K(K+1)/2 accumulations per haplotype there
+// GB300's FP64 units do 2 operations per clock and SM, 1/64 of the FP32
+// rate (a warp's operation takes 64 clocks of its quarter of an SM, however few lanes
+// work), so a pass that does its K(K+1)/2 accumulations per haplotype there
 // costs 90 to 160 clocks per (individual, block) pair (K = 5 .. 8).  These
 // passes keep on the FP64 unit only what has to be there, and only for the
 // haplotypes that a pair's genotypes allow (1.8 of 4 on average):
-//   qp_h = sum_k q[k,i] p[k,4j+h], r_h = 1 / qp_h, and the pair's weights
+//   qp_h = sum_k q[k,i] p[k,4j+h] and the pair's weights, from r_h = 1 / qp_h
+//   (which rcp64 forms in integers),
 //   W_h = c_h r_h^2 (Hessian) or U_h = c_h r_h (gradient only),
 // and form the sums H = sum W v v' (v = p on the Q side, q on the P side;
 // src/loops.jl:328-403) exactly on the tensor cores: the error-free splitting
@@ -368,10 +370,17 @@ __device__ __noinline__ void f64_rare(double w, const double* vrow, const unsign
 // 2 (w >> 2), +1.  PS = true (P side): CTA rows = the 128 columns m of 32
 // blocks, stage = 32 individuals; warp w: blocks 2w, 2w+1.  Chunks of the
 // reduction along grid.y, column groups along grid.z.
-// Bound by the FP64 unit: about (K + 5) operations per needed haplotype.  One
-// CTA per SM (480 of 512 TMEM columns at K = 8); the digit tiles need one
-// buffer only, because a stage's FP64 work (registers and warp-private shared
-// memory) runs while the MMAs of the stage before read it.
+// FP64 operations take 63% of the clocks (K + 1 per needed haplotype, 7 per pair
+// with qp-dependent counts; they were 80% to 88% with the reciprocals among them),
+// issue 43% and the MMAs about as much as FP64; the rest is a warp's own chain from
+// class to digits, in which the 16 warps move together.  One CTA per SM (480 of 512
+// TMEM columns at K = 8; shared memory has no room for a second set of digit
+// tiles): a stage's FP64 work (registers and warp-private shared memory) runs while
+// the MMAs of the stage before read the tiles.  Writing and issuing the digits in
+// three words, so that a stage's first MMAs need not wait for its last digits, gained
+// nothing (2.72 ms for 2.68).
+// 10,000 individuals x 5,000 blocks, K = 5: Q pass 3.43 ms with the reciprocals in
+// FP64, 2.68 now.
 template <int K, bool HESS, bool PS>
 __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args fa) {
     using D = FDim<K, HESS>;

@@ -14,7 +14,7 @@ int loglik_f32x2_blocks(int64_t Ipad, int K) {
 }
 
 int loglik_f32x2_resident(int K) {
-#define HX_CASE(KK) case KK: return resident_ctas((const void*)k_loglik2<KK, 2>, ACC_THREADS, 0, 0);
+#define HX_CASE(KK) case KK: return resident_ctas((const void*)k_loglik2<KK, 2>, ACC_THREADS, 0);
     switch (K) { HX_FOR_K(HX_CASE) default: return 1; }
 #undef HX_CASE
 }

@@ -602,7 +602,7 @@ cudaError_t launch_d2f(const double* a, int64_t n, float* out, cudaStream_t st) 
     k_d2f<<<nblk(n, 256), 256, 0, st>>>(a, n, out);
     return cudaGetLastError();
 }
-int resident_ctas(const void* kernel, int threads, size_t dyn_smem, int tmem_cols) {
+int resident_ctas(const void* kernel, int threads, size_t dyn_smem) {
     cudaFuncAttributes at{};
     int dev = 0, regs_sm = 0, smem_sm = 0, resv = 0, thr_sm = 0, blk_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaFuncGetAttributes(&at, kernel) != cudaSuccess) return 1;
@@ -620,7 +620,6 @@ int resident_ctas(const void* kernel, int threads, size_t dyn_smem, int tmem_col
     }
     const size_t per = at.sharedSizeBytes + dyn_smem + (size_t)resv;
     if (per > 0) n = std::min(n, (int)((size_t)smem_sm / per));
-    if (tmem_cols > 0) n = std::min(n, 512 / tmem_cols);
     return std::max(n, 1);
 }
 

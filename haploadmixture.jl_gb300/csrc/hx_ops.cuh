@@ -23,11 +23,9 @@ int loglik_f32x2_resident(int K);   // CTAs of launch_loglik_f32x2 resident on o
 // CTAs of a kernel resident on one SM of the current device, from its
 // registers (8-register steps per thread, 256-register steps per warp, a
 // quarter of the file per SM sub-partition), its shared memory (static +
-// dynamic + the driver's reserve), its threads and, for kernels that
-// allocate them, TMEM columns (512 per SM).  The runtime's occupancy
-// calculator reports one CTA for the tensor-core passes where the hardware
-// holds two, so the limits are applied here.
-int resident_ctas(const void* kernel, int threads, size_t dyn_smem, int tmem_cols);
+// dynamic + the driver's reserve) and its threads.  (The tensor-core passes'
+// counts are part of their chunk plans: TcDims::MINB.)
+int resident_ctas(const void* kernel, int threads, size_t dyn_smem);
 
 // tensor-core (tcgen05) Hessian+gradient passes of the mixed method (hx_tc.cu)
 // Host operations on the tensor-core instantiation of one K (hx_tc_impl.cuh);

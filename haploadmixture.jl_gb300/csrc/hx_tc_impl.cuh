@@ -10,7 +10,7 @@
 // with m = 4j+h, U = c_h/qp_h, W = c_h/qp_h^2, PP[m,(k,k2)] = p[k,m] p[k2,m]
 // (upper triangle) and QQ[i,(k,k2)] = q[k,i] q[k2,i].  The CUDA cores evaluate
 // each (individual, block) pair once (qp, class, U, W) and write 16-bit hi/lo
-// splits of U and W into shared memory; one thread issues
+// splits of U and W into shared memory; one warp issues
 // tcgen05.mma kind::f16 (16-bit x 16-bit -> fp32 in TMEM) for hi*hi + hi*lo + lo*hi.
 // The Hessian operands use BF16 (8-bit exponent) because W spans ~1 .. 2e10,
 // beyond FP16's range: hi+lo carries 16 significant bits.  The gradient
@@ -29,15 +29,18 @@
 // 1-D bulk copies (TMA engine) into a RING-deep shared-memory ring, completing
 // on an mbarrier with a transaction count.
 //
-// Pipeline per stage, with no CTA-wide barrier in the loop: every thread waits
-// for the stage's ring slot and until the MMAs that last read its A buffer
-// (stage s-2) are done; the first warp to get there refills the ring slot of
-// stage s-2 with stage s-2+RING; every warp generates its part of the A tiles and arrives on
-// a shared counter; the last arriving warp issues the stage's MMAs and commits
-// them to an mbarrier.  Warps therefore run up to two stages apart, and two CTAs (16 warps)
-// share an SM.  Every wait is bounded (PassArgs::budget cycles, by default
-// TC_BUDGET; the drain after a timeout always allows TC_BUDGET); a timeout sets
-// slots[S_TC_TIMEOUT] and the CTA drains and exits.
+// Pipeline per stage, with no CTA-wide barrier in the loop.  Eight warps generate; a
+// ninth keeps the rings of stage inputs filled, issues every MMA and commits them
+// to mbarriers.  It tells the generators by one barrier per stage buffer (go) that
+// the stage's inputs have landed and the MMAs that last read the buffer (stage
+// s-2) are done; each generating warp arrives on gen when its part of the A tiles
+// is written.  Warps therefore run up to two stages apart, and two CTAs (18 warps)
+// share an SM.  With the last arriving warp as the issuer, its own generation
+// stood behind the MMAs' issue (48 clocks each or more): per 1,000 pairs at K = 8
+// the Q pass took 4.6 ns instead of 4.1, the P pass 6.4 instead of 6.0.  Every wait
+// is bounded (PassArgs::budget cycles, by default TC_BUDGET; the drain after a
+// timeout always allows TC_BUDGET); a timeout sets slots[S_TC_TIMEOUT] and the CTA
+// drains and exits.
 #pragma once
 #include <algorithm>
 #include "hx_ops.cuh"
@@ -87,7 +90,8 @@ template <int K> struct TcDims {
     // of the Hessian side by side, then the same for the gradient
     static constexpr int WS = 2 * NHP + 2 * NG;
     static constexpr int TCOLS_S = (2 * WS <= 32) ? 32 : (2 * WS <= 64) ? 64 : (2 * WS <= 128) ? 128 : (2 * WS <= 256) ? 256 : 512;
-    // CTAs per SM: 2 while the generators fit in 128 registers, else 1
+    // CTAs per SM: 2 while the threads' sums fit beside the rest in 96 registers (18
+    // warps: five on one quarter of the SM), else 1
     static constexpr int MINB = K <= 8 ? 2 : 1;
 };
 
@@ -225,10 +229,9 @@ __device__ __forceinline__ void compensate(float* acc, const float* comp) {
 // The 3 split products of one 32-deep stage into D (TMEM cols dcol..):
 // Hessian (N = NHP, bf16) and gradient (N = 16, fp16).  A tiles W_hi, W_lo,
 // U_hi, U_lo at aBase + t*aStride; B tiles: hi at bBase, lo at bBase + B_TILE.
-// Issued in two groups with disjoint accumulator columns, by two issuers: the
-// Hessian's (HG = 0) and the gradient's (HG = 1).  Each column keeps one
-// issuer, issuing in stage order, so the FP32 accumulation order is fixed
-// (bit-reproducible).
+// In two groups with disjoint accumulator columns, the Hessian's (HG = 0) and the
+// gradient's (HG = 1), each issued in stage order, so the FP32 accumulation order
+// is fixed (bit-reproducible).
 template <int K, int HG>
 __device__ __forceinline__ void issue_stage_group(uint32_t tmem, int dcol, uint32_t aBase, int aStride, int aLBO,
                                                   int aSBO, uint32_t bBase, bool first, uint32_t el) {
