@@ -168,11 +168,11 @@ TRAFFIC_PER_PAIR = {"accum_q": 0.592, "accum_p": 0.588}
 
 # Warp instructions per (individual, block) pair that the mixed method's pass
 # kernels execute at K=8 (ncu smsp__inst_executed.sum over one launch at
-# I=100,000, J=5,000, divided by the 5e8 pairs).  These passes are bound by
+# I=100,000, J=20,000, divided by the 2e9 pairs).  These passes are bound by
 # instruction issue (the CUDA cores generate the tensor core's A operand), so
 # their third roofline is the issue rate: one warp instruction per clock in
 # each of an SM's 4 sub-partitions.
-ISSUE_INST_PER_PAIR = {("accum_q", 8): 4.12, ("accum_p", 8): 5.22, ("loglik", 8): 1.96}
+ISSUE_INST_PER_PAIR = {("accum_q", 8): 2.97, ("accum_p", 8): 4.18, ("loglik", 8): 1.90}
 SMS = 152
 
 
@@ -341,7 +341,7 @@ def issue_roofline(kind, I, J, K, per_launch_ms, sm_mhz):
     peak = SMS * 4 * sm_mhz * 1e6
     return {"achieved": achieved, "peak": peak, "unit": "warp instructions/s", "frac": achieved / peak,
             "warp_inst_per_pair": ipp, "sm_mhz": sm_mhz,
-            "source": "instructions per pair from ncu smsp__inst_executed.sum at I=1e5, J=5e3, K=8 (the same "
+            "source": "instructions per pair from ncu smsp__inst_executed.sum at I=1e5, J=2e4, K=8 (the same "
                       "kernel); peak = 152 SMs x 4 issue slots per clock at the median SM clock of this run"}
 
 
