@@ -811,12 +811,22 @@ __global__ void __launch_bounds__(TCI_THREADS, TcDims<K>::MINB) k_accum_p_tc(Pas
         const int64_t j = (int64_t)blockIdx.x * 32 + jl;
         const bool valid = j < a.J;
         const uint32_t taddr_lane = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+        // The block's 4 K frequencies in FP32: each of its eight lanes converts an eighth
+        // (a conversion takes 64 clocks of a quarter of an SM) and the others fetch it.
         uint64_t pr2[2 * K];
+        {
+            float pv[(K + 1) / 2];
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const double* pj = a.p + (int64_t)K * 4 * j + k;
-            pr2[2 * k] = valid ? f2_pack((float)pj[0], (float)pj[K]) : f2_dup(0.25f);
-            pr2[2 * k + 1] = valid ? f2_pack((float)pj[2 * K], (float)pj[3 * K]) : f2_dup(0.25f);
+            for (int u = 0; u < (K + 1) / 2; ++u) {
+                const int t = 8 * u + ig;
+                pv[u] = valid && t < 4 * K ? (float)a.p[(int64_t)K * 4 * j + t] : 0.25f;
+            }
+            auto at = [&](int t) { return __shfl_sync(0xffffffffu, pv[t / 8], t % 8, 8); };
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                pr2[2 * k] = f2_pack(at(k), at(K + k));
+                pr2[2 * k + 1] = f2_pack(at(2 * K + k), at(3 * K + k));
+            }
         }
         float acc[C::N], comp[8 * C::CG];
 #pragma unroll
