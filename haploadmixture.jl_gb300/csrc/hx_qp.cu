@@ -315,6 +315,7 @@ template <int K> struct PDim {
     // problems of a warp start in different banks
     static constexpr int LD = (RAW + 15) / 16 * 16 + (K % 4 == 0 ? 4 : K);
     static constexpr size_t SMEM = (size_t)WARPS * PW * LD * sizeof(double);
+    static_assert(PW * LD >= 16 * K * K + 44 * K, "a warp's memory holds the dense solver's work");
 };
 
 // One block on the dense solver, by a whole warp; base: 16 K^2 + 44 K doubles.
