@@ -81,7 +81,10 @@ size_t f64_image_bytes(int K, int64_t I, int64_t J);
 cudaError_t launch_f64_reduce(const double* part, int S, int K, bool hess, int64_t rows, int64_t ld, const double* x,
                               const unsigned long long* mx, int nmx, const F64Rare& rare, double* XtX, double* Xtz,
                               cudaStream_t st);
-constexpr int F64_MAX_STAGES = 2048;  // stages per chunk: bounds the 64-bit sums
+// Stages per chunk, 32 reduction indices each.  The 64-bit sums of orders 5 .. 9 take at
+// most 6 x 2^14 x 2^32 + 7 x 2^14 x 2^24 + ... < 2^48.6 per index in units of 2^-62, so
+// 2^14.3 indices (679 stages) stay below 2^63 whatever the digits are.
+constexpr int F64_MAX_STAGES = 512;
 
 cudaError_t launch_f2d(const float* a, int64_t n, double* out, cudaStream_t st);
 cudaError_t launch_d2f(const double* a, int64_t n, float* out, cudaStream_t st);
