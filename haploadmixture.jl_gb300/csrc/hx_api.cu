@@ -315,15 +315,17 @@ int stage_pf(hx_ctx* c, const double* p, PassArgs& a) {
     return HX_OK;
 }
 
-// The plain method's pass of one side: maxima, stage images, pass, reduction.
+// The plain method's pass of one side: range, stage images, digit pass or general
+// pass, reduction.
 int pass_f64(hx_ctx* c, bool p_side, const double* q, const double* p, bool hess, double* XtX, double* Xtz) {
-    F64Call f{p_side, hess, pass_args(c, q, p), c->f64_mx, c->rare, c->st};
+    F64Call f{p_side, hess, pass_args(c, q, p), p_side ? c->S_p : c->S_q, p_side ? c->ipc_p : c->wpc_q, c->f64_mx,
+              c->rare, c->st};
     f.a.S = p_side ? c->S_pf : c->S_qf;
     f.a.per_chunk = p_side ? c->spc_pf : c->spc_qf;
     f.a.part = p_side ? c->part_p : c->part_q;
     f.a.XtX = XtX;
     f.a.Xtz = Xtz;
-    HX_LAUNCH(p_side ? (hess ? HX_KIND_ACCUM_P : HX_KIND_EM_P) : (hess ? HX_KIND_ACCUM_Q : HX_KIND_EM_Q), 4,
+    HX_LAUNCH(p_side ? (hess ? HX_KIND_ACCUM_P : HX_KIND_EM_P) : (hess ? HX_KIND_ACCUM_Q : HX_KIND_EM_Q), 5,
               launch_f64_pass(c->K, f));
     return HX_OK;
 }
@@ -603,8 +605,8 @@ int create_common(const uint8_t* bed, bool bed_on_device, int64_t bps, int64_t n
     need(rq, &c->Xtzp, (size_t)K * 4 * J);
     const size_t NH = (size_t)K * (K + 1) / 2, rows = (size_t)std::max<int64_t>(I, 4 * J);
     if (c->prec == HX_PREC_FP64) {
-        need(rq, &c->part_q, (size_t)c->S_qf * NH * c->Ipad);
-        need(rq, &c->part_p, (size_t)c->S_pf * NH * 4 * J);
+        need(rq, &c->part_q, std::max<size_t>(c->S_qf * NH, (size_t)c->S_q * NVmax) * c->Ipad);
+        need(rq, &c->part_p, std::max<size_t>(c->S_pf * NH, (size_t)c->S_p * NVmax) * 4 * J);
         need(rq, &c->img, f64_image_bytes(K, I, J));
         need(rq, &c->f64_mx, (size_t)F_MAXB * F_MXS);
         need(rq, &c->rare.i, 2 * rows * NH);

@@ -181,6 +181,14 @@ __device__ __forceinline__ float pair_lik_tab(unsigned nib, const float qp[4], c
     return F1 * F2;
 }
 
+// Type-generic entry: FP32 uses the indicator table, FP64 the exact select form.
+__device__ __forceinline__ void pair_eval_t(unsigned nib, const float qp[4], float& L, float u[4], const float4* tab) {
+    pair_eval_tab(nib, qp, L, u, tab);
+}
+__device__ __forceinline__ void pair_eval_t(unsigned nib, const double qp[4], double& L, double u[4], const float4*) {
+    pair_eval<double>(nib, qp, L, u);
+}
+
 // Packed FP32x2 arithmetic (sm_100+): fma.rn.f32x2 performs two IEEE FMAs,
 // lane by lane, with the results of two fmaf calls.
 __device__ __forceinline__ uint64_t f2_dup(float x) {

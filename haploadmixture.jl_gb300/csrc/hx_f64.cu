@@ -34,87 +34,101 @@ size_t f64_image_bytes(int K, int64_t I, int64_t J) {
 }
 
 namespace {
-// Chunk sums -> XtX (both triangles) and Xtz = XtX x (see hx_f64.cuh), or Xtz
-// itself for the gradient-only pass.  Block: 32 rows; a warp sums one value
-// of 32 consecutive rows (coalesced), the results go out through shared memory,
-// so that the K x K blocks are written in order too.
+// Chunk sums -> XtX (both triangles) and Xtz.  Those of the digit passes (S chunks of
+// NH = NV - K values) give Xtz = XtX x (see hx_f64.cuh), or are Xtz itself for the
+// gradient-only pass; where the general passes ran (Sg chunks), Xtz leads each chunk.
+// Block: 32 rows; a warp sums one value of 32 consecutive rows (coalesced), the results
+// go out through shared memory, so that the K x K blocks are written in order too.
 constexpr int FR_ROWS = 32;
-__global__ void __launch_bounds__(256) k_f64_reduce(const double* __restrict__ part, int S, int K, int NV, bool hess,
+__global__ void __launch_bounds__(256) k_f64_reduce(const double* __restrict__ part, int S, int Sg, int K, bool hess,
                                                     int64_t rows, int64_t ld, const double* __restrict__ x,
                                                     const unsigned long long* __restrict__ mx, int nmx, F64Rare rare,
                                                     double* __restrict__ XtX, double* __restrict__ Xtz) {
-    extern __shared__ double tile[];   // [NV][FR_ROWS + 1]
+    extern __shared__ double tile[];   // [K + NH][FR_ROWS + 1]: Xtz, then the triangle
     __shared__ int se[HX_KMAX];
-    __shared__ bool bad;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid == 0) bad = false;
-    __syncthreads();
-    if (tid < K) {
-        unsigned long long m = 0ull;
-        for (int b = 0; b < nmx; ++b) m = max(m, mx[(int64_t)b * F_MXS + tid]);
-        const int f = (int)(m >> 52);
-        se[tid] = f == 0 || f == 0x7FF ? 0 : f - 1022;
-        if (f == 0x7FF) bad = true;
-    }
-    __syncthreads();
+    const bool general = __syncthreads_or(tid < nmx && mx[tid * F_MXS + HX_KMAX] != 0ull);
+    const int NH = hess ? K * (K + 1) / 2 : 0;
     const int64_t r0 = (int64_t)blockIdx.x * FR_ROWS, r = r0 + lane;
-    const int flag = *rare.flag;
-    int k = 0, k2 = 0;                 // of value v
-    for (int v = 0, left = warp; v < NV; ++v) {
-        if (left == 0) {
-            left = 8;
+    if (general) {
+        for (int v = warp; v < K + NH; v += 8) {
             double s = 0.0;
             if (r < rows) {
                 const double* src = part + (int64_t)v * ld + r;
 #pragma unroll 8
-                for (int c = 0; c < S; ++c) s += src[(int64_t)c * NV * ld];
-                if (flag) {            // products of out-of-range weights; left zero for the next pass
-                    const int64_t at = r * NV + v;
-                    s += scalbn((double)rare.i[2 * at], -8) + scalbn((double)rare.i[2 * at + 1], -56);
-                    rare.i[2 * at] = 0;
-                    rare.i[2 * at + 1] = 0;
-                    if (flag & 2) {
-                        s += rare.d[at];
-                        rare.d[at] = 0.0;
-                    }
-                }
-                s = bad ? NAN : scalbn(s, hess ? se[k] + se[k2] : se[v]);
+                for (int c = 0; c < Sg; ++c) s += src[(int64_t)c * (K + NH) * ld];
             }
             tile[v * (FR_ROWS + 1) + lane] = s;
         }
-        --left;
-        if (++k2 == K) { ++k; k2 = k; }
+    } else {
+        if (tid < K) {
+            unsigned long long m = 0ull;
+            for (int b = 0; b < nmx; ++b) m = max(m, mx[(int64_t)b * F_MXS + tid]);
+            se[tid] = (int)(m >> 52) - 1022;
+        }
+        __syncthreads();
+        const int NV = hess ? NH : K;
+        const int flag = *rare.flag;
+        int k = 0, k2 = 0;             // of value v
+        for (int v = 0, left = warp; v < NV; ++v) {
+            if (left == 0) {
+                left = 8;
+                double s = 0.0;
+                if (r < rows) {
+                    const double* src = part + (int64_t)v * ld + r;
+#pragma unroll 8
+                    for (int c = 0; c < S; ++c) s += src[(int64_t)c * NV * ld];
+                    if (flag) {        // products of out-of-range weights; left zero for the next pass
+                        const int64_t at = r * NV + v;
+                        s += scalbn((double)rare.i[2 * at], -8) + scalbn((double)rare.i[2 * at + 1], -56);
+                        rare.i[2 * at] = 0;
+                        rare.i[2 * at + 1] = 0;
+                        if (flag & 2) {
+                            s += rare.d[at];
+                            rare.d[at] = 0.0;
+                        }
+                    }
+                    s = scalbn(s, hess ? se[k] + se[k2] : se[v]);
+                }
+                tile[((hess ? K : 0) + v) * (FR_ROWS + 1) + lane] = s;
+            }
+            --left;
+            if (++k2 == K) { ++k; k2 = k; }
+        }
+        if (hess) {
+            __syncthreads();
+            for (int t = tid; t < FR_ROWS * K; t += 256) {
+                const int row = t / K, a = t - row * K;
+                double g = 0.0;
+                if (r0 + row < rows)
+                    for (int b = 0; b < K; ++b) {
+                        const int lo = min(a, b), hi = max(a, b);
+                        g = fma(tile[(K + lo * K - lo * (lo - 1) / 2 + hi - lo) * (FR_ROWS + 1) + row],
+                                x[(r0 + row) * K + b], g);
+                    }
+                tile[a * (FR_ROWS + 1) + row] = g;
+            }
+        }
     }
     __syncthreads();
     const int nr = (int)min((int64_t)FR_ROWS, rows - r0);
-    if (!hess) {
-        for (int t = tid; t < nr * K; t += 256) Xtz[r0 * K + t] = tile[(t % K) * (FR_ROWS + 1) + t / K];
-        return;
-    }
+    for (int t = tid; t < nr * K; t += 256) Xtz[r0 * K + t] = tile[(t % K) * (FR_ROWS + 1) + t / K];
+    if (!hess) return;
     const int KK = K * K;
     for (int t = tid; t < nr * KK; t += 256) {
         const int row = t / KK, e = t - row * KK, a = e / K, b = e - a * K;
         const int lo = min(a, b), hi = max(a, b);
-        XtX[r0 * KK + t] = tile[(lo * K - lo * (lo - 1) / 2 + hi - lo) * (FR_ROWS + 1) + row];
-    }
-    for (int t = tid; t < nr * K; t += 256) {
-        const int row = t / K, a = t - row * K;
-        double g = 0.0;
-        for (int b = 0; b < K; ++b) {
-            const int lo = min(a, b), hi = max(a, b);
-            g = fma(tile[(lo * K - lo * (lo - 1) / 2 + hi - lo) * (FR_ROWS + 1) + row], x[(r0 + row) * K + b], g);
-        }
-        Xtz[r0 * K + t] = g;
+        XtX[r0 * KK + t] = tile[(K + lo * K - lo * (lo - 1) / 2 + hi - lo) * (FR_ROWS + 1) + row];
     }
 }
 }  // namespace
 
-cudaError_t launch_f64_reduce(const double* part, int S, int K, bool hess, int64_t rows, int64_t ld, const double* x,
-                              const unsigned long long* mx, int nmx, const F64Rare& rare, double* XtX, double* Xtz,
-                              cudaStream_t st) {
-    const int NV = hess ? K * (K + 1) / 2 : K;
-    const size_t smem = (size_t)NV * (FR_ROWS + 1) * sizeof(double);   // <= 20.6 KB (K = 12)
-    k_f64_reduce<<<(unsigned)((rows + FR_ROWS - 1) / FR_ROWS), 256, smem, st>>>(part, S, K, NV, hess, rows, ld, x, mx,
+cudaError_t launch_f64_reduce(const double* part, int S, int Sg, int K, bool hess, int64_t rows, int64_t ld,
+                              const double* x, const unsigned long long* mx, int nmx, const F64Rare& rare, double* XtX,
+                              double* Xtz, cudaStream_t st) {
+    const int NV = K + (hess ? K * (K + 1) / 2 : 0);
+    const size_t smem = (size_t)NV * (FR_ROWS + 1) * sizeof(double);   // <= 23.8 KB (K = 12)
+    k_f64_reduce<<<(unsigned)((rows + FR_ROWS - 1) / FR_ROWS), 256, smem, st>>>(part, S, Sg, K, hess, rows, ld, x, mx,
                                                                                 nmx, rare, XtX, Xtz);
     return cudaGetLastError();
 }

@@ -88,42 +88,46 @@ template <int K, bool HESS, bool PS> constexpr size_t f_smem() {
            F_GEN_WARPS * 256 * (8 + 2) + sizeof(FSync);
 }
 
-// Largest |v[k]| of each of the K rows of v (K x n), as partial maxima of the
-// bit patterns per block (a NaN's pattern is above infinity's), and beside them
-// whether the block met a zero or a non-finite value; block 0 also clears the
-// flag of out-of-range weights.
-__global__ void __launch_bounds__(256) k_f64_colmax(const double* __restrict__ v, int K, int64_t n,
-                                                    unsigned long long* __restrict__ mx, int* __restrict__ flag) {
+// Largest v[k] of each of the K rows of v (K x n), as partial maxima of the bit
+// patterns per block, and beside them whether the block met an entry of v or w (the
+// nw entries of the other matrix) outside [lo, 1] (bit patterns; an ulp or two above 1
+// passes, which a projection onto the simplex of one variable leaves).  Block 0 also
+// clears the flag of out-of-range weights.
+__global__ void __launch_bounds__(256) k_f64_range(const double* __restrict__ v, int K, int64_t n,
+                                                   const double* __restrict__ w, int64_t nw, unsigned long long lo,
+                                                   unsigned long long* __restrict__ mx, int* __restrict__ flag) {
     __shared__ unsigned long long s[HX_KMAX + 1];
     if (threadIdx.x <= HX_KMAX) s[threadIdx.x] = 0ull;
     if (blockIdx.x == 0 && threadIdx.x == 0) *flag = 0;
     __syncthreads();
+    const unsigned long long span = 0x3FF0000000000010ull - lo;
+    bool out = false;
     // a stride that is a multiple of K keeps each thread on one k
     const int64_t stride = (int64_t)gridDim.x * blockDim.x / K * K;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t < stride) {
         unsigned long long m = 0ull;
-        bool odd = false;
         for (int64_t a = t; a < n * K; a += stride) {
-            const unsigned long long b = (unsigned long long)__double_as_longlong(v[a]) & 0x7FFFFFFFFFFFFFFFull;
+            const unsigned long long b = (unsigned long long)__double_as_longlong(v[a]);
             m = max(m, b);
-            odd |= b == 0ull || b >= 0x7FF0000000000000ull;
+            out |= b - lo > span;
         }
         atomicMax(&s[t % K], m);
-        if (odd) atomicMax(&s[HX_KMAX], 1ull);
+        for (int64_t a = t; a < nw; a += stride) out |= (unsigned long long)__double_as_longlong(w[a]) - lo > span;
     }
+    if (out) atomicMax(&s[HX_KMAX], 1ull);
     __syncthreads();
     if (threadIdx.x <= HX_KMAX) mx[(int64_t)blockIdx.x * F_MXS + threadIdx.x] = s[threadIdx.x];
 }
 
 // Exponents e_k with max |v_k| < 2^e_k, from the partial maxima; returns via
-// shared memory of HX_KMAX ints (INT_MAX where a value is not finite).
+// shared memory of HX_KMAX ints (where k_f64_range found no entry outside its range).
 __device__ __forceinline__ void f64_exponents(const unsigned long long* __restrict__ mx, int nb, int K, int* se) {
     if (threadIdx.x < (unsigned)K) {
         unsigned long long m = 0ull;
         for (int b = 0; b < nb; ++b) m = max(m, mx[(int64_t)b * F_MXS + threadIdx.x]);
         const int f = (int)(m >> 52);
-        se[threadIdx.x] = f == 0x7FF ? 0x7FFFFFFF : (f == 0 ? 0 : f - 1022);
+        se[threadIdx.x] = f - 1022;
     }
     __syncthreads();
 }
@@ -148,8 +152,7 @@ __global__ void __launch_bounds__(128) k_f64_img(const double* __restrict__ v, i
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         x[k] = a < n ? v[(int64_t)K * a + k] : 0.0;
-        const int e = se[k];
-        w[k] = e == 0x7FFFFFFF ? 0.0 : scalbn(x[k], -e);
+        w[k] = scalbn(x[k], -se[k]);
     }
     double* rows = reinterpret_cast<double*>(base + D::NG * D::B_TILE) + lane * D::KS;
 #pragma unroll
@@ -159,7 +162,7 @@ __global__ void __launch_bounds__(128) k_f64_img(const double* __restrict__ v, i
 #pragma unroll
     for (int k = 0; k < K; ++k) mw = fmax(mw, fabs(w[k]));
     const int fe = (int)((unsigned long long)__double_as_longlong(mw) >> 52);
-    const int f = fe == 0 || fe == 0x7FF ? 0 : fe - 1022;
+    const int f = fe == 0 ? 0 : fe - 1022;
     rows[K] = __longlong_as_double((long long)f);
 #pragma unroll
     for (int k = 0; k < K; ++k) w[k] = scalbn(w[k], -f);
@@ -241,12 +244,9 @@ __device__ __forceinline__ bool f_wait(FSync* sy, uint64_t* bar, int phase, doub
 // ballot and spread evenly over the lanes (4 rounds of 32 for 64 pairs instead
 // of 8); then the pairs whose counts depend on qp, again listed, are finished
 // from their reciprocals.  Results in rb[c][lane] (needed items only).
-// A frequency qp_h = 0 makes the Hessian NaN even where the genotypes do not
-// allow h (0 / 0), which the caller reports: with allh (P holds zeros or
-// non-finite values, the only way to such a qp) every haplotype is listed.
 template <int K, bool HESS>
 __device__ __forceinline__ void f64_weights(const unsigned (&nib)[2], const double* qrow, const double* prow,
-                                            double* rb, uint16_t* list, bool allh) {
+                                            double* rb, uint16_t* list) {
     constexpr int KS = FDim<K, HESS>::KS;
     const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
     int n = 0;
@@ -258,11 +258,9 @@ __device__ __forceinline__ void f64_weights(const unsigned (&nib)[2], const doub
         const unsigned tag = lane | (__popc(need[bb]) == 1 ? 256u : 0u) | (cpl[bb] ? 512u : 0u);
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
-            const bool own = (need[bb] >> h) & 1u;
-            const bool has = own || (allh && nib[bb] != NIB_MM);
+            const bool has = (need[bb] >> h) & 1u;
             const unsigned bal = __ballot_sync(0xffffffffu, has);
-            if (has)
-                list[n + __popc(bal & lt)] = (uint16_t)((own ? tag : lane | 1024u) | ((4 * bb + h) << 5));
+            if (has) list[n + __popc(bal & lt)] = (uint16_t)(tag | ((4 * bb + h) << 5));
             n += __popc(bal);
         }
     }
@@ -284,8 +282,6 @@ __device__ __forceinline__ void f64_weights(const unsigned (&nib)[2], const doub
                 const unsigned ex = ((unsigned)__double2hiint(w) >> 20) & 0x7FFu;
                 if (ex - 1u < 2045u) w = __hiloint2double(__double2hiint(w) + 0x00100000, __double2loint(w));
             }
-            // listed for a frequency of zero only (see allh)
-            if (HESS && (it & 1024u)) w = (__double2hiint(r) & 0x7FF00000) == 0x7FF00000 ? NAN : 0.0;
         }
         if (on) rb[(it & 255u)] = w;                    // it & 255 = 32 c + lane
     }
@@ -402,6 +398,8 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
     const int ns = (int)(min(fa.stages, s0 + a.per_chunk) - s0);
     const int nwc = PS ? (int)min((int64_t)4, (int64_t)a.JW - (int64_t)blockIdx.x * 4) : 1;
 
+    // inputs that the general passes take (k_accum_q, k_accum_p)
+    if (__syncthreads_or(tid < fa.nmx && fa.mx[tid * F_MXS + HX_KMAX] != 0ull)) return;
     if (warp == F_GEN_WARPS) tmem_alloc<D::TCOLS>(&sy->tslot);
     if (tid == 0) {
         for (int r = 0; r < F_RING; ++r) mbar_init(&sy->full[r], 1);
@@ -415,17 +413,12 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
     // the rows' own vectors
     const double* own = PS ? a.p : a.q;
     const int64_t nown = PS ? 4 * a.J : a.I;
-    bool odd_p = false;          // P side: zero or non-finite frequencies among the CTA's own columns
     for (int t = tid; t < 128 * K; t += F_THREADS) {
         const int r = t / K, k = t - r * K;
-        const double x = row0 + r < nown ? own[(row0 + r) * K + k] : 0.25;
-        fix[r * D::KS + k] = x;
-        odd_p |= PS && (x == 0.0 || !isfinite(x));
+        fix[r * D::KS + k] = row0 + r < nown ? own[(row0 + r) * K + k] : 0.25;
     }
-    if (!PS)                     // Q side: among all of P
-        for (int b = tid; b < fa.nmx; b += F_THREADS) odd_p |= fa.mx[(int64_t)b * F_MXS + HX_KMAX] != 0ull;
     fence_before();
-    const bool allh = __syncthreads_or(odd_p) && HESS;
+    __syncthreads();
     fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, sy->tslot, 0);
 
@@ -546,12 +539,11 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
                 qrow = fix + 32 * (warp & 3) * D::KS;
                 prow = srow + 8 * (warp >> 2) * D::KS;
             }
-            f64_weights<K, HESS>(nib, qrow, prow, rb, list, allh);
+            f64_weights<K, HESS>(nib, qrow, prow, rb, list);
             double W[8];
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
-                const unsigned nd = allh && nib[c >> 2] != NIB_MM ? 0xFu : (unsigned)(TAB_NEED >> (4 * nib[c >> 2])) & 0xFu;
-                W[c] = (nd >> (c & 3)) & 1u ? rb[32 * c + lane] : 0.0;
+                W[c] = (unsigned)(TAB_NEED >> (4 * nib[c >> 2] + (c & 3))) & 1u ? rb[32 * c + lane] : 0.0;
             }
             // powers of two to scale by: the exponents of the reduction indices
             auto sh = [&](int c) {

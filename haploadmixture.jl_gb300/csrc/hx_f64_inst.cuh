@@ -30,16 +30,26 @@ cudaError_t f64_launch(const F64Call& c) {
     const int64_t n = PS ? a.I : 4 * a.J;
     const int64_t stages = PS ? (a.I + F_KD - 1) / F_KD : a.JW;
     const int64_t tiles = PS ? (a.J + 31) / 32 : a.Ipad / 128;
-    const int nmx = (int)std::min<int64_t>(F_MAXB, (n * K + 2047) / 2048);
-    k_f64_colmax<<<nmx, 256, 0, c.st>>>(v, K, n, c.mx, c.rare.flag);
+    const double* w = PS ? a.p : a.q;             // the rows' own
+    const int64_t nw = (PS ? 4 * a.J : a.I) * K;
+    const int nmx = (int)std::min<int64_t>(F_MAXB, (n * K + nw + 2047) / 2048);
+    k_f64_range<<<nmx, 256, 0, c.st>>>(v, K, n, w, nw, HESS ? F_LO_HESS : F_LO_GRAD, c.mx, c.rare.flag);
     k_f64_img<K, HESS><<<(unsigned)((stages + 3) / 4), 128, 0, c.st>>>(v, n, stages, c.mx, nmx, a.img);
     F64Args fa{stages, c.mx, nmx, c.rare};
     dim3 grid((unsigned)tiles, (unsigned)a.S, D::NG);
     k_f64_pass<K, HESS, PS><<<grid, F_THREADS, f_smem<K, HESS, PS>(), c.st>>>(a, fa);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
+    PassArgs g = a;
+    g.S = c.Sg;
+    g.per_chunk = c.per_chunk_g;
+    g.run_if = c.mx + HX_KMAX;
+    g.n_run_if = nmx;
+    g.run_if_ld = F_MXS;
+    e = PS ? launch_accum_p_f64(K, HESS, g, c.st) : launch_accum_q_f64(K, HESS, g, c.st);
+    if (e != cudaSuccess) return e;
     const int64_t rows = PS ? 4 * a.J : a.I;
-    return launch_f64_reduce(a.part, a.S, K, HESS, rows, PS ? rows : a.Ipad, PS ? a.p : a.q, c.mx, nmx, c.rare,
+    return launch_f64_reduce(a.part, a.S, c.Sg, K, HESS, rows, PS ? rows : a.Ipad, PS ? a.p : a.q, c.mx, nmx, c.rare,
                              a.XtX, a.Xtz, c.st);
 }
 template <int K>

@@ -15,6 +15,9 @@ enum Slot {
 cudaError_t launch_loglik_f64(int K, const PassArgs& a, cudaStream_t st);
 // the same from BED bytes (first I individuals, 2J SNPs); a.G and a.Ipad unused
 cudaError_t launch_loglik_f64_bed(int K, const PassArgs& a, const uint8_t* bed, int64_t bps, cudaStream_t st);
+// general FP64 passes (partial sums in a.part whatever a.S is)
+cudaError_t launch_accum_q_f64(int K, bool hess, const PassArgs& a, cudaStream_t st);
+cudaError_t launch_accum_p_f64(int K, bool hess, const PassArgs& a, cudaStream_t st);
 cudaError_t launch_accum_q_f32(int K, bool hess, const PassArgs& a, cudaStream_t st);
 cudaError_t launch_accum_p_f32(int K, bool hess, const PassArgs& a, cudaStream_t st);
 cudaError_t launch_loglik_f32x2(int K, const PassArgs& a, cudaStream_t st);   // several individuals per thread
@@ -59,18 +62,24 @@ struct F64Rare {
     int* flag;             // bit 0: i was added to, bit 1: d was
 };
 constexpr int F_MXS = 16;  // partial maxima of one block: HX_KMAX values, then a flag
-constexpr int F_MAXB = 64; // blocks of partial maxima
+constexpr int F_MAXB = ACC_THREADS; // blocks of partial maxima (one thread of a CTA reads one)
+// Least entry of Q and P (bit pattern) that the digit passes take: 2^-17 with the
+// Hessian, whose products then stay above 2^-34, 2^-34 without.  The fit's own values
+// are above it (pseudocount 1e-5); all others go to the general passes.
+constexpr unsigned long long F_LO_HESS = (1023ull - 17) << 52, F_LO_GRAD = (1023ull - 34) << 52;
 struct F64Args {
     int64_t stages;                   // of 32 reduction indices
     const unsigned long long* mx;     // [nmx][F_MXS]
     int nmx;
     F64Rare rare;
 };
-// One pass: partial maxima of v, stage images, the pass (partial sums in
-// a.part, [S][NV][rows]) and their reduction to XtX and Xtz (a.XtX, a.Xtz).
+// One pass: range of the inputs, stage images, the digit pass (partial sums in a.part,
+// [S][NV][rows]), or the general one in its place ([Sg][K + NV][rows]), and their
+// reduction to XtX and Xtz (a.XtX, a.Xtz).
 struct F64Call {
     bool p_side, hess;
     PassArgs a;
+    int Sg, per_chunk_g;              // chunks of the general pass
     unsigned long long* mx;           // F_MAXB * F_MXS words
     F64Rare rare;
     cudaStream_t st;
@@ -78,9 +87,9 @@ struct F64Call {
 cudaError_t launch_f64_pass(int K, const F64Call& c);
 cudaError_t f64_attrs(int K);         // once per device before the first pass
 size_t f64_image_bytes(int K, int64_t I, int64_t J);
-cudaError_t launch_f64_reduce(const double* part, int S, int K, bool hess, int64_t rows, int64_t ld, const double* x,
-                              const unsigned long long* mx, int nmx, const F64Rare& rare, double* XtX, double* Xtz,
-                              cudaStream_t st);
+cudaError_t launch_f64_reduce(const double* part, int S, int Sg, int K, bool hess, int64_t rows, int64_t ld,
+                              const double* x, const unsigned long long* mx, int nmx, const F64Rare& rare, double* XtX,
+                              double* Xtz, cudaStream_t st);
 // Stages per chunk, 32 reduction indices each.  The 64-bit sums of orders 5 .. 9 take at
 // most 6 x 2^14 x 2^32 + 7 x 2^14 x 2^24 + ... < 2^48.6 per index in units of 2^-62, so
 // 2^14.3 indices (679 stages) stay below 2^63 whatever the digits are.

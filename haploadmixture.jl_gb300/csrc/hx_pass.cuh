@@ -2,8 +2,9 @@
 //
 // Kernels of the mixed method, templated on the number of ancestries K
 // (register-resident accumulators): FP32 products, FP64 cross-chunk totals and
-// FP64 stage-level promotion of the gradient.  (The plain FP64 method's are in
-// hx_f64.cuh and hx_pass_f64.cu.)
+// FP64 stage-level promotion of the gradient; and, with T = double, the plain
+// method's general passes.  (Those it takes for the values a fit works with, and its
+// log-likelihood, are in hx_f64.cuh and hx_pass_f64.cu.)
 //
 //   k_accum_q  : per individual i over a chunk of blocks (src/loops.jl:328-365,
 //                src/cuda/kernels.jl:104-138):
@@ -49,6 +50,8 @@ struct PassArgs {
     const float* pf;        // FP32 copy of p for the FP32 passes that stage p (or null): GB300's
                             // FP64 unit is narrow, and converting in every CTA kept it busy
     long long budget;       // tensor-core passes: clock64 cycles any one pipeline wait may take
+    const unsigned long long* run_if = nullptr;   // T = double: run if any of the n_run_if (at most
+    int n_run_if = 0, run_if_ld = 1;              // ACC_THREADS) words, run_if_ld apart, is not zero
 };
 
 template <int K> __device__ __forceinline__ constexpr int tri(int k, int k2) {
@@ -56,29 +59,36 @@ template <int K> __device__ __forceinline__ constexpr int tri(int k, int k2) {
 }
 
 // ------------------------------------------------------------------ Q side
-template <int K>
+// T = double (with its gradient-only form): the plain method's passes on inputs that
+// the digit sums of hx_f64.cuh do not take; run_if says on the device whether it is
+// one of them.
+template <typename T> __device__ __forceinline__ bool pass_idle(const PassArgs& a) {
+    return sizeof(T) == 8 && !__syncthreads_or((int)threadIdx.x < a.n_run_if && a.run_if[threadIdx.x * a.run_if_ld] != 0ull);
+}
+template <int K, typename T, bool HESS>
 __global__ void __launch_bounds__(ACC_THREADS)
 k_accum_q(PassArgs a) {
     constexpr int NH = K * (K + 1) / 2;
-    constexpr int NV = K + NH;
-    __shared__ float sp[QSTAGE_WORDS * 8 * 4 * K];
+    constexpr int NV = K + (HESS ? NH : 0);
+    __shared__ T sp[QSTAGE_WORDS * 8 * 4 * K];
     __shared__ float4 s_snp[4];
     const int tid = threadIdx.x;
+    if (pass_idle<T>(a)) return;
     snp_table_init(s_snp, tid);
     const int64_t i = (int64_t)blockIdx.x * ACC_THREADS + tid;
     const int w0 = blockIdx.y * a.per_chunk;
     const int w1 = min(a.JW, w0 + a.per_chunk);
     const bool active = i < a.I;
-    float qi[K];
+    T qi[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) qi[k] = active ? (float)a.q[(int64_t)K * i + k] : 1.f / K;
-    float gin[K];
+    for (int k = 0; k < K; ++k) qi[k] = active ? (T)a.q[(int64_t)K * i + k] : T(1) / T(K);
+    T gin[K];
     double gout[K];
-    float H[NH];
+    T H[HESS ? NH : 1];
 #pragma unroll
-    for (int k = 0; k < K; ++k) { gin[k] = 0.f; gout[k] = 0.0; }
+    for (int k = 0; k < K; ++k) { gin[k] = T(0); gout[k] = 0.0; }
 #pragma unroll
-    for (int v = 0; v < NH; ++v) H[v] = 0.f;
+    for (int v = 0; v < (HESS ? NH : 1); ++v) H[v] = T(0);
 
     for (int ws = w0; ws < w1; ws += QSTAGE_WORDS) {
         const int nw = min(QSTAGE_WORDS, w1 - ws);
@@ -91,7 +101,7 @@ k_accum_q(PassArgs a) {
         const int64_t base = (int64_t)ws * 8 * 4 * K;
         const int64_t limit = a.J * 4 * K;
         for (int t = tid; t < nval; t += ACC_THREADS)
-            sp[t] = (base + t < limit) ? (a.pf ? a.pf[base + t] : (float)a.p[base + t]) : 0.25f;
+            sp[t] = (base + t < limit) ? (sizeof(T) == 4 && a.pf ? (T)a.pf[base + t] : (T)a.p[base + t]) : T(0.25);
         __syncthreads();
         if (active) {
             for (int w = 0; w < nw; ++w) {
@@ -100,51 +110,55 @@ k_accum_q(PassArgs a) {
                 for (int b = 0; b < 8; ++b) {
                     const unsigned nib = (word >> (4 * b)) & 0xFu;
                     if (nib == NIB_MM) continue;
-                    const float* pb = sp + (w * 8 + b) * 4 * K;
-                    float qp[4];
+                    const T* pb = sp + (w * 8 + b) * 4 * K;
+                    T qp[4];
 #pragma unroll
                     for (int h = 0; h < 4; ++h) {
-                        float s = 0.f;
+                        T s = T(0);
 #pragma unroll
                         for (int k = 0; k < K; ++k) s = fma(qi[k], pb[h * K + k], s);
                         qp[h] = s;
                     }
-                    float L, u[4];
-                    pair_eval_tab(nib, qp, L, u, s_snp);
+                    T L, u[4];
+                    pair_eval_t(nib, qp, L, u, s_snp);
 #pragma unroll
                     for (int k = 0; k < K; ++k) {
-                        float g = gin[k];
+                        T g = gin[k];
                         g = fma(u[0], pb[k], g);
                         g = fma(u[1], pb[K + k], g);
                         g = fma(u[2], pb[2 * K + k], g);
                         g = fma(u[3], pb[3 * K + k], g);
                         gin[k] = g;
                     }
+                    if (HESS) {
 #pragma unroll
-                    for (int h = 0; h < 4; ++h) {
-                        const float wh = u[h] * __frcp_rn(qp[h]);
-                        float t[K];
+                        for (int h = 0; h < 4; ++h) {
+                            const T wh = u[h] * rcp<T>(qp[h]);
+                            T t[K];
 #pragma unroll
-                        for (int k = 0; k < K; ++k) t[k] = wh * pb[h * K + k];
+                            for (int k = 0; k < K; ++k) t[k] = wh * pb[h * K + k];
 #pragma unroll
-                        for (int k = 0; k < K; ++k)
+                            for (int k = 0; k < K; ++k)
 #pragma unroll
-                            for (int k2 = k; k2 < K; ++k2)
-                                H[tri<K>(k, k2)] = fma(t[k], pb[h * K + k2], H[tri<K>(k, k2)]);
+                                for (int k2 = k; k2 < K; ++k2)
+                                    H[tri<K>(k, k2)] = fma(t[k], pb[h * K + k2], H[tri<K>(k, k2)]);
+                        }
                     }
                 }
             }
         }
         // promote the stage's gradient partial to FP64
 #pragma unroll
-        for (int k = 0; k < K; ++k) { gout[k] += (double)gin[k]; gin[k] = 0.f; }
+        for (int k = 0; k < K; ++k) { gout[k] += (double)gin[k]; gin[k] = T(0); }
     }
     if (i < a.Ipad) {
         double* out = a.part + (int64_t)blockIdx.y * NV * a.Ipad;
 #pragma unroll
         for (int k = 0; k < K; ++k) out[(int64_t)k * a.Ipad + i] = gout[k];
+        if (HESS) {
 #pragma unroll
-        for (int v = 0; v < NH; ++v) out[(int64_t)(K + v) * a.Ipad + i] = (double)H[v];
+            for (int v = 0; v < (HESS ? NH : 1); ++v) out[(int64_t)(K + v) * a.Ipad + i] = (double)H[v];
+        }
     }
 }
 
@@ -242,39 +256,40 @@ k_grad_q(PassArgs a) {
 // ------------------------------------------------------------------ P side
 // Thread (b, h) of a CTA owns haplotype column m = 4*(32*blockIdx.x + b) + h;
 // the 4 threads of a block exchange their qp_h by warp shuffles.
-template <int K, bool HESS>
+template <int K, typename T, bool HESS>
 __global__ void __launch_bounds__(ACC_THREADS)
 k_accum_p(PassArgs a) {
     constexpr int NH = K * (K + 1) / 2;
     constexpr int NV = K + (HESS ? NH : 0);
-    __shared__ float sq[PSTAGE_IND * K];
+    __shared__ T sq[PSTAGE_IND * K];
     __shared__ uint32_t sg[4 * PSTAGE_IND];
     __shared__ float4 s_snp[4];
     const int tid = threadIdx.x;
+    if (pass_idle<T>(a)) return;
     snp_table_init(s_snp, tid);
     const int lane = tid & 31, warp = tid >> 5;
     const int b = tid >> 2, h = tid & 3;
     const int64_t j = (int64_t)blockIdx.x * 32 + b;
     const bool valid = j < a.J;
     const int64_t m = 4 * j + h;
-    float pr[K];
+    T pr[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) pr[k] = valid ? (float)a.p[(int64_t)K * m + k] : 0.25f;
+    for (int k = 0; k < K; ++k) pr[k] = valid ? (T)a.p[(int64_t)K * m + k] : T(0.25);
     const int64_t i0 = (int64_t)blockIdx.y * a.per_chunk;
     const int64_t i1 = min(a.I, i0 + (int64_t)a.per_chunk);
     const int bsh = 4 * (b & 7);
-    float gin[K];
+    T gin[K];
     double gout[K];
-    float H[HESS ? NH : 1];
+    T H[HESS ? NH : 1];
 #pragma unroll
-    for (int k = 0; k < K; ++k) { gin[k] = 0.f; gout[k] = 0.0; }
+    for (int k = 0; k < K; ++k) { gin[k] = T(0); gout[k] = 0.0; }
 #pragma unroll
-    for (int v = 0; v < (HESS ? NH : 1); ++v) H[v] = 0.f;
+    for (int v = 0; v < (HESS ? NH : 1); ++v) H[v] = T(0);
 
     for (int64_t is = i0; is < i1; is += PSTAGE_IND) {
         const int n = (int)min((int64_t)PSTAGE_IND, i1 - is);
         __syncthreads();
-        for (int t = tid; t < n * K; t += ACC_THREADS) sq[t] = (float)a.q[(int64_t)K * is + t];
+        for (int t = tid; t < n * K; t += ACC_THREADS) sq[t] = (T)a.q[(int64_t)K * is + t];
         for (int t = tid; t < 4 * PSTAGE_IND; t += ACC_THREADS) {
             const int w = t / PSTAGE_IND, r = t % PSTAGE_IND;
             const int64_t jw = (int64_t)blockIdx.x * 4 + w;
@@ -284,21 +299,21 @@ k_accum_p(PassArgs a) {
 #pragma unroll 1
         for (int r = 0; r < n; ++r) {
             const unsigned nib = (sg[warp * PSTAGE_IND + r] >> bsh) & 0xFu;
-            const float* qr = sq + r * K;
-            float own = 0.f;
+            const T* qr = sq + r * K;
+            T own = T(0);
 #pragma unroll
             for (int k = 0; k < K; ++k) own = fma(qr[k], pr[k], own);
-            float qp[4];
+            T qp[4];
 #pragma unroll
             for (int t = 0; t < 4; ++t) qp[t] = __shfl_sync(0xffffffffu, own, (lane & ~3) | t);
-            float L, u[4];
-            pair_eval_tab(nib, qp, L, u, s_snp);
-            const float uh = h == 0 ? u[0] : (h == 1 ? u[1] : (h == 2 ? u[2] : u[3]));
+            T L, u[4];
+            pair_eval_t(nib, qp, L, u, s_snp);
+            const T uh = h == 0 ? u[0] : (h == 1 ? u[1] : (h == 2 ? u[2] : u[3]));
 #pragma unroll
             for (int k = 0; k < K; ++k) gin[k] = fma(uh, qr[k], gin[k]);
             if (HESS) {
-                const float wh = uh * __frcp_rn(own);
-                float t[K];
+                const T wh = uh * rcp<T>(own);
+                T t[K];
 #pragma unroll
                 for (int k = 0; k < K; ++k) t[k] = wh * qr[k];
 #pragma unroll
@@ -308,10 +323,10 @@ k_accum_p(PassArgs a) {
             }
         }
 #pragma unroll
-        for (int k = 0; k < K; ++k) { gout[k] += (double)gin[k]; gin[k] = 0.f; }
+        for (int k = 0; k < K; ++k) { gout[k] += (double)gin[k]; gin[k] = T(0); }
     }
     if (!valid) return;
-    if (a.S == 1) {
+    if (sizeof(T) == 4 && a.S == 1) {
         double* X = a.XtX + (int64_t)K * K * m;
 #pragma unroll
         for (int k = 0; k < K; ++k) a.Xtz[(int64_t)K * m + k] = gout[k];
