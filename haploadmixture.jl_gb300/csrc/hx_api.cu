@@ -44,9 +44,9 @@ struct hx_ctx {
     double* h_slots = nullptr;   // pinned
     int pin_slot = -1;           // its place in the process's pinned page, or -1
     uint8_t* img = nullptr;      // B-operand image of the tensor-core passes
-    // plain method: partial maxima and out-of-range sums of the passes (hx_f64.cuh)
-    unsigned long long* f64_mx = nullptr;
-    F64Rare rare{nullptr, nullptr, nullptr};
+    // plain method: range flags and out-of-range sums of the passes (hx_f64.cuh)
+    unsigned* f64_off = nullptr;
+    F64Rare rare{nullptr, nullptr};
     int S_qf = 1, spc_qf = 1, S_pf = 1, spc_pf = 1;   // chunks, stages per chunk
     int8_t* qp_ws = nullptr;     // P-side QP working sets, warm start of the next solve
     hx_loop_opts lo{0, 0, 0, -1};  // admixture_qn!/init_em! options
@@ -269,7 +269,7 @@ void plan(hx_ctx* c) {
     ipc = (ipc + PSTAGE_IND - 1) / PSTAGE_IND * PSTAGE_IND;
     c->ipc_p = (int)ipc;
     c->S_p = (int)((c->I + ipc - 1) / ipc);
-    // plain method's passes: one CTA per SM, chunks within the 64-bit sums' range
+    // plain method's passes: one CTA per SM, chunks within the integer sums' range
     const int64_t nst_p = (c->I + 31) / 32;
     c->spc_qf = (int)pick_chunk_f64(tilesQ, c->JW, nsm);
     c->S_qf = (c->JW + c->spc_qf - 1) / c->spc_qf;
@@ -318,7 +318,7 @@ int stage_pf(hx_ctx* c, const double* p, PassArgs& a) {
 // The plain method's pass of one side: range, stage images, digit pass or general
 // pass, reduction.
 int pass_f64(hx_ctx* c, bool p_side, const double* q, const double* p, bool hess, double* XtX, double* Xtz) {
-    F64Call f{p_side, hess, pass_args(c, q, p), p_side ? c->S_p : c->S_q, p_side ? c->ipc_p : c->wpc_q, c->f64_mx,
+    F64Call f{p_side, hess, pass_args(c, q, p), p_side ? c->S_p : c->S_q, p_side ? c->ipc_p : c->wpc_q, c->f64_off,
               c->rare, c->st};
     f.a.S = p_side ? c->S_pf : c->S_qf;
     f.a.per_chunk = p_side ? c->spc_pf : c->spc_qf;
@@ -608,9 +608,8 @@ int create_common(const uint8_t* bed, bool bed_on_device, int64_t bps, int64_t n
         need(rq, &c->part_q, std::max<size_t>(c->S_qf * NH, (size_t)c->S_q * NVmax) * c->Ipad);
         need(rq, &c->part_p, std::max<size_t>(c->S_pf * NH, (size_t)c->S_p * NVmax) * 4 * J);
         need(rq, &c->img, f64_image_bytes(K, I, J));
-        need(rq, &c->f64_mx, (size_t)F_MAXB * F_MXS);
-        need(rq, &c->rare.i, 2 * rows * NH);
-        need(rq, &c->rare.d, rows * NH);
+        need(rq, &c->f64_off, (size_t)F_MAXB);
+        need(rq, &c->rare.i, 3 * rows * NH);
         need(rq, &c->rare.flag, 1);
     } else {
         need(rq, &c->part_q, (size_t)std::max(c->S_q, c->tc ? c->Sq_cap : 1) * NVmax * c->Ipad);
@@ -628,10 +627,7 @@ int create_common(const uint8_t* bed, bool bed_on_device, int64_t bps, int64_t n
     need(rq, &c->qp_ws, (size_t)4 * K * J);
     HX_ST(alloc_all(c, rq));
     c->V = c->U + nuv;
-    if (c->prec == HX_PREC_FP64) {
-        HX_CK(cudaMemsetAsync(c->rare.i, 0, 2 * rows * NH * sizeof(long long), c->st));
-        HX_CK(cudaMemsetAsync(c->rare.d, 0, rows * NH * sizeof(double), c->st));
-    }
+    if (c->prec == HX_PREC_FP64) HX_CK(cudaMemsetAsync(c->rare.i, 0, 3 * rows * NH * sizeof(long long), c->st));
     HX_CK(cudaMemsetAsync(c->qp_ws, 0, (size_t)4 * K * J, c->st));
     HX_CK(pin_get(c));
     for (int s = 0; s < HX_NSLOT; ++s) c->h_slots[s] = 0.0;

@@ -27,9 +27,8 @@ cudaError_t f64_attrs(int K) { return f64_run(K, nullptr); }
 // Bytes of the larger side's stage images (FDim::IMG of the Hessian form, the
 // larger one).
 size_t f64_image_bytes(int K, int64_t I, int64_t J) {
-    const int nv = K * (K + 1) / 2, ng = nv > 48 ? 2 : 1;
-    const int nhp = ((nv + ng - 1) / ng + 15) / 16 * 16;
-    const size_t img = (size_t)ng * 8 * nhp * 64 + (size_t)32 * ((K + 1) | 1) * 8;
+    const int nv = K * (K + 1) / 2, ng = f64_groups(nv), nhp = f64_nhp((nv + ng - 1) / ng);
+    const size_t img = (size_t)ng * F_NDB * nhp * 64 + (size_t)32 * ((K + 1) | 1) * 8;
     return img * (size_t)std::max((J + 7) / 8, (I + 31) / 32);
 }
 
@@ -41,13 +40,12 @@ namespace {
 // go out through shared memory, so that the K x K blocks are written in order too.
 constexpr int FR_ROWS = 32;
 __global__ void __launch_bounds__(256) k_f64_reduce(const double* __restrict__ part, int S, int Sg, int K, bool hess,
-                                                    int64_t rows, int64_t ld, const double* __restrict__ x,
-                                                    const unsigned long long* __restrict__ mx, int nmx, F64Rare rare,
+                                                    bool g, int64_t rows, int64_t ld, const double* __restrict__ x,
+                                                    const unsigned* __restrict__ off, int noff, F64Rare rare,
                                                     double* __restrict__ XtX, double* __restrict__ Xtz) {
     extern __shared__ double tile[];   // [K + NH][FR_ROWS + 1]: Xtz, then the triangle
-    __shared__ int se[HX_KMAX];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool general = __syncthreads_or(tid < nmx && mx[tid * F_MXS + HX_KMAX] != 0ull);
+    const bool general = __syncthreads_or(tid < noff && off[tid] != 0u);
     const int NH = hess ? K * (K + 1) / 2 : 0;
     const int64_t r0 = (int64_t)blockIdx.x * FR_ROWS, r = r0 + lane;
     if (general) {
@@ -61,39 +59,28 @@ __global__ void __launch_bounds__(256) k_f64_reduce(const double* __restrict__ p
             tile[v * (FR_ROWS + 1) + lane] = s;
         }
     } else {
-        if (tid < K) {
-            unsigned long long m = 0ull;
-            for (int b = 0; b < nmx; ++b) m = max(m, mx[(int64_t)b * F_MXS + tid]);
-            se[tid] = (int)(m >> 52) - 1022;
-        }
-        __syncthreads();
         const int NV = hess ? NH : K;
         const int flag = *rare.flag;
-        int k = 0, k2 = 0;             // of value v
-        for (int v = 0, left = warp; v < NV; ++v) {
-            if (left == 0) {
-                left = 8;
-                double s = 0.0;
-                if (r < rows) {
-                    const double* src = part + (int64_t)v * ld + r;
+        int sh = 0;                        // the row's exponent
+        if (g && r < rows) {
+            double m = 0.0;
+            for (int k = 0; k < K; ++k) m = fmax(m, x[r * K + k]);
+            sh = 1022 - (__double2hiint(m) >> 20);
+        }
+        for (int v = warp; v < NV; v += 8) {
+            double s = 0.0;
+            if (r < rows) {
+                const double* src = part + (int64_t)v * ld + r;
 #pragma unroll 8
-                    for (int c = 0; c < S; ++c) s += src[(int64_t)c * NV * ld];
-                    if (flag) {        // products of out-of-range weights; left zero for the next pass
-                        const int64_t at = r * NV + v;
-                        s += scalbn((double)rare.i[2 * at], -8) + scalbn((double)rare.i[2 * at + 1], -56);
-                        rare.i[2 * at] = 0;
-                        rare.i[2 * at + 1] = 0;
-                        if (flag & 2) {
-                            s += rare.d[at];
-                            rare.d[at] = 0.0;
-                        }
-                    }
-                    s = scalbn(s, hess ? se[k] + se[k2] : se[v]);
+                for (int c = 0; c < S; ++c) s += src[(int64_t)c * NV * ld];
+                if (flag) {                // products of out-of-range weights; left zero for the next pass
+                    long long* i = rare.i + 3 * (r * NV + v);
+                    s += scalbn((double)i[0], 2) + (scalbn((double)i[1], -35) + scalbn((double)i[2], -72));
+                    i[0] = i[1] = i[2] = 0;
                 }
-                tile[((hess ? K : 0) + v) * (FR_ROWS + 1) + lane] = s;
+                s = scalbn(s, sh);
             }
-            --left;
-            if (++k2 == K) { ++k; k2 = k; }
+            tile[((hess ? K : 0) + v) * (FR_ROWS + 1) + lane] = s;
         }
         if (hess) {
             __syncthreads();
@@ -123,13 +110,13 @@ __global__ void __launch_bounds__(256) k_f64_reduce(const double* __restrict__ p
 }
 }  // namespace
 
-cudaError_t launch_f64_reduce(const double* part, int S, int Sg, int K, bool hess, int64_t rows, int64_t ld,
-                              const double* x, const unsigned long long* mx, int nmx, const F64Rare& rare, double* XtX,
+cudaError_t launch_f64_reduce(const double* part, int S, int Sg, int K, bool hess, bool g, int64_t rows, int64_t ld,
+                              const double* x, const unsigned* off, int noff, const F64Rare& rare, double* XtX,
                               double* Xtz, cudaStream_t st) {
     const int NV = K + (hess ? K * (K + 1) / 2 : 0);
     const size_t smem = (size_t)NV * (FR_ROWS + 1) * sizeof(double);   // <= 23.8 KB (K = 12)
-    k_f64_reduce<<<(unsigned)((rows + FR_ROWS - 1) / FR_ROWS), 256, smem, st>>>(part, S, Sg, K, hess, rows, ld, x, mx,
-                                                                                nmx, rare, XtX, Xtz);
+    k_f64_reduce<<<(unsigned)((rows + FR_ROWS - 1) / FR_ROWS), 256, smem, st>>>(part, S, Sg, K, hess, g, rows, ld, x,
+                                                                                off, noff, rare, XtX, Xtz);
     return cudaGetLastError();
 }
 

@@ -11,31 +11,37 @@
 //   W_h = c_h r_h^2 (Hessian) or U_h = c_h r_h (gradient only),
 // and form the sums H = sum W v v' (v = p on the Q side, q on the P side;
 // src/loops.jl:328-403) exactly on the tensor cores: the error-free splitting
-// of Ozaki, Ogita, Oishi and Rump (2012).  The vectors are scaled by powers of
-// two, per k and then per reduction index, so that the largest entry is just
-// below 1 in both; W takes the inverse of the index's, which leaves
-// W' = c_h (s / qp_h)^2, s the index's scale: of the order of 1 even for rare
-// haplotypes.  W' is rounded to a multiple of 2^-56 and written as ND_A = 10
-// signed base-256 digits, the scaled products v_k v_k2 to a multiple of 2^-62
-// as ND_B = 8 digits.  Digits are integers in [-128, 127], exact in FP16; a
-// digit product is at most 2^14, and an FP32 accumulator column takes ND_B digit
-// pairs x 128 reduction indices x 2^14 = 2^24 before it is read out, so every
+// of Ozaki, Ogita, Oishi and Rump (2012).  Each index's vector is scaled by a power of
+// two 2^-f, so that its largest entry is just below 1, and W by 2^2f (2^f in the
+// gradient-only form), which leaves W' = c_h (2^f / qp_h)^2: of the order of 1 even for
+// rare haplotypes; on the P side the row's power of two 2^g (its largest frequency) is
+// a third factor, for the same reason.  W' is rounded to a multiple of 2^-56 and written
+// as ND_A = 9 signed base-256 digits, the scaled products v_k v_k2 to a multiple of
+// 2^-86 as ND_B = 11 digits.  Digits are integers in [-128, 127], exact in FP16; a
+// digit product is at most 2^14, and an FP32 accumulator column takes at most 9 digit
+// pairs x 96 reduction indices x 2^14 < 2^24 before it is read out, so every
 // accumulation is exact.  Digit pairs (a, b) of equal order a + b share a
-// column; orders 0 .. 9 are kept (an order-10 pair weighs 2^-56 at most, with
-// either sign).  The columns are read out to 64-bit integers, so a chunk's sum
+// column; orders 0 .. 12 are kept (an order-13 pair weighs 2^-88 at most, with
+// either sign).  The columns are read out to 128-bit integers, so a chunk's sum
 // does not depend on any order; only the chunk sums and the last digits' cut
-// are rounded, and the error against exact sums is below that of FP64
-// accumulation, whose every add rounds the running total.
+// are rounded.
+//
+// Which inputs: entries of Q and P in [2^-17, 1] (2^-34 without the Hessian), as a fit
+// has them; the general passes of hx_pass.cuh take all others (F_LO_HESS).  A product is
+// then at least 2^-34 and keeps 53 bits of its own, so that an entry made of small
+// products only (all carriers floored in both ancestries) is as accurate as an FP64 sum;
+// with 8 digits and 10 orders such entries had 24 to 27 bits.  W' is at least c / K^2
+// and keeps 50 bits there; a double heterozygote's c can be small (2^-17), and has that
+// many bits fewer, beside the other terms of its row.
 //
 // The gradient needs no sums of its own beside the Hessian: sum_k2 H[k,k2] x_k2
 // = sum W v_k qp = sum U v_k = g_k (x = the row's own vector, qp = v . x), all
 // terms of one sign, formed by the reduction of the chunks.
 //
-// A scaled weight of 2^22 or more (an observed haplotype 2,000 times rarer in
-// the individual's mixture than in one of the ancestries), a negative or a
-// non-finite one does not fit the digits: its products are added in fixed point
-// to 64-bit integers in global memory (order-independent, as every integer
-// sum), and from 2^42 on, or when not finite, to FP64 words there.
+// A scaled weight of 2^14 or more (an observed haplotype about 100 times rarer in
+// the individual's mixture than in one of the ancestries; 2^38 at most) does not fit
+// the digits: its products are added in fixed point to 64-bit integers in global memory
+// (order-independent, as every integer sum).
 #pragma once
 #include "hx_ops.cuh"
 #include "hx_tc.cuh"
@@ -48,26 +54,27 @@ using namespace tc;
 constexpr int F_GEN_WARPS = 16;                       // generator warps
 constexpr int F_THREADS = 32 * (F_GEN_WARPS + 1);     // + one warp that loads and issues
 constexpr int F_KD = 32;                              // reduction indices per stage
-constexpr int F_RING = 3;
-constexpr int F_WIN = 4;                              // stages per read-out (128 reduction indices)
-constexpr int F_NDA = 10, F_NDB = 8, F_NORD = 10;
-constexpr int F_SA = 56, F_SB = 62;                   // units 2^-SA of W', 2^-SB of the products
+constexpr int F_RING = 3;                             // vectors and class words of the next stages
+constexpr int F_BRING = 2;                            // B tiles: read by the MMAs only, a stage later
+constexpr int F_WIN = 3;                              // stages per read-out (96 reduction indices)
+constexpr int F_SA = 56, F_SB = 86;                   // units 2^-SA of W', 2^-SB of the products
 constexpr long long F_BUDGET = 4000000000LL;          // bound of any pipeline wait (clock64 cycles)
-constexpr int F_TOP = 22;                             // W' < 2^TOP: TOP + SA + 1 bits fit ND_A signed bytes
+constexpr int F_TOP = 14;                             // W' < 2^TOP: TOP + SA + 1 bits fit ND_A signed bytes
 
 template <int K, bool HESS> struct FDim {
     static constexpr int NV = HESS ? K * (K + 1) / 2 : K;    // sums per row
-    static constexpr int NG = NV > 48 ? 2 : 1;               // column groups (grid.z): NORD x 48 TMEM columns fit
+    static constexpr int NG = f64_groups(NV);                // column groups (grid.z)
     static constexpr int PER = (NV + NG - 1) / NG;           // sums per group
-    static constexpr int NHP = (PER + 15) / 16 * 16;
+    static constexpr int NHP = (PER + 15) / 16 * 16;         // MMA columns of one order, zero beyond PER
+    static constexpr int STR = f64_stride(PER);              // TMEM columns from one order to the next
     static constexpr int NPC = NHP / 4;                      // columns per order read out by one thread
-    static constexpr int TCOLS = F_NORD * NHP <= 256 ? 256 : 512;
+    static constexpr int TCOLS = (F_NORD - 1) * STR + NHP <= 256 ? 256 : 512;
     static constexpr int KS = (K + 1) | 1;                   // row stride (doubles): odd, so rows differ in banks;
-                                                             // entry K of a stage's row: the index's exponent
+                                                             // entry K of a row: its exponent
     static constexpr int B_TILE = F_NDB * NHP * F_KD * 2;
     static constexpr int ROWS = F_KD * KS * 8;
     static constexpr int IMG = NG * B_TILE + ROWS;           // image bytes per stage
-    static constexpr int SLOT = B_TILE + ROWS + 512;         // + 128 class words
+    static constexpr int SLOT = ROWS + 512;                  // + 128 class words
 };
 constexpr int F_LBO_B = 128, F_SBO_B = 512;
 template <bool PS> constexpr int f_lbo() { return PS ? 144 : 128; }   // P side: padded, so that a warp's
@@ -75,61 +82,56 @@ template <bool PS> constexpr int f_sbo() { return 4 * f_lbo<PS>(); }  // 32-bit 
 template <bool PS> constexpr int f_atile() { return 16 * f_sbo<PS>(); }
 
 struct FSync {
-    uint64_t full[F_RING];
+    uint64_t full[F_RING];    // vectors and class words landed
+    uint64_t fullb[F_BRING];  // B tile landed
     uint64_t gen;        // the generator warps have written a stage's digits (one arrival per warp)
     uint64_t mma;        // a stage's MMAs are done
     uint32_t tslot;
-    int bad, issued, loaded;
+    int bad, issued, loaded, loadedb;
 };
 
 template <int K, bool HESS, bool PS> constexpr size_t f_smem() {
     using D = FDim<K, HESS>;
-    return 128 + (size_t)F_NDA * f_atile<PS>() + (size_t)F_RING * D::SLOT + 128 * D::KS * 8 +
+    return 128 + (size_t)F_NDA * f_atile<PS>() + (size_t)F_BRING * D::B_TILE + (size_t)F_RING * D::SLOT + 128 * D::KS * 8 +
            F_GEN_WARPS * 256 * (8 + 2) + sizeof(FSync);
 }
 
-// Largest v[k] of each of the K rows of v (K x n), as partial maxima of the bit
-// patterns per block, and beside them whether the block met an entry of v or w (the
-// nw entries of the other matrix) outside [lo, 1] (bit patterns; an ulp or two above 1
-// passes, which a projection onto the simplex of one variable leaves).  Block 0 also
-// clears the flag of out-of-range weights.
-__global__ void __launch_bounds__(256) k_f64_range(const double* __restrict__ v, int K, int64_t n,
-                                                   const double* __restrict__ w, int64_t nw, unsigned long long lo,
-                                                   unsigned long long* __restrict__ mx, int* __restrict__ flag) {
-    __shared__ unsigned long long s[HX_KMAX + 1];
-    if (threadIdx.x <= HX_KMAX) s[threadIdx.x] = 0ull;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *flag = 0;
-    __syncthreads();
+// Per block: whether it met an entry of Q or P outside [lo, 1] (bit patterns; an ulp or
+// two above 1 passes, which a projection onto the simplex of one variable leaves).
+// Block 0 also clears the flag of out-of-range weights.
+__global__ void __launch_bounds__(256) k_f64_range(const double* __restrict__ q, int64_t nq,
+                                                   const double* __restrict__ p, int64_t np, unsigned long long lo,
+                                                   unsigned* __restrict__ off, int* __restrict__ flag) {
     const unsigned long long span = 0x3FF0000000000010ull - lo;
+    const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x, stride = (int64_t)gridDim.x * 256;
     bool out = false;
-    // a stride that is a multiple of K keeps each thread on one k
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x / K * K;
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < stride) {
-        unsigned long long m = 0ull;
-        for (int64_t a = t; a < n * K; a += stride) {
-            const unsigned long long b = (unsigned long long)__double_as_longlong(v[a]);
-            m = max(m, b);
-            out |= b - lo > span;
-        }
-        atomicMax(&s[t % K], m);
-        for (int64_t a = t; a < nw; a += stride) out |= (unsigned long long)__double_as_longlong(w[a]) - lo > span;
-    }
-    if (out) atomicMax(&s[HX_KMAX], 1ull);
-    __syncthreads();
-    if (threadIdx.x <= HX_KMAX) mx[(int64_t)blockIdx.x * F_MXS + threadIdx.x] = s[threadIdx.x];
+    for (int64_t a = t; a < nq; a += stride) out |= (unsigned long long)__double_as_longlong(q[a]) - lo > span;
+    for (int64_t a = t; a < np; a += stride) out |= (unsigned long long)__double_as_longlong(p[a]) - lo > span;
+    const int any = __syncthreads_or(out);
+    if (threadIdx.x == 0) off[blockIdx.x] = any ? 1u : 0u;
+    if (t == 0) *flag = 0;
 }
 
-// Exponents e_k with max |v_k| < 2^e_k, from the partial maxima; returns via
-// shared memory of HX_KMAX ints (where k_f64_range found no entry outside its range).
-__device__ __forceinline__ void f64_exponents(const unsigned long long* __restrict__ mx, int nb, int K, int* se) {
-    if (threadIdx.x < (unsigned)K) {
-        unsigned long long m = 0ull;
-        for (int b = 0; b < nb; ++b) m = max(m, mx[(int64_t)b * F_MXS + threadIdx.x]);
-        const int f = (int)(m >> 52);
-        se[threadIdx.x] = f - 1022;
-    }
-    __syncthreads();
+// Exponent f with x < 2^f, x >= 2^(f-1), of a positive x.
+__device__ __forceinline__ int f64_exponent(double x) { return (__double2hiint(x) >> 20) - 1022; }
+// The exponent kept with a row (entry K).
+__device__ __forceinline__ int f64_row_exp(const double* row, int K) { return __double2loint(row[K]); }
+
+// Fixed point of w 2^sh (w >= 0) in units of 2^-S, plus 128 in every one of the low
+// BYTES bytes: byte d minus 128 is then the signed digit of weight 256^d.
+template <int S, int BYTES>
+__device__ __forceinline__ void f64_fix(double w, int sh, uint32_t (&x)[3]) {
+    const uint32_t hi = (uint32_t)__double2hiint(w), lo = (uint32_t)__double2loint(w);
+    const int e = (int)(hi >> 20) - 1023 + (S - 52) + sh;   // of the 53-bit integer m
+    uint64_t m = ((uint64_t)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo;
+    if (hi < 0x100000u) m = 0;                             // zero (no subnormals here)
+    const int n = min(63, -e);
+    const uint64_t l = e >= 0 ? m << (e & 63) : (m + (1ull << ((n - 1) & 63))) >> (n & 63);   // rounded
+    const uint32_t h = e > 0 ? (uint32_t)(m >> ((64 - e) & 63)) : 0u;
+    constexpr uint32_t OFF = BYTES >= 12 ? 0x80808080u : 0x80808080u >> (8 * (12 - BYTES));
+    asm("add.cc.u32 %0, %3, %6;\n\t addc.cc.u32 %1, %4, %6;\n\t addc.u32 %2, %5, %7;"
+        : "=&r"(x[0]), "=&r"(x[1]), "=&r"(x[2])
+        : "r"((uint32_t)l), "r"((uint32_t)(l >> 32)), "r"(h), "r"(0x80808080u), "r"(OFF));
 }
 
 // Stage images: the digits of the products v_k v_k2 (or of v_k) of 32 reduction
@@ -138,42 +140,33 @@ __device__ __forceinline__ void f64_exponents(const unsigned long long* __restri
 // zeros (their class nibbles are padding).
 template <int K, bool HESS>
 __global__ void __launch_bounds__(128) k_f64_img(const double* __restrict__ v, int64_t n, int64_t stages,
-                                                 const unsigned long long* __restrict__ mx, int nb,
                                                  uint8_t* __restrict__ img) {
     using D = FDim<K, HESS>;
-    __shared__ int se[HX_KMAX];
-    f64_exponents(mx, nb, K, se);
     const int lane = threadIdx.x & 31;
     const int64_t st = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (st >= stages) return;
     const int64_t a = st * F_KD + lane;
     uint8_t* base = img + st * D::IMG;
-    double x[K], w[K];
+    double w[K], mx = 0.0;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        x[k] = a < n ? v[(int64_t)K * a + k] : 0.0;
-        w[k] = scalbn(x[k], -se[k]);
+        w[k] = a < n ? v[(int64_t)K * a + k] : 0.0;
+        mx = fmax(mx, w[k]);
     }
+    const int f = mx > 0.0 ? f64_exponent(mx) : 0;
     double* rows = reinterpret_cast<double*>(base + D::NG * D::B_TILE) + lane * D::KS;
 #pragma unroll
-    for (int k = 0; k < K; ++k) rows[k] = x[k];
-    // the index's exponent f: max |w| < 2^f
-    double mw = 0.0;
-#pragma unroll
-    for (int k = 0; k < K; ++k) mw = fmax(mw, fabs(w[k]));
-    const int fe = (int)((unsigned long long)__double_as_longlong(mw) >> 52);
-    const int f = fe == 0 ? 0 : fe - 1022;
+    for (int k = 0; k < K; ++k) rows[k] = w[k];
     rows[K] = __longlong_as_double((long long)f);
-#pragma unroll
-    for (int k = 0; k < K; ++k) w[k] = scalbn(w[k], -f);
-    auto put = [&](int c, double y) {   // sum c, value y in (-1, 1)
+    auto put = [&](int c, double y) {   // sum c, y 2^(-f or -2f) in [0, 1)
         const int g = c / D::PER, col = c - g * D::PER;
-        const unsigned long long u = (unsigned long long)__double2ll_rn(scalbn(y, F_SB)) + 0x8080808080808080ull;
+        uint32_t u[3];
+        f64_fix<F_SB, F_NDB>(y, HESS ? -2 * f : -f, u);
         uint8_t* tile = base + g * D::B_TILE;
 #pragma unroll
         for (int b = 0; b < F_NDB; ++b) {
-            const int row = b * D::NHP + col;
-            const int d = (int)((u >> (8 * (F_NDB - 1 - b))) & 0xFF) - 128;
+            const int row = b * D::NHP + col, byte = F_NDB - 1 - b;
+            const int d = (int)((u[byte >> 2] >> (8 * (byte & 3))) & 0xFF) - 128;
             uint16_t h;
             asm("cvt.rn.f16.s32 %0, %1;" : "=h"(h) : "r"(d));
             *reinterpret_cast<uint16_t*>(tile + (row >> 3) * F_SBO_B + (lane >> 3) * F_LBO_B + (row & 7) * 16 +
@@ -197,21 +190,6 @@ __global__ void __launch_bounds__(128) k_f64_img(const double* __restrict__ v, i
                 *reinterpret_cast<uint16_t*>(base + g * D::B_TILE + (row >> 3) * F_SBO_B + (lane >> 3) * F_LBO_B +
                                              (row & 7) * 16 + (lane & 7) * 2) = 0;
             }
-}
-
-// 80-bit fixed point of w 2^sh (0 <= w 2^sh < 2^TOP) in units of 2^-SA, plus 128
-// in every byte: byte d minus 128 is then the signed digit of weight 256^d.
-__device__ __forceinline__ void f64_fix(double w, int sh, uint32_t (&x)[3]) {
-    const uint32_t hi = (uint32_t)__double2hiint(w), lo = (uint32_t)__double2loint(w);
-    const int e = (int)(hi >> 20) - 1023 + (F_SA - 52) + sh;   // of the 53-bit integer m
-    uint64_t m = ((uint64_t)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo;
-    if (hi < 0x100000u) m = 0;                             // zero (subnormals vanish at 2^-SA)
-    const int n = min(63, -e);
-    const uint64_t l = e >= 0 ? m << (e & 63) : (m + (1ull << (n - 1))) >> n;   // rounded to a multiple of 2^-SA
-    const uint32_t h = e > 0 ? (uint32_t)(m >> (64 - e)) : 0u;
-    asm("add.cc.u32 %0, %3, %6;\n\t addc.cc.u32 %1, %4, %6;\n\t addc.u32 %2, %5, %7;"
-        : "=&r"(x[0]), "=&r"(x[1]), "=&r"(x[2])
-        : "r"((uint32_t)l), "r"((uint32_t)(l >> 32)), "r"(h), "r"(0x80808080u), "r"(0x8080u));
 }
 
 __device__ __forceinline__ uint32_t f64_h2(uint32_t pair_bytes, uint32_t sel) {
@@ -323,41 +301,34 @@ __device__ __forceinline__ void f64_weights(const unsigned (&nib)[2], const doub
     __syncwarp();
 }
 
-// Whether w 2^sh is outside the digits' range: too large, negative, not finite.
+// Whether w 2^sh is too large for the digits.
 __device__ __forceinline__ bool f64_out_of_range(double w, int sh) {
-    const int e = (int)((uint32_t)__double2hiint(w) >> 20);
-    return e >= 0x7FF || e + sh >= 1023 + F_TOP;
+    return (int)((uint32_t)__double2hiint(w) >> 20) + sh >= 1023 + F_TOP;
 }
 
-// A weight outside that range (see the top of the file): its products with the
-// group's vectors, in units of 2^-8 and 2^-56, to the row's integers.
+// A weight outside that range (see the top of the file), by a whole warp: its products
+// with the index's vector, times 2^s, each below 2^38, in units of 2^-72, as three
+// words of 37 bits, so that 2^26 of them fit the row's 64-bit integers.  The lanes take
+// one product each, and all of it is integer work but the products themselves.
 template <int K, bool HESS>
-__device__ __noinline__ void f64_rare(double w, const double* vrow, const unsigned long long* mx, int nb, int c0,
-                                      int c1, F64Rare ra, int64_t row) {
-    atomicOr(ra.flag, 1);
-    double v[K];
-    for (int k = 0; k < K; ++k) {
-        unsigned long long m = 0ull;
-        for (int b = 0; b < nb; ++b) m = max(m, mx[(int64_t)b * F_MXS + k]);
-        const int f = (int)(m >> 52);
-        v[k] = scalbn(vrow[k], f == 0 || f == 0x7FF ? 0 : 1022 - f);
+__device__ __noinline__ void f64_rare(double w, int s, const double* v, int c0, int c1, F64Rare ra, int64_t row) {
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) atomicOr(ra.flag, 1);
+    for (int c = c0 + lane; c < c1; c += 32) {
+        int k = c, k2 = c;
+        if (HESS) tri_pair<K>(c, k, k2);
+        const unsigned long long y = (unsigned long long)__double_as_longlong(HESS ? w * (v[k] * v[k2]) : w * v[k]);
+        const int e = (int)(y >> 52) - 1075 + 72 + s;
+        const unsigned long long m = (y & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+        const unsigned __int128 x = e >= 0 ? (unsigned __int128)m << e
+                                           : e > -54 ? (m + (1ull << (-e - 1))) >> -e : 0ull;
+        constexpr unsigned long long M37 = (1ull << 37) - 1;
+        unsigned long long* out = reinterpret_cast<unsigned long long*>(ra.i) + 3 * (row * FDim<K, HESS>::NV + c);
+        atomicAdd(out, (unsigned long long)(x >> 74));
+        atomicAdd(out + 1, (unsigned long long)(x >> 37) & M37);
+        atomicAdd(out + 2, (unsigned long long)x & M37);
     }
-    for (int k = 0; k < K; ++k)
-        for (int k2 = k; k2 < (HESS ? K : k + 1); ++k2) {
-            const int c = HESS ? tri_idx<K>(k, k2) : k;
-            if (c < c0 || c >= c1) continue;
-            const double y = HESS ? w * (v[k] * v[k2]) : w * v[k];
-            const int64_t at = row * FDim<K, HESS>::NV + c;
-            if (fabs(y) < 4398046511104.0) {           // 2^42
-                const long long A = __double2ll_rd(scalbn(y, 8));
-                const long long B = __double2ll_rn(scalbn(y - scalbn((double)A, -8), 56));
-                atomicAdd((unsigned long long*)ra.i + 2 * at, (unsigned long long)A);
-                atomicAdd((unsigned long long*)ra.i + 2 * at + 1, (unsigned long long)B);
-            } else {
-                atomicOr(ra.flag, 2);
-                atomicAdd(ra.d + at, y);
-            }
-        }
+    __syncwarp();
 }
 
 // ------------------------------------------------------------------ the pass
@@ -383,12 +354,12 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
     constexpr int LBO = f_lbo<PS>(), SBO = f_sbo<PS>(), AT = f_atile<PS>();
     extern __shared__ __align__(128) uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
-    uint8_t* ring = smem + F_NDA * AT;
+    uint8_t* ring = smem + F_NDA * AT + F_BRING * D::B_TILE;
     double* fix = reinterpret_cast<double*>(ring + F_RING * D::SLOT);      // [128][KS]
     double* rbuf = fix + 128 * D::KS;                                      // [GEN_WARPS][8][32]
     uint16_t* lists = reinterpret_cast<uint16_t*>(rbuf + F_GEN_WARPS * 256);
     FSync* sy = reinterpret_cast<FSync*>(lists + F_GEN_WARPS * 256);
-    const uint32_t sA = smem_u32(smem), sR = smem_u32(ring);
+    const uint32_t sA = smem_u32(smem), sB = sA + F_NDA * AT, sR = smem_u32(ring);
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int grp = blockIdx.z;
@@ -399,15 +370,17 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
     const int nwc = PS ? (int)min((int64_t)4, (int64_t)a.JW - (int64_t)blockIdx.x * 4) : 1;
 
     // inputs that the general passes take (k_accum_q, k_accum_p)
-    if (__syncthreads_or(tid < fa.nmx && fa.mx[tid * F_MXS + HX_KMAX] != 0ull)) return;
+    if (__syncthreads_or(tid < fa.noff && fa.off[tid] != 0u)) return;
     if (warp == F_GEN_WARPS) tmem_alloc<D::TCOLS>(&sy->tslot);
     if (tid == 0) {
         for (int r = 0; r < F_RING; ++r) mbar_init(&sy->full[r], 1);
+        for (int r = 0; r < F_BRING; ++r) mbar_init(&sy->fullb[r], 1);
         mbar_init(&sy->gen, F_GEN_WARPS);
         mbar_init(&sy->mma, 1);
         sy->bad = 0;
         sy->issued = 0;
         sy->loaded = 0;
+        sy->loadedb = 0;
         mbar_fence_init();
     }
     // the rows' own vectors
@@ -417,6 +390,15 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
         const int r = t / K, k = t - r * K;
         fix[r * D::KS + k] = row0 + r < nown ? own[(row0 + r) * K + k] : 0.25;
     }
+    if (PS && HESS && tid < 128) {        // the rows' exponents
+        double mx = 0.25;
+        if (row0 + tid < nown) {
+            mx = 0.0;
+#pragma unroll
+            for (int k = 0; k < K; ++k) mx = fmax(mx, own[(row0 + tid) * K + k]);
+        }
+        fix[tid * D::KS + K] = __longlong_as_double((long long)f64_exponent(mx));
+    }
     fence_before();
     __syncthreads();
     fence_after();
@@ -424,38 +406,53 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
 
     if (warp == F_GEN_WARPS) {
         const uint32_t el = elect_lane();
-        auto load = [&](int s) {
-            const int slot = s % F_RING;
-            const uint8_t* src = a.img + (s0 + s) * D::IMG;
-            const uint32_t dst = sR + slot * D::SLOT;
-            uint64_t* bar = &sy->full[slot];
-            const uint32_t wb = PS ? 128u * nwc : 512u;
+        auto copy = [&](uint32_t d, const void* g, uint32_t bytes, uint64_t* bar) {
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         :: "r"(d), "l"(g), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+        };
+        auto expect = [&](uint64_t* bar, uint32_t bytes) {
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                         :: "r"(smem_u32(bar)), "r"((uint32_t)(D::B_TILE + D::ROWS) + wb) : "memory");
-            auto copy = [&](uint32_t d, const void* g, uint32_t bytes) {
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                             :: "r"(d), "l"(g), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-            };
-            copy(dst, src + grp * D::B_TILE, D::B_TILE);
-            copy(dst + D::B_TILE, src + D::NG * D::B_TILE, D::ROWS);
+                         :: "r"(smem_u32(bar)), "r"(bytes) : "memory");
+        };
+        auto load_b = [&](int s) {
+            uint64_t* bar = &sy->fullb[s % F_BRING];
+            expect(bar, (uint32_t)D::B_TILE);
+            copy(sB + (s % F_BRING) * D::B_TILE, a.img + (s0 + s) * D::IMG + grp * D::B_TILE, D::B_TILE, bar);
+            *(volatile int*)&sy->loadedb = s + 1;
+        };
+        auto load = [&](int s) {          // vectors and class words
+            const uint32_t dst = sR + (s % F_RING) * D::SLOT;
+            uint64_t* bar = &sy->full[s % F_RING];
+            expect(bar, (uint32_t)D::ROWS + (PS ? 128u * nwc : 512u));
+            copy(dst, a.img + (s0 + s) * D::IMG + D::NG * D::B_TILE, D::ROWS, bar);
             if (PS) {
                 for (int w = 0; w < nwc; ++w)
-                    copy(dst + D::B_TILE + D::ROWS + 128 * w,
-                         a.G + ((int64_t)blockIdx.x * 4 + w) * a.Ipad + (s0 + s) * F_KD, 128);
+                    copy(dst + D::ROWS + 128 * w, a.G + ((int64_t)blockIdx.x * 4 + w) * a.Ipad + (s0 + s) * F_KD, 128,
+                         bar);
             } else {
-                copy(dst + D::B_TILE + D::ROWS, a.G + (s0 + s) * a.Ipad + row0, 512);
+                copy(dst + D::ROWS, a.G + (s0 + s) * a.Ipad + row0, 512, bar);
             }
             *(volatile int*)&sy->loaded = s + 1;
         };
-        if (el)
+        if (el) {
             for (int s = 0; s < F_RING && s < ns; ++s) load(s);
+            for (int s = 0; s < F_BRING && s < ns; ++s) load_b(s);
+        }
         for (int s = 0; s < ns; ++s) {
             // all digits of the stage written, and every warp past stage s-1
             if (!__all_sync(0xffffffffu, f_wait(sy, &sy->gen, s, a.slots))) break;
+            // the slots of stage s-1: its MMAs are done (every warp waited for
+            // them before it arrived for stage s) and its vectors are read
+            if (el && s >= 1) {
+                if (s + 2 < ns) load(s + 2);
+                if (s + 1 < ns) load_b(s + 1);
+            }
+            if (!__all_sync(0xffffffffu, f_wait(sy, &sy->fullb[s % F_BRING], s / F_BRING, a.slots))) break;
             fence_after();
-            const uint64_t dA = sdesc(sA, LBO, SBO), dB = sdesc(sR + (s % F_RING) * D::SLOT, F_LBO_B, F_SBO_B);
-            // one MMA per digit pair: all of one shape, so that those of one
-            // order (one accumulator) execute in issue order
+            const uint64_t dA = sdesc(sA, LBO, SBO), dB = sdesc(sB + (s % F_BRING) * D::B_TILE, F_LBO_B, F_SBO_B);
+            // One MMA per digit pair: all of one shape, so that those of one order
+            // (one accumulator) execute in issue order.  Where STR < NHP an order's
+            // zero columns add 0 to the next order's first ones, in the same order.
 #pragma unroll 1
             for (int d = 0; d < F_NDA; ++d)
 #pragma unroll
@@ -463,53 +460,65 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
                     if (d + b >= F_NORD) break;
 #pragma unroll
                     for (int ks = 0; ks < F_KD / 16; ++ks)
-                        mma_bf16(tmem + (d + b) * D::NHP, dA + (uint64_t)((d * AT + ks * 2 * LBO) >> 4),
+                        mma_bf16(tmem + (d + b) * D::STR, dA + (uint64_t)((d * AT + ks * 2 * LBO) >> 4),
                                  dB + (uint64_t)((b * (D::NHP / 8) * F_SBO_B + ks * 2 * F_LBO_B) >> 4),
                                  idesc_f16(D::NHP), 1u, el);
                 }
             commit(&sy->mma, el);
             if (el) *(volatile int*)&sy->issued = s + 1;
-            // the slot of stage s-1: its MMAs are done (every warp waited for
-            // them before it arrived for stage s) and its vectors are read
-            if (el && s >= 1 && s + 2 < ns) load(s + 2);
         }
         __syncwarp();
     } else {
         constexpr int NPC = D::NPC;
-        const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((warp >> 2) * NPC);
-        long long accA[NPC], accB[NPC];
+        const int col0 = (warp >> 2) * NPC;                  // this thread's columns of an order
+        const bool cols = col0 < D::STR;                     // (a quarter of the warps has none where STR < NHP)
+        const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)col0;
+        __int128 acc[NPC];                                   // units 2^-94, of order 12
 #pragma unroll
-        for (int c = 0; c < NPC; ++c) { accA[c] = 0; accB[c] = 0; }
-        // the window's columns go to the integer sums (orders 0-4 in units of
-        // 2^-22, orders 5-9 in units of 2^-62) and are cleared
+        for (int c = 0; c < NPC; ++c) acc[c] = 0;
+        // the window's columns go to the integer sums and are cleared
         auto zero_cols = [&]() {
+            if (cols)
 #pragma unroll
-            for (int o = 0; o < F_NORD; ++o)
+                for (int o = 0; o < F_NORD; ++o)
 #pragma unroll
-                for (int c = 0; c < NPC; c += 4)
-                    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %1, %1, %1};"
-                                 :: "r"(tl + (uint32_t)(o * D::NHP + c)), "r"(0u) : "memory");
+                    for (int c = 0; c < NPC; c += 4)
+                        asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %1, %1, %1};"
+                                     :: "r"(tl + (uint32_t)(o * D::STR + c)), "r"(0u) : "memory");
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             fence_before();
         };
+        // orders O0 .. O1 of four columns, Horner in base 256 (at most 2^24 each)
+        auto read_orders = [&](int c, int o0, int o1, long long (&t)[4]) {
+            uint32_t v[5][4];
+#pragma unroll
+            for (int o = 0; o < 5; ++o)
+                if (o0 + o <= o1)
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(v[o][0]), "=r"(v[o][1]), "=r"(v[o][2]), "=r"(v[o][3])
+                                 : "r"(tl + (uint32_t)((o0 + o) * D::STR + c)));
+            tmem_wait_ld();
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                t[x] = 0;
+#pragma unroll
+                for (int o = 0; o < 5; ++o)
+                    if (o0 + o <= o1) t[x] = t[x] * 256 + __float2int_rz(__uint_as_float(v[o][x]));
+            }
+        };
         auto read_out = [&]() {
             fence_after();
+            if (cols)
 #pragma unroll
-            for (int o = 0; o < F_NORD; ++o) {
-                uint32_t v[NPC];
+                for (int c = 0; c < NPC; c += 4) {
+                    long long t0[4], t1[4], t2[4];           // units 2^-30, 2^-62, 2^-94
+                    read_orders(c, 0, 4, t0);
+                    read_orders(c, 5, 8, t1);
+                    read_orders(c, 9, 12, t2);
 #pragma unroll
-                for (int c = 0; c < NPC; c += 4)
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                                 : "=r"(v[c]), "=r"(v[c + 1]), "=r"(v[c + 2]), "=r"(v[c + 3])
-                                 : "r"(tl + (uint32_t)(o * D::NHP + c)));
-                tmem_wait_ld();
-#pragma unroll
-                for (int c = 0; c < NPC; ++c) {
-                    const int x = __float2int_rz(__uint_as_float(v[c]));
-                    if (o < 5) accA[c] += (long long)x * (1ll << (8 * (4 - o)));
-                    else accB[c] += (long long)x * (1ll << (8 * (9 - o)));
+                    for (int x = 0; x < 4; ++x)
+                        acc[c + x] += ((__int128)t0[x] << 64) + ((__int128)t1[x] << 32) + t2[x];
                 }
-            }
         };
         zero_cols();
         const int lr = 32 * (warp & 3) + lane;                          // TMEM lane (row) of this thread
@@ -519,8 +528,8 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
         for (; s < ns; ++s) {
             const uint8_t* slot = ring + (s % F_RING) * D::SLOT;
             if (is_bad_f(sy) || !__all_sync(0xffffffffu, f_wait(sy, &sy->full[s % F_RING], s / F_RING, a.slots))) break;
-            const double* srow = reinterpret_cast<const double*>(slot + D::B_TILE);
-            const uint32_t* words = reinterpret_cast<const uint32_t*>(slot + D::B_TILE + D::ROWS);
+            const double* srow = reinterpret_cast<const double*>(slot);
+            const uint32_t* words = reinterpret_cast<const uint32_t*>(slot + D::ROWS);
             unsigned nib[2];
             const double *qrow, *prow;
             if (PS) {
@@ -545,26 +554,29 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
             for (int c = 0; c < 8; ++c) {
                 W[c] = (unsigned)(TAB_NEED >> (4 * nib[c >> 2] + (c & 3))) & 1u ? rb[32 * c + lane] : 0.0;
             }
-            // powers of two to scale by: the exponents of the reduction indices
-            auto sh = [&](int c) {
-                const double* row = PS ? qrow + lane * D::KS : prow + c * D::KS;
-                return (HESS ? 2 : 1) * (int)__double2loint(row[K]);
-            };
+            // powers of two to scale by: the exponents of the reduction indices, and the
+            // rows' on the P side
+            auto fexp = [&](int c) { return f64_row_exp(PS ? qrow + lane * D::KS : prow + c * D::KS, K); };
+            auto gexp = [&](int c) { return PS && HESS ? f64_row_exp(prow + c * D::KS, K) : 0; };
+            auto sh = [&](int c) { return (HESS ? 2 : 1) * fexp(c) + gexp(c); };
             bool big = false;
 #pragma unroll
             for (int c = 0; c < 8; ++c) big |= f64_out_of_range(W[c], sh(c));
-            if (big) {
+            if (__any_sync(0xffffffffu, big)) {
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    if (f64_out_of_range(W[c], sh(c))) {
-                        const int c0 = grp * D::PER, c1 = min(D::NV, c0 + D::PER);
-                        if (PS)
-                            f64_rare<K, HESS>(W[c], qrow + lane * D::KS, fa.mx, fa.nmx, c0, c1, fa.rare,
-                                              row0 + 8 * warp + c);
-                        else
-                            f64_rare<K, HESS>(W[c], prow + c * D::KS, fa.mx, fa.nmx, c0, c1, fa.rare, row0 + lr);
-                        W[c] = 0.0;
+                for (int c = 0; c < 8; ++c) {
+                    const bool mine = f64_out_of_range(W[c], sh(c));
+                    unsigned left = __ballot_sync(0xffffffffu, mine);
+                    while (left) {
+                        const int l = __ffs(left) - 1;
+                        left &= left - 1;
+                        f64_rare<K, HESS>(__shfl_sync(0xffffffffu, W[c], l), gexp(c),
+                                          PS ? qrow + l * D::KS : prow + c * D::KS, grp * D::PER,
+                                          min(D::NV, (grp + 1) * D::PER), fa.rare,
+                                          PS ? row0 + 8 * warp + c : row0 + 32 * (warp & 3) + l);
                     }
+                    if (mine) W[c] = 0.0;
+                }
             }
             __syncwarp();
             // the digit tiles and the accumulators are free once stage s-1's MMAs are done
@@ -579,14 +591,15 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
                 // lane pairs (2t, 2t+1) share 32-bit words of two reduction
                 // indices: the even lane stores block 0's rows, the odd one block 1's
                 const bool odd = lane & 1;
-                const int shm = sh(0), sho = __shfl_xor_sync(0xffffffffu, shm, 1);
+                const int shm = (HESS ? 2 : 1) * fexp(0), sho = __shfl_xor_sync(0xffffffffu, shm, 1);
                 uint32_t x0[4][3], x1[4][3];
 #pragma unroll
                 for (int h = 0; h < 4; ++h) {
                     const double mine = odd ? W[4 + h] : W[h];
                     const double other = __shfl_xor_sync(0xffffffffu, odd ? W[h] : W[4 + h], 1);
-                    f64_fix(odd ? other : mine, odd ? sho : shm, x0[h]);
-                    f64_fix(odd ? mine : other, odd ? shm : sho, x1[h]);
+                    const int g = gexp((odd ? 4 : 0) + h);
+                    f64_fix<F_SA, F_NDA>(odd ? other : mine, (odd ? sho : shm) + g, x0[h]);
+                    f64_fix<F_SA, F_NDA>(odd ? mine : other, (odd ? shm : sho) + g, x1[h]);
                 }
                 const uint32_t at = sA + warp * SBO + (lane >> 3) * LBO + (odd ? 64 : 0) + (lane & 6) * 2;
 #pragma unroll
@@ -596,7 +609,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
                         uint32_t dg[4];
                         f64_digits4(x0[h][w], x1[h][w], dg);
 #pragma unroll
-                        for (int t = 0; t < (w < 2 ? 4 : 2); ++t)
+                        for (int t = 0; t < (w < 2 ? 4 : F_NDA - 8); ++t)
                             asm volatile("st.shared.b32 [%0], %1;"
                                          :: "r"(at + (uint32_t)((F_NDA - 1 - (4 * w + t)) * AT + 16 * h)), "r"(dg[t])
                                          : "memory");
@@ -604,7 +617,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
             } else {
                 uint32_t x[8][3];
 #pragma unroll
-                for (int c = 0; c < 8; ++c) f64_fix(W[c], sh(c), x[c]);
+                for (int c = 0; c < 8; ++c) f64_fix<F_SA, F_NDA>(W[c], sh(c), x[c]);
                 const uint32_t at = sA + (lr >> 3) * SBO + (warp >> 2) * LBO + (lr & 7) * 16;
 #pragma unroll
                 for (int w = 0; w < 3; ++w) {
@@ -612,7 +625,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
 #pragma unroll
                     for (int e = 0; e < 4; ++e) f64_digits4(x[2 * e][w], x[2 * e + 1][w], dg[e]);
 #pragma unroll
-                    for (int t = 0; t < (w < 2 ? 4 : 2); ++t)
+                    for (int t = 0; t < (w < 2 ? 4 : F_NDA - 8); ++t)
                         sts128(at + (uint32_t)((F_NDA - 1 - (4 * w + t)) * AT), dg[0][t], dg[1][t], dg[2][t], dg[3][t]);
                 }
             }
@@ -628,10 +641,11 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
             double* out = a.part + (int64_t)blockIdx.y * D::NV * rows;
 #pragma unroll
             for (int c = 0; c < NPC; ++c) {
-                const int col = (warp >> 2) * NPC + c;
+                const int col = col0 + c;
                 const int v = grp * D::PER + col;
                 if (col < D::PER && v < D::NV)
-                    out[(int64_t)v * rows + row] = scalbn((double)accA[c], -22) + scalbn((double)accB[c], -62);
+                    out[(int64_t)v * rows + row] = scalbn((double)(long long)(acc[c] >> 64), -30) +
+                                                   scalbn((double)(unsigned long long)acc[c], -94);
             }
         }
     }
@@ -643,6 +657,9 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
         if (n > 0) mbar_wait(&sy->mma, (uint32_t)((n - 1) & 1), F_BUDGET);
         for (int t = (l >= F_RING ? l - F_RING : 0); t < l; ++t)
             mbar_wait(&sy->full[t % F_RING], (uint32_t)((t / F_RING) & 1), F_BUDGET);
+        const int lb = sy->loadedb;
+        for (int t = (lb >= F_BRING ? lb - F_BRING : 0); t < lb; ++t)
+            mbar_wait(&sy->fullb[t % F_BRING], (uint32_t)((t / F_BRING) & 1), F_BUDGET);
         __syncthreads();
     }
     fence_before();

@@ -25,17 +25,18 @@ cudaError_t f64_attrs_k() {
 template <int K, bool HESS, bool PS>
 cudaError_t f64_launch(const F64Call& c) {
     using D = FDim<K, HESS>;
+    static_assert(f_smem<K, HESS, PS>() <= 232448, "shared memory of one CTA");
+    static_assert((F_NORD - 1) * D::STR + D::NHP <= D::TCOLS && D::PER <= D::STR, "TMEM columns");
     const PassArgs& a = c.a;
     const double* v = PS ? a.q : a.p;             // the vectors along the reduction
     const int64_t n = PS ? a.I : 4 * a.J;
     const int64_t stages = PS ? (a.I + F_KD - 1) / F_KD : a.JW;
     const int64_t tiles = PS ? (a.J + 31) / 32 : a.Ipad / 128;
-    const double* w = PS ? a.p : a.q;             // the rows' own
-    const int64_t nw = (PS ? 4 * a.J : a.I) * K;
-    const int nmx = (int)std::min<int64_t>(F_MAXB, (n * K + nw + 2047) / 2048);
-    k_f64_range<<<nmx, 256, 0, c.st>>>(v, K, n, w, nw, HESS ? F_LO_HESS : F_LO_GRAD, c.mx, c.rare.flag);
-    k_f64_img<K, HESS><<<(unsigned)((stages + 3) / 4), 128, 0, c.st>>>(v, n, stages, c.mx, nmx, a.img);
-    F64Args fa{stages, c.mx, nmx, c.rare};
+    const int64_t nq = a.I * K, np = 4 * a.J * K;
+    const int noff = (int)std::min<int64_t>(F_MAXB, (nq + np + 1023) / 1024);
+    k_f64_range<<<noff, 256, 0, c.st>>>(a.q, nq, a.p, np, HESS ? F_LO_HESS : F_LO_GRAD, c.off, c.rare.flag);
+    k_f64_img<K, HESS><<<(unsigned)((stages + 3) / 4), 128, 0, c.st>>>(v, n, stages, a.img);
+    F64Args fa{stages, c.off, noff, c.rare};
     dim3 grid((unsigned)tiles, (unsigned)a.S, D::NG);
     k_f64_pass<K, HESS, PS><<<grid, F_THREADS, f_smem<K, HESS, PS>(), c.st>>>(a, fa);
     cudaError_t e = cudaGetLastError();
@@ -43,13 +44,12 @@ cudaError_t f64_launch(const F64Call& c) {
     PassArgs g = a;
     g.S = c.Sg;
     g.per_chunk = c.per_chunk_g;
-    g.run_if = c.mx + HX_KMAX;
-    g.n_run_if = nmx;
-    g.run_if_ld = F_MXS;
+    g.run_if = c.off;
+    g.n_run_if = noff;
     e = PS ? launch_accum_p_f64(K, HESS, g, c.st) : launch_accum_q_f64(K, HESS, g, c.st);
     if (e != cudaSuccess) return e;
     const int64_t rows = PS ? 4 * a.J : a.I;
-    return launch_f64_reduce(a.part, a.S, c.Sg, K, HESS, rows, PS ? rows : a.Ipad, PS ? a.p : a.q, c.mx, nmx, c.rare,
+    return launch_f64_reduce(a.part, a.S, c.Sg, K, HESS, PS && HESS, rows, PS ? rows : a.Ipad, PS ? a.p : a.q, c.off, noff, c.rare,
                              a.XtX, a.Xtz, c.st);
 }
 template <int K>

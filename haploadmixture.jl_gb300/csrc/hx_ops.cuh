@@ -57,22 +57,32 @@ int tc_resident(int K, bool p_side);
 // weights, kept zero between passes, and what the pass kernel takes beside
 // PassArgs (per_chunk counts stages there).
 struct F64Rare {
-    long long* i;          // [rows][NV][2] fixed-point sums
-    double* d;             // [rows][NV]
-    int* flag;             // bit 0: i was added to, bit 1: d was
+    long long* i;          // [rows][NV][3] fixed-point sums, units 2^2, 2^-35, 2^-72
+    int* flag;             // whether i was added to
 };
-constexpr int F_MXS = 16;  // partial maxima of one block: HX_KMAX values, then a flag
-constexpr int F_MAXB = ACC_THREADS; // blocks of partial maxima (one thread of a CTA reads one)
+constexpr int F_MAXB = ACC_THREADS;   // blocks of the range check (one thread of a CTA reads one)
 // Least entry of Q and P (bit pattern) that the digit passes take: 2^-17 with the
 // Hessian, whose products then stay above 2^-34, 2^-34 without.  The fit's own values
 // are above it (pseudocount 1e-5); all others go to the general passes.
 constexpr unsigned long long F_LO_HESS = (1023ull - 17) << 52, F_LO_GRAD = (1023ull - 34) << 52;
 struct F64Args {
     int64_t stages;                   // of 32 reduction indices
-    const unsigned long long* mx;     // [nmx][F_MXS]
-    int nmx;
+    const unsigned* off;              // [noff] inputs outside that range met
+    int noff;
     F64Rare rare;
 };
+// Digits of a weight and of a product, orders kept (hx_f64.cuh), and the columns of a
+// row's sums: `per` of them in F_NORD groups of TMEM columns, each as wide as the MMA
+// where that fits 512 columns, else overlapping by the MMA's zero columns.
+constexpr int F_NDA = 9, F_NDB = 11, F_NORD = 13;
+constexpr int f64_nhp(int per) { return (per + 15) / 16 * 16; }
+constexpr int f64_stride(int per) { return F_NORD * f64_nhp(per) <= 512 ? f64_nhp(per) : (per + 3) / 4 * 4; }
+// column groups (grid.z) of nv sums
+constexpr int f64_groups(int nv) {
+    int g = 1;
+    while ((F_NORD - 1) * f64_stride((nv + g - 1) / g) + f64_nhp((nv + g - 1) / g) > 512) ++g;
+    return g;
+}
 // One pass: range of the inputs, stage images, the digit pass (partial sums in a.part,
 // [S][NV][rows]), or the general one in its place ([Sg][K + NV][rows]), and their
 // reduction to XtX and Xtz (a.XtX, a.Xtz).
@@ -80,20 +90,20 @@ struct F64Call {
     bool p_side, hess;
     PassArgs a;
     int Sg, per_chunk_g;              // chunks of the general pass
-    unsigned long long* mx;           // F_MAXB * F_MXS words
+    unsigned* off;                    // F_MAXB words
     F64Rare rare;
     cudaStream_t st;
 };
 cudaError_t launch_f64_pass(int K, const F64Call& c);
 cudaError_t f64_attrs(int K);         // once per device before the first pass
 size_t f64_image_bytes(int K, int64_t I, int64_t J);
-cudaError_t launch_f64_reduce(const double* part, int S, int Sg, int K, bool hess, int64_t rows, int64_t ld,
-                              const double* x, const unsigned long long* mx, int nmx, const F64Rare& rare, double* XtX,
+// g: whether the rows' exponents scale the digit passes' sums (P side, Hessian)
+cudaError_t launch_f64_reduce(const double* part, int S, int Sg, int K, bool hess, bool g, int64_t rows, int64_t ld,
+                              const double* x, const unsigned* off, int noff, const F64Rare& rare, double* XtX,
                               double* Xtz, cudaStream_t st);
-// Stages per chunk, 32 reduction indices each.  The 64-bit sums of orders 5 .. 9 take at
-// most 6 x 2^14 x 2^32 + 7 x 2^14 x 2^24 + ... < 2^48.6 per index in units of 2^-62, so
-// 2^14.3 indices (679 stages) stay below 2^63 whatever the digits are.
-constexpr int F64_MAX_STAGES = 512;
+// Stages per chunk, 32 reduction indices each: a sum is at most 2^14 per index, and the
+// 128-bit integers hold 2^33.
+constexpr int F64_MAX_STAGES = 2048;
 
 cudaError_t launch_f2d(const float* a, int64_t n, double* out, cudaStream_t st);
 cudaError_t launch_d2f(const double* a, int64_t n, float* out, cudaStream_t st);

@@ -50,8 +50,8 @@ struct PassArgs {
     const float* pf;        // FP32 copy of p for the FP32 passes that stage p (or null): GB300's
                             // FP64 unit is narrow, and converting in every CTA kept it busy
     long long budget;       // tensor-core passes: clock64 cycles any one pipeline wait may take
-    const unsigned long long* run_if = nullptr;   // T = double: run if any of the n_run_if (at most
-    int n_run_if = 0, run_if_ld = 1;              // ACC_THREADS) words, run_if_ld apart, is not zero
+    const unsigned* run_if = nullptr;   // T = double: run if any of these n_run_if (at most
+    int n_run_if = 0;                   // ACC_THREADS) words is not zero
 };
 
 template <int K> __device__ __forceinline__ constexpr int tri(int k, int k2) {
@@ -63,7 +63,7 @@ template <int K> __device__ __forceinline__ constexpr int tri(int k, int k2) {
 // the digit sums of hx_f64.cuh do not take; run_if says on the device whether it is
 // one of them.
 template <typename T> __device__ __forceinline__ bool pass_idle(const PassArgs& a) {
-    return sizeof(T) == 8 && !__syncthreads_or((int)threadIdx.x < a.n_run_if && a.run_if[threadIdx.x * a.run_if_ld] != 0ull);
+    return sizeof(T) == 8 && !__syncthreads_or((int)threadIdx.x < a.n_run_if && a.run_if[threadIdx.x] != 0u);
 }
 template <int K, typename T, bool HESS>
 __global__ void __launch_bounds__(ACC_THREADS)

@@ -106,6 +106,19 @@ def vertices(c, floor):
     return np.asfortranarray(q), np.asfortranarray(np.maximum(p, floor).reshape(K, 4 * J))
 
 
+@pytest.mark.parametrize("K,I,J", [(3, 30, 40), (5, 250, 40), (8, 60, 30), (9, 90, 30), (11, 80, 24), (12, 129, 33)])
+def test_entries_of_small_products_only(hx, O, K, I, J):
+    """Floored rows at the fit's own pseudocount: where all carriers of a haplotype
+    are of one ancestry, an entry of two others sums products of two floors, 1e-10 of
+    the row's largest."""
+    c = small_cohort(I, J, K, seed=K + I, miss=0.03)
+    q, p = vertices(c, 1e-5)
+    d = handle(hx, c)
+    for g, w in zip(accums(d, q, p), oracle_accums(O, c, q, p)):
+        assert entry_err(g, w) < 1e-13
+    d.close()
+
+
 def test_zero_frequencies_leave_the_gradient(hx, O):
     """A haplotype of frequency zero that no genotype of its block allows: its terms
     are 0 in the gradient (and 0 / 0 in the Hessian only)."""
