@@ -58,7 +58,8 @@ constexpr int F_RING = 3;                             // vectors and class words
 constexpr int F_BRING = 2;                            // B tiles: read by the MMAs only, a stage later
 constexpr int F_WIN = 3;                              // stages per read-out (96 reduction indices)
 constexpr int F_SA = 56, F_SB = 86;                   // units 2^-SA of W', 2^-SB of the products
-constexpr long long F_BUDGET = 4000000000LL;          // bound of any pipeline wait (clock64 cycles)
+constexpr long long F_BUDGET = 4000000000LL;          // bound of the waits that drain a pass that timed out (clock64
+                                                      // cycles; the pipeline's own take PassArgs::budget)
 constexpr int F_TOP = 14;                             // W' < 2^TOP: TOP + SA + 1 bits fit ND_A signed bytes
 
 template <int K, bool HESS> struct FDim {
@@ -208,12 +209,15 @@ __device__ __forceinline__ void f64_digits4(uint32_t x0, uint32_t x1, uint32_t (
     out[3] = f64_h2(p23, 0x4342);
 }
 
-__device__ __forceinline__ bool is_bad_f(const FSync* sy) { return *(volatile const int*)&sy->bad != 0; }
-__device__ __forceinline__ bool f_wait(FSync* sy, uint64_t* bar, int phase, double* slots) {
-    if (mbar_wait(bar, (uint32_t)(phase & 1), F_BUDGET)) return true;
-    *(volatile int*)&sy->bad = 1;
-    slots[S_TC_TIMEOUT] = 1.0;
-    return false;
+// A wait of a whole warp: true if the phase is complete in time and no warp of the CTA
+// has given up.  The lanes decide together, so that they leave together.
+__device__ __forceinline__ bool f_wait(FSync* sy, uint64_t* bar, int phase, const PassArgs& a) {
+    const bool ok = mbar_wait(bar, (uint32_t)(phase & 1), a.budget);
+    if (!ok) {
+        *(volatile int*)&sy->bad = 1;
+        a.slots[S_TC_TIMEOUT] = 1.0;
+    }
+    return __all_sync(0xffffffffu, ok && *(volatile const int*)&sy->bad == 0);
 }
 
 // Weights of a warp's 2 x 32 pairs: lane = individual, blocks bb = 0, 1 of
@@ -440,14 +444,14 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
         }
         for (int s = 0; s < ns; ++s) {
             // all digits of the stage written, and every warp past stage s-1
-            if (!__all_sync(0xffffffffu, f_wait(sy, &sy->gen, s, a.slots))) break;
+            if (!f_wait(sy, &sy->gen, s, a)) break;
             // the slots of stage s-1: its MMAs are done (every warp waited for
             // them before it arrived for stage s) and its vectors are read
             if (el && s >= 1) {
                 if (s + 2 < ns) load(s + 2);
                 if (s + 1 < ns) load_b(s + 1);
             }
-            if (!__all_sync(0xffffffffu, f_wait(sy, &sy->fullb[s % F_BRING], s / F_BRING, a.slots))) break;
+            if (!f_wait(sy, &sy->fullb[s % F_BRING], s / F_BRING, a)) break;
             fence_after();
             const uint64_t dA = sdesc(sA, LBO, SBO), dB = sdesc(sB + (s % F_BRING) * D::B_TILE, F_LBO_B, F_SBO_B);
             // One MMA per digit pair: all of one shape, so that those of one order
@@ -527,7 +531,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
         int s = 0;
         for (; s < ns; ++s) {
             const uint8_t* slot = ring + (s % F_RING) * D::SLOT;
-            if (is_bad_f(sy) || !__all_sync(0xffffffffu, f_wait(sy, &sy->full[s % F_RING], s / F_RING, a.slots))) break;
+            if (!f_wait(sy, &sy->full[s % F_RING], s / F_RING, a)) break;
             const double* srow = reinterpret_cast<const double*>(slot);
             const uint32_t* words = reinterpret_cast<const uint32_t*>(slot + D::ROWS);
             unsigned nib[2];
@@ -581,7 +585,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
             __syncwarp();
             // the digit tiles and the accumulators are free once stage s-1's MMAs are done
             if (s > 0) {
-                if (is_bad_f(sy) || !__all_sync(0xffffffffu, f_wait(sy, &sy->mma, s - 1, a.slots))) break;
+                if (!f_wait(sy, &sy->mma, s - 1, a)) break;
                 if (s % F_WIN == 0) {
                     read_out();
                     zero_cols();
@@ -634,7 +638,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
             __syncwarp();
             if (lane == 0) mbar_arrive(&sy->gen);
         }
-        if (s == ns && ns > 0 && __all_sync(0xffffffffu, f_wait(sy, &sy->mma, ns - 1, a.slots))) read_out();
+        if (s == ns && ns > 0 && f_wait(sy, &sy->mma, ns - 1, a)) read_out();
         const int64_t rows = PS ? 4 * a.J : a.Ipad;
         const int64_t row = row0 + lr;
         if (row < rows) {
@@ -650,7 +654,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
         }
     }
     __syncthreads();
-    if (is_bad_f(sy)) {
+    if (sy->bad) {
         // a wait ran out: let the MMAs and copies that were issued end before
         // tensor and shared memory are released
         const int n = sy->issued, l = sy->loaded;

@@ -136,3 +136,25 @@ def test_zero_frequencies_leave_the_gradient(hx, O):
     p[p == 0.0] = 1e-300                      # 0 / p instead of 0 / 0
     assert entry_err(zq, O.accum_q(b, 3, q, p)[1]) < 1e-13
     assert entry_err(zp, O.accum_p(b, 3, q, p)[1]) < 1e-13
+
+
+@pytest.mark.parametrize("side", ["q", "p", "em"])
+def test_wait_budget(hx, O, side):
+    """The plain passes' pipeline waits are bounded by hx_set_wait_budget: with one
+    cycle the call returns HX_ETIMEOUT, and the handle works again afterwards."""
+    from haplo_gb300 import _lib
+    c = small_cohort(300, 900, 4, seed=37, miss=0.03)
+    q, p = draws(c, 13)
+    b = O.Bed(c["bed"], c["I"], c["J"])
+    d = handle(hx, c)
+    call = {"q": d.update_q_accum, "p": d.update_p_accum, "em": d.em_accum}[side]
+    want = {"q": O.accum_q, "p": O.accum_p, "em": O.em_accum}[side](b, c["K"], q, p)
+    for _ in range(2):
+        d.set_wait_budget(1)
+        with pytest.raises(hx.HxError) as e:
+            call(q, p)
+        assert e.value.status == _lib.HX_ETIMEOUT
+        d.set_wait_budget(0)
+        for g, w in zip(call(q, p), want):
+            assert entry_err(g, w) < 1e-13
+    d.close()
