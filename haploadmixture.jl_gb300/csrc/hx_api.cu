@@ -41,8 +41,9 @@ struct hx_ctx {
     double *part_q = nullptr, *part_p = nullptr, *part_ll = nullptr, *part_qn = nullptr, *coef = nullptr;
     float* pf = nullptr;                     // mixed: FP32 copy of the pass's p (K x 4J)
     double* slots = nullptr;
-    double* h_slots = nullptr;   // pinned
-    int pin_slot = -1;           // its place in the process's pinned page, or -1
+    // host copy of the scalar block.  Pageable: pinned memory of its own costs a context
+    // 270 us, and the copies are 128 bytes
+    double h_slots[HX_NSLOT] = {};
     uint8_t* img = nullptr;      // B-operand image of the tensor-core passes
     // plain method: range flags and out-of-range sums of the passes (hx_f64.cuh)
     unsigned* f64_off = nullptr;
@@ -133,48 +134,6 @@ void prof_resolve(hx_ctx* c) {
         HX_CK(expr);             \
         prof_end(c, kind, n);    \
     } while (0)
-
-// Pinned host memory of a context's scalar block.  Allocating and releasing it
-// costs 270 us, most of the time of opening a small cohort, so the process
-// keeps one page with room for PIN_SLOTS contexts; slots go back when their
-// context is destroyed, and further contexts allocate their own.  The page is
-// looked up before a slot is handed out: a device reset in between frees it.
-constexpr int PIN_SLOTS = 32;
-std::mutex g_pin_mu;
-double* g_pin = nullptr;
-uint32_t g_pin_used = 0;
-
-cudaError_t pin_get(hx_ctx* c) {
-    std::lock_guard<std::mutex> g(g_pin_mu);
-    if (g_pin && g_pin_used == 0) {
-        cudaPointerAttributes at{};
-        if (cudaPointerGetAttributes(&at, g_pin) != cudaSuccess || at.type != cudaMemoryTypeHost) {
-            cudaGetLastError();
-            g_pin = nullptr;
-        }
-    }
-    if (!g_pin) {
-        const cudaError_t e = cudaHostAlloc((void**)&g_pin, PIN_SLOTS * HX_NSLOT * sizeof(double), cudaHostAllocPortable);
-        if (e != cudaSuccess) { g_pin = nullptr; return e; }
-        g_pin_used = 0;
-    }
-    for (int s = 0; s < PIN_SLOTS; ++s)
-        if (!((g_pin_used >> s) & 1u)) {
-            g_pin_used |= 1u << s;
-            c->pin_slot = s;
-            c->h_slots = g_pin + s * HX_NSLOT;
-            return cudaSuccess;
-        }
-    return cudaMallocHost((void**)&c->h_slots, HX_NSLOT * sizeof(double));
-}
-void pin_put(hx_ctx* c) {
-    if (c->pin_slot < 0) {
-        if (c->h_slots) cudaFreeHost(c->h_slots);
-        return;
-    }
-    std::lock_guard<std::mutex> g(g_pin_mu);
-    g_pin_used &= ~(1u << c->pin_slot);
-}
 
 inline double* qof(double* x) { return x; }
 inline double* pof(hx_ctx* c, double* x) { return x + (int64_t)c->K * c->I; }
@@ -387,6 +346,7 @@ int loglik_to_slot(hx_ctx* c, const double* q, const double* p, int slot) {
 }
 
 int read_slots(hx_ctx* c) {
+    HX_CK(cudaStreamSynchronize(c->st));   // first, so that the copy does not wait inside the driver
     HX_CK(cudaMemcpyAsync(c->h_slots, c->slots, HX_NSLOT * sizeof(double), cudaMemcpyDeviceToHost, c->st));
     HX_CK(cudaStreamSynchronize(c->st));
     prof_resolve(c);
@@ -629,7 +589,6 @@ int create_common(const uint8_t* bed, bool bed_on_device, int64_t bps, int64_t n
     c->V = c->U + nuv;
     if (c->prec == HX_PREC_FP64) HX_CK(cudaMemsetAsync(c->rare.i, 0, 3 * rows * NH * sizeof(long long), c->st));
     HX_CK(cudaMemsetAsync(c->qp_ws, 0, (size_t)4 * K * J, c->st));
-    HX_CK(pin_get(c));
     for (int s = 0; s < HX_NSLOT; ++s) c->h_slots[s] = 0.0;
     c->h_slots[S_LL_NEW] = NAN;
     HX_CK(cudaMemcpyAsync(c->slots, c->h_slots, HX_NSLOT * sizeof(double), cudaMemcpyHostToDevice, c->st));
@@ -756,7 +715,6 @@ int hx_destroy(hx_ctx* c) {
     if (c->arena) cudaFree(c->arena);
     prof_resolve(c);
     for (cudaEvent_t e : c->pool) cudaEventDestroy(e);
-    pin_put(c);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->st) cudaStreamDestroy(c->st);
