@@ -426,7 +426,7 @@ int update_q(hx_ctx* c, bool update2) {
     HX_ST(pass_q(c, q, p, true, c->XtXq, c->Xtzq));
     HX_LAUNCH(HX_KIND_OTHER, 1, launch_nan_check(c->XtXq, (int64_t)c->K * c->K * c->I, c->slots, c->st));
     HX_LAUNCH(HX_KIND_OTHER, 1, launch_nan_check(c->Xtzq, (int64_t)c->K * c->I, c->slots, c->st));
-    HX_LAUNCH(HX_KIND_QP_Q, 1, launch_qp_q(c->K, c->I, c->XtXq, c->Xtzq, q, qof(c->xt), c->slots, c->st,
+    HX_LAUNCH(HX_KIND_QP_Q, 1, launch_qp_q(c->K, c->I, c->J, c->XtXq, c->Xtzq, q, qof(c->xt), c->slots, c->st,
                                            c->lo.penalty == 1 ? c->rho : -1.0));
     auto step = [&](double f) {
         HX_LAUNCH(HX_KIND_OTHER, 1, launch_step_q(q, qof(c->xt), c->K, c->I, c->eps, out, c->st, f));
@@ -448,7 +448,7 @@ int update_p(hx_ctx* c, bool update2) {
     }
     HX_ST(pass_p(c, q, p, true, c->XtXp, c->Xtzp));
     HX_LAUNCH(HX_KIND_QP_P, 1,
-              launch_qp_p(c->K, c->J, c->XtXp, c->Xtzp, p, c->rho, pof(c, c->xt), c->slots, c->qp_ws, c->st,
+              launch_qp_p(c->K, c->J, c->I, c->XtXp, c->Xtzp, p, c->rho, pof(c, c->xt), c->slots, c->qp_ws, c->st,
                           c->lo.penalty == 0));
     auto step = [&](double f) {
         HX_LAUNCH(HX_KIND_OTHER, 1, launch_step_p(p, pof(c, c->xt), c->K, c->J, c->eps, out, c->st, f));
@@ -881,7 +881,7 @@ int hx_qp_q(hx_ctx* c, int64_t n, const double* XtX, const double* Xtz, const do
     HX_CK(cudaMemcpyAsync(dX, XtX, (size_t)K * K * n * 8, cudaMemcpyHostToDevice, c->st));
     HX_CK(cudaMemcpyAsync(dz, Xtz, (size_t)K * n * 8, cudaMemcpyHostToDevice, c->st));
     HX_CK(cudaMemcpyAsync(dq, q, (size_t)K * n * 8, cudaMemcpyHostToDevice, c->st));
-    HX_CK(launch_qp_q(K, n, dX, dz, dq, dd, c->slots, c->st, c->lo.penalty == 1 ? c->rho : -1.0));
+    HX_CK(launch_qp_q(K, n, INT64_MAX, dX, dz, dq, dd, c->slots, c->st, c->lo.penalty == 1 ? c->rho : -1.0));
     HX_CK(cudaMemcpyAsync(qdiff, dd, (size_t)K * n * 8, cudaMemcpyDeviceToHost, c->st));
     HX_CK(cudaStreamSynchronize(c->st));
     return HX_OK;
@@ -900,7 +900,7 @@ int hx_qp_p(hx_ctx* c, int64_t n, const double* XtX, const double* Xtz, const do
     HX_CK(cudaMemcpyAsync(dX, XtX, (size_t)K * K * 4 * n * 8, cudaMemcpyHostToDevice, c->st));
     HX_CK(cudaMemcpyAsync(dz, Xtz, (size_t)K * 4 * n * 8, cudaMemcpyHostToDevice, c->st));
     HX_CK(cudaMemcpyAsync(dp, p, (size_t)K * 4 * n * 8, cudaMemcpyHostToDevice, c->st));
-    HX_CK(launch_qp_p(K, n, dX, dz, dp, c->rho, dd, c->slots, nullptr, c->st, c->lo.penalty == 0));
+    HX_CK(launch_qp_p(K, n, INT64_MAX, dX, dz, dp, c->rho, dd, c->slots, nullptr, c->st, c->lo.penalty == 0));
     HX_CK(cudaMemcpyAsync(pdiff, dd, (size_t)K * 4 * n * 8, cudaMemcpyDeviceToHost, c->st));
     HX_CK(cudaStreamSynchronize(c->st));
     return HX_OK;
@@ -1192,7 +1192,7 @@ int hx_lws_warm_start(hx_ctx* c, const float* params, int32_t p_step, int32_t* a
         // x_next.p holds the QP's step (x_next is rewritten by the next iteration)
         HX_ST(pass_p(c, qof(c->xt), pof(c, c->x), true, c->XtXp, c->Xtzp));
         HX_LAUNCH(HX_KIND_QP_P, 1,
-                  launch_qp_p(c->K, c->J, c->XtXp, c->Xtzp, pof(c, c->x), c->rho, pof(c, c->xn), c->slots, c->qp_ws,
+                  launch_qp_p(c->K, c->J, c->I, c->XtXp, c->Xtzp, pof(c, c->x), c->rho, pof(c, c->xn), c->slots, c->qp_ws,
                               c->st, c->lo.penalty == 0));
         HX_LAUNCH(HX_KIND_OTHER, 1,
                   launch_step_p(pof(c, c->x), pof(c, c->xn), c->K, c->J, c->eps, pof(c, c->xt), c->st));

@@ -628,9 +628,9 @@ cudaError_t init_kernel_attrs(int K) {
                                          (int)(QP_WARPS * qp_warp_bytes(4 * HX_KMAX, HX_KMAX)));
     return e == cudaSuccess ? init_qp_attrs(K) : e;
 }
-cudaError_t launch_qp_p(int K, int64_t n, const double* XtX, const double* Xtz, const double* p, double rho,
+cudaError_t launch_qp_p(int K, int64_t n, int64_t I, const double* XtX, const double* Xtz, const double* p, double rho,
                         double* pdiff, double* slots, int8_t* ws, cudaStream_t st, bool eq) {
-    if (!eq) return launch_qp_p_pen(K, n, XtX, Xtz, p, rho, pdiff, slots, ws, st);
+    if (!eq) return launch_qp_p_pen(K, n, I, XtX, Xtz, p, rho, pdiff, slots, ws, st);
     const size_t smem = QP_WARPS * qp_warp_bytes(4 * K, K);
     k_qp_p_eq<<<nblk(n, QP_WARPS), 32 * QP_WARPS, smem, st>>>(K, n, XtX, Xtz, p, pdiff, slots);
     return cudaGetLastError();

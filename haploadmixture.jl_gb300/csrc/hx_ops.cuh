@@ -153,12 +153,13 @@ cudaError_t launch_step_p(const double* p, const double* d, int K, int64_t J, do
 // batched QP (init_kernel_attrs: before the first launch for this K on a device)
 cudaError_t init_kernel_attrs(int K);
 cudaError_t init_qp_attrs(int K);
-cudaError_t launch_qp_p_pen(int K, int64_t n, const double* XtX, const double* Xtz, const double* p, double rho,
+// n problems; J blocks (Q) or I individuals (P) of data behind each
+cudaError_t launch_qp_p_pen(int K, int64_t n, int64_t I, const double* XtX, const double* Xtz, const double* p, double rho,
                             double* pdiff, double* slots, int8_t* ws, cudaStream_t st);
-cudaError_t launch_qp_q(int K, int64_t n, const double* XtX, const double* Xtz, const double* q, double* qdiff,
+cudaError_t launch_qp_q(int K, int64_t n, int64_t J, const double* XtX, const double* Xtz, const double* q, double* qdiff,
                         double* slots, cudaStream_t st, double pen_rho = -1.0);
 // eq: the equality form (K equalities per block, rho and ws unused)
-cudaError_t launch_qp_p(int K, int64_t n, const double* XtX, const double* Xtz, const double* p, double rho,
+cudaError_t launch_qp_p(int K, int64_t n, int64_t I, const double* XtX, const double* Xtz, const double* p, double rho,
                         double* pdiff, double* slots, int8_t* ws, cudaStream_t st, bool eq = false);
 // quasi-Newton point (ZAL or LBQN)
 int qn_dots_blocks(int64_t n);

@@ -16,10 +16,14 @@
 // out only those whose operands are exact zeros, so the results do not depend
 // on this arrangement (the mixed method rounds them to FP32 afterwards, which
 // would turn a last-bit difference into one of 6e-8).  A free block that is not
-// positive definite to rounding (a mixed-precision Hessian whose entries span
-// more than its 16 bits) has a pivot at its floor, and what follows grows without
-// bound: such a problem is handed to the dense solver, where it is solved from
-// the start.
+// positive definite to rounding (fewer data than variables, or a mixed-precision
+// Hessian whose entries span more than its 16 bits) has pivots at their floor; what
+// follows grows, and where it overflows, the zeros of fixed variables meet infinities
+// that the dense solver never forms: such a problem is handed to it by its warp and
+// solved from the start.  (Every floored pivot went there once, one after another:
+// 20,000 problems of rank 1, K = 8, Q side: 6.9 ms, 1.9 here.)
+// Calls of few problems and P steps of a handful of individuals go to the dense solver
+// as a whole, a warp per problem (see the launchers).
 #include "hx_ops.cuh"
 #include "hx_qp_dense.cuh"
 #include "hx_tc.cuh"
@@ -62,6 +66,7 @@ __device__ __forceinline__ double inv_root(double s) {
     R = R + (q > g) + (q > 3 * g) - (q < -g) - (q < -3 * g);
     return __longlong_as_double((i64)(R + ((u64)(1021 - half) << 52)));
 }
+__device__ __forceinline__ bool finite(double x) { return (__double2hiint(x) & 0x7FF00000) != 0x7FF00000; }
 // x > f for f > 0
 __device__ __forceinline__ bool above(double x, double f) {
     const long long b = __double_as_longlong(x);
@@ -175,7 +180,7 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
     }
     tol *= 1e-12;
     const int max_iter = 4 * K + 20;
-    bool done = !mine, floored = false;
+    bool done = !mine, over = false;
 #pragma unroll 1
     for (int it = 0; it < max_iter && !done; ++it) {
         double A[NT], y[K], o[K];
@@ -203,8 +208,7 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
         for (int a = 0; a < K; ++a) {
             const double pv = A[tri_idx<K>(a, a)];
             const bool fa = (fr >> a) & 1u;
-            if (fa && !above(pv, fl)) floored = true;
-            iv[a] = fa ? inv_root(pv) : 0.0;
+            iv[a] = fa ? inv_root(above(pv, fl) ? pv : fl) : 0.0;
             y[a] *= iv[a];
             o[a] *= iv[a];
 #pragma unroll
@@ -229,7 +233,6 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
                 o[b] = fma(-A[tri_idx<K>(b, a)], o[a], o[b]);
             }
         }
-        if (floored) break;
         double nu = 0.0;
         if (eq && fr) {
             double f[K];
@@ -245,6 +248,7 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
         for (int a = 0; a < K; ++a) {
             if (!((fr >> a) & 1u)) { y[a] = d[a]; continue; }
             if (eq) y[a] = fma(-nu, o[a], y[a]);
+            over |= !finite(y[a]);
             const double s = y[a] - d[a];
             bool u;
             double num;
@@ -253,6 +257,7 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
                 if (ra < best) { best = ra; bi = a; bup = u; }
             }
         }
+        if (over) break;
         if (bi < 0) {
 #pragma unroll
             for (int a = 0; a < K; ++a) d[a] = y[a];
@@ -283,12 +288,12 @@ k_qp_q(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz
             up = bup ? up | (1u << bi) : up & ~(1u << bi);
         }
     }
-    if (mine && !floored) {
+    if (mine && !over) {
 #pragma unroll
         for (int a = 0; a < K; ++a) qdiff[pr * K + a] = d[a];
         if (!done) atomicAdd(slots + S_QP_FAIL, 1.0);
     }
-    unsigned left = __ballot_sync(FULL, floored);
+    unsigned left = __ballot_sync(FULL, over);
     while (left) {
         const int b = __ffs(left) - 1;
         left &= left - 1;
@@ -395,7 +400,7 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
     double dk[4];                                   // diagonal of H
 #pragma unroll
     for (int h = 0; h < 4; ++h) dk[h] = D[h * KK + kc * K + kc] + rho;
-    bool done = !valid, floored = false;            // floored: left to the dense solver
+    bool done = !valid, over = false;               // over: left to the dense solver
 #pragma unroll 1
     for (int it = 0; it < max_iter; ++it) {
         if (__all_sync(FULL, done)) break;
@@ -458,8 +463,7 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
 #pragma unroll
             for (int c = 0; c < K; ++c) {
                 const double pv = __shfl_sync(FULL, M[c], base + c);
-                if (((fm >> c) & 1u) && !done && !above(pv, fl)) floored = true;
-                const double ivc = (fm >> c) & 1u ? inv_root(pv) : 0.0;
+                const double ivc = (fm >> c) & 1u ? inv_root(above(pv, fl) ? pv : fl) : 0.0;
                 const double l = k > c ? M[c] * ivc : 0.0;
                 if (row) Lh[c * K + k] = l;
                 if (k == c) iv[h * K + c] = ivc;
@@ -513,7 +517,6 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
             x[1] = (fr >> (h + 2)) & 1u ? x[2] : 0.0;
             x[2] = (fr >> (h + 3)) & 1u ? x[3] : 0.0;
         }
-        done |= floored;
         __syncwarp();
         // backward sweep, the same way: x[b] belongs to haplotype h - b
 #pragma unroll
@@ -542,6 +545,10 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
         }
 #pragma unroll
         for (int h = 0; h < 4; ++h) x[h] = vec[h * K + kc];
+        bool inf = false;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) inf |= row && ((fr >> h) & 1u) && !finite(x[h]);
+        if (((__ballot_sync(FULL, inf) >> base) & ((1u << K) - 1u)) && !done) { over = true; done = true; }
         // targets; ratio test: smallest step ratio < 1, lowest variable index (h, k) on ties
         double best = 1.0;
         int bidx = INT_MAX;
@@ -624,7 +631,7 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
             else if (rel % K == k && row) fr |= 1u << (rel / K);
         }
     }
-    if (valid && row && !floored) {
+    if (valid && row && !over) {
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
             const int64_t at = (j * 4 + h) * K + k;
@@ -633,7 +640,7 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
         }
     }
     if (valid && !done && k == 0) atomicAdd(slots + S_QP_FAIL, 1.0);
-    unsigned left = __ballot_sync(FULL, floored && k == 0);
+    unsigned left = __ballot_sync(FULL, over && k == 0);
     while (left) {
         const int b = __ffs(left) - 1;
         left &= left - 1;
@@ -641,11 +648,44 @@ k_qp_p4(int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xt
     }
 }
 
+// ------------------------------------------------------------------ dense
+// All problems of a call on the dense solver, a warp each.
+constexpr int QD_WARPS = 4;
+template <bool PS>
+__global__ void __launch_bounds__(32 * QD_WARPS)
+k_qp_dense(int K, int64_t n, const double* __restrict__ XtX, const double* __restrict__ Xtz, const double* __restrict__ x,
+           double rho, double* __restrict__ diff, double* slots, int8_t* __restrict__ ws) {
+    extern __shared__ double smem_d[];
+    const int warp = threadIdx.x >> 5;
+    const int64_t t = (int64_t)blockIdx.x * QD_WARPS + warp;
+    if (t >= n) return;
+    double* base = smem_d + warp * (qp_warp_bytes(PS ? 4 * K : K) / sizeof(double));
+    if (PS) qp_p_dense(K, t, XtX, Xtz, x, rho, diff, slots, ws, base);
+    else qp_q_dense(K, t, XtX, Xtz, x, diff, slots, rho, base);
+}
+template <bool PS>
+cudaError_t launch_dense(int K, int64_t n, const double* XtX, const double* Xtz, const double* x, double rho, double* diff,
+                         double* slots, int8_t* ws, cudaStream_t st) {
+    k_qp_dense<PS><<<(unsigned)((n + QD_WARPS - 1) / QD_WARPS), 32 * QD_WARPS, QD_WARPS * qp_warp_bytes(PS ? 4 * K : K),
+                     st>>>(K, n, XtX, Xtz, x, rho, diff, slots, ws);
+    return cudaGetLastError();
+}
+
 #define HX_FOR_K(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12)
 }  // namespace
 
-cudaError_t launch_qp_q(int K, int64_t n, const double* XtX, const double* Xtz, const double* q, double* qdiff,
+// A lane's solve takes as long for one problem as for 20,000, and goes through all K
+// variables however many are fixed; the dense solver's time grows with the problems and
+// shrinks with the variables that are fixed.  It is ahead, for the whole Q step, where
+// blocks are fewer than variables (many bounds met one after another; 2 blocks, K = 5:
+// 0.45 -> 0.34 ms at 2,000 individuals, 0.48 -> 0.67 at 10,000; K = 8: 1.05 -> 0.72 at
+// 4,000, 1.13 -> 1.53 at 10,000; K = 3 the same at 2,000), and from K = 11 on for small
+// cohorts (500 blocks, K = 12: 0.46 -> 0.37 ms at 500 individuals, 0.82 -> 0.78 at 3,000,
+// the same at 4,000; K = 8: 0.21 ms both at 1,000).  The results are the same bits.
+cudaError_t launch_qp_q(int K, int64_t n, int64_t J, const double* XtX, const double* Xtz, const double* q, double* qdiff,
                         double* slots, cudaStream_t st, double pen_rho) {
+    if (J < K ? K >= 4 && n <= 500 * K : K >= 11 && n <= 250 * K)
+        return launch_dense<false>(K, n, XtX, Xtz, q, pen_rho, qdiff, slots, nullptr, st);
     const unsigned g = (unsigned)((n + QQ_THREADS - 1) / QQ_THREADS);
 #define HX_CASE(KK) case KK: k_qp_q<KK><<<g, QQ_THREADS, 0, st>>>(n, XtX, Xtz, q, qdiff, slots, pen_rho); break;
     switch (K) { HX_FOR_K(HX_CASE) default: return cudaErrorInvalidValue; }
@@ -654,6 +694,9 @@ cudaError_t launch_qp_q(int K, int64_t n, const double* XtX, const double* Xtz, 
 }
 
 cudaError_t init_qp_attrs(int K) {
+    cudaError_t e = cudaFuncSetAttribute(k_qp_dense<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(QD_WARPS * qp_warp_bytes(4 * HX_KMAX)));
+    if (e != cudaSuccess) return e;
 #define HX_CASE(KK)                                                                                     \
     case KK:                                                                                            \
         return cudaFuncSetAttribute(k_qp_p4<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PDim<KK>::SMEM);
@@ -661,8 +704,13 @@ cudaError_t init_qp_attrs(int K) {
 #undef HX_CASE
 }
 
-cudaError_t launch_qp_p_pen(int K, int64_t n, const double* XtX, const double* Xtz, const double* p, double rho,
+// With fewer than 2 K individuals most variables end at bounds, met one after another
+// (see launch_qp_q): whole P step of 5 individuals x 1,000 blocks, dense against K lanes,
+// K = 5: 3.9 and 6.8 ms, K = 8: 11.3 and 25.7, K = 12: 37.6 and 58.8; of 24 individuals x
+// 10,000 blocks, K = 8: 11.9 and 6.0.
+cudaError_t launch_qp_p_pen(int K, int64_t n, int64_t I, const double* XtX, const double* Xtz, const double* p, double rho,
                             double* pdiff, double* slots, int8_t* ws, cudaStream_t st) {
+    if (K >= 4 && I < 2 * K) return launch_dense<true>(K, n, XtX, Xtz, p, rho, pdiff, slots, ws, st);
 #define HX_CASE(KK)                                                                                              \
     case KK: {                                                                                                   \
         constexpr int per = PDim<KK>::WARPS * PDim<KK>::PW;                                                      \
