@@ -88,6 +88,39 @@ __device__ __forceinline__ double rcp64(double x) {
     return __longlong_as_double(r + ((i64)(2044u - ex) << 52));
 }
 
+// 1 / sqrt(s) as the QPs' factorisation uses it: the reciprocal of the rounded root,
+// both correctly rounded.  In fixed point: with s = m 4^k, 1 <= m < 4, one
+// cubically convergent step y (1 + e/2 + 3 e^2/8), e = 1 - m y^2, from the
+// hardware's FP32 reciprocal root leaves y ~ 1 / sqrt(m) within 2^-53, and
+// G ~ sqrt(m) = m y; the remainders m - G^2 and 1 - G R, exact in the low 64 bits
+// of the products, then tell how far G and R are from the nearest 53-bit numbers
+// (1 and 2 units at most).  Outside 2^-600 .. 2^600 the operators, out of line.
+static __device__ __noinline__ double inv_root_edge(double s) { return 1.0 / sqrt(s); }
+__device__ __forceinline__ double inv_root(double s) {
+    typedef unsigned long long u64;
+    typedef long long i64;
+    const int hi = __double2hiint(s);
+    if (((unsigned)hi >> 20) - 423u > 1200u) return inv_root_edge(s);
+    const int ex = (hi >> 20) - 1023, odd = ex & 1, half = (ex - odd) >> 1;
+    const u64 b = ((u64)__double_as_longlong(s) & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+    const u64 m = b << (10 + odd);                                     // m 2^62
+    float y0;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(__uint2float_rn((unsigned)(m >> 32)) * 0x1p-30f));
+    const unsigned Y0 = __float2uint_rz(y0 * 0x1p31f);                 // y 2^31, at most 2^31 (1 + 2^-22)
+    const i64 e = (i64)((1ull << 60) - __umul64hi(m, (u64)Y0 * Y0));   // 2^60, |e| < 2^39
+    const int e1 = (int)(e >> 24);                                     // 2^36
+    const i64 t = (e >> 1) + (((i64)e1 * e1 * 3) >> 15);               // e/2 + 3 e^2/8, 2^60
+    const int t1 = (int)((t + 64) >> 7);                               // 2^53
+    const u64 y = ((u64)Y0 << 31) + (u64)(((i64)Y0 * t1) >> 22);       // 2^62
+    u64 G = (__umul64hi(m, y) + 128) >> 8;                             // sqrt(m) 2^52
+    const i64 r = (i64)((m << 42) - G * G);
+    G = G + (r > (i64)G) - (r <= -(i64)G);
+    u64 R = (y + 256) >> 9;                                            // 2^53 / sqrt(m)
+    const i64 g = (i64)G, q = -2 * (i64)(R * G);                       // 2 (2^105 - R G)
+    R = R + (q > g) + (q > 3 * g) - (q < -g) - (q < -3 * g);
+    return __longlong_as_double((i64)(R + ((u64)(1021 - half) << 52)));
+}
+
 // Per-pair evaluation.  Given the class nibble and the mixed haplotype
 // frequencies qp[h] = sum_k q[k,i] p[k,4j+h] it returns
 //   L    : the pair likelihood (src/loops.jl:85-104, 254),
