@@ -45,6 +45,8 @@ __global__ void __launch_bounds__(256) k_f64_reduce(const double* __restrict__ p
                                                     double* __restrict__ XtX, double* __restrict__ Xtz) {
     extern __shared__ double tile[];   // [K + NH][FR_ROWS + 1]: Xtz, then the triangle
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    __shared__ int mx[FR_ROWS];            // high word of the row's largest entry of x
+    if (tid < FR_ROWS) mx[tid] = 0;
     const bool general = __syncthreads_or(tid < noff && off[tid] != 0u);
     const int NH = hess ? K * (K + 1) / 2 : 0;
     const int64_t r0 = (int64_t)blockIdx.x * FR_ROWS, r = r0 + lane;
@@ -62,10 +64,11 @@ __global__ void __launch_bounds__(256) k_f64_reduce(const double* __restrict__ p
         const int NV = hess ? NH : K;
         const int flag = *rare.flag;
         int sh = 0;                        // the row's exponent
-        if (g && r < rows) {
-            double m = 0.0;
-            for (int k = 0; k < K; ++k) m = fmax(m, x[r * K + k]);
-            sh = 1022 - (__double2hiint(m) >> 20);
+        if (g) {
+            for (int t = tid; t < FR_ROWS * K; t += 256)
+                if (r0 * K + t < rows * K) atomicMax(&mx[t / K], __double2hiint(x[r0 * K + t]));
+            __syncthreads();
+            if (r < rows) sh = -f64_exponent(mx[lane]);
         }
         for (int v = warp; v < NV; v += 8) {
             double s = 0.0;
@@ -74,9 +77,13 @@ __global__ void __launch_bounds__(256) k_f64_reduce(const double* __restrict__ p
 #pragma unroll 8
                 for (int c = 0; c < S; ++c) s += src[(int64_t)c * NV * ld];
                 if (flag) {                // products of out-of-range weights; left zero for the next pass
-                    long long* i = rare.i + 3 * (r * NV + v);
-                    s += scalbn((double)i[0], 2) + (scalbn((double)i[1], -35) + scalbn((double)i[2], -72));
-                    i[0] = i[1] = i[2] = 0;
+                    long long* i = rare.i + (int64_t)v * rows + r;
+                    const int64_t word = NV * rows;
+                    const long long i0 = i[0], i1 = i[word], i2 = i[2 * word];
+                    if (i0 | i1 | i2) {
+                        s += scalbn((double)i0, 2) + (scalbn((double)i1, -35) + scalbn((double)i2, -72));
+                        i[0] = i[word] = i[2 * word] = 0;
+                    }
                 }
                 s = scalbn(s, sh);
             }

@@ -12,12 +12,12 @@
 // and form the sums H = sum W v v' (v = p on the Q side, q on the P side;
 // src/loops.jl:328-403) exactly on the tensor cores: the error-free splitting
 // of Ozaki, Ogita, Oishi and Rump (2012).  Each index's vector is scaled by a power of
-// two 2^-f, so that its largest entry is just below 1, and W by 2^2f (2^f in the
-// gradient-only form), which leaves W' = c_h (2^f / qp_h)^2: of the order of 1 even for
-// rare haplotypes; on the P side the row's power of two 2^g (its largest frequency) is
-// a third factor, for the same reason.  W' is rounded to a multiple of 2^-56 and written
-// as ND_A = 9 signed base-256 digits, the scaled products v_k v_k2 to a multiple of
-// 2^-86 as ND_B = 11 digits.  Digits are integers in [-128, 127], exact in FP16; a
+// two 2^-f, 2^f its largest entry (Q side) or its sum (P side, 1), rounded up, and W by
+// 2^2f (2^f in the gradient-only form), which leaves W' = c_h (2^f / qp_h)^2: c_h at
+// least, and not much more even for rare haplotypes; on the P side the row's power of
+// two 2^g (its largest frequency) is a third factor, for the same reason.  W' is rounded
+// to a multiple of 2^-56 and written as ND_A = 9 signed base-256 digits, the scaled
+// products v_k v_k2 to a multiple of 2^-86 as ND_B = 11 digits.  Digits are integers in [-128, 127], exact in FP16; a
 // digit product is at most 2^14, and an FP32 accumulator column takes at most 9 digit
 // pairs x 96 reduction indices x 2^14 < 2^24 before it is read out, so every
 // accumulation is exact.  Digit pairs (a, b) of equal order a + b share a
@@ -30,17 +30,17 @@
 // has them; the general passes of hx_pass.cuh take all others (F_LO_HESS).  A product is
 // then at least 2^-34 and keeps 53 bits of its own, so that an entry made of small
 // products only (all carriers floored in both ancestries) is as accurate as an FP64 sum;
-// with 8 digits and 10 orders such entries had 24 to 27 bits.  W' is at least c / K^2
-// and keeps 50 bits there; a double heterozygote's c can be small (2^-17), and has that
-// many bits fewer, beside the other terms of its row.
+// with 8 digits and 10 orders such entries had 24 to 27 bits.  A double heterozygote's c
+// can be small (2^-17): its W' keeps 40 bits then, and with units of 2^-52 the sums of
+// cohorts of 30 and 60 individuals were off by up to 4e-13.
 //
 // The gradient needs no sums of its own beside the Hessian: sum_k2 H[k,k2] x_k2
 // = sum W v_k qp = sum U v_k = g_k (x = the row's own vector, qp = v . x), all
 // terms of one sign, formed by the reduction of the chunks.
 //
-// A scaled weight of 2^14 or more (an observed haplotype about 100 times rarer in
-// the individual's mixture than in one of the ancestries; 2^38 at most) does not fit
-// the digits: its products are added in fixed point to 64-bit integers in global memory
+// A scaled weight of 2^14 or more (an observed haplotype about 100 times rarer in the
+// individual's mixture than in one of the ancestries; 2^38 at most) does not fit the
+// digits: its products are added in fixed point to 64-bit integers in global memory
 // (order-independent, as every integer sum).
 #pragma once
 #include "hx_ops.cuh"
@@ -113,8 +113,6 @@ __global__ void __launch_bounds__(256) k_f64_range(const double* __restrict__ q,
     if (t == 0) *flag = 0;
 }
 
-// Exponent f with x < 2^f, x >= 2^(f-1), of a positive x.
-__device__ __forceinline__ int f64_exponent(double x) { return (__double2hiint(x) >> 20) - 1022; }
 // The exponent kept with a row (entry K).
 __device__ __forceinline__ int f64_row_exp(const double* row, int K) { return __double2loint(row[K]); }
 
@@ -139,8 +137,10 @@ __device__ __forceinline__ void f64_fix(double w, int sh, uint32_t (&x)[3]) {
 // indices, in the shared-memory layout of the MMA's B operand, and the FP64
 // vectors.  One warp per stage, lane = reduction index.  Indices past n get
 // zeros (their class nibbles are padding).
+// The index's exponent: of the sum of its entries (by_sum; a sum of 1 with a few ulps
+// counts as 1), else of the largest.
 template <int K, bool HESS>
-__global__ void __launch_bounds__(128) k_f64_img(const double* __restrict__ v, int64_t n, int64_t stages,
+__global__ void __launch_bounds__(128) k_f64_img(const double* __restrict__ v, int64_t n, int64_t stages, bool by_sum,
                                                  uint8_t* __restrict__ img) {
     using D = FDim<K, HESS>;
     const int lane = threadIdx.x & 31;
@@ -148,18 +148,20 @@ __global__ void __launch_bounds__(128) k_f64_img(const double* __restrict__ v, i
     if (st >= stages) return;
     const int64_t a = st * F_KD + lane;
     uint8_t* base = img + st * D::IMG;
-    double w[K], mx = 0.0;
+    double w[K], sum = 0.0;
+    int mx = 0;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         w[k] = a < n ? v[(int64_t)K * a + k] : 0.0;
-        mx = fmax(mx, w[k]);
+        mx = max(mx, __double2hiint(w[k]));
+        if (by_sum) sum += w[k];
     }
-    const int f = mx > 0.0 ? f64_exponent(mx) : 0;
+    const int f = mx ? f64_exponent(by_sum ? __double2hiint(sum) - 1 : mx) : 0;
     double* rows = reinterpret_cast<double*>(base + D::NG * D::B_TILE) + lane * D::KS;
 #pragma unroll
     for (int k = 0; k < K; ++k) rows[k] = w[k];
     rows[K] = __longlong_as_double((long long)f);
-    auto put = [&](int c, double y) {   // sum c, y 2^(-f or -2f) in [0, 1)
+    auto put = [&](int c, double y) {   // sum c, y 2^(-f or -2f) in [0, 1.01)
         const int g = c / D::PER, col = c - g * D::PER;
         uint32_t u[3];
         f64_fix<F_SB, F_NDB>(y, HESS ? -2 * f : -f, u);
@@ -315,7 +317,8 @@ __device__ __forceinline__ bool f64_out_of_range(double w, int sh) {
 // words of 37 bits, so that 2^26 of them fit the row's 64-bit integers.  The lanes take
 // one product each, and all of it is integer work but the products themselves.
 template <int K, bool HESS>
-__device__ __noinline__ void f64_rare(double w, int s, const double* v, int c0, int c1, F64Rare ra, int64_t row) {
+__device__ __noinline__ void f64_rare(double w, int s, const double* v, int c0, int c1, F64Rare ra, int64_t rows,
+                                      int64_t row) {
     const int lane = threadIdx.x & 31;
     if (lane == 0) atomicOr(ra.flag, 1);
     for (int c = c0 + lane; c < c1; c += 32) {
@@ -327,10 +330,11 @@ __device__ __noinline__ void f64_rare(double w, int s, const double* v, int c0, 
         const unsigned __int128 x = e >= 0 ? (unsigned __int128)m << e
                                            : e > -54 ? (m + (1ull << (-e - 1))) >> -e : 0ull;
         constexpr unsigned long long M37 = (1ull << 37) - 1;
-        unsigned long long* out = reinterpret_cast<unsigned long long*>(ra.i) + 3 * (row * FDim<K, HESS>::NV + c);
+        unsigned long long* out = reinterpret_cast<unsigned long long*>(ra.i) + c * rows + row;
+        const int64_t word = FDim<K, HESS>::NV * rows;
         atomicAdd(out, (unsigned long long)(x >> 74));
-        atomicAdd(out + 1, (unsigned long long)(x >> 37) & M37);
-        atomicAdd(out + 2, (unsigned long long)x & M37);
+        atomicAdd(out + word, (unsigned long long)(x >> 37) & M37);
+        atomicAdd(out + 2 * word, (unsigned long long)x & M37);
     }
     __syncwarp();
 }
@@ -395,12 +399,10 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
         fix[r * D::KS + k] = row0 + r < nown ? own[(row0 + r) * K + k] : 0.25;
     }
     if (PS && HESS && tid < 128) {        // the rows' exponents
-        double mx = 0.25;
-        if (row0 + tid < nown) {
-            mx = 0.0;
+        int mx = 0;
 #pragma unroll
-            for (int k = 0; k < K; ++k) mx = fmax(mx, own[(row0 + tid) * K + k]);
-        }
+        for (int k = 0; k < K; ++k)
+            mx = max(mx, __double2hiint(row0 + tid < nown ? own[(row0 + tid) * K + k] : 0.25));
         fix[tid * D::KS + K] = __longlong_as_double((long long)f64_exponent(mx));
     }
     fence_before();
@@ -576,7 +578,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
                         left &= left - 1;
                         f64_rare<K, HESS>(__shfl_sync(0xffffffffu, W[c], l), gexp(c),
                                           PS ? qrow + l * D::KS : prow + c * D::KS, grp * D::PER,
-                                          min(D::NV, (grp + 1) * D::PER), fa.rare,
+                                          min(D::NV, (grp + 1) * D::PER), fa.rare, nown,
                                           PS ? row0 + 8 * warp + c : row0 + 32 * (warp & 3) + l);
                     }
                     if (mine) W[c] = 0.0;

@@ -35,7 +35,7 @@ cudaError_t f64_launch(const F64Call& c) {
     const int64_t nq = a.I * K, np = 4 * a.J * K;
     const int noff = (int)std::min<int64_t>(F_MAXB, (nq + np + 1023) / 1024);
     k_f64_range<<<noff, 256, 0, c.st>>>(a.q, nq, a.p, np, HESS ? F_LO_HESS : F_LO_GRAD, c.off, c.rare.flag);
-    k_f64_img<K, HESS><<<(unsigned)((stages + 3) / 4), 128, 0, c.st>>>(v, n, stages, a.img);
+    k_f64_img<K, HESS><<<(unsigned)((stages + 3) / 4), 128, 0, c.st>>>(v, n, stages, PS, a.img);
     F64Args fa{stages, c.off, noff, c.rare};
     dim3 grid((unsigned)tiles, (unsigned)a.S, D::NG);
     k_f64_pass<K, HESS, PS><<<grid, F_THREADS, f_smem<K, HESS, PS>(), c.st>>>(a, fa);

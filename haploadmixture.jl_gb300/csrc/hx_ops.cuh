@@ -57,7 +57,7 @@ int tc_resident(int K, bool p_side);
 // weights, kept zero between passes, and what the pass kernel takes beside
 // PassArgs (per_chunk counts stages there).
 struct F64Rare {
-    long long* i;          // [rows][NV][3] fixed-point sums, units 2^2, 2^-35, 2^-72
+    long long* i;          // [3][NV][rows] fixed-point sums, units 2^2, 2^-35, 2^-72
     int* flag;             // whether i was added to
 };
 constexpr int F_MAXB = ACC_THREADS;   // blocks of the range check (one thread of a CTA reads one)
@@ -71,6 +71,8 @@ struct F64Args {
     int noff;
     F64Rare rare;
 };
+// Exponent f with x < 2^f, x >= 2^(f-1), from the high word of a positive x.
+__host__ __device__ constexpr int f64_exponent(int hi) { return (hi >> 20) - 1022; }
 // Digits of a weight and of a product, orders kept (hx_f64.cuh), and the columns of a
 // row's sums: `per` of them in F_NORD groups of TMEM columns, each as wide as the MMA
 // where that fits 512 columns, else overlapping by the MMA's zero columns.
