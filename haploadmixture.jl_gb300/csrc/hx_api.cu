@@ -346,9 +346,10 @@ int loglik_to_slot(hx_ctx* c, const double* q, const double* p, int slot) {
 }
 
 int read_slots(hx_ctx* c) {
-    HX_CK(cudaStreamSynchronize(c->st));   // first, so that the copy does not wait inside the driver
-    HX_CK(cudaMemcpyAsync(c->h_slots, c->slots, HX_NSLOT * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    // the stream first, so that the copy (which returns when it is complete: the
+    // destination is pageable) does not wait inside the driver
     HX_CK(cudaStreamSynchronize(c->st));
+    HX_CK(cudaMemcpyAsync(c->h_slots, c->slots, HX_NSLOT * sizeof(double), cudaMemcpyDeviceToHost, c->st));
     prof_resolve(c);
     return HX_OK;
 }

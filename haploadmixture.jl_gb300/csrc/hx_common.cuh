@@ -320,7 +320,7 @@ __device__ __forceinline__ void pair_u_cls(unsigned off, uint64_t z01, uint64_t 
 }
 
 // Exact exponent/mantissa split used to accumulate products of likelihoods
-// without underflow (one log per thread instead of two per pair).
+// without underflow (one log per CTA instead of two per pair).
 __device__ __forceinline__ float renorm(float m, int& e) {
     unsigned b = __float_as_uint(m);
     e += (int)((b >> 23) & 0xFFu) - 127;

@@ -69,7 +69,12 @@ template <int K, bool HESS> struct FDim {
     static constexpr int NHP = (PER + 15) / 16 * 16;         // MMA columns of one order, zero beyond PER
     static constexpr int STR = f64_stride(PER);              // TMEM columns from one order to the next
     static constexpr int NPC = NHP / 4;                      // columns per order read out by one thread
-    static constexpr int TCOLS = (F_NORD - 1) * STR + NHP <= 256 ? 256 : 512;
+    // with 16 columns per order, one MMA takes a weight digit with all product digits
+    // (order d + b follows order d + b - 1 as the B rows do); orders from F_NORD on are
+    // formed too, and not read
+    static constexpr bool STACK = NHP == 16;
+    static constexpr int COLS = STACK ? (F_NDA + F_NDB - 1) * 16 : (F_NORD - 1) * STR + NHP;
+    static constexpr int TCOLS = COLS <= 256 ? 256 : 512;
     static constexpr int KS = (K + 1) | 1;                   // row stride (doubles): odd, so rows differ in banks;
                                                              // entry K of a row: its exponent
     static constexpr int B_TILE = F_NDB * NHP * F_KD * 2;
@@ -456,11 +461,17 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args f
             if (!f_wait(sy, &sy->fullb[s % F_BRING], s / F_BRING, a)) break;
             fence_after();
             const uint64_t dA = sdesc(sA, LBO, SBO), dB = sdesc(sB + (s % F_BRING) * D::B_TILE, F_LBO_B, F_SBO_B);
-            // One MMA per digit pair: all of one shape, so that those of one order
-            // (one accumulator) execute in issue order.  Where STR < NHP an order's
-            // zero columns add 0 to the next order's first ones, in the same order.
+            // One MMA per digit pair (or weight digit): all of one shape, so that they
+            // execute in issue order where they share accumulators.  Where STR < NHP an
+            // order's zero columns add 0 to the next order's first ones.
 #pragma unroll 1
             for (int d = 0; d < F_NDA; ++d)
+                if (D::STACK) {
+#pragma unroll
+                    for (int ks = 0; ks < F_KD / 16; ++ks)
+                        mma_bf16(tmem + d * 16, dA + (uint64_t)((d * AT + ks * 2 * LBO) >> 4),
+                                 dB + (uint64_t)((ks * 2 * F_LBO_B) >> 4), idesc_f16(F_NDB * 16), 1u, el);
+                } else
 #pragma unroll
                 for (int b = 0; b < F_NDB; ++b) {
                     if (d + b >= F_NORD) break;

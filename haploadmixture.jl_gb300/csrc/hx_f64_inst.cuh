@@ -26,7 +26,7 @@ template <int K, bool HESS, bool PS>
 cudaError_t f64_launch(const F64Call& c) {
     using D = FDim<K, HESS>;
     static_assert(f_smem<K, HESS, PS>() <= 232448, "shared memory of one CTA");
-    static_assert((F_NORD - 1) * D::STR + D::NHP <= D::TCOLS && D::PER <= D::STR, "TMEM columns");
+    static_assert(D::COLS <= D::TCOLS && D::PER <= D::STR, "TMEM columns");
     const PassArgs& a = c.a;
     const double* v = PS ? a.q : a.p;             // the vectors along the reduction
     const int64_t n = PS ? a.I : 4 * a.J;

@@ -16,7 +16,7 @@
 //                XtX_p[k2,k,m] = sum_i c_h q[k,i] q[k2,i] / qp_h^2
 //   k_loglik2  : sum over pairs of log L (src/loops.jl:236-258,
 //                src/cuda/kernels.jl:16-40), as the log of an exponent-
-//                renormalised running product (one log per thread).
+//                renormalised running product (one log per CTA).
 //
 // The EM numerators of em_loop!/em_kernel! (src/loops.jl:260-295,
 // src/cuda/kernels.jl:42-73) are q[k,i] * Xtz_q[k,i] and p[k,m] * Xtz_p[k,m],

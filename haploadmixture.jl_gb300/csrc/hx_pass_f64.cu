@@ -24,7 +24,7 @@ template <int K> struct LDim {
 // multiplies straight into the running product of whichever lane evaluates it
 // (homozygous pairs, whose qp counts twice, into one of their own); the other
 // classes are finished from the listed qp's.  Products are exponent-
-// renormalised: one log per lane and product.  Bound by the FP64 unit: K + 1
+// renormalised: one log per CTA.  Bound by the FP64 unit: K + 1
 // operations per needed haplotype (2 of 4 on average) against 4 K + 20 per
 // pair before.  BED: the two codes of each block are read from the BED bytes.
 template <int K, bool BED>

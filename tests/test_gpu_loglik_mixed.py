@@ -1,6 +1,7 @@
-"""Mixed log-likelihood where its chunks and its paired renormalisation can go
-wrong: ragged sizes, likelihoods below 2^-60 (evaluated pair by pair), zeros and
-NaN.  A pair's FP32 likelihood carries K + 8 roundings of 2^-24 at most (qp, two
+"""Mixed log-likelihood where its chunks and its renormalised products can go wrong:
+ragged sizes, small likelihoods (every pair is renormalised, so that products do not
+underflow; a pair's own likelihood has to be a normal FP32 number), zeros and NaN.  A
+pair's FP32 likelihood carries K + 8 roundings of 2^-24 at most (qp, two
 factors, products), which bounds the sum's error by (K + 8) 2^-24 per pair; only
 over many pairs do they average out to the mixed method's 1e-8."""
 import numpy as np
