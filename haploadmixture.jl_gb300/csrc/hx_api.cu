@@ -42,7 +42,8 @@ struct hx_ctx {
     float* pf = nullptr;                     // mixed: FP32 copy of the pass's p (K x 4J)
     double* slots = nullptr;
     // host copy of the scalar block.  Pageable: pinned memory of its own costs a context
-    // 270 us, and the copies are 128 bytes
+    // 270 us, and the copies are 128 bytes.  A copy to the device has left it when the call
+    // returns, a copy back is complete
     double h_slots[HX_NSLOT] = {};
     uint8_t* img = nullptr;      // B-operand image of the tensor-core passes
     // plain method: range flags and out-of-range sums of the passes (hx_f64.cuh)
@@ -346,18 +347,15 @@ int loglik_to_slot(hx_ctx* c, const double* q, const double* p, int slot) {
 }
 
 int read_slots(hx_ctx* c) {
-    // the stream first, so that the copy (which returns when it is complete: the
-    // destination is pageable) does not wait inside the driver
+    // the stream first, so that the copy does not wait inside the driver
     HX_CK(cudaStreamSynchronize(c->st));
     HX_CK(cudaMemcpyAsync(c->h_slots, c->slots, HX_NSLOT * sizeof(double), cudaMemcpyDeviceToHost, c->st));
     prof_resolve(c);
     return HX_OK;
 }
 int write_slot(hx_ctx* c, int slot, double v) {
-    HX_CK(cudaStreamSynchronize(c->st));
     c->h_slots[slot] = v;
     HX_CK(cudaMemcpyAsync(c->slots + slot, c->h_slots + slot, sizeof(double), cudaMemcpyHostToDevice, c->st));
-    HX_CK(cudaStreamSynchronize(c->st));
     return HX_OK;
 }
 
@@ -627,9 +625,7 @@ int reset_state(hx_ctx* c) {
     // a new trajectory starts from cold QP working sets, so that a fit from
     // given Q, P is reproducible regardless of earlier calls
     HX_CK(cudaMemsetAsync(c->qp_ws, 0, (size_t)4 * c->K * c->J, c->st));
-    HX_CK(cudaMemsetAsync(c->U, 0, (size_t)c->nx * c->Qs * sizeof(double), c->st));
-    HX_CK(cudaMemsetAsync(c->V, 0, (size_t)c->nx * c->Qs * sizeof(double), c->st));
-    HX_CK(cudaStreamSynchronize(c->st));
+    HX_CK(cudaMemsetAsync(c->U, 0, 2 * (size_t)c->nx * c->Qs * sizeof(double), c->st));   // and V behind it
     for (int s = 0; s < HX_NSLOT; ++s) c->h_slots[s] = 0.0;
     c->h_slots[S_LL_NEW] = NAN;
     HX_CK(cudaMemcpyAsync(c->slots, c->h_slots, HX_NSLOT * sizeof(double), cudaMemcpyHostToDevice, c->st));
