@@ -44,9 +44,8 @@ cudaError_t f64_launch(const F64Call& c) {
     PassArgs g = a;
     g.S = c.Sg;
     g.per_chunk = c.per_chunk_g;
-    g.run_if = c.off;
-    g.n_run_if = noff;
-    e = PS ? launch_accum_p_f64(K, HESS, g, c.st) : launch_accum_q_f64(K, HESS, g, c.st);
+    const RunIf r{c.off, noff};
+    e = PS ? launch_accum_p_f64(K, HESS, g, r, c.st) : launch_accum_q_f64(K, HESS, g, r, c.st);
     if (e != cudaSuccess) return e;
     const int64_t rows = PS ? 4 * a.J : a.I;
     return launch_f64_reduce(a.part, a.S, c.Sg, K, HESS, PS && HESS, rows, PS ? rows : a.Ipad, PS ? a.p : a.q, c.off, noff, c.rare,

@@ -16,8 +16,8 @@ cudaError_t launch_loglik_f64(int K, const PassArgs& a, cudaStream_t st);
 // the same from BED bytes (first I individuals, 2J SNPs); a.G and a.Ipad unused
 cudaError_t launch_loglik_f64_bed(int K, const PassArgs& a, const uint8_t* bed, int64_t bps, cudaStream_t st);
 // general FP64 passes (partial sums in a.part whatever a.S is)
-cudaError_t launch_accum_q_f64(int K, bool hess, const PassArgs& a, cudaStream_t st);
-cudaError_t launch_accum_p_f64(int K, bool hess, const PassArgs& a, cudaStream_t st);
+cudaError_t launch_accum_q_f64(int K, bool hess, const PassArgs& a, const RunIf& r, cudaStream_t st);
+cudaError_t launch_accum_p_f64(int K, bool hess, const PassArgs& a, const RunIf& r, cudaStream_t st);
 cudaError_t launch_accum_q_f32(int K, bool hess, const PassArgs& a, cudaStream_t st);
 cudaError_t launch_accum_p_f32(int K, bool hess, const PassArgs& a, cudaStream_t st);
 cudaError_t launch_loglik_f32x2(int K, const PassArgs& a, cudaStream_t st);   // several individuals per thread

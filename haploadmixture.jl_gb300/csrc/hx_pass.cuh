@@ -50,8 +50,6 @@ struct PassArgs {
     const float* pf;        // FP32 copy of p for the FP32 passes that stage p (or null): GB300's
                             // FP64 unit is narrow, and converting in every CTA kept it busy
     long long budget;       // tensor-core passes: clock64 cycles any one pipeline wait may take
-    const unsigned* run_if = nullptr;   // T = double: run if any of these n_run_if (at most
-    int n_run_if = 0;                   // ACC_THREADS) words is not zero
 };
 
 template <int K> __device__ __forceinline__ constexpr int tri(int k, int k2) {
@@ -60,20 +58,24 @@ template <int K> __device__ __forceinline__ constexpr int tri(int k, int k2) {
 
 // ------------------------------------------------------------------ Q side
 // T = double (with its gradient-only form): the plain method's passes on inputs that
-// the digit sums of hx_f64.cuh do not take; run_if says on the device whether it is
-// one of them.
-template <typename T> __device__ __forceinline__ bool pass_idle(const PassArgs& a) {
-    return sizeof(T) == 8 && !__syncthreads_or((int)threadIdx.x < a.n_run_if && a.run_if[threadIdx.x] != 0u);
+// the digit sums of hx_f64.cuh do not take, told on the device: they run if any of n
+// words (at most ACC_THREADS) is not zero.
+struct RunIf {
+    const unsigned* w;
+    int n;
+};
+template <typename T> __device__ __forceinline__ bool pass_idle(const RunIf& r) {
+    return sizeof(T) == 8 && !__syncthreads_or((int)threadIdx.x < r.n && r.w[threadIdx.x] != 0u);
 }
 template <int K, typename T, bool HESS>
 __global__ void __launch_bounds__(ACC_THREADS)
-k_accum_q(PassArgs a) {
+k_accum_q(PassArgs a, RunIf run) {
     constexpr int NH = K * (K + 1) / 2;
     constexpr int NV = K + (HESS ? NH : 0);
     __shared__ T sp[QSTAGE_WORDS * 8 * 4 * K];
     __shared__ float4 s_snp[4];
     const int tid = threadIdx.x;
-    if (pass_idle<T>(a)) return;
+    if (pass_idle<T>(run)) return;
     snp_table_init(s_snp, tid);
     const int64_t i = (int64_t)blockIdx.x * ACC_THREADS + tid;
     const int w0 = blockIdx.y * a.per_chunk;
@@ -258,14 +260,14 @@ k_grad_q(PassArgs a) {
 // the 4 threads of a block exchange their qp_h by warp shuffles.
 template <int K, typename T, bool HESS>
 __global__ void __launch_bounds__(ACC_THREADS)
-k_accum_p(PassArgs a) {
+k_accum_p(PassArgs a, RunIf run) {
     constexpr int NH = K * (K + 1) / 2;
     constexpr int NV = K + (HESS ? NH : 0);
     __shared__ T sq[PSTAGE_IND * K];
     __shared__ uint32_t sg[4 * PSTAGE_IND];
     __shared__ float4 s_snp[4];
     const int tid = threadIdx.x;
-    if (pass_idle<T>(a)) return;
+    if (pass_idle<T>(run)) return;
     snp_table_init(s_snp, tid);
     const int lane = tid & 31, warp = tid >> 5;
     const int b = tid >> 2, h = tid & 3;
