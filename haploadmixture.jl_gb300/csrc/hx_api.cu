@@ -50,6 +50,7 @@ struct hx_ctx {
     unsigned* f64_off = nullptr;
     F64Rare rare{nullptr, nullptr};
     int S_qf = 1, spc_qf = 1, S_pf = 1, spc_pf = 1;   // chunks, stages per chunk
+    int S_qg = 1, wpc_qg = 1, S_pg = 1, ipc_pg = 1;   // of the general passes: words, individuals
     int8_t* qp_ws = nullptr;     // P-side QP working sets, warm start of the next solve
     hx_loop_opts lo{0, 0, 0, -1};  // admixture_qn!/init_em! options
     double ll_tmp = NAN;         // d.ll_tmp of the step control
@@ -235,6 +236,18 @@ void plan(hx_ctx* c) {
     c->S_qf = (c->JW + c->spc_qf - 1) / c->spc_qf;
     c->spc_pf = (int)pick_chunk_f64(tilesP, nst_p, nsm);
     c->S_pf = (int)((nst_p + c->spc_pf - 1) / c->spc_pf);
+    // general passes: the CUDA-core splits, with fewer chunks where their sums would take
+    // more room than the digit passes' and more than 32 MB (allocating a context's memory
+    // takes some 0.3 us per MB)
+    const int64_t NH = (int64_t)c->K * (c->K + 1) / 2, NV = c->K + NH;
+    auto cap = [&](int64_t S, int64_t Sf, int64_t rows) {
+        return std::min(S, std::max<int64_t>({1, Sf * NH / NV, ((int64_t)32 << 20) / (NV * rows * 8)}));
+    };
+    const int64_t Sq = cap(c->S_q, c->S_qf, c->Ipad), Spg = cap(c->S_p, c->S_pf, 4 * c->J);
+    c->wpc_qg = (int)((c->JW + Sq - 1) / Sq);
+    c->S_qg = (c->JW + c->wpc_qg - 1) / c->wpc_qg;
+    c->ipc_pg = (int)(((c->I + Spg - 1) / Spg + PSTAGE_IND - 1) / PSTAGE_IND * PSTAGE_IND);
+    c->S_pg = (int)((c->I + c->ipc_pg - 1) / c->ipc_pg);
     // tensor-core passes (stages of one word column, Q, or 32 individuals, P)
     // and the FP32 log-likelihood pass: >= 8 waves with a full last wave
     const int64_t wpc = pick_chunk(tilesQ, c->JW, (int64_t)nsm * tc_resident(c->K, false), 8);
@@ -278,7 +291,7 @@ int stage_pf(hx_ctx* c, const double* p, PassArgs& a) {
 // The plain method's pass of one side: range, stage images, digit pass or general
 // pass, reduction.
 int pass_f64(hx_ctx* c, bool p_side, const double* q, const double* p, bool hess, double* XtX, double* Xtz) {
-    F64Call f{p_side, hess, pass_args(c, q, p), p_side ? c->S_p : c->S_q, p_side ? c->ipc_p : c->wpc_q, c->f64_off,
+    F64Call f{p_side, hess, pass_args(c, q, p), p_side ? c->S_pg : c->S_qg, p_side ? c->ipc_pg : c->wpc_qg, c->f64_off,
               c->rare, c->st};
     f.a.S = p_side ? c->S_pf : c->S_qf;
     f.a.per_chunk = p_side ? c->spc_pf : c->spc_qf;
@@ -564,8 +577,8 @@ int create_common(const uint8_t* bed, bool bed_on_device, int64_t bps, int64_t n
     need(rq, &c->Xtzp, (size_t)K * 4 * J);
     const size_t NH = (size_t)K * (K + 1) / 2, rows = (size_t)std::max<int64_t>(I, 4 * J);
     if (c->prec == HX_PREC_FP64) {
-        need(rq, &c->part_q, std::max<size_t>(c->S_qf * NH, (size_t)c->S_q * NVmax) * c->Ipad);
-        need(rq, &c->part_p, std::max<size_t>(c->S_pf * NH, (size_t)c->S_p * NVmax) * 4 * J);
+        need(rq, &c->part_q, std::max<size_t>(c->S_qf * NH, (size_t)c->S_qg * NVmax) * c->Ipad);
+        need(rq, &c->part_p, std::max<size_t>(c->S_pf * NH, (size_t)c->S_pg * NVmax) * 4 * J);
         need(rq, &c->img, f64_image_bytes(K, I, J));
         need(rq, &c->f64_off, (size_t)F_MAXB);
         need(rq, &c->rare.i, 3 * rows * NH);
