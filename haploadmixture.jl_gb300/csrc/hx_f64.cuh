@@ -350,17 +350,17 @@ __device__ __noinline__ void f64_rare(double w, int s, const double* v, int c0, 
 // 2 (w >> 2), +1.  PS = true (P side): CTA rows = the 128 columns m of 32
 // blocks, stage = 32 individuals; warp w: blocks 2w, 2w+1.  Chunks of the
 // reduction along grid.y, column groups along grid.z.
-// FP64 operations take 63% of the clocks (K + 1 per needed haplotype, 7 per pair
-// with qp-dependent counts; they were 80% to 88% with the reciprocals among them),
-// issue 43% and the MMAs about as much as FP64; the rest is a warp's own chain from
-// class to digits, in which the 16 warps move together.  One CTA per SM (480 of 512
-// TMEM columns at K = 8; shared memory has no room for a second set of digit
-// tiles): a stage's FP64 work (registers and warp-private shared memory) runs while
-// the MMAs of the stage before read the tiles.  Writing and issuing the digits in
-// three words, so that a stage's first MMAs need not wait for its last digits, gained
-// nothing (2.72 ms for 2.68).
-// 10,000 individuals x 5,000 blocks, K = 5: Q pass 3.43 ms with the reciprocals in
-// FP64, 2.68 now.
+// What bounds it: the FP64 unit, busy 74% of the clocks at K = 5 and 80% at K = 8 (K + 1
+// operations per needed haplotype, 7 per pair with qp-dependent counts), then a warp's
+// own chain from class to digits, in which the 16 warps move together; issue 42%.  One
+// CTA per SM: a stage's FP64 work (registers and warp-private shared memory) runs while
+// the MMAs of the stage before read the one set of digit tiles (two sets do not fit
+// beside the warps' buffers).  Writing and issuing the digits in three words, so that a
+// stage's first MMAs need not wait for its last digits, gained nothing.
+// 10,000 individuals x 5,000 blocks, K = 5, Q pass: 3.43 ms with the reciprocals in FP64
+// and 10 x 8 digits, 2.68 with integer reciprocals, 2.79 with 9 x 11 digits and an MMA per
+// digit pair, 2.32 with one per weight digit; P pass 2.43.  50,000 x 4,000, K = 8, where
+// every digit pair is an MMA of its own: 11.7 ms on either side.
 template <int K, bool HESS, bool PS>
 __global__ void __launch_bounds__(F_THREADS, 1) k_f64_pass(PassArgs a, F64Args fa) {
     using D = FDim<K, HESS>;

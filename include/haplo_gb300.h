@@ -142,7 +142,7 @@ int hx_update_p_accum(hx_ctx* ctx, const double* q, const double* p, double* XtX
 /* em_p!(d_cu, g_cu) raw P numerators only (runners.jl:51-55; kernels.jl:75-102). */
 int hx_em_p_accum(hx_ctx* ctx, const double* q, const double* p, double* p_next);
 
-/* Bound on any one pipeline wait of the tensor-core passes, in SM clock
+/* Bound on any one pipeline wait of the tensor-core passes (both methods), in SM clock
  * cycles (clock64).  No reference counterpart (CUDA.jl kernels never wait on
  * one another).  A wait that runs out makes the pass stop early: it drains the
  * copies and MMAs it issued (each such wait allowed HX_WAIT_BUDGET_DEFAULT
