@@ -649,7 +649,8 @@ cudaError_t launch_dense(int K, int64_t n, const double* XtX, const double* Xtz,
 // 0.45 -> 0.34 ms at 2,000 individuals, 0.48 -> 0.67 at 10,000; K = 8: 1.05 -> 0.72 at
 // 4,000, 1.13 -> 1.53 at 10,000; K = 3 the same at 2,000), and from K = 11 on for small
 // cohorts (500 blocks, K = 12: 0.46 -> 0.37 ms at 500 individuals, 0.82 -> 0.78 at 3,000,
-// the same at 4,000; K = 8: 0.21 ms both at 1,000).  The results are the same bits.
+// the same at 4,000; 2,750 problems, K = 11: 0.70 -> 0.67; K = 8: 0.21 ms both at 1,000).
+// The results are the same bits.
 cudaError_t launch_qp_q(int K, int64_t n, int64_t J, const double* XtX, const double* Xtz, const double* q, double* qdiff,
                         double* slots, cudaStream_t st, double pen_rho) {
     if (J < K ? K >= 4 && n <= 500 * K : K >= 11 && n <= 250 * K)
