@@ -17,14 +17,13 @@
 // least, and not much more even for rare haplotypes; on the P side the row's power of
 // two 2^g (its largest frequency) is a third factor, for the same reason.  W' is rounded
 // to a multiple of 2^-56 and written as ND_A = 9 signed base-256 digits, the scaled
-// products v_k v_k2 to a multiple of 2^-86 as ND_B = 11 digits.  Digits are integers in [-128, 127], exact in FP16; a
-// digit product is at most 2^14, and an FP32 accumulator column takes at most 9 digit
-// pairs x 96 reduction indices x 2^14 < 2^24 before it is read out, so every
-// accumulation is exact.  Digit pairs (a, b) of equal order a + b share a
-// column; orders 0 .. 12 are kept (an order-13 pair weighs 2^-88 at most, with
-// either sign).  The columns are read out to 128-bit integers, so a chunk's sum
-// does not depend on any order; only the chunk sums and the last digits' cut
-// are rounded.
+// products v_k v_k2 to a multiple of 2^-86 as ND_B = 11 digits.  Digits are integers in
+// [-128, 127], exact in FP16; a digit product is at most 2^14, and an FP32 accumulator
+// column takes at most 9 digit pairs x 96 reduction indices x 2^14 < 2^24 before it is
+// read out, so every accumulation is exact.  Digit pairs (a, b) of equal order a + b
+// share a column; orders 0 .. 12 are kept (an order-13 pair weighs 2^-88 at most, with
+// either sign).  The columns are read out to 128-bit integers, so a chunk's sum does not
+// depend on any order; only the chunk sums and the last digits' cut are rounded.
 //
 // Which inputs: entries of Q and P in [2^-17, 1] (2^-34 without the Hessian), as a fit
 // has them; the general passes of hx_pass.cuh take all others (F_LO_HESS).  A product is
